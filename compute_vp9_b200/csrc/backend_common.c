@@ -38,7 +38,7 @@ void cvp9_build_dct_basis(double *out)
 #define MAX_DEVICES 64
 static pthread_mutex_t g_setup_lock = PTHREAD_MUTEX_INITIALIZER;
 static int g_setup_done[MAX_DEVICES];
-static int g_ctas[MAX_DEVICES][2];
+static int g_ctas[MAX_DEVICES][3];
 static int g_lf_ctas[MAX_DEVICES];
 
 int cvp9_device_setup(int device)
@@ -55,6 +55,7 @@ int cvp9_device_setup(int device)
         } else {
             g_ctas[device][0] = cvp9k_recon_ctas_per_sm(CVP9_ARITH_REFCPU);
             g_ctas[device][1] = cvp9k_recon_ctas_per_sm(CVP9_ARITH_SPEC);
+            g_ctas[device][2] = cvp9k_recon_ctas_per_sm(CVP9_ARITH_FULL);
             g_lf_ctas[device] = cvp9k_lf_full_ctas_per_sm();
             g_setup_done[device] = 1;
         }
@@ -66,7 +67,7 @@ int cvp9_device_setup(int device)
 int cvp9_recon_ctas_per_sm(int device, int arith)
 {
     if (device < 0 || device >= MAX_DEVICES) return 1;
-    int v = g_ctas[device][arith != CVP9_ARITH_REFCPU ? 1 : 0];    /* FULL runs the SPEC kernel */
+    int v = g_ctas[device][arith >= 0 && arith <= CVP9_ARITH_FULL ? arith : 0];
     return v > 0 ? v : 1;
 }
 
@@ -120,12 +121,6 @@ int cvp9_env_inter_fast(void)
     const char *e = getenv("CVP9_INTER_FAST");
     if (e && *e >= '0' && *e <= '5' && !e[1]) return *e - '0';
     return 1;
-}
-
-int cvp9_env_recon_warp(void)
-{
-    const char *e = getenv("CVP9_RECON_WARP");
-    return !(e && e[0] == '0' && !e[1]);
 }
 
 int cvp9_env_arith(void)

@@ -1108,7 +1108,6 @@ static cvp9_err_t submit_impl(cvp9_batch_t *b, int n, const int *sids, const vp9
         L.recon_ctas = (int)s->n_tickets < width ? (int)s->n_tickets : width;
     }
     L.lf_tile_h = tc.lf32 ? 32 : 64;
-    L.warp_levels = cvp9_env_recon_warp();
     if (tc.inter) {
         L.general = s->d_fast;
         L.general_tickets = s->d_fast + s->n_tickets;
@@ -1135,7 +1134,6 @@ static cvp9_err_t submit_impl(cvp9_batch_t *b, int n, const int *sids, const vp9
     gkey = mix64(gkey, (uint64_t)(uintptr_t)L.general);
     gkey = mix64(gkey, ((uint64_t)L.inter_variant << 16) | (uint64_t)L.lf_tile_h);
     gkey = mix64(gkey, ((uint64_t)L.full << 32) | (uint64_t)L.lf_tickets);
-    gkey = mix64(gkey, (uint64_t)L.warp_levels);
     /* k_inter + k_compact, or k_pred + k_resid + k_compact (the split, both
      * profiles: cvp9k_launch_frame dispatches inter paths 3 and 4 to it) */
     const int split = L.inter_variant >= 3;     /* path 5: one more residual kernel */
