@@ -126,6 +126,7 @@ __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wa
 
 /* ── 32-bit wrap-around integer for the shader butterflies ───────────────── */
 struct wi {
+    using P = wi;           /* the type of a product with a Q14 multiplier */
     int v;
     __device__ __forceinline__ wi() : v(0) {}
     __device__ __forceinline__ wi(int x) : v(x) {}
@@ -140,6 +141,7 @@ __device__ __forceinline__ wi shr(wi x, int k) { return wi(x.v >> k); }
 /* 64-bit integer for the same butterflies at 10 bits (profile 2): products
  * of the +-2^17 dequantised range and the Q14 multipliers need 64 bits. */
 struct wl {
+    using P = wl;
     long long v;
     __device__ __forceinline__ wl() : v(0) {}
     __device__ __forceinline__ wl(long long x) : v(x) {}
@@ -150,6 +152,32 @@ __device__ __forceinline__ wl operator-(wl a) { return wl(-a.v); }
 __device__ __forceinline__ wl operator*(wl a, int k) { return wl(a.v * (long long)k); }
 __device__ __forceinline__ wl RS(wl x) { return wl((x.v + 8192) >> 14); }
 __device__ __forceinline__ wl shr(wl x, int k) { return wl(x.v >> k); }
+
+/* The same butterflies on values known to fit 32 bits: 32-bit values, 64-bit
+ * products and sums of products (one IMAD.WIDE a multiplier), one funnel
+ * shift to round back. Every value a butterfly forms is a sum of its inputs
+ * with factors below 2, so a 32-point row of |inputs| < 2^18 and the column
+ * after it stay below 2^30: the results are wl's. */
+struct wp {
+    long long v;
+    __device__ __forceinline__ wp() : v(0) {}
+    __device__ __forceinline__ wp(long long x) : v(x) {}
+};
+struct wn {
+    using P = wp;
+    int v;
+    __device__ __forceinline__ wn() : v(0) {}
+    __device__ __forceinline__ wn(int x) : v(x) {}
+};
+__device__ __forceinline__ wp operator+(wp a, wp b) { return wp(a.v + b.v); }
+__device__ __forceinline__ wp operator-(wp a, wp b) { return wp(a.v - b.v); }
+__device__ __forceinline__ wp operator-(wp a) { return wp(-a.v); }
+__device__ __forceinline__ wn operator+(wn a, wn b) { return wn(a.v + b.v); }
+__device__ __forceinline__ wn operator-(wn a, wn b) { return wn(a.v - b.v); }
+__device__ __forceinline__ wn operator-(wn a) { return wn(-a.v); }
+__device__ __forceinline__ wp operator*(wn a, int k) { return wp((long long)a.v * k); }
+__device__ __forceinline__ wn RS(wp x) { return wn((int)((x.v + 8192) >> 14)); }
+__device__ __forceinline__ wn shr(wn x, int k) { return wn(x.v >> k); }
 
 /* cos(k*pi/64) in Q14 */
 enum : int {
@@ -392,6 +420,7 @@ __device__ __forceinline__ ITask ld_task(const ITask *t)
 }
 
 constexpr int kMaxTasks = 384;       /* 4x4 TXs of an SB's three planes; 3 x kMaxBlocks */
+constexpr int kResidGrid = 64 * 64 + 2 * 32 * 32;
 constexpr int kMaxQuads = 2048;      /* 16 a luma row, at most 11 a chroma row */
 
 struct IntraWork {
@@ -478,8 +507,8 @@ __device__ __forceinline__ void plane_layout(const B &b, const cvp9_job_t &job, 
     int lim_w = ((job.mi_cols * 2) >> ss) - o4x, lim_h = ((job.mi_rows * 2) >> ss) - o4y;
     if (mw > lim_w) mw = lim_w;
     if (mh > lim_h) mh = lim_h;
-    nx = mw > 0 ? (mw + t4 - 1) / t4 : 0;
-    ny = mh > 0 ? (mh + t4 - 1) / t4 : 0;
+    nx = mw > 0 ? (mw + t4 - 1) >> tx : 0;
+    ny = mh > 0 ? (mh + t4 - 1) >> tx : 0;
     pbw = pw;
 }
 
@@ -1011,15 +1040,16 @@ enum : int { KS1 = 5283, KS2 = 9929, KS3 = 13377, KS4 = 15212 };
 template <class T>
 __device__ __forceinline__ void iadst4(T *x)
 {
-    T a = x[0] * KS1 + x[2] * KS4 + x[3] * KS2;
-    T b = x[0] * KS2 - x[2] * KS1 - x[3] * KS4;
-    T c = (x[0] - x[2] + x[3]) * KS3;
-    T d = x[1] * KS3;
+    using P = typename T::P;
+    P a = x[0] * KS1 + x[2] * KS4 + x[3] * KS2;
+    P b = x[0] * KS2 - x[2] * KS1 - x[3] * KS4;
+    P c = (x[0] - x[2] + x[3]) * KS3;
+    P d = x[1] * KS3;
     x[0] = RS(a + d); x[1] = RS(b + d); x[2] = RS(c); x[3] = RS(a + b - d);
 }
 
 template <class T>
-__device__ __forceinline__ void rot(T x, T y, int ca, int cb, T &o0, T &o1)
+__device__ __forceinline__ void rot(T x, T y, int ca, int cb, typename T::P &o0, typename T::P &o1)
 {
     o0 = x * ca + y * cb;
     o1 = x * cb - y * ca;
@@ -1029,7 +1059,7 @@ template <class T>
 __device__ __forceinline__ void iadst8(T *in)
 {
     T x0 = in[7], x1 = in[0], x2 = in[5], x3 = in[2], x4 = in[3], x5 = in[4], x6 = in[1], x7 = in[6];
-    T s0, s1, s2, s3, s4, s5, s6, s7;
+    typename T::P s0, s1, s2, s3, s4, s5, s6, s7;
     rot(x0, x1, K2, K30, s0, s1);
     rot(x2, x3, K10, K22, s2, s3);
     rot(x4, x5, K18, K14, s4, s5);
@@ -1040,19 +1070,20 @@ __device__ __forceinline__ void iadst8(T *in)
     s5 = x4 * K24 - x5 * K8;
     s6 = x7 * K8 - x6 * K24;
     s7 = x6 * K8 + x7 * K24;
-    s0 = x0 + x2; s1 = x1 + x3; s2 = x0 - x2; s3 = x1 - x3;
+    T u0 = x0 + x2, u1 = x1 + x3, u2 = x0 - x2, u3 = x1 - x3;
     x4 = RS(s4 + s6); x5 = RS(s5 + s7); x6 = RS(s4 - s6); x7 = RS(s5 - s7);
-    x2 = RS((s2 + s3) * K16);
-    x3 = RS((s2 - s3) * K16);
+    x2 = RS((u2 + u3) * K16);
+    x3 = RS((u2 - u3) * K16);
     T y6 = RS((x6 + x7) * K16), y7 = RS((x6 - x7) * K16);
-    in[0] = s0; in[1] = -x4; in[2] = y6; in[3] = -x2;
-    in[4] = x3; in[5] = -y7; in[6] = x5; in[7] = -s1;
+    in[0] = u0; in[1] = -x4; in[2] = y6; in[3] = -x2;
+    in[4] = x3; in[5] = -y7; in[6] = x5; in[7] = -u1;
 }
 
 template <class T>
 __device__ __forceinline__ void iadst16(T *in)
 {
-    T x[16], s[16];
+    T x[16], u[16];
+    typename T::P s[16];
     x[0] = in[15]; x[1] = in[0]; x[2] = in[13]; x[3] = in[2]; x[4] = in[11]; x[5] = in[4];
     x[6] = in[9]; x[7] = in[6]; x[8] = in[7]; x[9] = in[8]; x[10] = in[5]; x[11] = in[10];
     x[12] = in[3]; x[13] = in[12]; x[14] = in[1]; x[15] = in[14];
@@ -1067,7 +1098,7 @@ __device__ __forceinline__ void iadst16(T *in)
 #pragma unroll
     for (int k = 0; k < 8; k++) { x[k] = RS(s[k] + s[k + 8]); x[k + 8] = RS(s[k] - s[k + 8]); }
 #pragma unroll
-    for (int k = 0; k < 8; k++) s[k] = x[k];
+    for (int k = 0; k < 8; k++) u[k] = x[k];
     s[8] = x[8] * K4 + x[9] * K28;
     s[9] = x[8] * K28 - x[9] * K4;
     s[10] = x[10] * K20 + x[11] * K12;
@@ -1078,22 +1109,22 @@ __device__ __forceinline__ void iadst16(T *in)
     s[15] = x[14] * K20 + x[15] * K12;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        x[k] = s[k] + s[k + 4];
-        x[k + 4] = s[k] - s[k + 4];
+        x[k] = u[k] + u[k + 4];
+        x[k + 4] = u[k] - u[k + 4];
         x[k + 8] = RS(s[k + 8] + s[k + 12]);
         x[k + 12] = RS(s[k + 8] - s[k + 12]);
     }
 #pragma unroll
     for (int g = 0; g < 16; g += 8) {
-        s[g + 0] = x[g + 0]; s[g + 1] = x[g + 1]; s[g + 2] = x[g + 2]; s[g + 3] = x[g + 3];
+        u[g + 0] = x[g + 0]; u[g + 1] = x[g + 1]; u[g + 2] = x[g + 2]; u[g + 3] = x[g + 3];
         s[g + 4] = x[g + 4] * K8 + x[g + 5] * K24;
         s[g + 5] = x[g + 4] * K24 - x[g + 5] * K8;
         s[g + 6] = x[g + 7] * K8 - x[g + 6] * K24;
         s[g + 7] = x[g + 6] * K8 + x[g + 7] * K24;
-        x[g + 0] = s[g + 0] + s[g + 2];
-        x[g + 1] = s[g + 1] + s[g + 3];
-        x[g + 2] = s[g + 0] - s[g + 2];
-        x[g + 3] = s[g + 1] - s[g + 3];
+        x[g + 0] = u[g + 0] + u[g + 2];
+        x[g + 1] = u[g + 1] + u[g + 3];
+        x[g + 2] = u[g + 0] - u[g + 2];
+        x[g + 3] = u[g + 1] - u[g + 3];
         x[g + 4] = RS(s[g + 4] + s[g + 6]);
         x[g + 5] = RS(s[g + 5] + s[g + 7]);
         x[g + 6] = RS(s[g + 4] - s[g + 6]);
@@ -1189,54 +1220,6 @@ __device__ __forceinline__ int full_tile_start(int mi_col, int mi_cols, int log2
         if (o <= mi_col) start = o;
     }
     return start;
-}
-
-#define FAVG2(a, b) (((a) + (b) + 1) >> 1)
-#define FAVG3(a, b, c) (((a) + 2 * (b) + (c) + 2) >> 2)
-
-/* One sample of a VP9 intra predictor from the TX's edges: above[-1..2n-1]
- * (above[-1] the corner), left[0..n-1]; MAXV: the largest sample value (TM
- * clips to it). */
-template <int MAXV = 255, class E>
-__device__ __forceinline__ int full_pred(int mode, int r, int c, int n, const E *above, const E *left, int dc)
-{
-    switch (mode) {
-    case 1: return above[c];
-    case 2: return left[r];
-    case 3: {
-        const int k = r + c;
-        return k + 2 < 2 * n ? FAVG3(above[k], above[k + 1], above[k + 2]) : above[2 * n - 1];
-    }
-    case 4: {
-        const int t = c - r;
-        auto e = [&](int u) -> int { return u >= 0 ? above[u] : (u == -1 ? above[-1] : left[-u - 2]); };
-        return FAVG3(e(t - 2), e(t - 1), e(t));
-    }
-    case 5: {
-        const int k = min(r >> 1, c), rr = r - 2 * k, cc = c - k;
-        if (rr == 0) return FAVG2(above[cc - 1], above[cc]);
-        if (rr == 1) return cc == 0 ? FAVG3(left[0], above[-1], above[0]) : FAVG3(above[cc - 2], above[cc - 1], above[cc]);
-        return rr == 2 ? FAVG3(above[-1], left[0], left[1]) : FAVG3(left[rr - 3], left[rr - 2], left[rr - 1]);
-    }
-    case 6: {
-        const int k = min(r, c >> 1), rr = r - k, cc = c - 2 * k;
-        if (cc == 0) return rr == 0 ? FAVG2(above[-1], left[0]) : FAVG2(left[rr - 1], left[rr]);
-        if (cc == 1) return rr == 0 ? FAVG3(left[0], above[-1], above[0])
-                          : rr == 1 ? FAVG3(above[-1], left[0], left[1]) : FAVG3(left[rr - 2], left[rr - 1], left[rr]);
-        return FAVG3(above[cc - 3], above[cc - 2], above[cc - 1]);
-    }
-    case 7: {
-        const int k = r + (c >> 1);
-        auto L = [&](int i) -> int { return left[i < n ? i : n - 1]; };
-        return (c & 1) ? FAVG3(L(k), L(k + 1), L(k + 2)) : FAVG2(L(k), L(k + 1));
-    }
-    case 8: {
-        const int k = (r >> 1) + c;
-        return (r & 1) ? FAVG3(above[k], above[k + 1], above[k + 2]) : FAVG2(above[k], above[k + 1]);
-    }
-    case 9: return clampi((int)left[r] + (int)above[c] - (int)above[-1], 0, MAXV);
-    default: return dc;
-    }
 }
 
 /* Residual grid (and SPEC temp) index of a plane's sample. */
@@ -1567,6 +1550,27 @@ __device__ __forceinline__ void intra_halo(const IntraView<T> &V, const cvp9_job
             col[k] = v;
             tile[k * pitch - 1] = v;
         }
+    }
+}
+
+/* Claim the 4x4 cells of columns [c0x, c1x] and rows [c0y, c1y] for a block:
+ * a bit per cell, a word per row of the SB; true when another block has one
+ * of them. (A thread a block: a 64x64 block is 16 atomics.) */
+__device__ __forceinline__ bool claim_cells(uint32_t *rows, int c0x, int c1x, int c0y, int c1y)
+{
+    const uint32_t m = ((2u << c1x) - 1u) & ~((1u << c0x) - 1u);
+    uint32_t seen = 0;
+    for (int cy = c0y; cy <= c1y; cy++) seen |= atomicOr(&rows[cy], m);
+    return (seen & m) != 0;
+}
+
+/* The owner map of those cells: block + 1, one warp. */
+__device__ __forceinline__ void own_cells(uint16_t *cell, int b, int c0x, int c1x, int c0y, int c1y, int lane)
+{
+    const int w = c1x - c0x + 1, n = w * (c1y - c0y + 1);
+    for (int k = lane; k < n; k += 32) {
+        const int r = div_small(k, w);
+        cell[(c0y + r) * 16 + c0x + k - r * w] = (uint16_t)(b + 1);
     }
 }
 
@@ -4510,12 +4514,12 @@ __global__ void __launch_bounds__(128) k_lf_full(const cvp9_job_t *__restrict__ 
  * is k_lf_full<uint16_t, 2>.
  *
  * One CTA per superblock ticket (SB-diagonal order over the step's jobs,
- * persistent, as k_recon). Its inter blocks do not depend on one another or
- * on other superblocks, so they go first and together: prediction a thread
- * per column strip of up to 8 rows, then a thread per TX row, then per TX
- * column. The intra blocks follow by dependency level, the blocks of a
- * level on different warps, each block TX by TX (each TX predicted from the
- * reconstructed samples around it). A superblock whose blocks overlap, or
+ * persistent, as k_recon). What reads no neighbour goes first and together:
+ * the inter predictions a thread per column strip of up to 8 rows, then every
+ * residual a thread per TX row, then per TX column. The intra blocks follow
+ * as in k_recon, TX by TX in dependency levels over the whole CTA (8x1080p
+ * key step 15.6 -> 3.9 ms against a warp per block, prediction and
+ * transforms in turn). A superblock whose blocks overlap, or
  * whose intra blocks read samples of blocks later in the list, runs block by
  * block in list order, so every sample is what the list order makes it. */
 namespace {
@@ -4540,25 +4544,30 @@ struct HbdBlk {
 
 struct HbdTx {
     uint32_t coeff;
-    uint8_t  plane, txl, x, y;   /* plane-local tile position */
+    uint8_t  plane;              /* | TX type << 2, 16 intra, 32 no coefficients */
+    uint8_t  txl, x, y;          /* plane-local tile position */
 };
 
 struct HbdSmem {
     uint16_t ty[65 * kHYP];                /* luma tile, row 0 = the row above */
     uint16_t tc[2][33 * kHCP];
-    int32_t  tmp[64 * 64 + 2 * 32 * 32];   /* row-pass output at tile positions */
+    union {
+        int32_t i[64 * 64 + 2 * 32 * 32];  /* row-pass output at tile positions */
+        IntraWork w;                       /* then the intra tasks             */
+    } tmp;
+    int16_t  res[kResidGrid];              /* residuals of the intra blocks    */
+    uint16_t col[16 * 64 + 2 * 16 * 32];   /* left-column copies (IntraView)   */
     HbdBlk   blk[kHbdMaxBlocks];
     HbdTx    tx[kHbdMaxTx];
     uint16_t tx_base[kHbdMaxTx + 1];       /* prefix over TXs of their sizes   */
     uint16_t it_base[kHbdMaxBlocks + 1];   /* prefix over blocks of their items */
-    unsigned cell[256];                    /* claims of each 4x4 cell          */
-    uint8_t  owner[256];                   /* the block claiming it (one claim) */
-    uint8_t  lvl[kHbdMaxBlocks];           /* intra blocks: dependency level   */
-    uint8_t  txnz[kHbdMaxTx];
-    int32_t  edge[kHbdWarps][1 + 64 + 32]; /* intra, per warp: above[-1..2n-1], left */
+    uint16_t cell[256];                    /* owner block + 1 per 4x4          */
+    uint32_t rows[16];                     /* claimed cells, a bit each        */
+    uint8_t  txnz[kHbdMaxTx];              /* a TX has a nonzero coefficient   */
+    uint8_t  txwide[kHbdMaxTx];            /* and one that needs 64-bit values */
     int      scan[kHbdWarps];
     cvp9_job_t jc;
-    int      ticket, ntx, nlev, order_bad;
+    int      ticket;
 };
 
 __device__ __forceinline__ uint16_t &HT(HbdSmem &s, int p, int x, int y)
@@ -4568,12 +4577,7 @@ __device__ __forceinline__ uint16_t &HT(HbdSmem &s, int p, int x, int y)
 
 __device__ __forceinline__ int32_t *hbd_tmp(HbdSmem &s, int p, int x, int y)
 {
-    return p == 0 ? &s.tmp[y * 64 + x] : &s.tmp[4096 + (p - 1) * 1024 + y * 32 + x];
-}
-
-__device__ __forceinline__ long long clampll(long long v, long long lo, long long hi)
-{
-    return v < lo ? lo : (v > hi ? hi : v);
+    return &s.tmp.i[plane_at(p, x, y)];
 }
 
 /* Exclusive prefix of v over the CTA's threads (thread order); *total: the
@@ -4690,141 +4694,182 @@ __device__ void hbd_pred_strip(HbdSmem &s, const HbdBlk &b, int item, int sbx, i
         if (i < nr) HT(s, p, lx, ly0 + i) = (uint16_t)out[i];
 }
 
-/* The TX layout of one plane of a block (as plane_layout). */
-__device__ __forceinline__ void hbd_plane_layout(const HbdBlk &b, const cvp9_job_t &job, int gx, int gy, int p,
-                                                 int &tx, int &nx, int &ny, int &pbw)
+/* The residual TXs of a block in coefficient order (planes, then raster) as
+ * s.tx[at ...], by one warp; their number whatever the coefficients. A TX
+ * whose coefficients do not end inside num_coeffs is marked empty: offsets
+ * ascend, so every later one of the block is, too (as is one reaching past
+ * the SB, which no block that its TXs tile has). */
+__device__ int hbd_tx_count(const HbdBlk &b, const cvp9_job_t &job, int sbx, int sby)
 {
-    const int sub8 = b.w < 8 || b.h < 8;
-    const int ew = sub8 ? 8 : b.w, eh = sub8 ? 8 : b.h;
-    const int ss = p > 0;
-    int pw = ss ? ew / 2 : ew, ph = ss ? eh / 2 : eh;
-    pw = pw < 4 ? 4 : pw;
-    ph = ph < 4 ? 4 : ph;
-    tx = b.txl;
-    if (ss) { const int mt = max_tx_for(pw, ph); tx = sub8 ? 0 : (tx > mt ? mt : tx); }
-    const int t4 = 1 << tx;
-    const int o4x = ((gx >> 3) * 2) >> ss, o4y = ((gy >> 3) * 2) >> ss;
-    int mw = pw / 4, mh = ph / 4;
-    const int lim_w = ((job.mi_cols * 2) >> ss) - o4x, lim_h = ((job.mi_rows * 2) >> ss) - o4y;
-    if (mw > lim_w) mw = lim_w;
-    if (mh > lim_h) mh = lim_h;
-    nx = mw > 0 ? (mw + t4 - 1) / t4 : 0;
-    ny = mh > 0 ? (mh + t4 - 1) / t4 : 0;
-    pbw = pw;
-}
-
-/* Residual TXs of an inter block in coefficient order (planes, then raster),
- * written from s.tx[at] when `at` >= 0; returns their count. The running
- * offset stops at num_coeffs: a TX that does not fit and every later one of
- * the block are dropped. */
-__device__ int hbd_block_txs(HbdSmem &s, const HbdBlk &b, int sbx, int sby, int at)
-{
-    if ((b.flags & 2) || b.txl > 3) return 0;
-    const cvp9_job_t &job = s.jc;
-    const int gx = sbx + b.x, gy = sby + b.y;
-    uint64_t off = b.coeff;
     int n = 0;
     for (int p = 0; p < 3; p++) {
         int txl, nx, ny, pbw;
-        hbd_plane_layout(b, job, gx, gy, p, txl, nx, ny, pbw);
-        const int sz = 16 << (2 * txl), ts = 4 << txl;
-        const int ox = p ? (b.x >> 1) : b.x, oy = p ? (b.y >> 1) : b.y;
-        for (int ty = 0; ty < ny; ty++)
-            for (int tx = 0; tx < nx; tx++) {
-                if (off + (uint64_t)sz > (uint64_t)job.num_coeffs) { off = job.num_coeffs; continue; }
-                if (at >= 0 && at + n < kHbdMaxTx) {
-                    HbdTx &t = s.tx[at + n];
-                    t.coeff = (uint32_t)off;
-                    t.plane = (uint8_t)p;
-                    t.txl = (uint8_t)txl;
-                    t.x = (uint8_t)(ox + tx * ts);
-                    t.y = (uint8_t)(oy + ty * ts);
-                }
-                off += (uint64_t)sz;
-                n++;
-            }
+        plane_layout(b, job, sbx + b.x, sby + b.y, p, txl, nx, ny, pbw);
+        n += nx * ny;
     }
     return n;
 }
 
-/* Row pass of TX row i: the frame's dequantised coefficients through the
- * 1-D inverse (DCT, ADST along the row when row_adst, WHT when lossless),
- * 64-bit inside, 32-bit out into the temp rows. Returns whether the row had
- * a nonzero coefficient. */
-template <int N>
-__device__ __forceinline__ bool hbd_row(HbdSmem &s, const int32_t *X, int i, int p, int px0, int py0,
-                                        bool lossless, bool row_adst)
+__device__ void hbd_list_txs(HbdSmem &s, const HbdBlk &b, int sbx, int sby, int at, int lane)
 {
-    wl v[N];
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        const int c = __ldg(X + i * N + k);
-        any |= c != 0;
-        v[k] = wl(c);
+    const cvp9_job_t &job = s.jc;
+    const int gx = sbx + b.x, gy = sby + b.y;
+    uint64_t off = b.coeff;
+    for (int p = 0; p < 3; p++) {
+        int txl, nx, ny, pbw;
+        plane_layout(b, job, gx, gy, p, txl, nx, ny, pbw);
+        const int sz = 16 << (2 * txl), ts = 4 << txl;
+        const int ox = p ? (b.x >> 1) : b.x, oy = p ? (b.y >> 1) : b.y;
+        const int type = ((b.flags & 1) && p == 0 && !job.lossless && txl < 3 && b.ymode < 10) ? c_tx_type[b.ymode] : 0;
+        for (int k = lane; k < nx * ny && at + k < kHbdMaxTx; k += 32) {
+            const int ty = div_small(k, nx), tx = k - ty * nx;
+            const uint64_t o = off + (uint64_t)k * (uint64_t)sz;
+            HbdTx &t = s.tx[at + k];
+            t.coeff = (uint32_t)o;
+            const bool none = o + (uint64_t)sz > (uint64_t)job.num_coeffs || ox + (tx + 1) * ts > (p ? 32 : 64) ||
+                              oy + (ty + 1) * ts > (p ? 32 : 64);
+            t.plane = (uint8_t)(p | (type << 2) | ((b.flags & 1) << 4) | (none ? 0x20 : 0));
+            t.txl = (uint8_t)txl;
+            t.x = (uint8_t)(ox + tx * ts);
+            t.y = (uint8_t)(oy + ty * ts);
+        }
+        at += nx * ny;
+        off += (uint64_t)(nx * ny) * (uint64_t)sz;
     }
-    if (any) {
-        if (N == 4 && lossless) iwht4(v, true);
-        else itx1<N>(v, row_adst);
-    }
-    int32_t *d = hbd_tmp(s, p, px0, py0 + i);
-#pragma unroll
-    for (int k = 0; k < N; k++) d[k] = any ? (int32_t)v[k].v : 0;
-    return any;
 }
 
-/* Column pass of TX column j: the 1-D inverse down the column (64-bit),
- * rounding shift 4/5/6/6 (none after the WHT), add and clip to 10 bits. */
+/* Row pass of TX row i: the frame's dequantised coefficients through the
+ * 1-D inverse (DCT, ADST along the row when row_adst, WHT when lossless),
+ * 64-bit products inside, 32-bit out into the temp rows. Returns 0 when the
+ * row has no nonzero coefficient, 2 when one is outside +-2^18 (a 10-bit
+ * stream's reach +-2^17): then the row, and its TX's columns, run on 64-bit
+ * values (wl). The 32-bit values (wn) took six steps of six 2160p inter pictures
+ * from 30.1 to 29.6 ms. */
+template <int N, class T>
+__device__ __forceinline__ void hbd_row_as(T (&v)[N], int32_t *d, bool lossless, bool row_adst)
+{
+    if (N == 4 && lossless) iwht4(v, true);
+    else itx1<N>(v, row_adst);
+#pragma unroll
+    for (int k = 0; k < N; k++) d[k] = (int32_t)v[k].v;
+}
+
 template <int N>
-__device__ __forceinline__ void hbd_col(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst)
+__device__ __noinline__ void hbd_row_wide(const int32_t *X, int32_t *d, bool lossless, bool row_adst)
 {
     wl v[N];
+    for (int k = 0; k < N; k++) v[k] = wl(X[k]);
+    hbd_row_as<N>(v, d, lossless, row_adst);
+}
+
+template <int N>
+__device__ __forceinline__ int hbd_row(HbdSmem &s, const int32_t *X, int i, int p, int px0, int py0,
+                                       bool lossless, bool row_adst)
+{
+    wn v[N];
+    int any = 0;
+    unsigned wide = 0;
+    X += i * N;
 #pragma unroll
-    for (int k = 0; k < N; k++) v[k] = wl(*hbd_tmp(s, p, px0 + j, py0 + k));
+    for (int k = 0; k < N; k++) {
+        const int c = __ldg(X + k);
+        any |= c;
+        wide |= ((unsigned)c + (1u << 18)) >> 19;
+        v[k] = wn(c);
+    }
+    int32_t *d = hbd_tmp(s, p, px0, py0 + i);
+    if (!any) {
+#pragma unroll
+        for (int k = 0; k < N; k++) d[k] = 0;
+        return 0;
+    }
+    if (wide) {
+        hbd_row_wide<N>(X, d, lossless, row_adst);
+        return 2;
+    }
+    hbd_row_as<N>(v, d, lossless, row_adst);
+    return 1;
+}
+
+/* Column pass of TX column j: the 1-D inverse down the column, rounding
+ * shift 4/5/6/6 (none after the WHT); an inter block's residual is added and
+ * clipped to 10 bits, an intra block's (intra) goes to the residual grid,
+ * saturated to int16, which no sum with a sample notices. wide: a row of the
+ * TX left the 32-bit range. */
+template <int N, class T>
+__device__ __forceinline__ void hbd_col_as(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst,
+                                           bool intra)
+{
+    T v[N];
+    const int32_t *c = hbd_tmp(s, p, px0 + j, py0);
+    const int pitch = p ? 32 : 64;
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] = T(c[k * pitch]);
     const bool wht = N == 4 && lossless;
     if (wht) iwht4(v, false);
     else itx1<N>(v, col_adst);
-    const int sh = N == 4 ? 4 : (N == 8 ? 5 : 6);
+    const int sh = wht ? 0 : N == 4 ? 4 : (N == 8 ? 5 : 6);
+    const int round = wht ? 0 : 1 << (sh - 1);
+    int16_t *r = s.res + plane_at(p, px0 + j, py0);
+    uint16_t *px = &HT(s, p, px0 + j, py0);
 #pragma unroll
     for (int k = 0; k < N; k++) {
-        const long long r = wht ? v[k].v : (v[k].v + (1ll << (sh - 1))) >> sh;
-        uint16_t &px = HT(s, p, px0 + j, py0 + k);
-        px = (uint16_t)clampll((long long)px + r, 0, kHbdMax);
+        const auto x = (v[k].v + round) >> sh;
+        const int q = x < -32768 ? -32768 : (x > 32767 ? 32767 : (int)x);
+        if (intra) r[k * pitch] = (int16_t)q;
+        else px[k * (p ? kHCP : kHYP)] = (uint16_t)clampi((int)px[k * (p ? kHCP : kHYP)] + q, 0, kHbdMax);
     }
 }
 
-__device__ __forceinline__ void hbd_row_n(HbdSmem &s, int txl, const int32_t *X, int i, int p, int x, int y,
-                                          bool lossless, bool row_adst, bool &any)
+template <int N>
+__device__ __noinline__ void hbd_col_wide(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst,
+                                          bool intra)
+{
+    hbd_col_as<N, wl>(s, j, p, px0, py0, lossless, col_adst, intra);
+}
+
+template <int N>
+__device__ __forceinline__ void hbd_col(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst,
+                                        bool intra, bool wide)
+{
+    if (wide) hbd_col_wide<N>(s, j, p, px0, py0, lossless, col_adst, intra);
+    else hbd_col_as<N, wn>(s, j, p, px0, py0, lossless, col_adst, intra);
+}
+
+__device__ __forceinline__ int hbd_row_n(HbdSmem &s, int txl, const int32_t *X, int i, int p, int x, int y,
+                                         bool lossless, bool row_adst)
 {
     switch (txl) {
-    case 0: any = hbd_row<4>(s, X, i, p, x, y, lossless, row_adst); break;
-    case 1: any = hbd_row<8>(s, X, i, p, x, y, lossless, row_adst); break;
-    case 2: any = hbd_row<16>(s, X, i, p, x, y, lossless, row_adst); break;
-    default: any = hbd_row<32>(s, X, i, p, x, y, lossless, false); break;
+    case 0: return hbd_row<4>(s, X, i, p, x, y, lossless, row_adst);
+    case 1: return hbd_row<8>(s, X, i, p, x, y, lossless, row_adst);
+    case 2: return hbd_row<16>(s, X, i, p, x, y, lossless, row_adst);
+    default: return hbd_row<32>(s, X, i, p, x, y, lossless, false);
     }
 }
 
 __device__ __forceinline__ void hbd_col_n(HbdSmem &s, int txl, int j, int p, int x, int y, bool lossless,
-                                          bool col_adst)
+                                          bool col_adst, bool intra, bool wide)
 {
     switch (txl) {
-    case 0: hbd_col<4>(s, j, p, x, y, lossless, col_adst); break;
-    case 1: hbd_col<8>(s, j, p, x, y, lossless, col_adst); break;
-    case 2: hbd_col<16>(s, j, p, x, y, lossless, col_adst); break;
-    default: hbd_col<32>(s, j, p, x, y, lossless, false); break;
+    case 0: hbd_col<4>(s, j, p, x, y, lossless, col_adst, intra, wide); break;
+    case 1: hbd_col<8>(s, j, p, x, y, lossless, col_adst, intra, wide); break;
+    case 2: hbd_col<16>(s, j, p, x, y, lossless, col_adst, intra, wide); break;
+    default: hbd_col<32>(s, j, p, x, y, lossless, false, intra, wide); break;
     }
 }
 
-/* Inter blocks [lo, hi) of the SB, whole CTA: predictions, then the TX rows,
- * then the TX columns of their residuals. */
-__device__ void hbd_inter_blocks(HbdSmem &s, int lo, int hi, int nb, int sbx, int sby)
+/* Blocks [lo, hi) of the SB, whole CTA: the inter blocks' predictions, then
+ * the TX rows and the TX columns of every block's residual (an intra block's
+ * into the residual grid, which starts at zero). */
+__device__ __noinline__ void hbd_blocks(HbdSmem &s, int lo, int hi, int nb, int sbx, int sby)
 {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const cvp9_job_t &job = s.jc;
-    const bool mine = tid >= lo && tid < hi && tid < nb && !(s.blk[tid].flags & 1);
+    const bool in = tid >= lo && tid < hi && tid < nb;
+    const bool inter = in && !(s.blk[tid].flags & 1);
     int total;
     /* 1. predictions */
-    int cnt = mine ? hbd_pred_items(s.blk[tid]) : 0;
+    int cnt = inter ? hbd_pred_items(s.blk[tid]) : 0;
     int base = hbd_scan(s, cnt, &total);
     if (tid < kHbdMaxBlocks) s.it_base[tid] = (uint16_t)min(base, 0xFFFF);
     __syncthreads();
@@ -4832,14 +4877,19 @@ __device__ void hbd_inter_blocks(HbdSmem &s, int lo, int hi, int nb, int sbx, in
         const int bi = hbd_find(s.it_base, nb, it);
         hbd_pred_strip(s, s.blk[bi], it - s.it_base[bi], sbx, sby);
     }
-    /* 2. the residual TXs, a thread per block listing its own */
-    cnt = mine ? hbd_block_txs(s, s.blk[tid], sbx, sby, -1) : 0;
+    for (int i = tid; i < kResidGrid / 8; i += kHbdThreads) reinterpret_cast<uint4 *>(s.res)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    /* 2. the residual TXs, a warp per block listing them */
+    cnt = in && !(s.blk[tid].flags & 2) && s.blk[tid].txl <= 3 ? hbd_tx_count(s.blk[tid], job, sbx, sby) : 0;
     base = hbd_scan(s, cnt, &total);
     if (total > kHbdMaxTx) {
         if (tid == 0) atomicOr(job.status, (unsigned)CVP9_JOB_TOO_MANY);
         total = kHbdMaxTx;
     }
-    if (mine && cnt) hbd_block_txs(s, s.blk[tid], sbx, sby, base);
+    if (tid < kHbdMaxBlocks) s.it_base[tid] = (uint16_t)min(base, 0xFFFF);
+    __syncthreads();
+    for (int b = lo + warp; b < min(hi, nb); b += kHbdWarps)
+        if (!(s.blk[b].flags & 2) && s.blk[b].txl <= 3) hbd_list_txs(s, s.blk[b], sbx, sby, s.it_base[b], lane);
     __syncthreads();
     const int ntx = total;
     /* prefix over TXs of their edge length (their rows, and columns), two
@@ -4851,102 +4901,30 @@ __device__ void hbd_inter_blocks(HbdSmem &s, int lo, int hi, int nb, int sbx, in
         const int b0 = hbd_scan(s, a + c, &nrow_all);
         if (t0 <= ntx) s.tx_base[t0] = (uint16_t)b0;
         if (t1 <= ntx) s.tx_base[t1] = (uint16_t)(b0 + a);
-        if (t0 < ntx) s.txnz[t0] = 0;
-        if (t1 < ntx) s.txnz[t1] = 0;
+        if (t0 < ntx) s.txnz[t0] = s.txwide[t0] = 0;
+        if (t1 < ntx) s.txnz[t1] = s.txwide[t1] = 0;
     }
     if (ntx > 0) {
         __syncthreads();
         const int nrow = s.tx_base[ntx];
         for (int it = tid; it < nrow; it += kHbdThreads) {
             const int t = hbd_find(s.tx_base, ntx, it);
-            const HbdTx &x = s.tx[t];
-            bool any;
-            hbd_row_n(s, x.txl, job.coeffs32 + x.coeff, it - s.tx_base[t], x.plane, x.x, x.y, job.lossless, false,
-                      any);
-            if (any) s.txnz[t] = 1;
+            const HbdTx x = s.tx[t];
+            if (x.plane & 0x20) continue;
+            const int got = hbd_row_n(s, x.txl, job.coeffs32 + x.coeff, it - s.tx_base[t], x.plane & 3, x.x, x.y,
+                                      job.lossless, ((x.plane >> 2) & 3) >= 2);
+            if (got) s.txnz[t] = 1;
+            if (got == 2) s.txwide[t] = 1;
         }
         __syncthreads();
         for (int it = tid; it < nrow; it += kHbdThreads) {
             const int t = hbd_find(s.tx_base, ntx, it);
-            const HbdTx &x = s.tx[t];
-            if (s.txnz[t]) hbd_col_n(s, x.txl, it - s.tx_base[t], x.plane, x.x, x.y, job.lossless, false);
+            const HbdTx x = s.tx[t];
+            if (s.txnz[t]) hbd_col_n(s, x.txl, it - s.tx_base[t], x.plane & 3, x.x, x.y, job.lossless,
+                                     (x.plane >> 2) & 1, (x.plane >> 4) & 1, s.txwide[t] != 0);
         }
     }
     __syncthreads();
-}
-
-/* Intra prediction of one n x n TX of plane p (tile position lx, ly; plane
- * position X0, Y0 in a pw x ph plane) by one warp, the FULL edge rules at 10
- * bits: 511 above and 513 on the left when unavailable, above-right only for
- * a 4x4 TX with have_right, samples past the plane's edge repeating the
- * last one inside. */
-__device__ void hbd_intra_tx(HbdSmem &s, int p, int lx, int ly, int X0, int Y0, int pw, int ph, int n, int mode,
-                             bool have_top, bool have_left, bool have_right, int lane, int warp)
-{
-    int32_t *edge = s.edge[warp];
-    int32_t *above = edge + 1, *left = edge + 65;
-    if (have_top) {
-        const int want = n + ((n == 4 && have_right) ? 4 : 0);
-        const int cnt = min(want, pw - X0);
-        for (int i = lane; i < 2 * n; i += 32) above[i] = HT(s, p, lx + (i < cnt ? i : cnt - 1), ly - 1);
-        if (lane == 0) above[-1] = have_left ? HT(s, p, lx - 1, ly - 1) : kHbdMid + 1;
-    } else {
-        for (int i = lane; i < 2 * n + 1; i += 32) edge[i] = kHbdMid - 1;
-    }
-    for (int i = lane; i < n; i += 32) left[i] = have_left ? HT(s, p, lx - 1, ly + min(i, ph - 1 - Y0)) : kHbdMid + 1;
-    __syncwarp();
-    int dc = kHbdMid;
-    if (mode == 0) {
-        const unsigned sa = __reduce_add_sync(0xffffffffu, lane < n ? (unsigned)above[lane] : 0u);
-        const unsigned sl = __reduce_add_sync(0xffffffffu, lane < n ? (unsigned)left[lane] : 0u);
-        if (have_top && have_left) dc = (int)((sa + sl + (unsigned)n) / (unsigned)(2 * n));
-        else if (have_top) dc = (int)((sa + (unsigned)n / 2) / (unsigned)n);
-        else if (have_left) dc = (int)((sl + (unsigned)n / 2) / (unsigned)n);
-    }
-    const int lg = n == 4 ? 2 : n == 8 ? 3 : n == 16 ? 4 : 5;
-    for (int idx = lane; idx < n * n; idx += 32) {
-        const int r = idx >> lg, c = idx & (n - 1);
-        HT(s, p, lx + c, ly + r) = (uint16_t)full_pred<kHbdMax>(mode, r, c, n, above, left, dc);
-    }
-    __syncwarp();
-}
-
-/* One intra block by one warp: each plane's TXs in raster order, each
- * predicted and given its residual before the next. */
-__device__ void hbd_intra_block(HbdSmem &s, const HbdBlk &b, int sbx, int sby, int lane, int warp)
-{
-    const cvp9_job_t &job = s.jc;
-    const int gx = sbx + b.x, gy = sby + b.y;
-    const int mi_col = gx >> 3, mi_row = gy >> 3;
-    const bool left_ok = mi_col > full_tile_start(mi_col, job.mi_cols, job.log2_tile_cols);
-    const bool resid = !(b.flags & 2) && b.txl <= 3;
-    uint64_t off = b.coeff;
-    for (int p = 0; p < 3; p++) {
-        int txl, nx, ny, pbw;
-        hbd_plane_layout(b, job, gx, gy, p, txl, nx, ny, pbw);
-        const int n = 4 << txl, sz = n * n;
-        const int mode = p ? (b.uvmode > 9 ? 0 : b.uvmode) : (b.ymode > 9 ? 0 : b.ymode);
-        const int tx_type = (p == 0 && !job.lossless && txl < 3 && b.ymode < 10) ? c_tx_type[b.ymode] : 0;
-        const int pw = p ? job.CW : job.W, ph = p ? job.CH : job.H;
-        const int ox = p ? (b.x >> 1) : b.x, oy = p ? (b.y >> 1) : b.y;
-        const int gox = p ? (gx >> 1) : gx, goy = p ? (gy >> 1) : gy;
-        for (int ty = 0; ty < ny; ty++)
-            for (int tx = 0; tx < nx; tx++) {
-                const int lx = ox + tx * n, ly = oy + ty * n;
-                hbd_intra_tx(s, p, lx, ly, gox + tx * n, goy + ty * n, pw, ph, n, mode, ty > 0 || mi_row > 0,
-                             tx > 0 || left_ok, (tx + 1) * n < pbw, lane, warp);
-                if (!resid) continue;
-                if (off + (uint64_t)sz > (uint64_t)job.num_coeffs) { off = job.num_coeffs; continue; }
-                const int32_t *X = job.coeffs32 + off;
-                off += (uint64_t)sz;
-                bool any = false;
-                if (lane < n) hbd_row_n(s, txl, X, lane, p, lx, ly, job.lossless, tx_type == 2 || tx_type == 3, any);
-                any = __any_sync(0xffffffffu, any);
-                __syncwarp();
-                if (any && lane < n) hbd_col_n(s, txl, lane, p, lx, ly, job.lossless, tx_type == 1 || tx_type == 3);
-                __syncwarp();
-            }
-    }
 }
 
 } /* namespace */
@@ -4983,14 +4961,18 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
                          (groups && end - start > (uint32_t)kHbdMaxBlocks);
         int nb = (groups && !bad && !layout_bad) ? (int)(end - start) : 0;
         /* the tile at 512, no cell claimed */
-        for (int i = tid; i < 65 * kHYP; i += kHbdThreads) s.ty[i] = kHbdMid;
-        for (int i = tid; i < 2 * 33 * kHCP; i += kHbdThreads) (&s.tc[0][0])[i] = kHbdMid;
+        {
+            const uint4 mid = make_uint4(0x02000200u, 0x02000200u, 0x02000200u, 0x02000200u);
+            uint4 *t4 = reinterpret_cast<uint4 *>(s.ty);
+            for (int i = tid; i < (65 * kHYP + 2 * 33 * kHCP) / 8; i += kHbdThreads) t4[i] = mid;
+        }
         for (int i = tid; i < 256; i += kHbdThreads) s.cell[i] = 0;
+        if (tid < 16) s.rows[tid] = 0;
         __syncthreads();
 
         /* 1. blocks (each inside this SB, 4-aligned, 4..64 px, tx_size <= 3,
          * sub-8x8 ones on the 8x8 grid), and the 4x4 cells they write */
-        bool my_intra = false, my_bad = false;
+        bool my_intra = false, my_bad = false, my_seq = false;
         if (tid < nb) {
             const vp9_macroblock_info_t g = job.blocks[start + tid];
             const int lx = (int)g.x - sbx, ly = (int)g.y - sby;
@@ -5022,152 +5004,141 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
             b.coeff = g.coeff_offset;
             s.blk[tid] = b;
             my_intra = g.is_intra != 0;
+            /* TXs that do not tile their block, or whose chroma TXs straddle
+             * 4x4 cells: list order */
+            const int n = 4 << (g.tx_size & 3), m = min(n, 4 << max_tx_for(max(4, bw / 2), max(4, bh / 2)));
+            my_seq = (bw % n) || (bh % n) || (!sub8 && ((bw / 2) % m || (bh / 2) % m)) || (lx & 7) || (ly & 7);
         }
         if (__syncthreads_or(my_bad)) {
             if (tid == 0) atomicOr(job.status, (unsigned)CVP9_JOB_BAD_BLOCK);
             nb = 0;
-            my_intra = false;
+            my_intra = my_seq = false;
         }
         if (tid < nb) {
             /* cells of the luma region a block writes (a sub-8x8 block its 8x8) */
             const HbdBlk &b = s.blk[tid];
-            for (int cy = b.y >> 2; cy < min(16, (b.y + b.ch + 3) >> 2); cy++)
-                for (int cx = b.x >> 2; cx < min(16, (b.x + b.cw + 3) >> 2); cx++) {
-                    atomicAdd(&s.cell[cy * 16 + cx], 1u);
-                    s.owner[cy * 16 + cx] = (uint8_t)tid;
-                }
+            my_seq |= claim_cells(s.rows, b.x >> 2, (b.x + b.cw - 1) >> 2, b.y >> 2, (b.y + b.ch - 1) >> 2);
         }
-        __syncthreads();
-        bool my_over = false;
-        for (int i = tid; i < 256; i += kHbdThreads) my_over |= s.cell[i] > 1;
-        bool overlap = __syncthreads_or(my_over) != 0;
         const bool any_intra = __syncthreads_or(my_intra) != 0;
-        if (any_intra && !overlap) {
-            /* dependency levels of the intra blocks: 1 + the deepest intra
-             * block owning a sample of the row above, the column to the
-             * left or the corner (inter blocks, reconstructed first, count
-             * 0). A block reading samples of a block later in the list runs
-             * the superblock in list order instead. */
-            if (tid == 0) {
-                int nlev = 0, bad = 0;
-                for (int i = 0; i < nb; i++) {
-                    const HbdBlk &b = s.blk[i];
-                    s.lvl[i] = 0;
-                    if (!(b.flags & 1)) continue;
-                    int lv = 0;
-                    const int cx0 = b.x >> 2, cy0 = b.y >> 2;
-                    const int cx1 = (b.x + b.cw - 1) >> 2, cy1 = (b.y + b.ch - 1) >> 2;
-                    auto dep = [&](int cx, int cy) {
-                        if (cx < 0 || cy < 0 || cx > 15 || cy > 15) return;
-                        const int c = cy * 16 + cx;
-                        if (!s.cell[c]) return;
-                        const int j = s.owner[c];
-                        if (j > i) bad = 1;
-                        else if (j < i) lv = max(lv, (int)s.lvl[j]);
-                    };
-                    for (int cx = cx0 - 1; cx <= cx1; cx++) dep(cx, cy0 - 1);
-                    for (int cy = cy0; cy <= cy1; cy++) dep(cx0 - 1, cy);
-                    s.lvl[i] = (uint8_t)(lv + 1);
-                    nlev = max(nlev, lv + 1);
-                }
-                s.nlev = nlev;
-                s.order_bad = bad;
-            }
-            __syncthreads();
-            overlap = s.order_bad != 0;
-        }
-
-        /* 2. intra blocks read the neighbour SBs' samples: wait for them,
-         * then load the row above (x = -1..63) and the column to the left */
         if (any_intra) {
-            if (tid == 0) {
-                bool ok = true;
-                if (sbc > 0) ok &= wait_flag(job.sb_done + sb - 1, job.epoch);
-                if (sbr > 0) ok &= wait_flag(job.sb_done + sb - job.sb_cols, job.epoch);
-                if (sbr > 0 && sbc > 0) ok &= wait_flag(job.sb_done + sb - job.sb_cols - 1, job.epoch);
-                if (!ok) atomicOr(job.status, (unsigned)CVP9_JOB_TIMEOUT);
+            for (int i = warp; i < nb; i += kHbdWarps) {
+                const HbdBlk &b = s.blk[i];
+                own_cells(s.cell, i, b.x >> 2, (b.x + b.cw - 1) >> 2, b.y >> 2, (b.y + b.ch - 1) >> 2, lane);
             }
             __syncthreads();
-            const uint16_t *Y = reinterpret_cast<const uint16_t *>(job.out);
-            const uint16_t *U = Y + (size_t)job.W * job.H;
-            const uint16_t *V = U + (size_t)job.CW * job.CH;
-            if (sby > 0) {
-                for (int i = tid - 1; i < 64; i += kHbdThreads) {
-                    const int gx = sbx + i;
-                    if (gx >= 0 && gx < job.W) HT(s, 0, i, -1) = __ldcg(Y + (size_t)(sby - 1) * job.W + gx);
-                }
-                for (int i = tid - 1; i < 32; i += kHbdThreads) {
-                    const int gx = (sbx >> 1) + i;
-                    if (gx >= 0 && gx < job.CW) {
-                        HT(s, 1, i, -1) = __ldcg(U + (size_t)((sby >> 1) - 1) * job.CW + gx);
-                        HT(s, 2, i, -1) = __ldcg(V + (size_t)((sby >> 1) - 1) * job.CW + gx);
-                    }
-                }
-            }
-            if (sbx > 0) {
-                for (int i = tid; i < 64; i += kHbdThreads) {
-                    const int gy = sby + i;
-                    if (gy < job.H) HT(s, 0, -1, i) = __ldcg(Y + (size_t)gy * job.W + sbx - 1);
-                }
-                for (int i = tid; i < 32; i += kHbdThreads) {
-                    const int gy = (sby >> 1) + i;
-                    if (gy < job.CH) {
-                        HT(s, 1, -1, i) = __ldcg(U + (size_t)gy * job.CW + (sbx >> 1) - 1);
-                        HT(s, 2, -1, i) = __ldcg(V + (size_t)gy * job.CW + (sbx >> 1) - 1);
-                    }
-                }
-            }
         }
-        __syncthreads();
+        /* an intra block reading samples of a block later in the list: the
+         * superblock runs in list order */
+        unsigned needs = 0;
+        if (tid < nb && my_intra) {
+            const HbdBlk &b = s.blk[tid];
+            const int cx0 = b.x >> 2, cy0 = b.y >> 2, cx1 = (b.x + b.cw - 1) >> 2, cy1 = (b.y + b.ch - 1) >> 2;
+            if (cy0 > 0) for (int cx = max(0, cx0 - 1); cx <= cx1; cx++) my_seq |= s.cell[(cy0 - 1) * 16 + cx] > tid;
+            if (cx0 > 0) for (int cy = cy0; cy <= cy1; cy++) my_seq |= s.cell[cy * 16 + cx0 - 1] > tid;
+            needs = intra_needs(b.x, b.y);
+        }
+        const bool seq = __syncthreads_or(my_seq) != 0;
 
-        /* 3. reconstruct: inter blocks together, then intra blocks in order;
-         * overlapping blocks one by one in list order */
-        if (!overlap) {
-            hbd_inter_blocks(s, 0, nb, nb, sbx, sby);
-            /* intra blocks level by level, the blocks of a level one warp each */
-            const int nlev = any_intra ? s.nlev : 0;
-            for (int L = 1; L <= nlev; L++) {
-                int k = 0;
-                for (int i = 0; i < nb; i++) {
-                    if (s.lvl[i] != L) continue;
-                    if (k++ % kHbdWarps == warp) hbd_intra_block(s, s.blk[i], sbx, sby, lane, warp);
-                }
+        IntraWork &W = s.tmp.w;
+        IntraView<uint16_t> V;
+        V.ty = &HT(s, 0, 0, 0);
+        V.tc[0] = &HT(s, 1, 0, 0);
+        V.tc[1] = &HT(s, 2, 0, 0);
+        V.cy = s.col;
+        V.cc[0] = s.col + 16 * 64;
+        V.cc[1] = s.col + 16 * 64 + 16 * 32;
+        V.res = s.res;
+        const bool have_l = (sbx >> 3) > full_tile_start(sbx >> 3, job.mi_cols, job.log2_tile_cols);
+        auto neighbours = [&](unsigned need) {
+            if (tid < 3 && ((need >> tid) & 1u)) {
+                const int dc = tid == 1 ? 0 : 1, dr = tid == 0 ? 0 : 1;
+                if (sbc >= dc && sbr >= dr && (have_l || tid == 1) &&
+                    !wait_flag(job.sb_done + sb - dr * job.sb_cols - dc, job.epoch))
+                    atomicOr(job.status, (unsigned)CVP9_JOB_TIMEOUT);
+            }
+            __syncthreads();
+            intra_halo<uint16_t>(V, job, sbx, sby, sby > 0, have_l, kHbdMid - 1, kHbdMid + 1, tid, kHbdThreads);
+            __syncthreads();
+        };
+
+        /* 2. reconstruct: what reads no neighbour, then the intra blocks level
+         * by level; or block by block in list order */
+        if (!seq) {
+            hbd_blocks(s, 0, nb, nb, sbx, sby);
+            if (any_intra) {
+                intra_fill_cols(V, tid, kHbdThreads);
+                int ntask;
+                const int at = hbd_scan(s, tid < nb && my_intra ? hbd_tx_count(s.blk[tid], job, sbx, sby) : 0, &ntask);
+                s.it_base[tid] = (uint16_t)min(at, 0xFFFF);
+                for (int i = tid; i < kMaxTasks; i += kHbdThreads) W.own[i] = 0;
                 __syncthreads();
+                for (int b = warp; b < nb; b += kHbdWarps)
+                    if (s.blk[b].flags & 1) intra_tx_tasks(W, s.blk[b], job, sbx, sby, s.it_base[b], true, lane);
+                ntask = min(ntask, kMaxTasks);
+                __syncthreads();
+                intra_tx_levels(W, ntask, tid, kHbdThreads);
+                intra_sort(W, ntask, tid, kHbdThreads);
+                needs = __reduce_or_sync(0xffffffffu, needs);
+                needs = (unsigned)(__syncthreads_or(needs & 1u) ? 1u : 0u) | (__syncthreads_or(needs & 2u) ? 2u : 0u) |
+                        (__syncthreads_or(needs & 4u) ? 4u : 0u);
+                neighbours(needs);
+                intra_run<CVP9_ARITH_FULL, kHbdMax, uint16_t>(W, V, tid, kHbdThreads);
             }
         } else {
+            if (any_intra) neighbours(7u);
             for (int i = 0; i < nb; i++) {
+                hbd_blocks(s, i, i + 1, nb, sbx, sby);
                 if (s.blk[i].flags & 1) {
-                    if (warp == 0) hbd_intra_block(s, s.blk[i], sbx, sby, lane, warp);
+                    intra_fill_cols(V, tid, kHbdThreads);
+                    if (warp == 0) {
+                        const int n = intra_tx_tasks(W, s.blk[i], job, sbx, sby, 0, false, lane);
+                        if (lane == 0) W.ntask = min(n, kMaxTasks);
+                    }
                     __syncthreads();
-                } else {
-                    hbd_inter_blocks(s, i, i + 1, nb, sbx, sby);
+                    intra_run_ordered<CVP9_ARITH_FULL, kHbdMax, uint16_t>(W, V, W.ntask, tid, kHbdThreads);
+                    __syncthreads();
                 }
             }
         }
 
-        /* 4. write the tile (clipped to the frame) and release the SB */
+        /* 3. the samples the neighbours read, release the SB, then the whole
+         * tile (clipped to the frame) */
         {
-            uint16_t *Y = reinterpret_cast<uint16_t *>(job.out);
-            uint16_t *U = Y + (size_t)job.W * job.H;
-            uint16_t *V = U + (size_t)job.CW * job.CH;
+            uint16_t *out = reinterpret_cast<uint16_t *>(job.out);
             const int vw = min(64, job.W - sbx), vh = min(64, job.H - sby);
-            for (int i = tid; i < 64 * 64; i += kHbdThreads) {
-                const int r = i >> 6, c = i & 63;
-                if (r < vh && c < vw) Y[(size_t)(sby + r) * job.W + sbx + c] = HT(s, 0, c, r);
+            {
+                const int p = tid < 128 ? 0 : 1 + ((tid >> 5) & 1), n = p ? 32 : 64;
+                const bool row = tid < 128 ? tid >= 64 : tid >= 192;
+                const int k = p ? tid & 31 : tid & 63;
+                const int pw = p ? job.CW : job.W, ph = p ? job.CH : job.H;
+                const int X = (p ? sbx >> 1 : sbx) + (row ? k : n - 1), Y = (p ? sby >> 1 : sby) + (row ? n - 1 : k);
+                if (X < pw && Y < ph && (row ? vh == 64 : vw == 64))
+                    out[(p ? (size_t)job.W * job.H + (size_t)(p - 1) * job.CW * job.CH : 0) + (size_t)Y * pw + X] =
+                        HT(s, p, row ? k : n - 1, row ? n - 1 : k);
+            }
+            __syncthreads();
+            if (tid == 0) {
+                if (bad)
+                    atomicOr(job.status, (unsigned)CVP9_JOB_BAD_ORDER |
+                                         ((groups && end >= start && end - start > (uint32_t)kHbdMaxBlocks) ? (unsigned)CVP9_JOB_TOO_MANY : 0u));
+                __threadfence();
+                st_release(job.sb_done + sb, job.epoch);
+            }
+            /* four samples a store: sizes are multiples of 8 */
+            uint16_t *U = out + (size_t)job.W * job.H, *Vp = U + (size_t)job.CW * job.CH;
+            for (int i = tid; i < 64 * 16; i += kHbdThreads) {
+                const int r = i >> 4, c = (i & 15) * 4;
+                if (r < vh && c < vw)
+                    *reinterpret_cast<uint2 *>(out + (size_t)(sby + r) * job.W + sbx + c) =
+                        *reinterpret_cast<const uint2 *>(&HT(s, 0, c, r));
             }
             const int cvw = min(32, job.CW - (sbx >> 1)), cvh = min(32, job.CH - (sby >> 1));
-            for (int i = tid; i < 2 * 32 * 32; i += kHbdThreads) {
-                const int p = i >> 10, k = i & 1023, r = k >> 5, c = k & 31;
-                if (r < cvh && c < cvw) (p ? V : U)[(size_t)((sby >> 1) + r) * job.CW + (sbx >> 1) + c] = HT(s, 1 + p, c, r);
+            for (int i = tid; i < 2 * 32 * 8; i += kHbdThreads) {
+                const int p = i >> 8, r = (i >> 3) & 31, c = (i & 7) * 4;
+                if (r < cvh && c < cvw)
+                    *reinterpret_cast<uint2 *>((p ? Vp : U) + (size_t)((sby >> 1) + r) * job.CW + (sbx >> 1) + c) =
+                        *reinterpret_cast<const uint2 *>(&HT(s, 1 + p, c, r));
             }
-        }
-        if (tid == 0 && bad)
-            atomicOr(job.status, (unsigned)CVP9_JOB_BAD_ORDER |
-                                 ((groups && end >= start && end - start > (uint32_t)kHbdMaxBlocks) ? (unsigned)CVP9_JOB_TOO_MANY : 0u));
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            st_release(job.sb_done + sb, job.epoch);
         }
     }
 }

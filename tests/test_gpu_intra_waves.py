@@ -9,7 +9,8 @@ import numpy as np
 import pytest
 
 from compute_vp9_b200 import ARITH_FULL, ARITH_REFCPU, ARITH_SPEC, CVP9_OK, BlockInfo, CudaBackend, Synth, synth_config
-from oracle.oracle_py import FULL, REFCPU, SPEC, OracleStream
+from compute_vp9_b200.hbd import HbdEngine, hbd_frames
+from oracle.oracle_py import FULL, REFCPU, SPEC, HbdOracleStream, OracleStream
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +58,24 @@ def test_intra_waves(arith, size, content, reverse):
         assert rc == CVP9_OK, gpu.last_error()
         assert np.array_equal(got, want), "frame %d: %d bytes differ" % (f, int((got != want).sum()))
     gpu.close()
+
+
+@pytest.mark.parametrize("step", [64, 2000])      # 2000: dequantised values past +-2^18 among smaller ones
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("content", list(CONTENT))
+@pytest.mark.parametrize("size", [(64, 64), (136, 72), (328, 200)])
+def test_intra_waves_10bit(size, content, reverse, step):
+    w, h = size
+    eng = HbdEngine()
+    sid = eng.open_stream(w, h)
+    orc = HbdOracleStream()
+    over = dict(CONTENT[content], gop=2, intra_in_inter=0.5, all_intra_modes=1)
+    for f, (pf, c32) in enumerate(hbd_frames(2, w, h, 3, seed=w + h, step=step, **over)):
+        if reverse:
+            _reverse_superblocks(pf)
+        want = orc.decode(pf, c32)
+        assert eng.submit([sid], [(pf, c32.ctypes.data)]) == CVP9_OK
+        assert eng.wait() == CVP9_OK
+        got = eng.get_frame(sid)
+        assert np.array_equal(got, want), "frame %d: %d samples differ" % (f, int((got != want).sum()))
+    eng.close()
