@@ -51,22 +51,17 @@ constexpr int kMaxItems = 1536;      /* TX columns per SB: 4x4 TXs on all three 
 constexpr int kYPitch = 72;          /* luma tile row pitch; x = 0 at byte 4 */
 constexpr int kCPitch = 40;          /* chroma tile row pitch; x = 0 at byte 4 */
 constexpr int kTempPitch = 65;       /* doubles per REFCPU temp row */
-constexpr int kStagePerWarp = 768;   /* bytes of MC staging per warp */
 constexpr int kTyBytes = (65 * kYPitch + 15) / 16 * 16;
 constexpr int kTcBytes = (33 * kCPitch + 15) / 16 * 16;
 constexpr long long kSpinLimit = 1ll << 20;   /* ~0.25 s of polling */
 
 __constant__ double c_dct[16 + 64 + 256 + 1024];      /* N = 4, 8, 16, 32 */
-__constant__ int c_subpel[16][8] = CVP9_SUBPEL_REGULAR_INIT;
-/* FULL: the frame header's filter, interp_filter 0..3 */
-__constant__ int c_subpel4[4][16][8] = { CVP9_SUBPEL_REGULAR_INIT, CVP9_SUBPEL_SMOOTH_INIT,
-                                         CVP9_SUBPEL_SHARP_INIT, CVP9_SUBPEL_BILINEAR_INIT };
 __constant__ uint8_t c_tx_type[10] = CVP9_INTRA_TX_TYPE_INIT;
-/* the same taps as signed bytes, taps 0-3 and 4-7 in two words, for dp4a
+/* the regular filter's taps as signed bytes, taps 0-3 and 4-7 in two words, for dp4a
  * (phase 0's 128 does not fit a byte: callers take the centre sample for
  * it, which is what its filter computes); uploaded by cvp9k_configure */
 __constant__ uint32_t c_subpel_pk[16][2];
-/* the four VP9 filters (c_subpel4) packed the same way, for the FULL profile */
+/* the four VP9 filters (interp_filter 0..3) packed the same way, for the FULL profile */
 __constant__ uint32_t c_subpel4_pk[4][16][2];
 
 __device__ __forceinline__ const double *dct_basis(int txl)
@@ -397,47 +392,72 @@ struct BlkS {
  * key) 21.5 -> 6.0 ms, a step of 24 1366x768 REFCPU inter pictures with 5%
  * intra blocks 2.2 -> 1.4 ms. */
 
-struct alignas(16) ITask {
-    uint8_t x, y;        /* plane position in the SB tile                    */
-    uint8_t w, h;        /* samples written                                  */
-    uint8_t pw, ph;      /* of them predicted (the rest keep the tile's: the
-                          * residual of a SPEC sub-8x8 block covers its MI)  */
-    uint8_t pm;          /* plane | mode << 2                                */
-    uint8_t acl, lcl;    /* last sample read of the row above, of the left
-                          * column: later ones repeat it                     */
-    uint8_t dcw, dch;    /* edge lengths (DC sums; directional modes: n)     */
-    uint8_t avail;       /* 1: samples above, 2: to the left (DC)            */
-    uint8_t spare[5];
+struct ITask {           /* four words, read as one 16-byte load            */
+    uint32_t xywh;       /* plane position in the SB tile; samples written   */
+    uint32_t edge;       /* plane | mode << 2; last sample read of the row
+                          * above, of the left column (later ones repeat it);
+                          * DC: 1 counts the row above, 2 the left column    */
+    uint32_t area;       /* edge lengths: the TX size (FULL), the predicted
+                          * area (others: samples past it keep the tile's,
+                          * the residual of a SPEC sub-8x8 block covers its
+                          * whole MI)                                        */
+    uint32_t inv;        /* DC: ceil(2^32 / samples counted); 0: one sample  */
+    __device__ __forceinline__ int x() const { return (int)(xywh & 255u); }
+    __device__ __forceinline__ int y() const { return (int)((xywh >> 8) & 255u); }
+    __device__ __forceinline__ int w() const { return (int)((xywh >> 16) & 255u); }
+    __device__ __forceinline__ int h() const { return (int)(xywh >> 24); }
+    __device__ __forceinline__ int plane() const { return (int)(edge & 3u); }
+    __device__ __forceinline__ int mode() const { return (int)((edge >> 2) & 63u); }
+    __device__ __forceinline__ int acl() const { return (int)((edge >> 8) & 255u); }
+    __device__ __forceinline__ int lcl() const { return (int)((edge >> 16) & 255u); }
+    __device__ __forceinline__ unsigned avail() const { return edge >> 24; }
+    __device__ __forceinline__ int pw() const { return (int)(area & 255u); }
+    __device__ __forceinline__ int ph() const { return (int)(area >> 8); }
 };
 
-/* A task as one 16-byte shared-memory load. */
-__device__ __forceinline__ ITask ld_task(const ITask *t)
+__device__ __forceinline__ ITask ld_task(const uint4 *t)
 {
-    const uint4 w = *reinterpret_cast<const uint4 *>(t);
-    ITask o;
-    __builtin_memcpy(&o, &w, sizeof(o));
-    return o;
+    const uint4 w = *t;
+    return ITask{ w.x, w.y, w.z, w.w };
+}
+
+__device__ __forceinline__ void st_task(uint4 *t, int x, int y, int w, int h, int plane, int mode, int acl, int lcl,
+                                        int avail, int pw, int ph, uint32_t inv)
+{
+    *t = make_uint4((uint32_t)(x | y << 8 | w << 16) | (uint32_t)h << 24,
+                    (uint32_t)(plane | mode << 2 | acl << 8 | lcl << 16) | (uint32_t)avail << 24,
+                    (uint32_t)(pw | ph << 8), inv);
 }
 
 constexpr int kMaxTasks = 384;       /* 4x4 TXs of an SB's three planes; 3 x kMaxBlocks */
+constexpr uint32_t kNoQuad = 0xFFFFFFFFu;
 constexpr int kResidGrid = 64 * 64 + 2 * 32 * 32;
 constexpr int kMaxQuads = 2048;      /* 16 a luma row, at most 11 a chroma row */
 
 struct IntraWork {
     uint32_t qtab[kMaxQuads];        /* by level: task | row << 9 | quad << 15 */
     uint32_t lvlq[kMaxTasks + 1];    /* quads per level, then each level's first */
-    ITask    task[kMaxTasks];
+    uint4    task[kMaxTasks];        /* ITask                                */
     uint16_t lvl[kMaxTasks];
     uint16_t qat[kMaxTasks];         /* a task's first quad in its level     */
-    uint16_t own[kMaxTasks];         /* FULL: task + 1 owning each 4x4 cell (luma 256, U 64, V 64) */
+    uint16_t own[kMaxTasks];         /* FULL: task + 1 owning each 4x4 cell (luma 256, U 64, V 64);
+                                      * others: task of each block's luma, 0xFFFF none */
+    uint32_t prow[3][16], pcol[3][16];   /* intra_levels: cells still open, by row and by column */
     int      ntask, nlev;
 };
 
+/* A superblock's tile for the intra tasks. The planes of the tile, and the
+ * left columns (luma before x = 4k at [k * 64 + y], chroma before x = 2k at
+ * [k * 32 + y]), lie at fixed distances, so that a plane is an offset and not
+ * a pointer picked from an array (which would go through local memory). */
 template <class T>
 struct IntraView {
-    T *ty, *tc[2];                   /* sample (0, 0) of each plane's tile   */
-    T *cy, *cc[2];                   /* left columns: luma before x = 4k at [k * 64 + y], chroma before x = 2k at [k * 32 + y] */
+    static constexpr int kU = sizeof(T) == 1 ? kTyBytes + kCPitch - kYPitch : 65 * kYPitch + kCPitch - kYPitch;
+    static constexpr int kUV = sizeof(T) == 1 ? kTcBytes : 33 * kCPitch;
+    T *tile0, *col0;                 /* luma sample (0, 0); column 0          */
     const int16_t *res;              /* residuals: 64x64 luma, 32x32 U, V    */
+    __device__ __forceinline__ T *tile(int p) const { return tile0 + (p ? kU + (p - 1) * kUV : 0); }
+    __device__ __forceinline__ T *col(int p) const { return col0 + (p ? 16 * 64 + (p - 1) * 16 * 32 : 0); }
 };
 
 struct ReconSmem {
@@ -456,15 +476,16 @@ struct ReconSmem {
     BlkS     blk[kMaxBlocks];
     uint32_t txmask[256 + 64 + 64];              /* per-TX column-nonzero bits  */
     uint16_t cell[256];                          /* owner block + 1 per 4x4     */
-    uint16_t lvl[kMaxBlocks];                    /* block levels; FULL: first task */
+    uint32_t rows[16];                           /* claimed cells, a bit each   */
+    uint16_t first[kMaxBlocks];                  /* FULL: a block's first task  */
     uint16_t chunk_off[kMaxBlocks + 1];          /* inter chunks before a block */
     uint16_t item_off[kMaxBlocks + 1];           /* TX items before a block     */
     uint8_t  chunk_blk[256];                     /* chunk -> block              */
     uint8_t  item_blk[kMaxItems];                /* TX column/row -> block      */
     uint8_t  col[16 * 64 + 2 * 16 * 32];         /* left-column copies (IntraView) */
-    alignas(16) uint8_t stage[kWarps][kStagePerWarp];
     int      scan_tmp[2 * kWarps];
     unsigned c_lo, c_hi;                         /* coefficient span of the SB  */
+    unsigned needs;                              /* intra_needs of its blocks   */
     int      ticket;
 };
 
@@ -513,7 +534,7 @@ __device__ __forceinline__ void plane_layout(const B &b, const cvp9_job_t &job, 
 }
 
 template <int A>
-__device__ void residual_layout(BlkS &b, const cvp9_job_t &job, int gx, int gy)
+__device__ __forceinline__ void residual_layout(BlkS &b, const cvp9_job_t &job, int gx, int gy)
 {
     b.pnt[0] = b.pnt[1] = b.pnt[2] = 0;
     b.pnx[0] = b.pnx[1] = b.pnx[2] = 0;
@@ -541,42 +562,298 @@ __device__ __forceinline__ int block_items(const BlkS &b)
     return b.pnt[0] * (4 << b.ptxl[0]) + b.pnt[1] * (4 << b.ptxl[1]) + b.pnt[2] * (4 << b.ptxl[2]);
 }
 
+__device__ __forceinline__ int mc_chunks(int cw, int ch, int ccw, int cch);
+
+/* Inter chunks of a block: REFCPU an 8x8 of luma with its chroma, the others
+ * of one plane each (mc_chunks). */
+template <int A>
 __device__ __forceinline__ int block_chunks(const BlkS &b)
 {
-    return ((b.cw + 7) >> 3) * ((b.ch + 7) >> 3);
+    return A == CVP9_ARITH_REFCPU ? ((b.cw + 7) >> 3) * ((b.ch + 7) >> 3)
+                                  : mc_chunks(b.cw, b.ch, (b.cw + 1) >> 1, (b.ch + 1) >> 1);
 }
 
-/* Stage a (sw x sh) window of a reference plane starting at (x0, y0), at
- * most 16 wide and 2*MAXI high, every sample clamped into [0, pw-1] x
- * [0, ph-1], in two steps: every lane's loads first, then its shared-memory
- * stores. (Loaded and stored one by one, each load waits for the store
- * before it, which may alias: a round trip to L2 per row.) */
-template <int MAXI>
-struct WinRows {
-    uint32_t v[MAXI];
-    __device__ __forceinline__ void load(const uint8_t *__restrict__ plane, int stride, int pw, int ph,
-                                         int x0, int y0, int sw, int sh, int lane)
+/* c + the dot product of four signed taps with four unsigned samples */
+
+
+/* 4x4 byte transpose: rows a..d (one word of four columns each) to four
+ * words, one column each (its bytes in row order) */
+__device__ __forceinline__ void tr4(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t col[4])
+{
+    const uint32_t x0 = __byte_perm(a, b, 0x5140), x1 = __byte_perm(a, b, 0x7362);
+    const uint32_t y0 = __byte_perm(c, d, 0x5140), y1 = __byte_perm(c, d, 0x7362);
+    col[0] = __byte_perm(x0, y0, 0x5410);
+    col[1] = __byte_perm(x0, y0, 0x7632);
+    col[2] = __byte_perm(x1, y1, 0x5410);
+    col[3] = __byte_perm(x1, y1, 0x7632);
+}
+
+/* ── 8-tap inter prediction, eight lanes a chunk (SPEC, FULL, 10-bit) ─────
+ *
+ * A chunk is up to 8x8 samples of one plane of an inter block. Lane k of its
+ * eight runs the horizontal pass on rows k and k + 8 of the (h + 7)-row
+ * window — a row comes as a few 8-byte loads, shifted into place, and a
+ * sample is two dp4a (8 bits) or four dp2a (16 bits) — into shared rows, then
+ * the vertical pass of output row k, the window's rows transposed by byte
+ * permutes. Both passes round and clip, as vp9_mc.comp.glsl:61-110 does;
+ * every fetch is clamped into the reference plane. What bounded this was
+ * instructions and L1 requests, not bytes: a warp per chunk with a load per
+ * sample took 50 k cycles a superblock (8 bits), a load per tap and sample 75 k
+ * (10 bits), this 25 k and 42 k. */
+template <class T> struct McRow;
+
+template <> struct McRow<uint8_t> {
+    static constexpr int kWords = 4, kLoads = 3;      /* 16 samples; 15 + 7 bytes */
+    /* 8 outputs of the horizontal pass, packed as two words */
+    static __device__ __forceinline__ void filter(const uint32_t (&w)[4], int f, uint32_t ta, uint32_t tb, uint8_t *d)
     {
-        const int xm = pw > 0 ? pw - 1 : 0, ym = ph > 0 ? ph - 1 : 0;
-        const int sx = lane & 15;
-        const int xx = clampi(x0 + sx, 0, xm);
+        uint32_t *o = reinterpret_cast<uint32_t *>(d);
+        if (f == 0) {
+            o[0] = __funnelshift_r(w[0], w[1], 24);
+            o[1] = __funnelshift_r(w[1], w[2], 24);
+            return;
+        }
+        uint32_t s[12];
 #pragma unroll
-        for (int k = 0; k < MAXI; k++) {
-            const int sy = (lane >> 4) + 2 * k;
-            v[k] = (sx < sw && sy < sh) ? (uint32_t)__ldg(plane + (size_t)clampi(y0 + sy, 0, ym) * stride + xx) : 0u;
+        for (int c = 0; c < 12; c++) s[c] = (c & 3) ? __funnelshift_r(w[c >> 2], w[(c >> 2) + 1], 8 * (c & 3)) : w[c >> 2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint32_t r[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) r[c] = tap_round(dp4a_su(tb, s[4 * h + c + 4], dp4a_su(ta, s[4 * h + c], 0)));
+            o[h] = r[0] | r[1] << 8 | r[2] << 16 | r[3] << 24;
         }
     }
-    __device__ __forceinline__ void store(uint8_t *st, int sp, int sw, int sh, int lane) const
+    /* output row from the 8 rows at h (8 samples each) */
+    static __device__ __forceinline__ void down(const uint8_t *h, int f, uint32_t ta, uint32_t tb, int (&v)[8])
     {
-        const int sx = lane & 15;
-        if (sx >= sw) return;
+        const uint2 *r = reinterpret_cast<const uint2 *>(h);
+        if (f == 0) {
+            const uint2 m = r[3];
 #pragma unroll
-        for (int k = 0; k < MAXI; k++) {
-            const int sy = (lane >> 4) + 2 * k;
-            if (sy < sh) st[sy * sp + sx] = (uint8_t)v[k];
+            for (int c = 0; c < 4; c++) {
+                v[c] = (int)((m.x >> (8 * c)) & 255u);
+                v[4 + c] = (int)((m.y >> (8 * c)) & 255u);
+            }
+            return;
+        }
+        uint2 a[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) a[t] = r[t];
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            uint32_t lo[4], hi[4];
+            tr4(s ? a[0].y : a[0].x, s ? a[1].y : a[1].x, s ? a[2].y : a[2].x, s ? a[3].y : a[3].x, lo);
+            tr4(s ? a[4].y : a[4].x, s ? a[5].y : a[5].x, s ? a[6].y : a[6].x, s ? a[7].y : a[7].x, hi);
+#pragma unroll
+            for (int c = 0; c < 4; c++) v[4 * s + c] = (int)tap_round(dp4a_su(tb, hi[c], dp4a_su(ta, lo[c], 0)));
         }
     }
 };
+
+__device__ __forceinline__ int dp2a_lo_su(uint32_t px, uint32_t taps, int c)
+{
+    int d;
+    asm("dp2a.lo.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(px), "r"(taps), "r"(c));
+    return d;
+}
+__device__ __forceinline__ int dp2a_hi_su(uint32_t px, uint32_t taps, int c)
+{
+    int d;
+    asm("dp2a.hi.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(px), "r"(taps), "r"(c));
+    return d;
+}
+
+template <> struct McRow<uint16_t> {
+    static constexpr int kWords = 8, kLoads = 5;      /* 16 samples; 30 + 6 bytes */
+    static __device__ __forceinline__ int tap(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t ta, uint32_t tb)
+    {
+        const int s = dp2a_hi_su(d, tb, dp2a_lo_su(c, tb, dp2a_hi_su(b, ta, dp2a_lo_su(a, ta, 64))));
+        return clampi(s >> 7, 0, 1023);
+    }
+    static __device__ __forceinline__ void filter(const uint32_t (&w)[8], int f, uint32_t ta, uint32_t tb, uint16_t *d)
+    {
+        uint4 *o = reinterpret_cast<uint4 *>(d);
+        uint32_t s[7];                                /* the words one sample on */
+#pragma unroll
+        for (int i = 0; i < 7; i++) s[i] = __funnelshift_r(w[i], w[i + 1], 16);
+        if (f == 0) {
+            *o = make_uint4(s[1], s[2], s[3], s[4]);
+            return;
+        }
+        uint32_t r[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            r[i] = (uint32_t)tap(w[i], w[i + 1], w[i + 2], w[i + 3], ta, tb) |
+                   (uint32_t)tap(s[i], s[i + 1], s[i + 2], s[i + 3], ta, tb) << 16;
+        *o = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+    static __device__ __forceinline__ void down(const uint16_t *h, int f, uint32_t ta, uint32_t tb, int (&v)[8])
+    {
+        const uint4 *r = reinterpret_cast<const uint4 *>(h);
+        if (f == 0) {
+            const uint4 m = r[3];
+            const uint32_t x[4] = { m.x, m.y, m.z, m.w };
+#pragma unroll
+            for (int i = 0; i < 4; i++) { v[2 * i] = (int)(x[i] & 0xffffu); v[2 * i + 1] = (int)(x[i] >> 16); }
+            return;
+        }
+        int acc[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) acc[c] = 64;
+#pragma unroll
+        for (int t = 0; t < 4; t++) {                 /* rows 2t and 2t + 1 side by side */
+            const uint4 a = r[2 * t], b = r[2 * t + 1];
+            const uint32_t x[4] = { a.x, a.y, a.z, a.w }, y[4] = { b.x, b.y, b.z, b.w };
+            const uint32_t tp = t < 2 ? ta : tb;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t e = __byte_perm(x[i], y[i], 0x5410), o = __byte_perm(x[i], y[i], 0x7632);
+                acc[2 * i] = t & 1 ? dp2a_hi_su(e, tp, acc[2 * i]) : dp2a_lo_su(e, tp, acc[2 * i]);
+                acc[2 * i + 1] = t & 1 ? dp2a_hi_su(o, tp, acc[2 * i + 1]) : dp2a_lo_su(o, tp, acc[2 * i + 1]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; c++) v[c] = clampi(acc[c] >> 7, 0, 1023);
+    }
+};
+
+/* 16 samples of a reference row from column X (the last may be beyond the
+ * window), as words. */
+template <class T>
+__device__ __forceinline__ void mc_load(const T *row, int X, int pw, uint32_t (&w)[McRow<T>::kWords])
+{
+    constexpr int kW = McRow<T>::kWords, kL = McRow<T>::kLoads, kPer = 4 / (int)sizeof(T);
+    if (X >= 0 && X + 16 + 8 / (int)sizeof(T) <= pw) {   /* every byte read is the row's */
+        const uintptr_t at = (uintptr_t)(row + X);
+        const uint2 *q = reinterpret_cast<const uint2 *>(at & ~(uintptr_t)7);
+        uint32_t u[2 * kL];
+#pragma unroll
+        for (int i = 0; i < kL; i++) {
+            const uint2 x = __ldg(q + i);
+            u[2 * i] = x.x;
+            u[2 * i + 1] = x.y;
+        }
+        const unsigned sh = 8u * (unsigned)(at & 3);
+        const bool odd = at & 4;
+        /* one word on when the row starts in the upper half of its 8 bytes */
+#pragma unroll
+        for (int i = 0; i < 2 * kL - 1; i++) u[i] = odd ? u[i + 1] : u[i];
+#pragma unroll
+        for (int i = 0; i < kW; i++) w[i] = __funnelshift_r(u[i], i + 1 < 2 * kL ? u[i + 1] : 0u, sh);
+    } else {
+        const int xm = pw > 0 ? pw - 1 : 0;
+#pragma unroll
+        for (int i = 0; i < kW; i++) {
+            uint32_t x = 0;
+#pragma unroll
+            for (int j = 0; j < kPer; j++)
+                x |= (uint32_t)__ldg(row + clampi(X + i * kPer + j, 0, xm)) << (8 * (int)sizeof(T) * j);
+            w[i] = x;
+        }
+    }
+}
+
+/* A chunk's part of one reference: its window's origin and phases. */
+struct McRef {
+    const void *plane;
+    int pw, ph, X, Y, fx, fy;
+};
+
+template <class T>
+__device__ __forceinline__ McRef mc_ref(const cvp9_ref_t &R, int p, int gx, int gy, int mvx, int mvy)
+{
+    McRef m;
+    const T *q = reinterpret_cast<const T *>(R.plane);
+    m.pw = R.w;
+    m.ph = R.h;
+    if (p) {
+        m.pw = (R.w + 1) >> 1;
+        m.ph = (R.h + 1) >> 1;
+        q += (size_t)R.w * R.h + (p == 2 ? (size_t)m.pw * m.ph : 0);
+    }
+    m.plane = q;
+    m.X = gx + (p ? mvx >> 4 : mvx >> 3) - 3;
+    m.Y = gy + (p ? mvy >> 4 : mvy >> 3) - 3;
+    m.fx = p ? mvx & 15 : (mvx & 7) << 1;
+    m.fy = p ? mvy & 15 : (mvy & 7) << 1;
+    return m;
+}
+
+/* One chunk by lane k of its eight (`on`: they have one; all lanes of the
+ * warp call it): 8 samples of row k of a w x h chunk at (lx, ly) of plane p
+ * into the tile row `dst`. rows: the group's 15 rows of 8 samples in shared
+ * memory, 16-byte aligned. A missing first reference predicts `mid`, a missing
+ * second one leaves the single prediction. */
+template <class T, class B>
+__device__ __forceinline__ void mc_chunk(const cvp9_job_t &job, const uint32_t (*P)[2], const B &b, bool on, int p, int gx,
+                                         int gy, int w, int h, int mid, T *rows, T *dst, int k)
+{
+    int v[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) v[c] = mid;
+    for (int q = 0; q < 2; q++) {
+        const int rf = on ? (q ? b.ref1 : b.ref0) : 0;
+        if (q && !__any_sync(0xffffffffu, on && rf != 0)) break;
+        const cvp9_ref_t &R = job.ref[job.ref_slot_of[clampi(rf - 1, 0, 2)] & 7];
+        on = on && R.plane;
+        const bool go = on && (q == 0 || rf != 0);
+        McRef m;
+        if (go) {
+            m = mc_ref<T>(R, p, gx, gy, q ? b.mv1x : b.mvx, q ? b.mv1y : b.mvy);
+            const uint32_t ta = P[m.fx][0], tb = P[m.fx][1];
+            const int ym = m.ph > 0 ? m.ph - 1 : 0;
+            for (int j = k; j < h + 7; j += 8) {
+                uint32_t x[McRow<T>::kWords];
+                mc_load<T>((const T *)m.plane + (size_t)clampi(m.Y + j, 0, ym) * m.pw, m.X, m.pw, x);
+                McRow<T>::filter(x, m.fx, ta, tb, rows + j * 8);
+            }
+        }
+        __syncwarp();
+        if (go && k < h) {
+            int u[8];
+            McRow<T>::down(rows + k * 8, m.fy, P[m.fy][0], P[m.fy][1], u);
+#pragma unroll
+            for (int c = 0; c < 8; c++) v[c] = q ? (v[c] + u[c] + 1) >> 1 : u[c];
+        }
+        __syncwarp();
+    }
+    if (k < h) {
+        if (w == 8 && !((uintptr_t)dst & 3)) {
+            uint32_t *d = reinterpret_cast<uint32_t *>(dst);
+            if (sizeof(T) == 1) {
+                d[0] = (uint32_t)v[0] | (uint32_t)v[1] << 8 | (uint32_t)v[2] << 16 | (uint32_t)v[3] << 24;
+                d[1] = (uint32_t)v[4] | (uint32_t)v[5] << 8 | (uint32_t)v[6] << 16 | (uint32_t)v[7] << 24;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++) d[i] = (uint32_t)v[2 * i] | (uint32_t)v[2 * i + 1] << 16;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; c++) if (c < w) dst[c] = (T)v[c];
+        }
+    }
+}
+
+/* A block's chunks: luma, then U, then V, raster of 8x8 each. */
+__device__ __forceinline__ int mc_chunks(int cw, int ch, int ccw, int cch)
+{
+    return ((cw + 7) >> 3) * ((ch + 7) >> 3) + 2 * ((ccw + 7) >> 3) * ((cch + 7) >> 3);
+}
+
+/* Chunk i of them: plane, position in the block, size. */
+__device__ __forceinline__ void mc_chunk_at(int i, int cw, int ch, int ccw, int cch, int &p, int &x, int &y, int &w, int &h)
+{
+    const int nl = ((cw + 7) >> 3) * ((ch + 7) >> 3), nc = ((ccw + 7) >> 3) * ((cch + 7) >> 3);
+    p = i < nl ? 0 : (i < nl + nc ? 1 : 2);
+    i -= p == 0 ? 0 : nl + (p - 1) * nc;
+    const int bw = p ? ccw : cw, bh = p ? cch : ch, nx = (bw + 7) >> 3;
+    const int r = div_small(i, nx);
+    x = (i - r * nx) * 8;
+    y = r * 8;
+    w = min(8, bw - x);
+    h = min(8, bh - y);
+}
 
 /* Geometry of one chunk's REFCPU bilinear prediction: integer positions and
  * fractions of the luma and chroma windows (vp9_reconstruct.c:94-131,
@@ -740,141 +1017,6 @@ __device__ __forceinline__ void refcpu_fill8(ReconSmem &s, int v, int lx0, int l
     const int p = 1 + (k >> 2), r = k & 3;
     if (r < clh)
         for (int c = 0; c < clw; c++) TC(s, p, cx0 + c, cy0 + r) = (uint8_t)v;
-}
-
-/* A reference that is absent predicts as a flat value (127 REFCPU, 128 SPEC). */
-__device__ __forceinline__ void fill_chunk(ReconSmem &s, int v, int lx0, int ly0, int lw, int lh,
-                                          int cx0, int cy0, int clw, int clh, int lane)
-{
-    for (int idx = lane; idx < 64; idx += 32) {
-        int r = idx >> 3, c = idx & 7;
-        if (r < lh && c < lw) TY(s, lx0 + c, ly0 + r) = (uint8_t)v;
-    }
-    int p = 1 + (lane >> 4), r = (lane >> 2) & 3, c = lane & 3;
-    if (r < clh && c < clw) TC(s, p, cx0 + c, cy0 + r) = (uint8_t)v;
-}
-
-/* SPEC inter prediction of one chunk from one reference: 8-tap on luma
- * (even phases of the 1/8-pel MV) and chroma (1/16 chroma pel), every fetch
- * clamped into the reference plane, horizontal pass rounded and clipped to 8
- * bits before the vertical pass (vp9_mc.comp.glsl:61-110). F: the filter
- * (the regular one under SPEC). avg: round-average into the tile (the
- * second prediction of a FULL compound block). */
-/* One 8-tap output of a staged row (4-byte aligned in shared memory) at
- * column c: samples c..c+7 as two words, two dp4a (tap8). The same value as
- * the scalar sum: clamp((sum + 64) >> 7, 0, 255). */
-__device__ __forceinline__ uint32_t htap8(const uint8_t *row, int c, const uint32_t *pk, int phase)
-{
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(row) + (c >> 2);
-    const unsigned sh = 8u * (unsigned)(c & 3);
-    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
-    return tap8(pk[0], pk[1], phase, __funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
-}
-
-__device__ void spec_inter_pass(ReconSmem &s, const cvp9_ref_t &R, int mvx, int mvy, const int (*F)[8],
-                                const uint32_t (*P)[2], bool avg,
-                                int sbx, int sby, int lx0, int ly0, int lw, int lh,
-                                int cx0, int cy0, int clw, int clh, int warp, int lane)
-{
-    const uint8_t *rp = R.plane;
-    const int rw = R.w, rh = R.h;
-    const int rcs = (rw + 1) >> 1;
-    const uint8_t *ru = rp + (size_t)rw * rh;
-    const uint8_t *rv = ru + (size_t)rcs * ((rh + 1) >> 1);
-    uint8_t *st = s.stage[warp];
-        /* luma: (lw+7) x (lh+7) window at pitch 16; H pass into 15 x 8 */
-        int bx = sbx + lx0 + (mvx >> 3), by = sby + ly0 + (mvy >> 3);
-        int fx = (mvx & 7) << 1, fy = (mvy & 7) << 1;
-        int gcx = (sbx >> 1) + cx0, gcy = (sby >> 1) + cy0;
-        int cbx = gcx + (mvx >> 4), cby = gcy + (mvy >> 4);
-        int cfx = mvx & 15, cfy = mvy & 15;
-        int cw2 = (rw + 1) >> 1, ch2 = (rh + 1) >> 1;
-        uint8_t *sy_ = st;              /* 15 x 16 */
-        uint8_t *hy = st + 240;         /* 15 x 8  */
-        uint8_t *su = st + 360;         /* 11 x 12 */
-        uint8_t *sv = st + 492;         /* 11 x 12 */
-        uint8_t *hu = st + 624;         /* 11 x 4  */
-        uint8_t *hv = st + 668;         /* 11 x 4  */
-        {
-            /* all three windows' reads in flight at once */
-            WinRows<8> wl;
-            WinRows<6> wu, wv;
-            wl.load(rp, rw, rw, rh, bx - 3, by - 3, lw + 7, lh + 7, lane);
-            wu.load(ru, rcs, cw2, ch2, cbx - 3, cby - 3, clw + 7, clh + 7, lane);
-            wv.load(rv, rcs, cw2, ch2, cbx - 3, cby - 3, clw + 7, clh + 7, lane);
-            wl.store(sy_, 16, lw + 7, lh + 7, lane);
-            wu.store(su, 12, clw + 7, clh + 7, lane);
-            wv.store(sv, 12, clw + 7, clh + 7, lane);
-        }
-        __syncwarp();
-        /* horizontal pass (rounded, clipped to 8 bits) */
-        for (int i = lane; i < (lh + 7) * lw; i += 32) {
-            int r = lw == 8 ? i >> 3 : i / lw, c = i - r * lw;
-            hy[r * 8 + c] = (uint8_t)htap8(sy_ + r * 16, c, P[fx], fx);
-        }
-        for (int i = lane; i < 2 * (clh + 7) * clw; i += 32) {
-            int pl = i >= (clh + 7) * clw;
-            int j = pl ? i - (clh + 7) * clw : i;
-            int r = clw == 4 ? j >> 2 : j / clw, c = j - r * clw;
-            const uint8_t *src = pl ? sv : su;
-            (pl ? hv : hu)[r * 4 + c] = (uint8_t)htap8(src + r * 12, c, P[cfx], cfx);
-        }
-        __syncwarp();
-        for (int idx = lane; idx < 64; idx += 32) {
-            int r = idx >> 3, c = idx & 7;
-            if (r >= lh || c >= lw) continue;
-            int v;
-            if (fx == 0 && fy == 0) {
-                v = sy_[(r + 3) * 16 + c + 3];
-            } else {
-                int acc = 0;
-#pragma unroll
-                for (int t = 0; t < 8; t++) acc += F[fy][t] * hy[(r + t) * 8 + c];
-                v = clampi((acc + 64) >> 7, 0, 255);
-            }
-            uint8_t &d = TY(s, lx0 + c, ly0 + r);
-            d = (uint8_t)(avg ? ((int)d + v + 1) >> 1 : v);
-        }
-        {
-            int p = 1 + (lane >> 4), r = (lane >> 2) & 3, c = lane & 3;
-            if (r < clh && c < clw) {
-                int v;
-                if (cfx == 0 && cfy == 0) {
-                    v = (p == 1 ? su : sv)[(r + 3) * 12 + c + 3];
-                } else {
-                    const uint8_t *h = p == 1 ? hu : hv;
-                    int acc = 0;
-#pragma unroll
-                    for (int t = 0; t < 8; t++) acc += F[cfy][t] * h[(r + t) * 4 + c];
-                    v = clampi((acc + 64) >> 7, 0, 255);
-                }
-                uint8_t &d = TC(s, p, cx0 + c, cy0 + r);
-                d = (uint8_t)(avg ? ((int)d + v + 1) >> 1 : v);
-            }
-        }
-        __syncwarp();
-}
-
-/* SPEC inter prediction of one chunk; FULL also takes the header's filter
- * and averages in a second reference's prediction (compound blocks). A
- * missing first reference predicts flat 128; a missing second one leaves
- * the single prediction. */
-__device__ void spec_inter_chunk(ReconSmem &s, const BlkS &b, int sbx, int sby,
-                                 int lx0, int ly0, int lw, int lh,
-                                 int cx0, int cy0, int clw, int clh, int warp, int lane)
-{
-    const cvp9_job_t &job = s.jc;
-    const cvp9_ref_t &R = job.ref[job.ref_slot_of[clampi((int)b.ref0 - 1, 0, 2)] & 7];
-    if (!R.plane) { fill_chunk(s, 128, lx0, ly0, lw, lh, cx0, cy0, clw, clh, lane); return; }
-    const int (*F)[8] = job.full ? c_subpel4[job.interp_filter & 3] : c_subpel;
-    const uint32_t (*P)[2] = job.full ? c_subpel4_pk[job.interp_filter & 3] : c_subpel_pk;
-    spec_inter_pass(s, R, b.mvx, b.mvy, F, P, false, sbx, sby, lx0, ly0, lw, lh, cx0, cy0, clw, clh, warp, lane);
-    if (b.ref1) {
-        const cvp9_ref_t &R1 = job.ref[job.ref_slot_of[clampi((int)b.ref1 - 1, 0, 2)] & 7];
-        if (R1.plane)
-            spec_inter_pass(s, R1, b.mv1x, b.mv1y, F, P, true, sbx, sby, lx0, ly0, lw, lh, cx0, cy0, clw, clh,
-                            warp, lane);
-    }
 }
 
 /* ── Residual: one item = one TX column (pass 1) or one TX row (pass 2) ── */
@@ -1228,222 +1370,302 @@ __device__ __forceinline__ int plane_at(int p, int x, int y)
     return p == 0 ? y * 64 + x : 4096 + (p - 1) * 1024 + y * 32 + x;
 }
 
-/* Sum of e[min(i, last)] over i < n. */
-__device__ __forceinline__ unsigned edge_sum(const uint8_t *e, int n, int last)
+/* Sum of e[min(i, last)] over i < n (n <= 64). An aligned edge without
+ * repeats goes as independent word loads, as many as its size needs. */
+template <class T>
+__device__ __forceinline__ unsigned edge_sum(const T *e, int n, int last)
 {
-    const int m = min(n, last + 1);
+    constexpr int kPer = 4 / (int)sizeof(T);
     unsigned s = 0;
-    int i = 0;
-    if (!((uintptr_t)e & 3))
-        for (; i + 4 <= m; i += 4) s = __dp4a(*reinterpret_cast<const uint32_t *>(e + i), 0x01010101u, s);
-    for (; i < m; i++) s += e[i];
-    return s + (n > m ? (unsigned)(n - m) * e[m - 1] : 0u);
-}
-__device__ __forceinline__ unsigned edge_sum(const uint16_t *e, int n, int last)
-{
-    const int m = min(n, last + 1);
-    unsigned s = 0;
-    int i = 0;
-    if (!((uintptr_t)e & 3))
-        for (; i + 2 <= m; i += 2) {
-            const uint32_t w = *reinterpret_cast<const uint32_t *>(e + i);
-            s += (w & 0xffffu) + (w >> 16);
+    if (last >= n - 1 && !((uintptr_t)e & 3) && !(n & (kPer - 1))) {
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(e);
+        auto add = [&](uint32_t v) { s = sizeof(T) == 1 ? __dp4a(v, 0x01010101u, s) : s + (v & 0xffffu) + (v >> 16); };
+        const int m = n / kPer;
+        int k = 0;
+        for (; k + 4 <= m; k += 4) {
+            const uint32_t a = w[k], b = w[k + 1], c = w[k + 2], d = w[k + 3];
+            add(a); add(b); add(c); add(d);
         }
-    for (; i < m; i++) s += e[i];
-    return s + (n > m ? (unsigned)(n - m) * e[m - 1] : 0u);
+        if (m & 2) {
+            const uint32_t a = w[k], b = w[k + 1];
+            add(a); add(b);
+            k += 2;
+        }
+        if (m & 1) add(w[k]);
+    } else {
+        for (int i = 0; i < n; i++) s += e[min(i, last)];
+    }
+    return s;
 }
 
-/* Four samples of a task: predict, add the residual, clip, store. A: the
- * profile (REFCPU's DC counts the filled edges, the others' only available
- * ones); directional modes are FULL's. Every directional sample is a copy, a
- * two-tap or a three-tap average at one place of the edge E: E(i) = above[i]
- * for i >= -1 (-1 the corner), left[-i - 2] below. */
-template <int A, int MAXV, class T>
-__device__ __forceinline__ void intra_quad(const IntraView<T> &V, const ITask t, int r, int q)
+/* The samples that a task's DC counts, as the reciprocal of its division:
+ * (sum * inv) >> 32 is sum / n for sum < 2^32 / n. */
+__device__ __forceinline__ uint32_t dc_inverse(int n)
 {
-    const int p = t.pm & 3, mode = t.pm >> 2;
-    const int pitch = p ? kCPitch : kYPitch;
-    const int x = t.x, y = t.y;
-    T *const tile = p == 0 ? V.ty : V.tc[p - 1];
-    T *const col = p == 0 ? V.cy : V.cc[p - 1];
-    const T *up = tile + (y - 1) * pitch + x;
-    const T *lf = col + (p ? (x >> 1) * 32 : (x >> 2) * 64) + y;
-    const int c0 = 4 * q, nc = min(4, (int)t.w - c0);
-    T *dst = tile + (y + r) * pitch + x + c0;
-    int v[4];
-    if (mode == 0) {
-        const unsigned sa = edge_sum(up, t.dcw, t.acl), sl = edge_sum(lf, t.dch, t.lcl);
-        unsigned dc;
-        if (A == CVP9_ARITH_REFCPU) {
-            const unsigned n = t.dcw + t.dch;
-            dc = (sa + sl + (n >> 1)) / n;
-        } else {
-            const unsigned n = (t.avail & 1 ? t.dcw : 0) + (t.avail & 2 ? t.dch : 0);
-            dc = n ? ((t.avail & 1 ? sa : 0u) + (t.avail & 2 ? sl : 0u) + (n >> 1)) / n : (unsigned)(MAXV + 1) / 2;
-        }
+    return n > 1 ? (uint32_t)((0x100000000ull + (unsigned)n - 1u) / (unsigned)n) : 0u;
+}
+
+/* Four samples of a task, in two parts: what does not wait for other samples
+ * (where they are, their residuals), then the prediction. */
+template <class T>
+struct IntraQuad {
+    const T *up, *lf;                /* the task's row above, left column    */
+    T *dst, *col;                    /* the samples; column copies of their row */
+    uint32_t r0, r1;                 /* their residuals                      */
+    ITask t;
+    int r, c0, nc;
+    __device__ __forceinline__ void load(const IntraView<T> &V, const ITask &task, int row, int q)
+    {
+        t = task;
+        r = row;
+        c0 = 4 * q;
+        const int p = t.plane(), pitch = p ? kCPitch : kYPitch, x = t.x(), y = t.y();
+        T *const tile = V.tile(p);
+        nc = min(4, t.w() - c0);
+        up = tile + (y - 1) * pitch + x;
+        lf = V.col(p) + (p ? (x >> 1) * 32 : (x >> 2) * 64) + y;
+        dst = tile + (y + r) * pitch + x + c0;
+        col = V.col(p) + y + r;
+        /* x is even: two words of residuals */
+        const uint32_t *rs = reinterpret_cast<const uint32_t *>(V.res + plane_at(p, x + c0, y + r));
+        r0 = rs[0];
+        r1 = nc > 2 ? rs[1] : 0u;
+    }
+    /* A: the profile; directional modes are FULL's. Every directional sample
+     * is a copy, a two-tap or a three-tap average at one place of the edge E:
+     * E(i) = above[i] for i >= -1 (-1 the corner), left[-i - 2] below. */
+    template <int A, int MAXV>
+    __device__ __forceinline__ void run() const
+    {
+        const int mode = t.mode();
+        int v[4];
+        if (mode == 0) {
+            const unsigned av = t.avail(), n = (av & 1u ? t.pw() : 0) + (av & 2u ? t.ph() : 0);
+            const unsigned sum = (av & 1u ? edge_sum(up, t.pw(), t.acl()) : 0u) +
+                                 (av & 2u ? edge_sum(lf, t.ph(), t.lcl()) : 0u) + (n >> 1);
+            const unsigned dc = n == 0 ? (unsigned)(MAXV + 1) / 2 : t.inv ? __umulhi(sum, t.inv) : sum;
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = (int)dc;
-    } else if (A != CVP9_ARITH_FULL || mode == 9 || mode <= 2) {
-        const int l = lf[min(r, (int)t.lcl)], tl = up[-1], acl = t.acl;
+            for (int i = 0; i < 4; i++) v[i] = (int)dc;
+        } else if (A != CVP9_ARITH_FULL || mode == 9 || mode <= 2) {
+            const int l = lf[min(r, t.lcl())], tl = up[-1], acl = t.acl();
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int a = up[min(c0 + i, acl)];
-            v[i] = mode == 1 ? a : mode == 2 ? l : clampi(a + l - tl, 0, MAXV);
-        }
-    } else {
-        const int n = t.dcw, acl = t.acl, lcl = t.lcl;
-        auto E = [&](int i) -> int { return *(i >= -1 ? up + min(i, acl) : lf + min(-i - 2, lcl)); };
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int c = c0 + k;
-            int i, taps = 3;             /* E(i), E(i) E(i+1), or E(i) E(i+1) E(i+2) */
-            if (mode == 3) {
-                i = r + c;
-                if (i + 2 >= 2 * n) { i = 2 * n - 1; taps = 1; }
-            } else if (mode == 8) {
-                i = (r >> 1) + c;
-                if (!(r & 1)) taps = 2;
-            } else if (mode == 4) {
-                i = c - r - 2;
-            } else if (mode == 5) {
-                const int d = r - 2 * c, j = c - (r >> 1);
-                i = d >= 2 ? -d - 1 : j - 2 + !(r & 1);
-                if (d < 2 && !(r & 1)) taps = 2;
-            } else if (mode == 6) {
-                const int d = c - 2 * r, rr = r - (c >> 1);
-                i = d >= 2 ? d - 3 : -rr - 2;
-                if (d < 2 && !(c & 1)) taps = 2;
-            } else {
-                const int j = r + (c >> 1);
-                i = -j - 4 + !(c & 1);
-                if (!(c & 1)) taps = 2;
+            for (int i = 0; i < 4; i++) {
+                const int a = up[min(c0 + i, acl)];
+                v[i] = mode == 1 ? a : mode == 2 ? l : clampi(a + l - tl, 0, MAXV);
             }
-            const int e0 = E(i), e1 = E(i + 1), e2 = E(i + 2);
-            v[k] = taps == 1 ? e0 : taps == 2 ? (e0 + e1 + 1) >> 1 : (e0 + 2 * e1 + e2 + 2) >> 2;
-        }
-    }
-    if (A == CVP9_ARITH_SPEC && (r >= t.ph || c0 + 4 > t.pw)) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) if (r >= t.ph || c0 + i >= t.pw) v[i] = i < nc ? dst[i] : 0;
-    }
-    /* x is even: two words of residuals */
-    const uint32_t *rs = reinterpret_cast<const uint32_t *>(V.res + plane_at(p, x + c0, y + r));
-    const uint32_t r0 = rs[0], r1 = nc > 2 ? rs[1] : 0u;
-    v[0] = clampi(v[0] + (int16_t)(r0 & 0xffffu), 0, MAXV);
-    v[1] = clampi(v[1] + ((int)r0 >> 16), 0, MAXV);
-    v[2] = clampi(v[2] + (int16_t)(r1 & 0xffffu), 0, MAXV);
-    v[3] = clampi(v[3] + ((int)r1 >> 16), 0, MAXV);
-    if (nc == 4 && !(x & 3)) {
-        if (sizeof(T) == 1) {
-            *reinterpret_cast<uint32_t *>(dst) = (uint32_t)v[0] | (uint32_t)v[1] << 8 | (uint32_t)v[2] << 16 | (uint32_t)v[3] << 24;
         } else {
-            *reinterpret_cast<uint2 *>(dst) = make_uint2((uint32_t)v[0] | (uint32_t)v[1] << 16,
-                                                         (uint32_t)v[2] | (uint32_t)v[3] << 16);
-        }
-    } else {
+            const int n = t.pw(), acl = t.acl(), lcl = t.lcl();
+            auto E = [&](int i) -> int { return *(i >= -1 ? up + min(i, acl) : lf + min(-i - 2, lcl)); };
 #pragma unroll
-        for (int i = 0; i < 4; i++) if (i < nc) dst[i] = (T)v[i];
+            for (int k = 0; k < 4; k++) {
+                const int c = c0 + k;
+                int i, taps = 3;             /* E(i), E(i) E(i+1), or E(i) E(i+1) E(i+2) */
+                if (mode == 3) {
+                    i = r + c;
+                    if (i + 2 >= 2 * n) { i = 2 * n - 1; taps = 1; }
+                } else if (mode == 8) {
+                    i = (r >> 1) + c;
+                    if (!(r & 1)) taps = 2;
+                } else if (mode == 4) {
+                    i = c - r - 2;
+                } else if (mode == 5) {
+                    const int d = r - 2 * c, j = c - (r >> 1);
+                    i = d >= 2 ? -d - 1 : j - 2 + !(r & 1);
+                    if (d < 2 && !(r & 1)) taps = 2;
+                } else if (mode == 6) {
+                    const int d = c - 2 * r, rr = r - (c >> 1);
+                    i = d >= 2 ? d - 3 : -rr - 2;
+                    if (d < 2 && !(c & 1)) taps = 2;
+                } else {
+                    const int j = r + (c >> 1);
+                    i = -j - 4 + !(c & 1);
+                    if (!(c & 1)) taps = 2;
+                }
+                const int e0 = E(i), e1 = E(i + 1), e2 = E(i + 2);
+                v[k] = taps == 1 ? e0 : taps == 2 ? (e0 + e1 + 1) >> 1 : (e0 + 2 * e1 + e2 + 2) >> 2;
+            }
+        }
+        if (A == CVP9_ARITH_SPEC && (r >= t.ph() || c0 + 4 > t.pw())) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) if (r >= t.ph() || c0 + i >= t.pw()) v[i] = i < nc ? dst[i] : 0;
+        }
+        v[0] = clampi(v[0] + (int16_t)(r0 & 0xffffu), 0, MAXV);
+        v[1] = clampi(v[1] + ((int)r0 >> 16), 0, MAXV);
+        v[2] = clampi(v[2] + (int16_t)(r1 & 0xffffu), 0, MAXV);
+        v[3] = clampi(v[3] + ((int)r1 >> 16), 0, MAXV);
+        const int x = t.x(), cx = x + c0;
+        if (nc == 4 && !(x & 3)) {
+            if (sizeof(T) == 1) {
+                *reinterpret_cast<uint32_t *>(dst) = (uint32_t)v[0] | (uint32_t)v[1] << 8 | (uint32_t)v[2] << 16 |
+                                                     (uint32_t)v[3] << 24;
+            } else {
+                *reinterpret_cast<uint2 *>(dst) = make_uint2((uint32_t)v[0] | (uint32_t)v[1] << 16,
+                                                             (uint32_t)v[2] | (uint32_t)v[3] << 16);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) if (i < nc) dst[i] = (T)v[i];
+        }
+        if (t.plane() == 0) {
+            if (nc == 4 && cx < 60) col[((cx + 4) >> 2) * 64] = (T)v[3];
+        } else {
+            if (nc >= 2 && cx < 30) col[((cx + 2) >> 1) * 32] = (T)v[1];
+            if (nc == 4 && cx < 28) col[((cx + 4) >> 1) * 32] = (T)v[3];
+        }
     }
-    const int cx = x + c0;
-    if (p == 0) {
-        if (nc == 4 && cx < 60) col[((cx + 4) >> 2) * 64 + y + r] = (T)v[3];
-    } else {
-        if (nc >= 2 && cx < 30) col[((cx + 2) >> 1) * 32 + y + r] = (T)v[1];
-        if (nc == 4 && cx < 28) col[((cx + 4) >> 1) * 32 + y + r] = (T)v[3];
-    }
-}
+};
 
-/* FULL: the TXs of an intra block as tasks at, at + 1, ... in coding order
- * (planes, then raster), by one warp; own: mark the cells each one writes.
- * Returns their number. */
+/* FULL: TXs of a block. */
 template <class B>
-__device__ int intra_tx_tasks(IntraWork &W, const B &b, const cvp9_job_t &job, int sbx, int sby, int at, bool own,
-                              int lane)
+__device__ __forceinline__ int intra_tx_count(const B &b, const cvp9_job_t &job, int sbx, int sby)
 {
-    const int gx = sbx + b.x, gy = sby + b.y;
-    const bool left_ok = (gx >> 3) > full_tile_start(gx >> 3, job.mi_cols, job.log2_tile_cols);
-    int id0 = at;
+    int n = 0;
+#pragma unroll
     for (int p = 0; p < 3; p++) {
         int txl, nx, ny, pbw;
-        plane_layout(b, job, gx, gy, p, txl, nx, ny, pbw);
-        const int n = 4 << txl, mode = p ? (b.uvmode > 9 ? 0 : b.uvmode) : (b.ymode > 9 ? 0 : b.ymode);
-        const int pw = p ? job.CW : job.W, ph = p ? job.CH : job.H, tile = p ? 32 : 64;
-        const int ox = p ? (b.x >> 1) : b.x, oy = p ? (b.y >> 1) : b.y;
-        const int gox = p ? (gx >> 1) : gx, goy = p ? (gy >> 1) : gy;
-        for (int k = lane; k < nx * ny && id0 + k < kMaxTasks; k += 32) {
-            const int ty = div_small(k, nx), tx = k - ty * nx;
-            const int lx = ox + tx * n, ly = oy + ty * n, X0 = gox + tx * n, Y0 = goy + ty * n;
-            ITask t;
-            t.x = (uint8_t)lx;
-            t.y = (uint8_t)ly;
-            t.w = t.pw = (uint8_t)max(0, min(n, min(pw - X0, tile - lx)));
-            t.h = t.ph = (uint8_t)max(0, min(n, min(ph - Y0, tile - ly)));
-            t.pm = (uint8_t)(p | (mode << 2));
-            const bool top = Y0 > 0, right = n == 4 && (tx + 1) * n < pbw;
-            t.acl = (uint8_t)(top ? max(1, min(n + (right ? 4 : 0), pw - X0)) - 1 : n - 1);
-            t.lcl = (uint8_t)max(0, min(n - 1, ph - 1 - Y0));
-            t.dcw = t.dch = (uint8_t)n;
-            t.avail = (uint8_t)((top ? 1 : 0) | (tx > 0 || left_ok ? 2 : 0));
-            W.task[id0 + k] = t;
-            if (own) {
-                uint16_t *o = W.own + (p == 0 ? 0 : 192 + 64 * p);
-                const int wpt = p ? 8 : 16;
-                for (int cy = ly >> 2; cy < (ly + n) >> 2; cy++)
-                    for (int cx = lx >> 2; cx < (lx + n) >> 2; cx++) o[cy * wpt + cx] = (uint16_t)(id0 + k + 1);
-            }
-        }
-        id0 += nx * ny;
+        plane_layout(b, job, sbx + b.x, sby + b.y, p, txl, nx, ny, pbw);
+        n += nx * ny;
     }
-    return id0 - at;
+    return n;
 }
 
-/* FULL: levels of the tasks, whole CTA. A task reads the cells above it (a
- * 4x4 one also above to its right), to its left and at its corner; their
- * tasks come before it in coding order, so relaxing every task until none
- * changes ends with the longest paths. */
+/* FULL: TX k (coding order: planes, then raster) of an intra block as task
+ * `id`, a thread each; own: mark the cells it writes. */
+template <class B>
+__device__ __forceinline__ void intra_tx_task(IntraWork &W, const B &b, const cvp9_job_t &job, int sbx, int sby, int k,
+                                              int id, bool own)
+{
+    const int gx = sbx + b.x, gy = sby + b.y;
+    int p = 0, txl, nx, ny, pbw;
+    for (;; p++) {
+        plane_layout(b, job, gx, gy, p, txl, nx, ny, pbw);
+        if (k < nx * ny || p == 2) break;
+        k -= nx * ny;
+    }
+    const bool left_ok = (gx >> 3) > full_tile_start(gx >> 3, job.mi_cols, job.log2_tile_cols);
+    const int n = 4 << txl, mode = p ? (b.uvmode > 9 ? 0 : b.uvmode) : (b.ymode > 9 ? 0 : b.ymode);
+    const int pw = p ? job.CW : job.W, ph = p ? job.CH : job.H, tile = p ? 32 : 64;
+    const int ty = div_small(k, nx), tx = k - ty * nx;
+    const int lx = (p ? (b.x >> 1) : b.x) + tx * n, ly = (p ? (b.y >> 1) : b.y) + ty * n;
+    const int X0 = (p ? (gx >> 1) : gx) + tx * n, Y0 = (p ? (gy >> 1) : gy) + ty * n;
+    const bool top = Y0 > 0, right = n == 4 && (tx + 1) * n < pbw;
+    const int avail = (top ? 1 : 0) | (tx > 0 || left_ok ? 2 : 0);
+    st_task(&W.task[id], lx, ly, max(0, min(n, min(pw - X0, tile - lx))), max(0, min(n, min(ph - Y0, tile - ly))), p, mode,
+            top ? max(1, min(n + (right ? 4 : 0), pw - X0)) - 1 : n - 1, max(0, min(n - 1, ph - 1 - Y0)), avail, n, n,
+            1u << (32 - (2 + txl + (avail == 3))));
+    if (own) {
+        uint16_t *o = W.own + (p == 0 ? 0 : 192 + 64 * p);
+        const int wpt = p ? 8 : 16;
+        for (int cy = ly >> 2; cy < (ly + n) >> 2; cy++)
+            for (int cx = lx >> 2; cx < (lx + n) >> 2; cx++) o[cy * wpt + cx] = (uint16_t)(id + 1);
+    }
+}
+
+/* Largest k in [0, n) with base[k] <= v (base ascending, base[0] = 0). */
+__device__ __forceinline__ int find_base(const uint16_t *base, int n, int v)
+{
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (base[mid] <= v) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+/* Levels, whole CTA. A thread's tasks are rectangles of 4x4 cells; each reads
+ * the cells above it (up to column `up`), to its left and at its corner, of
+ * which only bottom rows and right columns of tasks matter. Those of unplaced
+ * tasks are bits of two maps, so a task sees with two words whether all it
+ * reads is placed; every pass places the tasks that see nothing open, the
+ * pass's number their level. (Relaxing levels cell by cell took 33 k cycles a
+ * superblock of 64 8x8 blocks, this 8 k.) */
+struct LvlTask {
+    uint32_t *ur, *lc, *br, *rc;     /* row above, column left; own bottom row, right column */
+    uint32_t um, lm, cm, rm;         /* cells read there; own columns and rows */
+    int      level;                  /* -1: not placed yet                   */
+    __device__ __forceinline__ void set(uint32_t *prow, uint32_t *pcol, int x0, int x1, int y0, int y1, int up)
+    {
+        cm = ((2u << x1) - 1u) & ~((1u << x0) - 1u);
+        rm = ((2u << y1) - 1u) & ~((1u << y0) - 1u);
+        um = y0 > 0 ? ((2u << up) - 1u) & ~((1u << max(0, x0 - 1)) - 1u) : 0u;
+        lm = x0 > 0 ? rm : 0u;
+        ur = prow + max(0, y0 - 1);
+        lc = pcol + max(0, x0 - 1);
+        br = prow + y1;
+        rc = pcol + x1;
+        level = -1;
+        atomicOr(br, cm);
+        atomicOr(rc, rm);
+    }
+};
+
+/* W.prow and W.pcol zero, then every task set, then a barrier, before this. */
+template <int N>
+__device__ __forceinline__ void intra_levels(LvlTask (&k)[N], const bool (&have)[N])
+{
+    for (int L = 0; L < kMaxTasks; L++) {
+        bool go[N], open = false;
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            go[i] = have[i] && k[i].level < 0 &&
+                    !((*(volatile uint32_t *)k[i].ur & k[i].um) | (*(volatile uint32_t *)k[i].lc & k[i].lm));
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            if (go[i]) {
+                atomicAnd(k[i].br, ~k[i].cm);
+                atomicAnd(k[i].rc, ~k[i].rm);
+                k[i].level = L;
+            }
+            open |= have[i] && k[i].level < 0;
+        }
+        if (!__syncthreads_or(open)) break;
+    }
+}
+
+/* FULL: the levels of the TX tasks (two a thread: at most kMaxTasks of them
+ * on at least kMaxTasks / 2 threads). */
 __device__ __forceinline__ void intra_tx_levels(IntraWork &W, int ntask, int tid, int nthreads)
 {
-    volatile uint16_t *lvl = W.lvl;
-    for (int t = tid; t < ntask; t += nthreads) lvl[t] = 0;
-    __syncthreads();
-    for (int it = 0; it <= kMaxTasks; it++) {
-        bool changed = false;
-        for (int t = tid; t < ntask; t += nthreads) {
-            const ITask k = ld_task(&W.task[t]);
-            const int p = k.pm & 3, wpt = p ? 8 : 16, n = k.dcw;
-            const uint16_t *o = W.own + (p == 0 ? 0 : 192 + 64 * p);
-            const int cx0 = k.x >> 2, cy0 = k.y >> 2;
-            const int cx1 = min(wpt - 1, ((k.x + n - 1) >> 2) + (k.acl >= n)), cy1 = (k.y + k.lcl) >> 2;
-            int L = 0;
-            if (cy0 > 0)
-                for (int cx = max(0, cx0 - 1); cx <= cx1; cx++) {
-                    const int j = o[(cy0 - 1) * wpt + cx];
-                    if (j) L = max(L, lvl[j - 1] + 1);
-                }
-            if (cx0 > 0)
-                for (int cy = cy0; cy <= cy1; cy++) {
-                    const int j = o[cy * wpt + cx0 - 1];
-                    if (j) L = max(L, lvl[j - 1] + 1);
-                }
-            if (L != lvl[t]) { lvl[t] = (uint16_t)L; changed = true; }
-        }
-        if (!__syncthreads_or(changed)) break;
+    LvlTask lt[2];
+    bool have[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int t = tid + i * nthreads;
+        have[i] = t < ntask;
+        if (!have[i]) continue;
+        const ITask k = ld_task(&W.task[t]);
+        const int p = k.plane(), n = k.pw(), x1 = (k.x() + n - 1) >> 2;
+        lt[i].set(W.prow[p], W.pcol[p], k.x() >> 2, x1, k.y() >> 2, (k.y() + n - 1) >> 2,
+                  min(p ? 7 : 15, x1 + (k.acl() >= n)));
     }
+    __syncthreads();
+    intra_levels<2>(lt, have);
+#pragma unroll
+    for (int i = 0; i < 2; i++) if (have[i]) W.lvl[tid + i * nthreads] = (uint16_t)max(0, lt[i].level);
 }
 
 /* Sort the quads of all tasks by level, whole CTA: W.lvlq[L] .. W.lvlq[L + 1]
- * of W.qtab are level L's. */
-__device__ __forceinline__ void intra_sort(IntraWork &W, int ntask, int tid, int nthreads)
+ * of W.qtab are level L's. A thread per four-sample group of the SB finds its
+ * task from the owner map of the cells: W.own of each plane's (FULL), or the
+ * block map `cell` of the luma ones, whose chroma groups start at even
+ * samples. */
+template <int A>
+__device__ __forceinline__ void intra_sort(IntraWork &W, const uint16_t *cell, int ntask, int tid, int nthreads)
 {
     const int lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i <= kMaxTasks; i += nthreads) W.lvlq[i] = 0;
+    for (int i = tid; i < kMaxQuads; i += nthreads) W.qtab[i] = kNoQuad;
     if (tid == 0) W.nlev = 0;
     __syncthreads();
+    int top = 0;
     for (int t = tid; t < ntask; t += nthreads) {
         const ITask k = ld_task(&W.task[t]);
-        W.qat[t] = (uint16_t)atomicAdd(&W.lvlq[W.lvl[t]], (unsigned)(((k.w + 3) >> 2) * k.h));
-        atomicMax(&W.nlev, (int)W.lvl[t] + 1);
+        W.qat[t] = (uint16_t)atomicAdd(&W.lvlq[W.lvl[t]], (unsigned)(((k.w() + 3) >> 2) * k.h()));
+        top = max(top, (int)W.lvl[t] + 1);
     }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0 && top) atomicMax(&W.nlev, top);
     __syncthreads();
     if (warp == 0) {
         const int nlev = W.nlev, per = (nlev + 31) >> 5, b0 = lane * per;
@@ -1464,28 +1686,64 @@ __device__ __forceinline__ void intra_sort(IntraWork &W, int ntask, int tid, int
         if (lane == 31) W.lvlq[nlev] = x;
     }
     __syncthreads();
-    for (int t = warp; t < ntask; t += nthreads >> 5) {
-        const ITask k = ld_task(&W.task[t]);
-        const int qw = (k.w + 3) >> 2, nq = qw * k.h;
-        const unsigned at = W.lvlq[W.lvl[t]] + W.qat[t];
-        for (int i = lane; i < nq; i += 32) {
-            const int r = div_small(i, qw);
-            if (at + i < (unsigned)kMaxQuads) W.qtab[at + i] = (uint32_t)t | (uint32_t)r << 9 | (uint32_t)(i - r * qw) << 15;
+    constexpr int kGroups = A == CVP9_ARITH_FULL ? 1024 + 2 * 256 : 1024 + 2 * 512;
+    for (int i = tid; i < kGroups; i += nthreads) {
+        int t, x, y;
+        if (i < 1024) {
+            y = i >> 4;
+            x = (i & 15) * 4;
+            const int c = (y >> 2) * 16 + (x >> 2);
+            t = A == CVP9_ARITH_FULL ? (int)W.own[c] - 1 : cell[c] ? (int)W.own[cell[c] - 1] : -1;
+        } else if (A == CVP9_ARITH_FULL) {
+            const int p = (i - 1024) >> 8, j = i & 255;
+            y = j >> 3;
+            x = (j & 7) * 4;
+            t = (int)W.own[256 + 64 * p + (y >> 2) * 8 + (x >> 2)] - 1;
+        } else {
+            const int p = (i - 1024) >> 9, j = i & 511;
+            y = j >> 4;
+            x = (j & 15) * 2;
+            const int o = cell[(y >> 1) * 16 + (x >> 1)];
+            t = o ? (int)W.own[o - 1] : -1;
+            if (t >= 0 && t != 0xFFFF) t += 1 + p;
         }
+        if (t < 0 || t >= ntask) continue;
+        const ITask k = ld_task(&W.task[t]);
+        const int r = y - k.y(), c = x - k.x();
+        if (r >= k.h() || c >= k.w() || (c & 3)) continue;
+        const unsigned at = W.lvlq[W.lvl[t]] + W.qat[t] + (unsigned)(r * ((k.w() + 3) >> 2) + (c >> 2));
+        if (at < (unsigned)kMaxQuads) W.qtab[at] = (uint32_t)t | (uint32_t)r << 9 | (uint32_t)(c >> 2) << 15;
     }
     __syncthreads();
 }
 
-/* The levels, whole CTA: one barrier each. */
+/* The levels, whole CTA: one barrier each. The next level's first quad and
+ * its task are loaded before the barrier. */
 template <int A, int MAXV, class T>
 __device__ __forceinline__ void intra_run(const IntraWork &W, const IntraView<T> &V, int tid, int nthreads)
 {
     const int nlev = W.nlev;
+    int q = tid, q1 = min((int)W.lvlq[1], kMaxQuads);
+    uint32_t e = q < q1 ? W.qtab[q] : kNoQuad;
+    ITask t = ld_task(&W.task[e != kNoQuad ? e & 511u : 0u]);
     for (int L = 0; L < nlev; L++) {
-        const int q1 = min((int)W.lvlq[L + 1], kMaxQuads);
-        for (int q = (int)W.lvlq[L] + tid; q < q1; q += nthreads) {
-            const uint32_t e = W.qtab[q];
-            intra_quad<A, MAXV, T>(V, ld_task(&W.task[e & 511u]), (int)(e >> 9) & 63, (int)(e >> 15));
+        while (q < q1) {
+            if (e != kNoQuad) {
+                IntraQuad<T> k;
+                k.load(V, t, (int)(e >> 9) & 63, (int)(e >> 15));
+                k.template run<A, MAXV>();
+            }
+            q += nthreads;
+            if (q < q1) {
+                e = W.qtab[q];
+                t = ld_task(&W.task[e != kNoQuad ? e & 511u : 0u]);
+            }
+        }
+        if (L + 1 < nlev) {
+            q = q1 + tid;
+            q1 = min((int)W.lvlq[L + 2], kMaxQuads);
+            e = q < q1 ? W.qtab[q] : kNoQuad;
+            t = ld_task(&W.task[e != kNoQuad ? e & 511u : 0u]);
         }
         __syncthreads();
     }
@@ -1499,10 +1757,12 @@ __device__ __forceinline__ void intra_run_ordered(const IntraWork &W, const Intr
 {
     for (int t = 0; t < ntask; t++) {
         const ITask k = ld_task(&W.task[t]);
-        const int qw = (k.w + 3) >> 2, nq = qw * k.h;
+        const int qw = (k.w() + 3) >> 2, nq = qw * k.h();
         for (int i = tid; i < nq; i += nthreads) {
             const int r = div_small(i, qw);
-            intra_quad<A, MAXV, T>(V, k, r, i - r * qw);
+            IntraQuad<T> quad;
+            quad.load(V, k, r, i - r * qw);
+            quad.template run<A, MAXV>();
         }
         __syncthreads();
     }
@@ -1514,11 +1774,11 @@ __device__ __forceinline__ void intra_fill_cols(const IntraView<T> &V, int tid, 
 {
     for (int i = tid; i < 15 * 64; i += nthreads) {
         const int k = 1 + (i >> 6), y = i & 63;
-        V.cy[k * 64 + y] = V.ty[y * kYPitch + 4 * k - 1];
+        V.col0[k * 64 + y] = V.tile0[y * kYPitch + 4 * k - 1];
     }
     for (int i = tid; i < 2 * 15 * 32; i += nthreads) {
-        const int p = i >= 15 * 32, j = p ? i - 15 * 32 : i, k = 1 + (j >> 5), y = j & 31;
-        V.cc[p][k * 32 + y] = V.tc[p][y * kCPitch + 2 * k - 1];
+        const int p = 1 + (i >= 15 * 32), j = p == 2 ? i - 15 * 32 : i, k = 1 + (j >> 5), y = j & 31;
+        V.col(p)[k * 32 + y] = V.tile(p)[y * kCPitch + 2 * k - 1];
     }
 }
 
@@ -1538,7 +1798,7 @@ __device__ __forceinline__ void intra_halo(const IntraView<T> &V, const cvp9_job
         const int w = p ? job.CW : job.W, h = p ? job.CH : job.H;
         const int X = p ? sbx >> 1 : sbx, Y = p ? sby >> 1 : sby;
         const T *g = base + (p ? (size_t)job.W * job.H + (size_t)(p - 1) * job.CW * job.CH : 0);
-        T *tile = p == 0 ? V.ty : V.tc[p - 1], *col = p == 0 ? V.cy : V.cc[p - 1];
+        T *tile = V.tile(p), *col = V.col(p);
         const int pitch = p ? kCPitch : kYPitch;
         if (!half) {
             T v = (T)(top ? fill_l : fill_a);
@@ -1681,7 +1941,7 @@ __device__ __forceinline__ void st_release(unsigned *p, unsigned v)
 }
 
 /* Bounded wait until flag == epoch; returns false on timeout. */
-__device__ bool wait_flag(const unsigned *flag, unsigned epoch)
+__device__ __forceinline__ bool wait_flag(const unsigned *flag, unsigned epoch)
 {
     for (long long it = 0; it < kSpinLimit; it++) {
         if (ld_acquire(flag) == epoch) return true;
@@ -1698,23 +1958,23 @@ __device__ __forceinline__ void pf_l2(const void *p)
 /* Prefetch into L2 the rows of a reference window (clamped like the
  * prediction reads) — first and last 128-byte line of each row. */
 __device__ __forceinline__ void pf_window(const uint8_t *plane, int stride, int pw, int ph,
-                                          int x0, int y0, int w, int h)
+                                          int x0, int y0, int w, int h, int lane)
 {
     int xm = pw > 0 ? pw - 1 : 0, ym = ph > 0 ? ph - 1 : 0;
     int xa = clampi(x0, 0, xm), xb = clampi(x0 + w - 1, 0, xm);
-    for (int r = 0; r < h; r++) {
+    for (int r = lane; r < h; r += 32) {
         const uint8_t *row = plane + (size_t)clampi(y0 + r, 0, ym) * stride;
         pf_l2(row + xa);
         if ((xb >> 7) != (xa >> 7)) pf_l2(row + xb);
     }
 }
 
-/* One thread per block, right after the descriptors are read: pull the
+/* One warp per block, right after the descriptors are read: pull the
  * block's reference windows towards L2 so the prediction phase finds them
  * there. Addresses are clamped into the buffers exactly as the later reads
  * are. */
 template <int A>
-__device__ void prefetch_block(const BlkS &b, const cvp9_job_t &job, int sbx, int sby)
+__device__ void prefetch_block(const BlkS &b, const cvp9_job_t &job, int sbx, int sby, int lane)
 {
     if (b.flags & 1) return;
     const cvp9_ref_t *R;
@@ -1731,15 +1991,15 @@ __device__ void prefetch_block(const BlkS &b, const cvp9_job_t &job, int sbx, in
     const int gx = sbx + b.x, gy = sby + b.y, cbw = (b.cw + 1) >> 1, cbh = (b.ch + 1) >> 1;
     if (A == CVP9_ARITH_REFCPU) {
         int px8 = gx * 8 + b.mvx, py8 = gy * 8 + b.mvy;
-        pf_window(R->plane, rw, rw, rh, px8 >> 3, py8 >> 3, b.cw + 1, b.ch + 1);
+        pf_window(R->plane, rw, rw, rh, px8 >> 3, py8 >> 3, b.cw + 1, b.ch + 1, lane);
         int cx8 = (gx >> 1) * 8 + b.mvx / 2, cy8 = (gy >> 1) * 8 + b.mvy / 2;
-        pf_window(ru, rcs, rw >> 1, rh >> 1, cx8 >> 3, cy8 >> 3, cbw + 1, cbh + 1);
-        pf_window(rv, rcs, rw >> 1, rh >> 1, cx8 >> 3, cy8 >> 3, cbw + 1, cbh + 1);
+        pf_window(ru, rcs, rw >> 1, rh >> 1, cx8 >> 3, cy8 >> 3, cbw + 1, cbh + 1, lane);
+        pf_window(rv, rcs, rw >> 1, rh >> 1, cx8 >> 3, cy8 >> 3, cbw + 1, cbh + 1, lane);
     } else {
-        pf_window(R->plane, rw, rw, rh, gx + (b.mvx >> 3) - 3, gy + (b.mvy >> 3) - 3, b.cw + 7, b.ch + 7);
+        pf_window(R->plane, rw, rw, rh, gx + (b.mvx >> 3) - 3, gy + (b.mvy >> 3) - 3, b.cw + 7, b.ch + 7, lane);
         int cx = (gx >> 1) + (b.mvx >> 4) - 3, cy = (gy >> 1) + (b.mvy >> 4) - 3;
-        pf_window(ru, rcs, rcs, (rh + 1) >> 1, cx, cy, cbw + 7, cbh + 7);
-        pf_window(rv, rcs, rcs, (rh + 1) >> 1, cx, cy, cbw + 7, cbh + 7);
+        pf_window(ru, rcs, rcs, (rh + 1) >> 1, cx, cy, cbw + 7, cbh + 7, lane);
+        pf_window(rv, rcs, rcs, (rh + 1) >> 1, cx, cy, cbw + 7, cbh + 7, lane);
     }
 }
 
@@ -1833,11 +2093,11 @@ __global__ void __launch_bounds__(256) k_scan_blocks(const cvp9_job_t *__restric
 template <int A>
 __device__ __forceinline__ void recon_inter(ReconSmem &s, const BlkS *one, int n, int sbx, int sby, int warp, int lane)
 {
-    auto params = [&](int chk) {
-        const int b = one ? 0 : s.chunk_blk[chk];
-        return one ? chunk_params(*one, chk) : chunk_params(s.blk[b], chk - s.chunk_off[b]);
-    };
     if (A == CVP9_ARITH_REFCPU) {
+        auto params = [&](int chk) {
+            const int b = one ? 0 : s.chunk_blk[chk];
+            return one ? chunk_params(*one, chk) : chunk_params(s.blk[b], chk - s.chunk_off[b]);
+        };
         constexpr int kRound = 4;
         uint8_t *wst = reinterpret_cast<uint8_t *>(s.temp.d) + warp * (kRound * kChunkStage);
         const int q = lane >> 3, k = lane & 7;
@@ -1866,9 +2126,23 @@ __device__ __forceinline__ void recon_inter(ReconSmem &s, const BlkS *one, int n
             __syncwarp();
         }
     } else {
-        for (int chk = warp; chk < n; chk += kWarps) {
-            const ChunkP c = params(chk);
-            spec_inter_chunk(s, *c.b, sbx, sby, c.lx0, c.ly0, c.lw, c.lh, c.cx0, c.cy0, c.clw, c.clh, warp, lane);
+        /* SPEC and FULL: four chunks a warp */
+        const cvp9_job_t &job = s.jc;
+        const uint32_t (*P)[2] = A == CVP9_ARITH_FULL ? c_subpel4_pk[job.interp_filter & 3] : c_subpel_pk;
+        const int g = lane >> 3, k = lane & 7;
+        uint8_t *rows = reinterpret_cast<uint8_t *>(s.temp.i) + (warp * 4 + g) * 128;
+        for (int base = warp * 4; base < n; base += 4 * kWarps) {
+            const int chk = base + g;
+            const bool on = chk < n;
+            const int bi = one || !on ? 0 : s.chunk_blk[chk];
+            const BlkS &b = one ? *one : s.blk[bi];
+            const int ccw = (b.cw + 1) >> 1, cch = (b.ch + 1) >> 1;
+            int p = 0, x = 0, y = 0, w = 0, h = 0;
+            if (on) mc_chunk_at(one ? chk : chk - s.chunk_off[bi], b.cw, b.ch, ccw, cch, p, x, y, w, h);
+            const int lx = (p ? b.x >> 1 : b.x) + x, ly = (p ? b.y >> 1 : b.y) + y;
+            uint8_t *dst = p == 0 ? &TY(s, lx, ly + k) : &TC(s, p, lx, ly + k);
+            mc_chunk<uint8_t>(job, P, b, on, p, (p ? sbx >> 1 : sbx) + lx, (p ? sby >> 1 : sby) + ly, w, h, 128, rows,
+                              dst, k);
         }
     }
 }
@@ -1882,23 +2156,17 @@ __device__ __forceinline__ void intra_block_tasks(IntraWork &W, const BlkS &b, c
     for (int p = 0; p < 3; p++) {
         const int m = p ? b.uvmode : b.ymode;
         const int mode = A == CVP9_ARITH_REFCPU ? (m <= 2 ? m : 9) : (m == 0 || m == 2 || m == 9 ? m : 1);
-        ITask t;
-        t.x = (uint8_t)(p ? b.x >> 1 : b.x);
-        t.y = (uint8_t)(p ? b.y >> 1 : b.y);
-        t.pw = (uint8_t)(p ? (b.cw + 1) >> 1 : b.cw);
-        t.ph = (uint8_t)(p ? (b.ch + 1) >> 1 : b.ch);
-        t.w = t.pw;
-        t.h = t.ph;
+        const int pw = p ? (b.cw + 1) >> 1 : b.cw, ph = p ? (b.ch + 1) >> 1 : b.ch;
+        int w = pw, h = ph;
         if (A == CVP9_ARITH_SPEC && (b.w < 8 || b.h < 8)) {   /* the residual's area: the whole MI */
-            t.w = (uint8_t)(p ? 4 : 8);
-            t.h = t.w;
+            const int ow = min(8, job.W - (sbx + b.x)), oh = min(8, job.H - (sby + b.y));
+            w = p ? (ow + 1) >> 1 : ow;
+            h = p ? (oh + 1) >> 1 : oh;
         }
-        t.pm = (uint8_t)(p | (mode << 2));
-        t.acl = t.lcl = 255;
-        t.dcw = t.pw;
-        t.dch = t.ph;
-        t.avail = (uint8_t)((sby + b.y > 0 ? 1 : 0) | (sbx + b.x > 0 ? 2 : 0));
-        W.task[at + p] = t;
+        /* REFCPU's DC counts the filled edges too */
+        const int avail = (A == CVP9_ARITH_REFCPU || sby + b.y > 0 ? 1 : 0) | (A == CVP9_ARITH_REFCPU || sbx + b.x > 0 ? 2 : 0);
+        st_task(&W.task[at + p], p ? b.x >> 1 : b.x, p ? b.y >> 1 : b.y, w, h, p, mode, 255, 255, avail, pw, ph,
+                dc_inverse((avail & 1 ? pw : 0) + (avail & 2 ? ph : 0)));
         W.lvl[at + p] = (uint16_t)level;
     }
 }
@@ -1954,6 +2222,184 @@ __device__ __forceinline__ int cta_scan1(ReconSmem &s, int v, int *total)
     return ea;
 }
 
+/* The phases of a superblock are functions of their own, each with the whole
+ * register budget of the kernel for its loops: inlined into one body, the
+ * values that live across phases were kept in local memory inside the hot
+ * loops, where the small L1 that the shared memory leaves (28 KB) misses. They
+ * name the shared memory themselves, since a pointer parameter would make
+ * every access a generic one. */
+template <class S>
+__device__ __forceinline__ S &smem_as()
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    return *reinterpret_cast<S *>(smem_raw);
+}
+
+__device__ __forceinline__ IntraView<uint8_t> recon_view(ReconSmem &s)
+{
+    IntraView<uint8_t> V;
+    V.tile0 = &TY(s, 0, 0);
+    V.col0 = s.col;
+    V.res = s.coef;
+    return V;
+}
+
+/* The 4x4 cells of a block: its prediction area; under SPEC and FULL a
+ * sub-8x8 block's residual spans the whole 8x8 MI (vp9_kf_tile.c:327-330),
+ * so it owns that area too. */
+template <int A>
+__device__ __forceinline__ void block_cells(const BlkS &b, const cvp9_job_t &job, int sbx, int sby, int &c0x, int &c1x,
+                                            int &c0y, int &c1y)
+{
+    int ow = b.cw, oh = b.ch;
+    if (A != CVP9_ARITH_REFCPU && (b.w < 8 || b.h < 8)) {
+        ow = min(8, job.W - (sbx + b.x));
+        oh = min(8, job.H - (sby + b.y));
+    }
+    c0x = b.x >> 2;
+    c0y = b.y >> 2;
+    c1x = (b.x + ow - 1) >> 2;
+    c1y = (b.y + oh - 1) >> 2;
+}
+
+/* Inter predictions: of n chunks of the whole SB (one < 0), or of block `one`. */
+template <int A>
+__device__ __noinline__ void phase_inter(int one, int n, int sbx, int sby)
+{
+    ReconSmem &s = smem_as<ReconSmem>();
+    recon_inter<A>(s, one < 0 ? nullptr : &s.blk[one], n, sbx, sby, threadIdx.x >> 5, threadIdx.x & 31);
+}
+
+/* Both transform passes of n items of the whole SB (one < 0), or of block
+ * `one`; zero: clear the residual grid (the coefficient staging, spent after
+ * the first pass) in between. Barriers at both ends. */
+template <int A>
+__device__ __noinline__ void phase_residual(int one, int n, bool staged, unsigned c_base, bool zero)
+{
+    ReconSmem &s = smem_as<ReconSmem>();
+    const int tid = threadIdx.x;
+    __syncthreads();
+    for (int it = tid; it < n; it += kThreads) {
+        const int b = one < 0 ? s.item_blk[it] : one;
+        item_pass1<A>(s, s.blk[b], one < 0 ? it - s.item_off[b] : it, staged, c_base);
+    }
+    __syncthreads();
+    if (zero) {
+        uint4 *z = reinterpret_cast<uint4 *>(s.coef);
+        for (int i = tid; i < kCoefStage / 8; i += kThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+    }
+    for (int it = tid; it < n; it += kThreads) {
+        const int b = one < 0 ? s.item_blk[it] : one;
+        item_pass2<A>(s, s.blk[b], one < 0 ? it - s.item_off[b] : it);
+    }
+    __syncthreads();
+}
+
+/* The intra tasks of the SB's nb blocks, their levels, the sorted quads. */
+template <int A>
+__device__ __noinline__ void phase_plan(int nb, int sbx, int sby)
+{
+    ReconSmem &s = smem_as<ReconSmem>();
+    const cvp9_job_t &job = s.jc;
+    IntraWork &W = s.temp.w;
+    const int tid = threadIdx.x;
+    const bool mine = tid < nb && (s.blk[tid].flags & 1);
+    intra_fill_cols(recon_view(s), tid, kThreads);
+    int ntask;
+    if (A == CVP9_ARITH_FULL) {
+        const int at = cta_scan1(s, mine ? intra_tx_count(s.blk[tid], job, sbx, sby) : 0, &ntask);
+        ntask = min(ntask, kMaxTasks);
+        if (tid < nb) s.first[tid] = (uint16_t)at;
+        for (int i = tid; i < kMaxTasks; i += kThreads) W.own[i] = 0;
+        if (tid < 96) (&W.prow[0][0])[tid] = 0u;
+        __syncthreads();
+        for (int t = tid; t < ntask; t += kThreads) {
+            const int b = find_base(s.first, nb, t);
+            intra_tx_task(W, s.blk[b], job, sbx, sby, t - s.first[b], t, true);
+        }
+        __syncthreads();
+        intra_tx_levels(W, ntask, tid, kThreads);
+    } else {
+        /* a block's three planes share its level */
+        const int at = cta_scan1(s, mine ? 3 : 0, &ntask);
+        if (tid < 96) (&W.prow[0][0])[tid] = 0u;
+        if (tid < nb) W.own[tid] = mine ? (uint16_t)at : (uint16_t)0xFFFF;
+        __syncthreads();
+        LvlTask lt[1];
+        const bool have[1] = { mine };
+        if (mine) {
+            const BlkS &b = s.blk[tid];
+            int c0x, c1x, c0y, c1y;
+            block_cells<A>(b, job, sbx, sby, c0x, c1x, c0y, c1y);
+            lt[0].set(W.prow[0], W.pcol[0], c0x, c1x, c0y, c1y, (b.x + b.cw - 1) >> 2);
+        }
+        __syncthreads();
+        intra_levels<1>(lt, have);
+        if (mine) intra_block_tasks<A>(W, s.blk[tid], job, sbx, sby, at, max(0, lt[0].level));
+    }
+    __syncthreads();
+    intra_sort<A>(W, s.cell, ntask, tid, kThreads);
+}
+
+template <int A>
+__device__ __noinline__ void phase_levels()
+{
+    ReconSmem &s = smem_as<ReconSmem>();
+    intra_run<A, 255, uint8_t>(s.temp.w, recon_view(s), threadIdx.x, kThreads);
+}
+
+/* Intra block b on its own, its residual in the grid. */
+template <int A>
+__device__ __noinline__ void phase_ordered(int b, int sbx, int sby)
+{
+    ReconSmem &s = smem_as<ReconSmem>();
+    const cvp9_job_t &job = s.jc;
+    IntraWork &W = s.temp.w;
+    const int tid = threadIdx.x;
+    const IntraView<uint8_t> V = recon_view(s);
+    intra_fill_cols(V, tid, kThreads);
+    if (A == CVP9_ARITH_FULL) {
+        const int n = min(intra_tx_count(s.blk[b], job, sbx, sby), kMaxTasks);
+        for (int k = tid; k < n; k += kThreads) intra_tx_task(W, s.blk[b], job, sbx, sby, k, k, false);
+        if (tid == 0) W.ntask = n;
+    } else if (tid == 0) {
+        intra_block_tasks<A>(W, s.blk[b], job, sbx, sby, 0, 0);
+        W.ntask = 3;
+    }
+    __syncthreads();
+    intra_run_ordered<A, 255, uint8_t>(W, V, W.ntask, tid, kThreads);
+    __syncthreads();
+}
+
+/* Wait (bounded) for the neighbour SBs whose samples are read (intra_needs
+ * bits), a lane a neighbour, then load the halo. */
+template <class S, class T>
+__device__ __forceinline__ void wait_halo(S &s, const IntraView<T> &V, unsigned need, int sb, bool full, int fill_a,
+                                          int fill_l, int tid, int nthreads)
+{
+    const cvp9_job_t &job = s.jc;
+    const int sbr = sb / job.sb_cols, sbc = sb - sbr * job.sb_cols;
+    const bool have_l = full ? sbc * 8 > full_tile_start(sbc * 8, job.mi_cols, job.log2_tile_cols) : sbc > 0;
+    if (tid < 3 && ((need >> tid) & 1u)) {
+        const int dc = tid == 1 ? 0 : 1, dr = tid == 0 ? 0 : 1;
+        if (sbc >= dc && sbr >= dr && (have_l || tid == 1) &&
+            !wait_flag(job.sb_done + sb - dr * job.sb_cols - dc, job.epoch))
+            atomicOr(job.status, (unsigned)CVP9_JOB_TIMEOUT);
+    }
+    __syncthreads();
+    intra_halo<T>(V, job, sbc * 64, sbr * 64, sbr > 0, have_l, fill_a, fill_l, tid, nthreads);
+    __syncthreads();
+}
+
+template <int A>
+__device__ __noinline__ void phase_neighbours(unsigned need, int sb)
+{
+    ReconSmem &s = smem_as<ReconSmem>();
+    constexpr int fill_a = A == CVP9_ARITH_SPEC ? 128 : 127, fill_l = A == CVP9_ARITH_FULL ? 129 : fill_a;
+    wait_halo<ReconSmem, uint8_t>(s, recon_view(s), need, sb, A == CVP9_ARITH_FULL, fill_a, fill_l, threadIdx.x, kThreads);
+}
+
 template <int A>
 __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restrict__ jobs,
                                                    const uint32_t *__restrict__ tickets,
@@ -1962,8 +2408,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
 {
     /* with the inter fast path the general ticket count is known on the device */
     if (n_dev) n_tickets = *n_dev;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ReconSmem &s = *reinterpret_cast<ReconSmem *>(smem_raw);
+    ReconSmem &s = smem_as<ReconSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const cvp9_job_t &job = s.jc;     /* valid after the reset barrier */
 
@@ -2000,7 +2445,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
         }
         for (int i = tid; i < 256 + 128; i += kThreads) s.txmask[i] = 0;
         for (int i = tid; i < 256; i += kThreads) s.cell[i] = 0;
-        if (tid == 0) { s.c_lo = 0xFFFFFFFFu; s.c_hi = 0u; }
+        if (tid < 16) s.rows[tid] = 0;
+        if (tid == 0) { s.c_lo = 0xFFFFFFFFu; s.c_hi = 0u; s.needs = 0u; }
         __syncthreads();
 
         /* 1. load and re-check blocks (a block must sit inside this SB,
@@ -2058,7 +2504,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             residual_layout<A>(mb, job, g.x, g.y);
             s.blk[tid] = mb;
             my_intra = g.is_intra != 0;
-            nch = my_intra ? 0 : block_chunks(mb);
+            nch = my_intra ? 0 : block_chunks<A>(mb);
             nit = block_items(mb);
         }
         if (__syncthreads_or(my_bad)) {
@@ -2067,7 +2513,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             nb = 0;
             my_intra = my_seq = false;
         }
-        if (tid < nb) prefetch_block<A>(mb, job, sbx, sby);
+        for (int b = warp; b < nb; b += kWarps) prefetch_block<A>(s.blk[b], job, sbx, sby, lane);
         {
             /* span of coefficients the residual pass reads */
             unsigned lo = 0xFFFFFFFFu, hi = 0u;
@@ -2082,20 +2528,14 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             hi = __reduce_max_sync(0xffffffffu, hi);
             if (lane == 0) { atomicMin(&s.c_lo, lo); atomicMax(&s.c_hi, hi); }
         }
+        int c0x = 0, c1x = 0, c0y = 0, c1y = 0;
         if (tid < nb) {
-            /* cells a block writes: its prediction area; under SPEC a
-             * sub-8x8 block's residual spans the whole 8x8 MI
-             * (vp9_kf_tile.c:327-330), so it owns that area too */
-            int ow = mb.cw, oh = mb.ch;
-            if (A != CVP9_ARITH_REFCPU && (mb.w < 8 || mb.h < 8)) {
-                ow = min(8, job.W - (sbx + mb.x));
-                oh = min(8, job.H - (sby + mb.y));
-            }
-            int c0x = mb.x >> 2, c0y = mb.y >> 2;
-            int c1x = (mb.x + ow - 1) >> 2, c1y = (mb.y + oh - 1) >> 2;
-            for (int cy = c0y; cy <= c1y; cy++)
-                for (int cx = c0x; cx <= c1x; cx++)
-                    if (atomicCAS(&s.cell[cy * 16 + cx], (uint16_t)0, (uint16_t)(tid + 1)) != 0) my_seq = true;
+            block_cells<A>(mb, job, sbx, sby, c0x, c1x, c0y, c1y);
+            my_seq |= claim_cells(s.rows, c0x, c1x, c0y, c1y);
+        }
+        {
+            const unsigned need = __reduce_or_sync(0xffffffffu, tid < nb && my_intra ? intra_needs(mb.x, mb.y) : 0u);
+            if (lane == 0 && need) atomicOr(&s.needs, need);
         }
         const int any_intra = __syncthreads_or(my_intra);
         bool seq = __syncthreads_or(my_seq) != 0;
@@ -2104,7 +2544,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
          * copies */
         const unsigned c_lo = s.c_lo, c_hi = s.c_hi;
         const unsigned c_base = c_lo & ~7u;
-        bool staged = c_hi > c_lo && c_hi <= job.num_coeffs && c_hi - c_base <= (unsigned)kCoefStage;
+        const bool staged = c_hi > c_lo && c_hi <= job.num_coeffs && c_hi - c_base <= (unsigned)kCoefStage;
         const bool c_vec = !((uintptr_t)job.coeffs & 15);
         constexpr int kStageIt = kCoefStage / 8 / kThreads;
 #pragma unroll
@@ -2119,15 +2559,18 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
         /* 2. an intra block reads the blocks above it, to its left and at its
          * corner: where one of them comes later in the list, the superblock
          * runs in list order (as it does when blocks overlap) */
-        unsigned needs = 0;
         if (any_intra) {
+            for (int b = warp; b < nb; b += kWarps) {
+                int x0, x1, y0, y1;
+                block_cells<A>(s.blk[b], job, sbx, sby, x0, x1, y0, y1);
+                own_cells(s.cell, b, x0, x1, y0, y1, lane);
+            }
+            __syncthreads();
             bool late = false;
             if (tid < nb && my_intra) {
-                const int c0x = mb.x >> 2, c0y = mb.y >> 2;
-                const int c1x = (mb.x + mb.cw - 1) >> 2, c1y = (mb.y + mb.ch - 1) >> 2;
-                if (c0y > 0) for (int cx = max(0, c0x - 1); cx <= c1x; cx++) late |= s.cell[(c0y - 1) * 16 + cx] > tid;
-                if (c0x > 0) for (int cy = c0y; cy <= c1y; cy++) late |= s.cell[cy * 16 + c0x - 1] > tid;
-                needs = intra_needs(mb.x, mb.y);
+                const int x1 = (mb.x + mb.cw - 1) >> 2, y1 = (mb.y + mb.ch - 1) >> 2;
+                if (c0y > 0) for (int cx = max(0, c0x - 1); cx <= x1; cx++) late |= s.cell[(c0y - 1) * 16 + cx] > tid;
+                if (c0x > 0) for (int cy = c0y; cy <= y1; cy++) late |= s.cell[cy * 16 + c0x - 1] > tid;
             }
             seq |= __syncthreads_or(late) != 0;
         }
@@ -2151,149 +2594,33 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
         }
         __syncthreads();
 
-        IntraWork &W = s.temp.w;
-        IntraView<uint8_t> V;
-        V.ty = &TY(s, 0, 0);
-        V.tc[0] = &TC(s, 1, 0, 0);
-        V.tc[1] = &TC(s, 2, 0, 0);
-        V.cy = s.col;
-        V.cc[0] = s.col + 16 * 64;
-        V.cc[1] = s.col + 16 * 64 + 16 * 32;
-        V.res = s.coef;
-        constexpr int fill_a = A == CVP9_ARITH_SPEC ? 128 : 127;
-        constexpr int fill_l = A == CVP9_ARITH_FULL ? 129 : fill_a;
-        const bool have_l = A == CVP9_ARITH_FULL
-            ? (sbx >> 3) > full_tile_start(sbx >> 3, job.mi_cols, job.log2_tile_cols) : sbx > 0;
-        /* wait (bounded) for the neighbour SBs whose samples are read, a lane
-         * a neighbour, then load the halo */
-        auto neighbours = [&](unsigned need) {
-            if (tid < 3 && ((need >> tid) & 1u)) {
-                const int dc = tid == 1 ? 0 : 1, dr = tid == 0 ? 0 : 1;
-                if (sbc >= dc && sbr >= dr && (have_l || tid == 1) &&
-                    !wait_flag(job.sb_done + sb - dr * job.sb_cols - dc, job.epoch))
-                    atomicOr(job.status, (unsigned)CVP9_JOB_TIMEOUT);
-            }
-            __syncthreads();
-            intra_halo<uint8_t>(V, job, sbx, sby, sby > 0, have_l, fill_a, fill_l, tid, kThreads);
-            __syncthreads();
-        };
-
         if (!seq) {
             /* 3. everything that reads no neighbour: inter predictions, the
              * first transform pass of every TX, then the second, which adds
              * to the inter blocks and leaves the intra blocks' residuals in
              * the (spent) coefficient staging */
-            recon_inter<A>(s, nullptr, min((int)s.chunk_off[nb], 256), sbx, sby, warp, lane);
+            const int n_chunks = min((int)s.chunk_off[nb], 256), n_items = min((int)s.item_off[nb], kMaxItems);
+            if (n_chunks) phase_inter<A>(-1, n_chunks, sbx, sby);
             cp_async_wait_all();
-            __syncthreads();
-            const int n_items = min((int)s.item_off[nb], kMaxItems);
-            for (int it = tid; it < n_items; it += kThreads) {
-                const int lo = s.item_blk[it];
-                item_pass1<A>(s, s.blk[lo], it - s.item_off[lo], staged, c_base);
-            }
-            __syncthreads();
+            phase_residual<A>(-1, n_items, staged, c_base, any_intra);
             if (any_intra) {
-                uint4 *z = reinterpret_cast<uint4 *>(s.coef);
-                for (int i = tid; i < kCoefStage / 8; i += kThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
-                __syncthreads();
-            }
-            for (int it = tid; it < n_items; it += kThreads) {
-                const int lo = s.item_blk[it];
-                item_pass2<A>(s, s.blk[lo], it - s.item_off[lo]);
-            }
-            __syncthreads();
-            if (any_intra) {
-                /* 4. the intra tasks and their levels */
-                intra_fill_cols(V, tid, kThreads);
-                int ntask;
-                if (A == CVP9_ARITH_FULL) {
-                    int cnt = 0;
-                    if (tid < nb && my_intra) {
-#pragma unroll
-                        for (int p = 0; p < 3; p++) {
-                            int txl, nx, ny, pbw;
-                            plane_layout(mb, job, sbx + mb.x, sby + mb.y, p, txl, nx, ny, pbw);
-                            cnt += nx * ny;
-                        }
-                    }
-                    const int at = cta_scan1(s, cnt, &ntask);
-                    if (tid < nb) s.lvl[tid] = (uint16_t)at;
-                    for (int i = tid; i < kMaxTasks; i += kThreads) W.own[i] = 0;
-                    __syncthreads();
-                    for (int b = warp; b < nb; b += kWarps)
-                        if (s.blk[b].flags & 1) intra_tx_tasks(W, s.blk[b], job, sbx, sby, s.lvl[b], true, lane);
-                    ntask = min(ntask, kMaxTasks);
-                    __syncthreads();
-                    intra_tx_levels(W, ntask, tid, kThreads);
-                } else {
-                    /* block levels: inter blocks 0, an intra one above the
-                     * deepest block it reads */
-                    const int at = cta_scan1(s, tid < nb && my_intra ? 3 : 0, &ntask);
-                    volatile uint16_t *lvl = s.lvl;
-                    if (tid < nb) lvl[tid] = my_intra ? 1 : 0;
-                    __syncthreads();
-                    for (int it = 0; it <= kMaxBlocks; it++) {
-                        bool changed = false;
-                        if (tid < nb && my_intra) {
-                            const int c0x = mb.x >> 2, c0y = mb.y >> 2;
-                            const int c1x = (mb.x + mb.cw - 1) >> 2, c1y = (mb.y + mb.ch - 1) >> 2;
-                            int L = 1;
-                            if (c0y > 0)
-                                for (int cx = max(0, c0x - 1); cx <= c1x; cx++) {
-                                    const int o = s.cell[(c0y - 1) * 16 + cx];
-                                    if (o) L = max(L, lvl[o - 1] + 1);
-                                }
-                            if (c0x > 0)
-                                for (int cy = c0y; cy <= c1y; cy++) {
-                                    const int o = s.cell[cy * 16 + c0x - 1];
-                                    if (o) L = max(L, lvl[o - 1] + 1);
-                                }
-                            if (L != lvl[tid]) { lvl[tid] = (uint16_t)L; changed = true; }
-                        }
-                        if (!__syncthreads_or(changed)) break;
-                    }
-                    if (tid < nb && my_intra) intra_block_tasks<A>(W, mb, job, sbx, sby, at, lvl[tid] - 1);
-                }
-                intra_sort(W, ntask, tid, kThreads);
-                /* 5. the neighbours' samples, then level by level */
-                needs = __reduce_or_sync(0xffffffffu, needs);
-                needs = (unsigned)(__syncthreads_or(needs & 1u) ? 1u : 0u) | (__syncthreads_or(needs & 2u) ? 2u : 0u) |
-                        (__syncthreads_or(needs & 4u) ? 4u : 0u);
-                neighbours(needs);
-                intra_run<A, 255, uint8_t>(W, V, tid, kThreads);
+                /* 4. the intra tasks and their levels; 5. the neighbours'
+                 * samples, then level by level */
+                phase_plan<A>(nb, sbx, sby);
+                phase_neighbours<A>(s.needs, sb);
+                phase_levels<A>();
             }
         } else {
             /* list order, block by block; the staging holds residuals only */
             cp_async_wait_all();
-            staged = false;
             __syncthreads();
-            if (any_intra) neighbours(7u);
+            if (any_intra) phase_neighbours<A>(7u, sb);
             for (int b = 0; b < nb; b++) {
-                const BlkS &blk = s.blk[b];
-                if (!(blk.flags & 1)) recon_inter<A>(s, &blk, block_chunks(blk), sbx, sby, warp, lane);
+                const bool intra = s.blk[b].flags & 1;
+                if (!intra) phase_inter<A>(b, block_chunks<A>(s.blk[b]), sbx, sby);
                 for (int i = tid; i < 256 + 128; i += kThreads) s.txmask[i] = 0;
-                for (int i = tid; i < kCoefStage; i += kThreads) s.coef[i] = 0;
-                __syncthreads();
-                const int n_it = block_items(blk);
-                for (int k = tid; k < n_it; k += kThreads) item_pass1<A>(s, blk, k, false, 0u);
-                __syncthreads();
-                for (int k = tid; k < n_it; k += kThreads) item_pass2<A>(s, blk, k);
-                __syncthreads();
-                if (blk.flags & 1) {
-                    intra_fill_cols(V, tid, kThreads);
-                    if (A == CVP9_ARITH_FULL) {
-                        if (warp == 0) {
-                            const int n = intra_tx_tasks(W, blk, job, sbx, sby, 0, false, lane);
-                            if (lane == 0) W.ntask = min(n, kMaxTasks);
-                        }
-                    } else if (tid == 0) {
-                        intra_block_tasks<A>(W, blk, job, sbx, sby, 0, 0);
-                        W.ntask = 3;
-                    }
-                    __syncthreads();
-                    intra_run_ordered<A, 255, uint8_t>(W, V, W.ntask, tid, kThreads);
-                    __syncthreads();
-                }
+                phase_residual<A>(b, block_items(s.blk[b]), false, 0u, true);
+                if (intra) phase_ordered<A>(b, sbx, sby);
             }
         }
 
@@ -2978,20 +3305,6 @@ __device__ __forceinline__ uint32_t win4(const uint32_t o[4], int k)
     return (k & 3) ? __funnelshift_r(o[k >> 2], o[(k >> 2) + 1], 8 * (k & 3)) : o[k >> 2];
 }
 
-/* c + the dot product of four signed taps with four unsigned samples */
-
-
-/* 4x4 byte transpose: rows a..d (one word of four columns each) to four
- * words, one column each (its bytes in row order) */
-__device__ __forceinline__ void tr4(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t col[4])
-{
-    const uint32_t x0 = __byte_perm(a, b, 0x5140), x1 = __byte_perm(a, b, 0x7362);
-    const uint32_t y0 = __byte_perm(c, d, 0x5140), y1 = __byte_perm(c, d, 0x7362);
-    col[0] = __byte_perm(x0, y0, 0x5410);
-    col[1] = __byte_perm(x0, y0, 0x7632);
-    col[2] = __byte_perm(x1, y1, 0x5410);
-    col[3] = __byte_perm(x1, y1, 0x7632);
-}
 
 /* Luma prediction of four chunks (vp9_mc.comp.glsl:61-110): lane = (chunk
  * c0 + lane/8, k = lane%8). Horizontal 8-tap rows k and k+8 of each chunk's
@@ -4567,6 +4880,7 @@ struct HbdSmem {
     uint8_t  txwide[kHbdMaxTx];            /* and one that needs 64-bit values */
     int      scan[kHbdWarps];
     cvp9_job_t jc;
+    unsigned needs;                        /* intra_needs of its blocks        */
     int      ticket;
 };
 
@@ -4582,7 +4896,7 @@ __device__ __forceinline__ int32_t *hbd_tmp(HbdSmem &s, int p, int x, int y)
 
 /* Exclusive prefix of v over the CTA's threads (thread order); *total: the
  * sum. Every thread calls it. */
-__device__ int hbd_scan(HbdSmem &s, int v, int *total)
+__device__ __forceinline__ int hbd_scan(HbdSmem &s, int v, int *total)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int x = v;
@@ -4605,112 +4919,12 @@ __device__ int hbd_scan(HbdSmem &s, int v, int *total)
     return off + x - v;
 }
 
-/* Largest k in [0, n) with base[k] <= v (base ascending, base[0] = 0). */
-__device__ __forceinline__ int hbd_find(const uint16_t *base, int n, int v)
-{
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (base[mid] <= v) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-/* Prediction items of an inter block: a column strip of up to 8 rows of
- * one plane. */
-__device__ __forceinline__ int hbd_pred_items(const HbdBlk &b)
-{
-    return (int)b.cw * (((int)b.ch + 7) >> 3) + 2 * (int)b.ccw * (((int)b.cch + 7) >> 3);
-}
-
-/* One column strip of one plane of an inter block: both 8-tap passes (the
- * frame's filter), each rounded and clipped to 10 bits, every fetch clamped
- * into the reference plane; a compound block averages its second
- * prediction in with rounding. A missing first reference predicts 512. */
-__device__ void hbd_pred_strip(HbdSmem &s, const HbdBlk &b, int item, int sbx, int sby)
-{
-    const cvp9_job_t &job = s.jc;
-    const int nl = (int)b.cw * (((int)b.ch + 7) >> 3), nc = (int)b.ccw * (((int)b.cch + 7) >> 3);
-    int p, k;
-    if (item < nl) { p = 0; k = item; }
-    else { p = 1 + (item - nl >= nc); k = item - nl - (p - 1) * nc; }
-    const int cols = p ? b.ccw : b.cw, rows = p ? b.cch : b.ch;
-    const int grp = k / cols, c = k - grp * cols;
-    const int r0 = grp * 8, nr = min(8, rows - r0);
-    const int lx = (p ? (b.x >> 1) : b.x) + c, ly0 = (p ? (b.y >> 1) : b.y) + r0;
-    const int gx = (p ? (sbx >> 1) : sbx) + lx, gy0 = (p ? (sby >> 1) : sby) + ly0;
-    const int (*F)[8] = c_subpel4[job.interp_filter & 3];
-    int out[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) out[i] = kHbdMid;
-    for (int q = 0; q < 2; q++) {
-        const int rf = q ? b.ref1 : b.ref0;
-        if (q == 1 && rf == 0) break;
-        const cvp9_ref_t &R = job.ref[job.ref_slot_of[clampi(rf - 1, 0, 2)] & 7];
-        if (!R.plane) break;
-        const uint16_t *rp = reinterpret_cast<const uint16_t *>(R.plane);
-        int pw = R.w, ph = R.h;
-        if (p) {
-            rp += (size_t)R.w * R.h;
-            pw = (R.w + 1) >> 1;
-            ph = (R.h + 1) >> 1;
-            if (p == 2) rp += (size_t)pw * ph;
-        }
-        const int mvx = q ? b.mv1x : b.mvx, mvy = q ? b.mv1y : b.mvy;
-        const int X = gx + (p ? (mvx >> 4) : (mvx >> 3)), Y0 = gy0 + (p ? (mvy >> 4) : (mvy >> 3));
-        const int fx = p ? (mvx & 15) : ((mvx & 7) << 1), fy = p ? (mvy & 15) : ((mvy & 7) << 1);
-        int cx[8];
-#pragma unroll
-        for (int t = 0; t < 8; t++) cx[t] = clampi(X + t - 3, 0, pw - 1);
-        int h[15];
-#pragma unroll
-        for (int j = 0; j < 15; j++) {
-            h[j] = 0;
-            if (j >= nr + 7) continue;
-            const uint16_t *row = rp + (size_t)clampi(Y0 - 3 + j, 0, ph - 1) * pw;
-            if (fx == 0) {
-                h[j] = __ldg(row + cx[3]);
-            } else {
-                int a = 0;
-#pragma unroll
-                for (int t = 0; t < 8; t++) a += F[fx][t] * (int)__ldg(row + cx[t]);
-                h[j] = clampi((a + 64) >> 7, 0, kHbdMax);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            int v = h[i + 3];
-            if (fy != 0) {
-                int a = 0;
-#pragma unroll
-                for (int t = 0; t < 8; t++) a += F[fy][t] * h[i + t];
-                v = clampi((a + 64) >> 7, 0, kHbdMax);
-            }
-            out[i] = q ? (out[i] + v + 1) >> 1 : v;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-        if (i < nr) HT(s, p, lx, ly0 + i) = (uint16_t)out[i];
-}
-
 /* The residual TXs of a block in coefficient order (planes, then raster) as
- * s.tx[at ...], by one warp; their number whatever the coefficients. A TX
+ * s.tx[at ...], by one warp. A TX
  * whose coefficients do not end inside num_coeffs is marked empty: offsets
  * ascend, so every later one of the block is, too (as is one reaching past
  * the SB, which no block that its TXs tile has). */
-__device__ int hbd_tx_count(const HbdBlk &b, const cvp9_job_t &job, int sbx, int sby)
-{
-    int n = 0;
-    for (int p = 0; p < 3; p++) {
-        int txl, nx, ny, pbw;
-        plane_layout(b, job, sbx + b.x, sby + b.y, p, txl, nx, ny, pbw);
-        n += nx * ny;
-    }
-    return n;
-}
-
-__device__ void hbd_list_txs(HbdSmem &s, const HbdBlk &b, int sbx, int sby, int at, int lane)
+__device__ __forceinline__ void hbd_list_txs(HbdSmem &s, const HbdBlk &b, int sbx, int sby, int at, int lane)
 {
     const cvp9_job_t &job = s.jc;
     const int gx = sbx + b.x, gy = sby + b.y;
@@ -4822,17 +5036,17 @@ __device__ __forceinline__ void hbd_col_as(HbdSmem &s, int j, int p, int px0, in
 }
 
 template <int N>
-__device__ __noinline__ void hbd_col_wide(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst,
+__device__ __noinline__ void hbd_col_wide(int j, int p, int px0, int py0, bool lossless, bool col_adst,
                                           bool intra)
 {
-    hbd_col_as<N, wl>(s, j, p, px0, py0, lossless, col_adst, intra);
+    hbd_col_as<N, wl>(smem_as<HbdSmem>(), j, p, px0, py0, lossless, col_adst, intra);
 }
 
 template <int N>
 __device__ __forceinline__ void hbd_col(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst,
                                         bool intra, bool wide)
 {
-    if (wide) hbd_col_wide<N>(s, j, p, px0, py0, lossless, col_adst, intra);
+    if (wide) hbd_col_wide<N>(j, p, px0, py0, lossless, col_adst, intra);
     else hbd_col_as<N, wn>(s, j, p, px0, py0, lossless, col_adst, intra);
 }
 
@@ -4858,30 +5072,48 @@ __device__ __forceinline__ void hbd_col_n(HbdSmem &s, int txl, int j, int p, int
     }
 }
 
-/* Blocks [lo, hi) of the SB, whole CTA: the inter blocks' predictions, then
- * the TX rows and the TX columns of every block's residual (an intra block's
- * into the residual grid, which starts at zero). */
-__device__ __noinline__ void hbd_blocks(HbdSmem &s, int lo, int hi, int nb, int sbx, int sby)
+/* The inter predictions of blocks [lo, hi) of the SB, whole CTA, four chunks
+ * a warp. */
+__device__ __noinline__ void hbd_predict(int lo, int hi, int nb, int sbx, int sby)
 {
+    HbdSmem &s = smem_as<HbdSmem>();
+    const cvp9_job_t &job = s.jc;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 3, k = lane & 7;
+    const bool inter = tid >= lo && tid < hi && tid < nb && !(s.blk[tid].flags & 1);
+    int n;
+    const int at = hbd_scan(s, inter ? mc_chunks(s.blk[tid].cw, s.blk[tid].ch, s.blk[tid].ccw, s.blk[tid].cch) : 0, &n);
+    if (tid < kHbdMaxBlocks) s.it_base[tid] = (uint16_t)min(at, 0xFFFF);
+    __syncthreads();
+    const uint32_t (*P)[2] = c_subpel4_pk[job.interp_filter & 3];
+    uint16_t *rows = reinterpret_cast<uint16_t *>(s.tmp.i) + (warp * 4 + g) * 128;
+    for (int base = warp * 4; base < n; base += 4 * kHbdWarps) {
+        const int chk = base + g;
+        const bool on = chk < n;
+        const int bi = on ? find_base(s.it_base, nb, chk) : 0;
+        const HbdBlk &b = s.blk[bi];
+        int p = 0, x = 0, y = 0, w = 0, h = 0;
+        if (on) mc_chunk_at(chk - s.it_base[bi], b.cw, b.ch, b.ccw, b.cch, p, x, y, w, h);
+        const int lx = (p ? b.x >> 1 : b.x) + x, ly = (p ? b.y >> 1 : b.y) + y;
+        mc_chunk<uint16_t>(job, P, b, on, p, (p ? sbx >> 1 : sbx) + lx, (p ? sby >> 1 : sby) + ly, w, h, kHbdMid, rows,
+                           &HT(s, p, lx, ly + k), k);
+    }
+    __syncthreads();
+}
+
+/* Blocks [lo, hi) of the SB, whole CTA: the TX rows and the TX columns of every block's residual (an intra block's
+ * into the residual grid, which starts at zero). */
+__device__ __noinline__ void hbd_residual(int lo, int hi, int nb, int sbx, int sby)
+{
+    HbdSmem &s = smem_as<HbdSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const cvp9_job_t &job = s.jc;
     const bool in = tid >= lo && tid < hi && tid < nb;
-    const bool inter = in && !(s.blk[tid].flags & 1);
     int total;
-    /* 1. predictions */
-    int cnt = inter ? hbd_pred_items(s.blk[tid]) : 0;
-    int base = hbd_scan(s, cnt, &total);
-    if (tid < kHbdMaxBlocks) s.it_base[tid] = (uint16_t)min(base, 0xFFFF);
-    __syncthreads();
-    for (int it = tid; it < total; it += kHbdThreads) {
-        const int bi = hbd_find(s.it_base, nb, it);
-        hbd_pred_strip(s, s.blk[bi], it - s.it_base[bi], sbx, sby);
-    }
     for (int i = tid; i < kResidGrid / 8; i += kHbdThreads) reinterpret_cast<uint4 *>(s.res)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    /* 2. the residual TXs, a warp per block listing them */
-    cnt = in && !(s.blk[tid].flags & 2) && s.blk[tid].txl <= 3 ? hbd_tx_count(s.blk[tid], job, sbx, sby) : 0;
-    base = hbd_scan(s, cnt, &total);
+    /* the residual TXs, a warp per block listing them */
+    int cnt = in && !(s.blk[tid].flags & 2) && s.blk[tid].txl <= 3 ? intra_tx_count(s.blk[tid], job, sbx, sby) : 0;
+    int base = hbd_scan(s, cnt, &total);
     if (total > kHbdMaxTx) {
         if (tid == 0) atomicOr(job.status, (unsigned)CVP9_JOB_TOO_MANY);
         total = kHbdMaxTx;
@@ -4908,7 +5140,7 @@ __device__ __noinline__ void hbd_blocks(HbdSmem &s, int lo, int hi, int nb, int 
         __syncthreads();
         const int nrow = s.tx_base[ntx];
         for (int it = tid; it < nrow; it += kHbdThreads) {
-            const int t = hbd_find(s.tx_base, ntx, it);
+            const int t = find_base(s.tx_base, ntx, it);
             const HbdTx x = s.tx[t];
             if (x.plane & 0x20) continue;
             const int got = hbd_row_n(s, x.txl, job.coeffs32 + x.coeff, it - s.tx_base[t], x.plane & 3, x.x, x.y,
@@ -4918,7 +5150,7 @@ __device__ __noinline__ void hbd_blocks(HbdSmem &s, int lo, int hi, int nb, int 
         }
         __syncthreads();
         for (int it = tid; it < nrow; it += kHbdThreads) {
-            const int t = hbd_find(s.tx_base, ntx, it);
+            const int t = find_base(s.tx_base, ntx, it);
             const HbdTx x = s.tx[t];
             if (s.txnz[t]) hbd_col_n(s, x.txl, it - s.tx_base[t], x.plane & 3, x.x, x.y, job.lossless,
                                      (x.plane >> 2) & 1, (x.plane >> 4) & 1, s.txwide[t] != 0);
@@ -4927,14 +5159,75 @@ __device__ __noinline__ void hbd_blocks(HbdSmem &s, int lo, int hi, int nb, int 
     __syncthreads();
 }
 
+__device__ __forceinline__ IntraView<uint16_t> hbd_view(HbdSmem &s)
+{
+    IntraView<uint16_t> V;
+    V.tile0 = &HT(s, 0, 0, 0);
+    V.col0 = s.col;
+    V.res = s.res;
+    return V;
+}
+
+/* The intra TXs of the SB's nb blocks, their levels, the sorted quads. */
+__device__ __noinline__ void hbd_plan(int nb, int sbx, int sby)
+{
+    HbdSmem &s = smem_as<HbdSmem>();
+    const cvp9_job_t &job = s.jc;
+    IntraWork &W = s.tmp.w;
+    const int tid = threadIdx.x;
+    intra_fill_cols(hbd_view(s), tid, kHbdThreads);
+    int ntask;
+    const int at = hbd_scan(s, tid < nb && (s.blk[tid].flags & 1) ? intra_tx_count(s.blk[tid], job, sbx, sby) : 0, &ntask);
+    ntask = min(ntask, kMaxTasks);
+    s.it_base[tid] = (uint16_t)min(at, 0xFFFF);
+    for (int i = tid; i < kMaxTasks; i += kHbdThreads) W.own[i] = 0;
+    if (tid < 96) (&W.prow[0][0])[tid] = 0u;
+    __syncthreads();
+    for (int t = tid; t < ntask; t += kHbdThreads) {
+        const int b = find_base(s.it_base, nb, t);
+        intra_tx_task(W, s.blk[b], job, sbx, sby, t - s.it_base[b], t, true);
+    }
+    __syncthreads();
+    intra_tx_levels(W, ntask, tid, kHbdThreads);
+    __syncthreads();
+    intra_sort<CVP9_ARITH_FULL>(W, s.cell, ntask, tid, kHbdThreads);
+}
+
+__device__ __noinline__ void hbd_levels()
+{
+    HbdSmem &s = smem_as<HbdSmem>();
+    intra_run<CVP9_ARITH_FULL, kHbdMax, uint16_t>(s.tmp.w, hbd_view(s), threadIdx.x, kHbdThreads);
+}
+
+/* Intra block b on its own, its residual in the grid. */
+__device__ __noinline__ void hbd_ordered(int b, int sbx, int sby)
+{
+    HbdSmem &s = smem_as<HbdSmem>();
+    IntraWork &W = s.tmp.w;
+    const int tid = threadIdx.x;
+    const IntraView<uint16_t> V = hbd_view(s);
+    intra_fill_cols(V, tid, kHbdThreads);
+    const int n = min(intra_tx_count(s.blk[b], s.jc, sbx, sby), kMaxTasks);
+    for (int k = tid; k < n; k += kHbdThreads) intra_tx_task(W, s.blk[b], s.jc, sbx, sby, k, k, false);
+    if (tid == 0) W.ntask = n;
+    __syncthreads();
+    intra_run_ordered<CVP9_ARITH_FULL, kHbdMax, uint16_t>(W, V, W.ntask, tid, kHbdThreads);
+    __syncthreads();
+}
+
+__device__ __noinline__ void hbd_neighbours(unsigned need, int sb)
+{
+    HbdSmem &s = smem_as<HbdSmem>();
+    wait_halo<HbdSmem, uint16_t>(s, hbd_view(s), need, sb, true, kHbdMid - 1, kHbdMid + 1, threadIdx.x, kHbdThreads);
+}
+
 } /* namespace */
 
 __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *__restrict__ jobs,
                                                               const uint32_t *__restrict__ tickets,
                                                               uint32_t n_tickets, uint32_t *ticket_counter)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    HbdSmem &s = *reinterpret_cast<HbdSmem *>(smem_raw);
+    HbdSmem &s = smem_as<HbdSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const cvp9_job_t &job = s.jc;
     for (;;) {
@@ -4968,6 +5261,7 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
         }
         for (int i = tid; i < 256; i += kHbdThreads) s.cell[i] = 0;
         if (tid < 16) s.rows[tid] = 0;
+        if (tid == 0) s.needs = 0u;
         __syncthreads();
 
         /* 1. blocks (each inside this SB, 4-aligned, 4..64 px, tx_size <= 3,
@@ -5029,75 +5323,34 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
         }
         /* an intra block reading samples of a block later in the list: the
          * superblock runs in list order */
-        unsigned needs = 0;
+        unsigned need = 0;
         if (tid < nb && my_intra) {
             const HbdBlk &b = s.blk[tid];
             const int cx0 = b.x >> 2, cy0 = b.y >> 2, cx1 = (b.x + b.cw - 1) >> 2, cy1 = (b.y + b.ch - 1) >> 2;
             if (cy0 > 0) for (int cx = max(0, cx0 - 1); cx <= cx1; cx++) my_seq |= s.cell[(cy0 - 1) * 16 + cx] > tid;
             if (cx0 > 0) for (int cy = cy0; cy <= cy1; cy++) my_seq |= s.cell[cy * 16 + cx0 - 1] > tid;
-            needs = intra_needs(b.x, b.y);
+            need = intra_needs(b.x, b.y);
         }
+        need = __reduce_or_sync(0xffffffffu, need);
+        if (lane == 0 && need) atomicOr(&s.needs, need);
         const bool seq = __syncthreads_or(my_seq) != 0;
-
-        IntraWork &W = s.tmp.w;
-        IntraView<uint16_t> V;
-        V.ty = &HT(s, 0, 0, 0);
-        V.tc[0] = &HT(s, 1, 0, 0);
-        V.tc[1] = &HT(s, 2, 0, 0);
-        V.cy = s.col;
-        V.cc[0] = s.col + 16 * 64;
-        V.cc[1] = s.col + 16 * 64 + 16 * 32;
-        V.res = s.res;
-        const bool have_l = (sbx >> 3) > full_tile_start(sbx >> 3, job.mi_cols, job.log2_tile_cols);
-        auto neighbours = [&](unsigned need) {
-            if (tid < 3 && ((need >> tid) & 1u)) {
-                const int dc = tid == 1 ? 0 : 1, dr = tid == 0 ? 0 : 1;
-                if (sbc >= dc && sbr >= dr && (have_l || tid == 1) &&
-                    !wait_flag(job.sb_done + sb - dr * job.sb_cols - dc, job.epoch))
-                    atomicOr(job.status, (unsigned)CVP9_JOB_TIMEOUT);
-            }
-            __syncthreads();
-            intra_halo<uint16_t>(V, job, sbx, sby, sby > 0, have_l, kHbdMid - 1, kHbdMid + 1, tid, kHbdThreads);
-            __syncthreads();
-        };
 
         /* 2. reconstruct: what reads no neighbour, then the intra blocks level
          * by level; or block by block in list order */
         if (!seq) {
-            hbd_blocks(s, 0, nb, nb, sbx, sby);
+            hbd_predict(0, nb, nb, sbx, sby);
+            hbd_residual(0, nb, nb, sbx, sby);
             if (any_intra) {
-                intra_fill_cols(V, tid, kHbdThreads);
-                int ntask;
-                const int at = hbd_scan(s, tid < nb && my_intra ? hbd_tx_count(s.blk[tid], job, sbx, sby) : 0, &ntask);
-                s.it_base[tid] = (uint16_t)min(at, 0xFFFF);
-                for (int i = tid; i < kMaxTasks; i += kHbdThreads) W.own[i] = 0;
-                __syncthreads();
-                for (int b = warp; b < nb; b += kHbdWarps)
-                    if (s.blk[b].flags & 1) intra_tx_tasks(W, s.blk[b], job, sbx, sby, s.it_base[b], true, lane);
-                ntask = min(ntask, kMaxTasks);
-                __syncthreads();
-                intra_tx_levels(W, ntask, tid, kHbdThreads);
-                intra_sort(W, ntask, tid, kHbdThreads);
-                needs = __reduce_or_sync(0xffffffffu, needs);
-                needs = (unsigned)(__syncthreads_or(needs & 1u) ? 1u : 0u) | (__syncthreads_or(needs & 2u) ? 2u : 0u) |
-                        (__syncthreads_or(needs & 4u) ? 4u : 0u);
-                neighbours(needs);
-                intra_run<CVP9_ARITH_FULL, kHbdMax, uint16_t>(W, V, tid, kHbdThreads);
+                hbd_plan(nb, sbx, sby);
+                hbd_neighbours(s.needs, sb);
+                hbd_levels();
             }
         } else {
-            if (any_intra) neighbours(7u);
+            if (any_intra) hbd_neighbours(7u, sb);
             for (int i = 0; i < nb; i++) {
-                hbd_blocks(s, i, i + 1, nb, sbx, sby);
-                if (s.blk[i].flags & 1) {
-                    intra_fill_cols(V, tid, kHbdThreads);
-                    if (warp == 0) {
-                        const int n = intra_tx_tasks(W, s.blk[i], job, sbx, sby, 0, false, lane);
-                        if (lane == 0) W.ntask = min(n, kMaxTasks);
-                    }
-                    __syncthreads();
-                    intra_run_ordered<CVP9_ARITH_FULL, kHbdMax, uint16_t>(W, V, W.ntask, tid, kHbdThreads);
-                    __syncthreads();
-                }
+                hbd_predict(i, i + 1, nb, sbx, sby);
+                hbd_residual(i, i + 1, nb, sbx, sby);
+                if (s.blk[i].flags & 1) hbd_ordered(i, sbx, sby);
             }
         }
 
