@@ -58,7 +58,7 @@ size_t cvp9k_recon_smem_bytes(void);
 int    cvp9k_upload_dct_basis(const double *basis, int count);
 int    cvp9k_configure(void);
 int    cvp9k_recon_ctas_per_sm(int arith);
-/* CTAs of k_lf_full (128 threads, static shared memory) resident per SM. */
+/* CTAs of k_lf_full resident per SM. */
 int    cvp9k_lf_full_ctas_per_sm(void);
 /* CTAs of k_hbd_recon resident per SM. */
 int    cvp9k_hbd_ctas_per_sm(void);
