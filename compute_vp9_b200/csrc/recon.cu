@@ -50,12 +50,14 @@ constexpr int kCoefStage = 6144;     /* int16 coefficients staged per SB (64x64 
 constexpr int kMaxItems = 1536;      /* TX columns per SB: 4x4 TXs on all three planes */
 constexpr int kYPitch = 72;          /* luma tile row pitch; x = 0 at byte 4 */
 constexpr int kCPitch = 40;          /* chroma tile row pitch; x = 0 at byte 4 */
-constexpr int kTempPitch = 65;       /* doubles per REFCPU temp row */
 constexpr int kTyBytes = (65 * kYPitch + 15) / 16 * 16;
 constexpr int kTcBytes = (33 * kCPitch + 15) / 16 * 16;
 constexpr long long kSpinLimit = 1ll << 20;   /* ~0.25 s of polling */
 
 __constant__ double c_dct[16 + 64 + 256 + 1024];      /* N = 4, 8, 16, 32 */
+/* The basis again in global memory: lane-varying reads are served by L1
+ * instead of being serialised by the constant cache. */
+__device__ __align__(16) double g_dct[16 + 64 + 256 + 1024];
 __constant__ uint8_t c_tx_type[10] = CVP9_INTRA_TX_TYPE_INIT;
 /* the regular filter's taps as signed bytes, taps 0-3 and 4-7 in two words, for dp4a
  * (phase 0's 128 does not fit a byte: callers take the centre sample for
@@ -63,11 +65,6 @@ __constant__ uint8_t c_tx_type[10] = CVP9_INTRA_TX_TYPE_INIT;
 __constant__ uint32_t c_subpel_pk[16][2];
 /* the four VP9 filters (interp_filter 0..3) packed the same way, for the FULL profile */
 __constant__ uint32_t c_subpel4_pk[4][16][2];
-
-__device__ __forceinline__ const double *dct_basis(int txl)
-{
-    return c_dct + (txl == 0 ? 0 : txl == 1 ? 16 : txl == 2 ? 80 : 336);
-}
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
@@ -462,16 +459,20 @@ struct IntraView {
 
 struct ReconSmem {
     union {
-        double  d[64 * kTempPitch];              /* REFCPU first-pass output    */
-        int32_t i[64 * 64 + 2 * 32 * 32];        /* SPEC column-pass output     */
-        IntraWork w;                             /* then the intra tasks        */
+        uint8_t mc[kWarps * 4 * 608];            /* REFCPU: windows of the chunks in flight */
+        int32_t i[64 * 64 + 2 * 32 * 32];        /* SPEC, FULL: first-pass output */
+        struct {
+            IntraWork w;                         /* then the intra tasks        */
+            int16_t res[kResidGrid];             /* REFCPU: intra residuals     */
+        } a;
     } temp;
     /* tiles, contiguous and 16-byte sized so they fill with vector stores */
     uint8_t  ty[kTyBytes];                       /* luma tile, row 0 = halo     */
     uint8_t  tu[kTcBytes];
     uint8_t  tv[kTcBytes];
     int16_t  coef[kCoefStage];                   /* the SB's coefficient span; then
-                                                  * its intra blocks' residuals */
+                                                  * (SPEC, FULL) its intra blocks'
+                                                  * residuals                   */
     cvp9_job_t jc;                               /* this ticket's job           */
     BlkS     blk[kMaxBlocks];
     uint32_t txmask[256 + 64 + 64];              /* per-TX column-nonzero bits  */
@@ -481,7 +482,11 @@ struct ReconSmem {
     uint16_t chunk_off[kMaxBlocks + 1];          /* inter chunks before a block */
     uint16_t item_off[kMaxBlocks + 1];           /* TX items before a block     */
     uint8_t  chunk_blk[256];                     /* chunk -> block              */
-    uint8_t  item_blk[kMaxItems];                /* TX column/row -> block      */
+    union {
+        uint8_t item_blk[kMaxItems];             /* TX column/row -> block      */
+        uint2   tx[256];                         /* REFCPU: the SB's TXs (RefTx) */
+    };
+    int      ntx[4];                             /* REFCPU: TXs of each size    */
     uint8_t  col[16 * 64 + 2 * 16 * 32];         /* left-column copies (IntraView) */
     int      scan_tmp[2 * kWarps];
     unsigned c_lo, c_hi;                         /* coefficient span of the SB  */
@@ -541,8 +546,7 @@ __device__ __forceinline__ void residual_layout(BlkS &b, const cvp9_job_t &job, 
     b.ptxl[0] = b.ptxl[1] = b.ptxl[2] = 0;
     if (b.flags & 2) return;
     if (A == CVP9_ARITH_REFCPU) {
-        int n = 4 << b.txl;
-        int nx = b.cw / n, ny = b.ch / n;
+        const int nx = b.cw >> (2 + b.txl), ny = b.ch >> (2 + b.txl);
         b.ptxl[0] = b.txl;
         b.pnx[0] = (uint8_t)nx;
         b.pnt[0] = (uint16_t)(nx * ny);
@@ -1056,32 +1060,6 @@ __device__ __forceinline__ TxRef locate_item(const BlkS &b, int item, int *lane_
     return t;
 }
 
-/* REFCPU pass 1: T[:, j] = M^T X[:, j] over the nonzero X[k][j], k ascending
- * (vp9_reconstruct.c:31-40). Skipped zero terms add +-0 to a sum that is
- * never -0, so the result is bit-identical to the full sum. */
-template <int N>
-__device__ __forceinline__ void refcpu_col(ReconSmem &s, const int16_t *X, int j,
-                                           int px0, int py0, int mask_idx, const double *M)
-{
-    unsigned nzm = 0;
-#pragma unroll
-    for (int k = 0; k < N; k++) nzm |= (X[k * N + j] != 0 ? 1u : 0u) << k;
-    if (!nzm) return;
-    double acc[N];
-#pragma unroll
-    for (int i = 0; i < N; i++) acc[i] = 0.0;
-    while (nzm) {
-        const int k = __ffs(nzm) - 1;
-        nzm &= nzm - 1;
-        const double xd = (double)X[k * N + j];
-#pragma unroll
-        for (int i = 0; i < N; i++) acc[i] = __dadd_rn(acc[i], __dmul_rn(M[k * N + i], xd));
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++) s.temp.d[(py0 + i) * kTempPitch + px0 + j] = acc[i];
-    atomicOr(&s.txmask[mask_idx], 1u << j);
-}
-
 /* Residual of one sample: saturated to int16 (which no sum with a sample
  * notices) into the residual grid of an intra block, or added into the tile
  * of an inter block (res null). */
@@ -1092,30 +1070,6 @@ __device__ __forceinline__ void put_residual(ReconSmem &s, int p, int x, int y, 
     } else {
         uint8_t &px = p == 0 ? TY(s, x, y) : TC(s, p, x, y);
         px = (uint8_t)clampi((int)px + r, 0, 255);
-    }
-}
-
-/* REFCPU pass 2: O[i, :] = T[i, :] M over the nonzero columns, round half
- * away from zero, saturate to int16, add and clamp (:42-59, :351-360). */
-template <int N>
-__device__ __forceinline__ void refcpu_row(ReconSmem &s, int i, int px0, int py0, unsigned mask,
-                                           const double *M, int16_t *res)
-{
-    double acc[N];
-#pragma unroll
-    for (int j = 0; j < N; j++) acc[j] = 0.0;
-    while (mask) {
-        const int k = __ffs(mask) - 1;
-        mask &= mask - 1;
-        double t = s.temp.d[(py0 + i) * kTempPitch + px0 + k];
-#pragma unroll
-        for (int j = 0; j < N; j++) acc[j] = __dadd_rn(acc[j], __dmul_rn(t, M[k * N + j]));
-    }
-#pragma unroll
-    for (int j = 0; j < N; j++) {
-        double v = acc[j];
-        int r = __double2int_rz(__dadd_rn(v, v >= 0.0 ? 0.5 : -0.5));
-        put_residual(s, 0, px0 + j, py0 + i, clampi(r, -32768, 32767), res);
     }
 }
 
@@ -1858,17 +1812,9 @@ __device__ __forceinline__ void item_pass1(ReconSmem &s, const BlkS &b, int item
     int j;
     TxRef t = locate_item(b, item, &j);
     if (t.coeff + (uint64_t)(t.n * t.n) > (uint64_t)job.num_coeffs) return;
-    if (A != CVP9_ARITH_REFCPU && (t.px0 + t.n > (t.plane ? 32 : 64) || t.py0 + t.n > (t.plane ? 32 : 64))) return;
+    if ((t.px0 + t.n > (t.plane ? 32 : 64) || t.py0 + t.n > (t.plane ? 32 : 64))) return;
     const int16_t *X = staged ? s.coef + (t.coeff - c_base) : job.coeffs + t.coeff;
-    if (A == CVP9_ARITH_REFCPU) {
-        const double *M = dct_basis(t.txl);
-        switch (t.txl) {
-        case 0: refcpu_col<4>(s, X, j, t.px0, t.py0, t.mask_idx, M); break;
-        case 1: refcpu_col<8>(s, X, j, t.px0, t.py0, t.mask_idx, M); break;
-        case 2: refcpu_col<16>(s, X, j, t.px0, t.py0, t.mask_idx, M); break;
-        default: refcpu_col<32>(s, X, j, t.px0, t.py0, t.mask_idx, M); break;
-        }
-    } else if (A == CVP9_ARITH_FULL) {
+    if (A == CVP9_ARITH_FULL) {
         /* FULL: rows first, item j = row j; intra luma by its mode's type */
         const int qdc = t.plane ? job.q_dc_uv : job.q_dc, qac = t.plane ? job.q_ac_uv : job.q_ac;
         const bool adst = full_tx_type(b, job, t) >= 2;
@@ -1899,15 +1845,7 @@ __device__ __forceinline__ void item_pass2(ReconSmem &s, const BlkS &b, int item
     unsigned mask = s.txmask[t.mask_idx];
     if (!mask) return;
     int16_t *res = (b.flags & 1) ? s.coef : nullptr;
-    if (A == CVP9_ARITH_REFCPU) {
-        const double *M = dct_basis(t.txl);
-        switch (t.txl) {
-        case 0: refcpu_row<4>(s, i, t.px0, t.py0, mask, M, res); break;
-        case 1: refcpu_row<8>(s, i, t.px0, t.py0, mask, M, res); break;
-        case 2: refcpu_row<16>(s, i, t.px0, t.py0, mask, M, res); break;
-        default: refcpu_row<32>(s, i, t.px0, t.py0, mask, M, res); break;
-        }
-    } else if (A == CVP9_ARITH_FULL) {
+    if (A == CVP9_ARITH_FULL) {
         /* item i = column i */
         const bool adst = full_tx_type(b, job, t) & 1;
         switch (t.txl) {
@@ -2099,7 +2037,7 @@ __device__ __forceinline__ void recon_inter(ReconSmem &s, const BlkS *one, int n
             return one ? chunk_params(*one, chk) : chunk_params(s.blk[b], chk - s.chunk_off[b]);
         };
         constexpr int kRound = 4;
-        uint8_t *wst = reinterpret_cast<uint8_t *>(s.temp.d) + warp * (kRound * kChunkStage);
+        uint8_t *wst = s.temp.mc + warp * (kRound * kChunkStage);
         const int q = lane >> 3, k = lane & 7;
         for (int base = warp; base < n; base += kRound * kWarps) {
             /* lane group q works on chunk base + q * kWarps */
@@ -2235,12 +2173,13 @@ __device__ __forceinline__ S &smem_as()
     return *reinterpret_cast<S *>(smem_raw);
 }
 
+template <int A>
 __device__ __forceinline__ IntraView<uint8_t> recon_view(ReconSmem &s)
 {
     IntraView<uint8_t> V;
     V.tile0 = &TY(s, 0, 0);
     V.col0 = s.col;
-    V.res = s.coef;
+    V.res = A == CVP9_ARITH_REFCPU ? s.temp.a.res : s.coef;
     return V;
 }
 
@@ -2296,16 +2235,175 @@ __device__ __noinline__ void phase_residual(int one, int n, bool staged, unsigne
     __syncthreads();
 }
 
+/* REFCPU: the residual of a TX, both passes at once, a warp for 32 / N TXs
+ * (N = 32: half the columns of one). Lane i of a TX owns its row i:
+ * for each column k with a nonzero coefficient it forms T[i][k] = sum over l
+ * of M[l][i] X[l][k] over the nonzero X[l][k], l ascending
+ * (vp9_reconstruct.c:31-40), and adds T[i][k] M[k][j] to its O[i][j], k
+ * ascending (:42-50) — the reference's operands, order and separate
+ * roundings; skipped zero terms add +-0 to a sum that is never -0. Then round
+ * half away from zero, saturate to int16, add and clamp (:51-59, :351-360),
+ * or leave it in the grid (an intra block's). What bounds it is the FP64 pipe
+ * and its latency; a thread per column and then per row, with the basis read
+ * from constant memory at addresses that differ from lane to lane, took 56 k
+ * cycles a superblock of mixed sizes, this 27 k. */
+struct RefTx {                       /* x: first coefficient; y: */
+    static constexpr uint32_t kIntra = 1u << 8, kNone = 1u << 9;   /* x / 4 | y / 4 << 4 | flags */
+};
+
+template <int N>
+__device__ __forceinline__ void ref_tx_unit(ReconSmem &s, int first, int count, int half, bool staged, unsigned c_base, int lane)
+{
+    constexpr int kCols = N == 32 ? 16 : N;
+    const int sub = lane / N, i = lane & (N - 1), j0 = half * kCols;
+    const bool on = sub < count;
+    const uint2 tx = s.tx[first + (on ? sub : 0)];
+    const int16_t *X = staged ? s.coef + (tx.x - c_base) : s.jc.coeffs + tx.x;
+    const double *M = g_dct + (N == 4 ? 0 : N == 8 ? 16 : N == 16 ? 80 : 336);
+    uint32_t nz = 0;                 /* this row's nonzero columns */
+    if (on && !(tx.y & RefTx::kNone)) {
+        const int16_t *row = X + i * N;
+        if (!((uintptr_t)row & (N == 4 ? 7 : 15))) {
+            uint32_t w[N / 2];
+            if (N == 4) {
+                const uint2 v = *reinterpret_cast<const uint2 *>(row);
+                w[0] = v.x;
+                w[1] = v.y;
+            } else {
+#pragma unroll
+                for (int k = 0; k < N / 8; k++) {
+                    const uint4 v = reinterpret_cast<const uint4 *>(row)[k];
+                    w[4 * k] = v.x;
+                    w[(4 * k + 1) % (N / 2)] = v.y;
+                    w[(4 * k + 2) % (N / 2)] = v.z;
+                    w[(4 * k + 3) % (N / 2)] = v.w;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < N / 2; k++)
+                nz |= ((w[k] & 0xffffu ? 1u : 0u) | (w[k] >> 16 ? 2u : 0u)) << (2 * k);
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; k++) nz |= (row[k] != 0 ? 1u : 0u) << k;
+        }
+    }
+    uint32_t cols = nz;              /* the TX's */
+#pragma unroll
+    for (int o = 1; o < N; o <<= 1) cols |= __shfl_xor_sync(0xffffffffu, cols, o);
+    const bool any = cols != 0;
+    double acc[kCols];
+#pragma unroll
+    for (int j = 0; j < kCols; j++) acc[j] = 0.0;
+    while (__any_sync(0xffffffffu, cols != 0)) {
+        const int k = cols ? __ffs(cols) - 1 : 0;
+        uint32_t rows = __ballot_sync(0xffffffffu, cols && ((nz >> k) & 1u));
+        if (N < 32) rows = (rows >> (sub * N)) & ((1u << (N & 31)) - 1u);
+        if (cols) {
+            double t = 0.0;
+            while (rows) {
+                const int l = __ffs(rows) - 1;
+                rows &= rows - 1;
+                t = __dadd_rn(t, __dmul_rn(__ldg(M + l * N + i), (double)X[l * N + k]));
+            }
+            const double2 *b = reinterpret_cast<const double2 *>(M + k * N + j0);
+#pragma unroll
+            for (int j = 0; j < kCols / 2; j++) {
+                const double2 m = __ldg(b + j);
+                acc[2 * j] = __dadd_rn(acc[2 * j], __dmul_rn(t, m.x));
+                acc[2 * j + 1] = __dadd_rn(acc[2 * j + 1], __dmul_rn(t, m.y));
+            }
+            cols &= cols - 1;
+        }
+    }
+    if (!any) return;
+    const int px = (int)(tx.y & 15u) * 4 + j0, py = (int)((tx.y >> 4) & 15u) * 4 + i;
+    const bool intra = tx.y & RefTx::kIntra;
+#pragma unroll
+    for (int j = 0; j < kCols; j += 4) {
+        int r[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const double v = acc[j + q];
+            r[q] = clampi(__double2int_rz(__dadd_rn(v, v >= 0.0 ? 0.5 : -0.5)), -32768, 32767);
+        }
+        if (intra) {
+            *reinterpret_cast<uint2 *>(&s.temp.a.res[py * 64 + px + j]) =
+                make_uint2((uint32_t)(r[0] & 0xffff) | (uint32_t)r[1] << 16, (uint32_t)(r[2] & 0xffff) | (uint32_t)r[3] << 16);
+        } else {
+            uint32_t *d = reinterpret_cast<uint32_t *>(&TY(s, px + j, py));
+            const uint32_t o = *d;
+            *d = (uint32_t)clampi((int)(o & 255u) + r[0], 0, 255) | (uint32_t)clampi((int)((o >> 8) & 255u) + r[1], 0, 255) << 8 |
+                 (uint32_t)clampi((int)((o >> 16) & 255u) + r[2], 0, 255) << 16 |
+                 (uint32_t)clampi((int)(o >> 24) + r[3], 0, 255) << 24;
+        }
+    }
+}
+
+/* REFCPU: every residual of blocks [lo, hi) of the SB. Barriers at both ends. */
+__device__ __noinline__ void phase_residual_ref(int lo, int hi, bool staged, unsigned c_base)
+{
+    ReconSmem &s = smem_as<ReconSmem>();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < 4) s.ntx[tid] = 0;
+    __syncthreads();
+    {
+        uint4 *z = reinterpret_cast<uint4 *>(s.temp.a.res);
+        for (int k = tid; k < kResidGrid / 8; k += kThreads) z[k] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    /* the TXs, largest first: count each size, then list them, a warp a block */
+    const bool in = tid >= lo && tid < hi && s.blk[tid].pnt[0];
+    int at = 0;
+    if (in) at = atomicAdd(&s.ntx[s.blk[tid].txl], (int)s.blk[tid].pnt[0]);
+    __syncthreads();
+    const int n32 = s.ntx[3], n16 = s.ntx[2], n8 = s.ntx[1], n4 = s.ntx[0];
+    if (n32 + n16 + n8 + n4 <= 256) {
+        if (in) {
+            const int c = s.blk[tid].txl;
+            s.chunk_off[tid] = (uint16_t)(at + (c < 3 ? n32 : 0) + (c < 2 ? n16 : 0) + (c < 1 ? n8 : 0));
+        }
+        __syncthreads();
+        for (int b = lo + warp; b < hi; b += kWarps) {
+            const BlkS &k = s.blk[b];
+            const int n = 4 << k.txl, nx = k.pnx[0];
+            for (int t = lane; t < k.pnt[0]; t += 32) {
+                const int ty = div_small(t, nx), tx = t - ty * nx;
+                const uint64_t co = (uint64_t)k.coeff + (uint64_t)t * (uint64_t)(n * n);
+                s.tx[s.chunk_off[b] + t] = make_uint2(
+                    (uint32_t)co, (uint32_t)((k.x + tx * n) >> 2) | (uint32_t)((k.y + ty * n) >> 2) << 4 |
+                                      (k.flags & 1 ? RefTx::kIntra : 0u) |
+                                      (co + (uint64_t)(n * n) > (uint64_t)s.jc.num_coeffs ? RefTx::kNone : 0u));
+            }
+        }
+        __syncthreads();
+        const int u16 = 2 * n32, u8 = u16 + ((n16 + 1) >> 1), u4 = u8 + ((n8 + 3) >> 2), end = u4 + ((n4 + 7) >> 3);
+        for (int u = warp; u < end; u += kWarps) {
+            if (u < u16) {
+                ref_tx_unit<32>(s, u >> 1, 1, u & 1, staged, c_base, lane);
+            } else if (u < u8) {
+                const int f = (u - u16) * 2;
+                ref_tx_unit<16>(s, n32 + f, min(2, n16 - f), 0, staged, c_base, lane);
+            } else if (u < u4) {
+                const int f = (u - u8) * 4;
+                ref_tx_unit<8>(s, n32 + n16 + f, min(4, n8 - f), 0, staged, c_base, lane);
+            } else {
+                const int f = (u - u4) * 8;
+                ref_tx_unit<4>(s, n32 + n16 + n8 + f, min(8, n4 - f), 0, staged, c_base, lane);
+            }
+        }
+    }
+    __syncthreads();
+}
+
 /* The intra tasks of the SB's nb blocks, their levels, the sorted quads. */
 template <int A>
 __device__ __noinline__ void phase_plan(int nb, int sbx, int sby)
 {
     ReconSmem &s = smem_as<ReconSmem>();
     const cvp9_job_t &job = s.jc;
-    IntraWork &W = s.temp.w;
+    IntraWork &W = s.temp.a.w;
     const int tid = threadIdx.x;
     const bool mine = tid < nb && (s.blk[tid].flags & 1);
-    intra_fill_cols(recon_view(s), tid, kThreads);
+    intra_fill_cols(recon_view<A>(s), tid, kThreads);
     int ntask;
     if (A == CVP9_ARITH_FULL) {
         const int at = cta_scan1(s, mine ? intra_tx_count(s.blk[tid], job, sbx, sby) : 0, &ntask);
@@ -2346,7 +2444,7 @@ template <int A>
 __device__ __noinline__ void phase_levels()
 {
     ReconSmem &s = smem_as<ReconSmem>();
-    intra_run<A, 255, uint8_t>(s.temp.w, recon_view(s), threadIdx.x, kThreads);
+    intra_run<A, 255, uint8_t>(s.temp.a.w, recon_view<A>(s), threadIdx.x, kThreads);
 }
 
 /* Intra block b on its own, its residual in the grid. */
@@ -2355,9 +2453,9 @@ __device__ __noinline__ void phase_ordered(int b, int sbx, int sby)
 {
     ReconSmem &s = smem_as<ReconSmem>();
     const cvp9_job_t &job = s.jc;
-    IntraWork &W = s.temp.w;
+    IntraWork &W = s.temp.a.w;
     const int tid = threadIdx.x;
-    const IntraView<uint8_t> V = recon_view(s);
+    const IntraView<uint8_t> V = recon_view<A>(s);
     intra_fill_cols(V, tid, kThreads);
     if (A == CVP9_ARITH_FULL) {
         const int n = min(intra_tx_count(s.blk[b], job, sbx, sby), kMaxTasks);
@@ -2397,7 +2495,7 @@ __device__ __noinline__ void phase_neighbours(unsigned need, int sb)
 {
     ReconSmem &s = smem_as<ReconSmem>();
     constexpr int fill_a = A == CVP9_ARITH_SPEC ? 128 : 127, fill_l = A == CVP9_ARITH_FULL ? 129 : fill_a;
-    wait_halo<ReconSmem, uint8_t>(s, recon_view(s), need, sb, A == CVP9_ARITH_FULL, fill_a, fill_l, threadIdx.x, kThreads);
+    wait_halo<ReconSmem, uint8_t>(s, recon_view<A>(s), need, sb, A == CVP9_ARITH_FULL, fill_a, fill_l, threadIdx.x, kThreads);
 }
 
 template <int A>
@@ -2499,13 +2597,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
                 const bool sub8 = g.width < 8 || g.height < 8;
                 const int ew = sub8 ? 8 : g.width, eh = sub8 ? 8 : g.height, n = 4 << g.tx_size;
                 const int m = min(n, 4 << max_tx_for(max(4, ew / 2), max(4, eh / 2)));
-                my_seq = (ew % n) || (eh % n) || (!sub8 && ((ew / 2) % m || (eh / 2) % m)) || (lx & 7) || (ly & 7);
+                my_seq = ((ew | eh) & (n - 1)) || (!sub8 && (((ew | eh) >> 1) & (m - 1))) || ((lx | ly) & 7);
             }
             residual_layout<A>(mb, job, g.x, g.y);
             s.blk[tid] = mb;
             my_intra = g.is_intra != 0;
             nch = my_intra ? 0 : block_chunks<A>(mb);
-            nit = block_items(mb);
+            nit = A == CVP9_ARITH_REFCPU ? 0 : block_items(mb);
         }
         if (__syncthreads_or(my_bad)) {
             /* leave the tile at 128 and flag the frame */
@@ -2602,7 +2700,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             const int n_chunks = min((int)s.chunk_off[nb], 256), n_items = min((int)s.item_off[nb], kMaxItems);
             if (n_chunks) phase_inter<A>(-1, n_chunks, sbx, sby);
             cp_async_wait_all();
-            phase_residual<A>(-1, n_items, staged, c_base, any_intra);
+            if (A == CVP9_ARITH_REFCPU) phase_residual_ref(0, nb, staged, c_base);
+            else phase_residual<A>(-1, n_items, staged, c_base, any_intra);
             if (any_intra) {
                 /* 4. the intra tasks and their levels; 5. the neighbours'
                  * samples, then level by level */
@@ -2619,7 +2718,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
                 const bool intra = s.blk[b].flags & 1;
                 if (!intra) phase_inter<A>(b, block_chunks<A>(s.blk[b]), sbx, sby);
                 for (int i = tid; i < 256 + 128; i += kThreads) s.txmask[i] = 0;
-                phase_residual<A>(b, block_items(s.blk[b]), false, 0u, true);
+                if (A == CVP9_ARITH_REFCPU) phase_residual_ref(b, b + 1, false, 0u);
+                else phase_residual<A>(b, block_items(s.blk[b]), false, 0u, true);
                 if (intra) phase_ordered<A>(b, sbx, sby);
             }
         }
@@ -2710,10 +2810,6 @@ struct __align__(16) FastSmem {                   /* one per warp; 16-byte vecto
         };
     };
 };
-
-/* The basis again in global memory: lane-varying reads are served by L1
- * instead of being serialised by the constant cache. */
-__device__ __align__(16) double g_dct[16 + 64 + 256 + 1024];
 
 static_assert(sizeof(FastSmem) % 16 == 0, "per-warp tiles must stay 16-byte aligned");
 static_assert(sizeof(FastSmem) * kFastWarps + 1024 <= 233472 / 5, "five CTAs of k_inter per SM");
@@ -5466,7 +5562,7 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
             /* TXs that do not tile their block, or whose chroma TXs straddle
              * 4x4 cells: list order */
             const int n = 4 << (g.tx_size & 3), m = min(n, 4 << max_tx_for(max(4, bw / 2), max(4, bh / 2)));
-            my_seq = (bw % n) || (bh % n) || (!sub8 && ((bw / 2) % m || (bh / 2) % m)) || (lx & 7) || (ly & 7);
+            my_seq = ((bw | bh) & (n - 1)) || (!sub8 && (((bw | bh) >> 1) & (m - 1))) || ((lx | ly) & 7);
         }
         if (__syncthreads_or(my_bad)) {
             if (tid == 0) atomicOr(job.status, (unsigned)CVP9_JOB_BAD_BLOCK);
