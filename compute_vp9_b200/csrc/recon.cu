@@ -47,7 +47,6 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxBlocks = 128;      /* blocks per SB (the tile parser emits at most 64) */
 constexpr int kCoefStage = 6144;     /* int16 coefficients staged per SB (64x64 luma + chroma) */
-constexpr int kMaxItems = 1536;      /* TX columns per SB: 4x4 TXs on all three planes */
 constexpr int kYPitch = 72;          /* luma tile row pitch; x = 0 at byte 4 */
 constexpr int kCPitch = 40;          /* chroma tile row pitch; x = 0 at byte 4 */
 constexpr int kTyBytes = (65 * kYPitch + 15) / 16 * 16;
@@ -357,9 +356,8 @@ struct BlkS {
     uint8_t  ymode, uvmode;
     uint8_t  ref0;
     uint8_t  ptxl[3];       /* residual TX log2-4 per plane                */
-    uint8_t  pnx[3];        /* residual TXs per row per plane              */
+    uint8_t  pnx[3], pny[3];    /* residual TXs per row and column, per plane */
     uint8_t  ref1;          /* FULL: second reference of a compound block  */
-    uint16_t pnt[3];        /* residual TX count per plane                 */
     int16_t  mvx, mvy;
     int16_t  mv1x, mv1y;    /* FULL: its MV                                */
     uint32_t coeff;
@@ -459,40 +457,34 @@ struct IntraView {
 
 struct ReconSmem {
     union {
-        uint8_t mc[kWarps * 4 * 608];            /* REFCPU: windows of the chunks in flight */
-        int32_t i[64 * 64 + 2 * 32 * 32];        /* SPEC, FULL: first-pass output */
-        struct {
-            IntraWork w;                         /* then the intra tasks        */
-            int16_t res[kResidGrid];             /* REFCPU: intra residuals     */
-        } a;
+        uint8_t   mc[kWarps * 4 * 608];          /* REFCPU: windows of the chunks in flight */
+        int32_t   tx[kWarps][32 * 32];           /* SPEC, FULL: a warp's TXs between the passes */
+        IntraWork w;                             /* then the intra tasks        */
     } temp;
     /* tiles, contiguous and 16-byte sized so they fill with vector stores */
     uint8_t  ty[kTyBytes];                       /* luma tile, row 0 = halo     */
     uint8_t  tu[kTcBytes];
     uint8_t  tv[kTcBytes];
-    int16_t  coef[kCoefStage];                   /* the SB's coefficient span; then
-                                                  * (SPEC, FULL) its intra blocks'
-                                                  * residuals                   */
+    int16_t  coef[kCoefStage];                   /* the SB's coefficient span   */
+    int16_t  res[kResidGrid];                    /* residuals of intra blocks   */
     cvp9_job_t jc;                               /* this ticket's job           */
     BlkS     blk[kMaxBlocks];
-    uint32_t txmask[256 + 64 + 64];              /* per-TX column-nonzero bits  */
-    uint16_t cell[256];                          /* owner block + 1 per 4x4     */
+    uint8_t  cell[256];                          /* owner block + 1 per 4x4     */
     uint32_t rows[16];                           /* claimed cells, a bit each   */
     uint16_t first[kMaxBlocks];                  /* FULL: a block's first task  */
     uint16_t chunk_off[kMaxBlocks + 1];          /* inter chunks before a block */
-    uint16_t item_off[kMaxBlocks + 1];           /* TX items before a block     */
+    uint16_t tx_at[3][kMaxBlocks];               /* first TX of a block's plane in tx */
     uint8_t  chunk_blk[256];                     /* chunk -> block              */
-    union {
-        uint8_t item_blk[kMaxItems];             /* TX column/row -> block      */
-        uint2   tx[256];                         /* REFCPU: the SB's TXs (RefTx) */
-    };
-    int      ntx[4];                             /* REFCPU: TXs of each size    */
+    uint2    tx[kMaxTasks];                      /* residual TXs by size (TxRef) */
+    int      ntx[4];                             /* TXs of each size            */
     uint8_t  col[16 * 64 + 2 * 16 * 32];         /* left-column copies (IntraView) */
     int      scan_tmp[2 * kWarps];
     unsigned c_lo, c_hi;                         /* coefficient span of the SB  */
     unsigned needs;                              /* intra_needs of its blocks   */
     int      ticket;
 };
+
+static_assert(sizeof(ReconSmem) <= 75 * 1024, "three CTAs per SM");
 
 __device__ __forceinline__ uint8_t &TY(ReconSmem &s, int x, int y) { return s.ty[(y + 1) * kYPitch + x + 4]; }
 __device__ __forceinline__ uint8_t &TC(ReconSmem &s, int p, int x, int y)
@@ -541,29 +533,24 @@ __device__ __forceinline__ void plane_layout(const B &b, const cvp9_job_t &job, 
 template <int A>
 __device__ __forceinline__ void residual_layout(BlkS &b, const cvp9_job_t &job, int gx, int gy)
 {
-    b.pnt[0] = b.pnt[1] = b.pnt[2] = 0;
     b.pnx[0] = b.pnx[1] = b.pnx[2] = 0;
+    b.pny[0] = b.pny[1] = b.pny[2] = 0;
     b.ptxl[0] = b.ptxl[1] = b.ptxl[2] = 0;
     if (b.flags & 2) return;
     if (A == CVP9_ARITH_REFCPU) {
         const int nx = b.cw >> (2 + b.txl), ny = b.ch >> (2 + b.txl);
         b.ptxl[0] = b.txl;
         b.pnx[0] = (uint8_t)nx;
-        b.pnt[0] = (uint16_t)(nx * ny);
+        b.pny[0] = (uint8_t)ny;
     } else {
         for (int p = 0; p < 3; p++) {
             int tx, nx, ny, pbw;
             plane_layout(b, job, gx, gy, p, tx, nx, ny, pbw);
             b.ptxl[p] = (uint8_t)tx;
             b.pnx[p] = (uint8_t)nx;
-            b.pnt[p] = (uint16_t)(nx * ny);
+            b.pny[p] = (uint8_t)ny;
         }
     }
-}
-
-__device__ __forceinline__ int block_items(const BlkS &b)
-{
-    return b.pnt[0] * (4 << b.ptxl[0]) + b.pnt[1] * (4 << b.ptxl[1]) + b.pnt[2] * (4 << b.ptxl[2]);
 }
 
 __device__ __forceinline__ int mc_chunks(int cw, int ch, int ccw, int cch);
@@ -789,14 +776,15 @@ __device__ __forceinline__ McRef mc_ref(const cvp9_ref_t &R, int p, int gx, int 
  * into the tile row `dst`. rows: the group's 15 rows of 8 samples in shared
  * memory, 16-byte aligned. A missing first reference predicts `mid`, a missing
  * second one leaves the single prediction. */
-template <class T, class B>
+template <class T, bool COMPOUND, class B>
 __device__ __forceinline__ void mc_chunk(const cvp9_job_t &job, const uint32_t (*P)[2], const B &b, bool on, int p, int gx,
                                          int gy, int w, int h, int mid, T *rows, T *dst, int k)
 {
     int v[8];
 #pragma unroll
     for (int c = 0; c < 8; c++) v[c] = mid;
-    for (int q = 0; q < 2; q++) {
+#pragma unroll 1
+    for (int q = 0; q < (COMPOUND ? 2 : 1); q++) {
         const int rf = on ? (q ? b.ref1 : b.ref0) : 0;
         if (q && !__any_sync(0xffffffffu, on && rf != 0)) break;
         const cvp9_ref_t &R = job.ref[job.ref_slot_of[clampi(rf - 1, 0, 2)] & 7];
@@ -1023,55 +1011,7 @@ __device__ __forceinline__ void refcpu_fill8(ReconSmem &s, int v, int lx0, int l
         for (int c = 0; c < clw; c++) TC(s, p, cx0 + c, cy0 + r) = (uint8_t)v;
 }
 
-/* ── Residual: one item = one TX column (pass 1) or one TX row (pass 2) ── */
-
-struct TxRef {
-    int plane, txl, n;
-    int px0, py0;      /* TX origin in the SB tile of its plane */
-    uint64_t coeff;    /* first coefficient of the TX            */
-    int mask_idx;
-};
-
-__device__ __forceinline__ TxRef locate_item(const BlkS &b, int item, int *lane_idx)
-{
-    TxRef t;
-    uint64_t off = b.coeff;
-    int p = 0;
-    for (; p < 2; p++) {
-        int cnt = b.pnt[p] * (4 << b.ptxl[p]);
-        if (item < cnt) break;
-        item -= cnt;
-        off += (uint64_t)b.pnt[p] * (uint64_t)(16 << (2 * b.ptxl[p]));
-    }
-    int txl = b.ptxl[p], n = 4 << txl;
-    int tx = item >> (2 + txl);
-    *lane_idx = item & (n - 1);
-    int nx = b.pnx[p];
-    int tx_y = nx == 1 ? tx : div_small(tx, nx), tx_x = tx - tx_y * nx;
-    t.plane = p;
-    t.txl = txl;
-    t.n = n;
-    int ox = p ? (b.x >> 1) : b.x, oy = p ? (b.y >> 1) : b.y;
-    t.px0 = ox + tx_x * n;
-    t.py0 = oy + tx_y * n;
-    t.coeff = off + (uint64_t)tx * (uint64_t)(n * n);
-    t.mask_idx = p == 0 ? (t.py0 >> 2) * 16 + (t.px0 >> 2)
-                        : 256 + (p - 1) * 64 + (t.py0 >> 2) * 8 + (t.px0 >> 2);
-    return t;
-}
-
-/* Residual of one sample: saturated to int16 (which no sum with a sample
- * notices) into the residual grid of an intra block, or added into the tile
- * of an inter block (res null). */
-__device__ __forceinline__ void put_residual(ReconSmem &s, int p, int x, int y, int r, int16_t *res)
-{
-    if (res) {
-        res[p == 0 ? y * 64 + x : 4096 + (p - 1) * 1024 + y * 32 + x] = (int16_t)clampi(r, -32768, 32767);
-    } else {
-        uint8_t &px = p == 0 ? TY(s, x, y) : TC(s, p, x, y);
-        px = (uint8_t)clampi((int)px + r, 0, 255);
-    }
-}
+/* ── Residual ──────────────────────────────────────────────────────────── */
 
 template <class T>
 __device__ __forceinline__ void idct_n(T *x, int n)
@@ -1080,51 +1020,6 @@ __device__ __forceinline__ void idct_n(T *x, int n)
     else if (n == 8) idct8(x);
     else if (n == 16) idct16(x);
     else idct32(x);
-}
-
-__device__ __forceinline__ int32_t *spec_temp(ReconSmem &s, int plane, int x, int y)
-{
-    if (plane == 0) return &s.temp.i[y * 64 + x];
-    return &s.temp.i[4096 + (plane - 1) * 1024 + y * 32 + x];
-}
-
-/* SPEC pass 1: dequantise column j (DC step at [0][0] only) and run the
- * 1-D transform down the column (vp9_idct.comp.glsl:666-679). */
-template <int N>
-__device__ __forceinline__ void spec_col(ReconSmem &s, const int16_t *X, int j,
-                                         const TxRef &t, int q_dc, int q_ac)
-{
-    wi v[N];
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        int c = X[k * N + j];
-        any |= c != 0;
-        v[k] = wi(c) * ((k == 0 && j == 0) ? q_dc : q_ac);
-    }
-    if (any) {
-        idct_n(v, N);
-        atomicOr(&s.txmask[t.mask_idx], 1u);
-    }
-#pragma unroll
-    for (int k = 0; k < N; k++) *spec_temp(s, t.plane, t.px0 + j, t.py0 + k) = any ? v[k].v : 0;
-}
-
-/* SPEC pass 2: row transform, final rounding shift 4/5/6/6, add and clamp;
- * samples outside the frame are left alone (tile write-back clips them). */
-template <int N>
-__device__ __forceinline__ void spec_row(ReconSmem &s, int i, const TxRef &t, int16_t *res)
-{
-    wi v[N];
-#pragma unroll
-    for (int k = 0; k < N; k++) v[k] = wi(*spec_temp(s, t.plane, t.px0 + k, t.py0 + i));
-    idct_n(v, N);
-    const int sh = N == 4 ? 4 : (N == 8 ? 5 : 6);
-#pragma unroll
-    for (int j = 0; j < N; j++) {
-        int r = ((int)((unsigned)v[j].v + (1u << (sh - 1)))) >> sh;
-        put_residual(s, t.plane, t.px0 + j, t.py0 + i, r, res);
-    }
 }
 
 /* ── FULL profile: ADST and WHT, rows-then-columns residual, per-TX intra ── */
@@ -1257,52 +1152,6 @@ __device__ __forceinline__ void itx1(T *v, bool adst)
     else if (N == 8 && adst) iadst8(v);
     else if (N == 16 && adst) iadst16(v);
     else idct_n(v, N);
-}
-
-/* FULL pass 1 on TX row i: dequantise (the plane's steps, DC at [0][0];
- * 32x32 values halved toward zero) and transform along the row (DCT, or
- * ADST when row_adst; WHT when lossless) into the temp rows. Returns
- * whether the row had a nonzero coefficient. */
-template <int N>
-__device__ __forceinline__ bool full_row(ReconSmem &s, const int16_t *X, int i, int plane, int px0, int py0,
-                                         int qdc, int qac, bool lossless, bool row_adst)
-{
-    wi v[N];
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        int c = X[i * N + k];
-        any |= c != 0;
-        int d = c * ((i == 0 && k == 0) ? qdc : qac);
-        v[k] = wi(N == 32 ? d / 2 : d);
-    }
-    if (any) {
-        if (N == 4 && lossless) iwht4(v, true);
-        else itx1<N>(v, row_adst);
-    }
-#pragma unroll
-    for (int k = 0; k < N; k++) *spec_temp(s, plane, px0 + k, py0 + i) = any ? v[k].v : 0;
-    return any;
-}
-
-/* FULL pass 2 on TX column j: transform down the column, final rounding
- * shift 4/5/6/6 (none after the WHT), add and clamp into the tile. */
-template <int N>
-__device__ __forceinline__ void full_col(ReconSmem &s, int j, int plane, int px0, int py0, bool lossless,
-                                         bool col_adst, int16_t *res)
-{
-    wi v[N];
-#pragma unroll
-    for (int k = 0; k < N; k++) v[k] = wi(*spec_temp(s, plane, px0 + j, py0 + k));
-    const bool wht = N == 4 && lossless;
-    if (wht) iwht4(v, false);
-    else itx1<N>(v, col_adst);
-    const int sh = N == 4 ? 4 : (N == 8 ? 5 : 6);
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        int r = wht ? v[k].v : ((int)((unsigned)v[k].v + (1u << (sh - 1)))) >> sh;
-        put_residual(s, plane, px0 + j, py0 + k, r, res);
-    }
 }
 
 /* First MI column of the tile column holding mi_col (VP9 tile offsets). */
@@ -1604,8 +1453,8 @@ __device__ __forceinline__ void intra_tx_levels(IntraWork &W, int ntask, int tid
  * task from the owner map of the cells: W.own of each plane's (FULL), or the
  * block map `cell` of the luma ones, whose chroma groups start at even
  * samples. */
-template <int A>
-__device__ __forceinline__ void intra_sort(IntraWork &W, const uint16_t *cell, int ntask, int tid, int nthreads)
+template <int A, class C>
+__device__ __forceinline__ void intra_sort(IntraWork &W, const C *cell, int ntask, int tid, int nthreads)
 {
     const int lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i <= kMaxTasks; i += nthreads) W.lvlq[i] = 0;
@@ -1767,6 +1616,19 @@ __device__ __forceinline__ void intra_halo(const IntraView<T> &V, const cvp9_job
     }
 }
 
+/* f(i, k) for k < count of each of the warp's lanes (i: the lane's own number
+ * or the lane in turn): up to four by the lane itself, more by the whole warp. */
+template <class F>
+__device__ __forceinline__ void warp_spread(int count, int lane, F f)
+{
+    if (count <= 4)
+        for (int k = 0; k < count; k++) f(lane, k);
+    for (uint32_t m = __ballot_sync(0xffffffffu, count > 4); m; m &= m - 1) {
+        const int from = __ffs(m) - 1, n = __shfl_sync(0xffffffffu, count, from);
+        for (int k = lane; k < n; k += 32) f(from, k);
+    }
+}
+
 /* Claim the 4x4 cells of columns [c0x, c1x] and rows [c0y, c1y] for a block:
  * a bit per cell, a word per row of the SB; true when another block has one
  * of them. (A thread a block: a 64x64 block is 16 atomics.) */
@@ -1778,14 +1640,12 @@ __device__ __forceinline__ bool claim_cells(uint32_t *rows, int c0x, int c1x, in
     return (seen & m) != 0;
 }
 
-/* The owner map of those cells: block + 1, one warp. */
-__device__ __forceinline__ void own_cells(uint16_t *cell, int b, int c0x, int c1x, int c0y, int c1y, int lane)
+/* Cell k of a block's, in its owner map. */
+template <class C>
+__device__ __forceinline__ void own_cell(C *cell, int b, int c0x, int c1x, int c0y, int k)
 {
-    const int w = c1x - c0x + 1, n = w * (c1y - c0y + 1);
-    for (int k = lane; k < n; k += 32) {
-        const int r = div_small(k, w);
-        cell[(c0y + r) * 16 + c0x + k - r * w] = (uint16_t)(b + 1);
-    }
+    const int w = c1x - c0x + 1, r = div_small(k, w);
+    cell[(c0y + r) * 16 + c0x + k - r * w] = (C)(b + 1);
 }
 
 /* Which neighbours (1 left, 2 above, 4 above-left) the intra blocks of a
@@ -1794,74 +1654,6 @@ __device__ __forceinline__ void own_cells(uint16_t *cell, int b, int c0x, int c1
 __device__ __forceinline__ unsigned intra_needs(int x, int y)
 {
     return (x == 0 ? 1u : 0u) | (y == 0 ? 2u : 0u) | (x == 0 && y == 0 ? 4u : 0u);
-}
-
-/* The two transform passes of one residual item (a TX column, then a TX
- * row; FULL: a row, then a column) of block b, item index `item` inside the
- * block. Pass 1 reads the coefficients (staged span or global), pass 2 adds
- * the residual into the tile, or leaves it in `res` for an intra block. */
-__device__ __forceinline__ int full_tx_type(const BlkS &b, const cvp9_job_t &job, const TxRef &t)
-{
-    return ((b.flags & 1) && t.plane == 0 && !job.lossless && t.txl < 3 && b.ymode < 10) ? c_tx_type[b.ymode] : 0;
-}
-
-template <int A>
-__device__ __forceinline__ void item_pass1(ReconSmem &s, const BlkS &b, int item, bool staged, unsigned c_base)
-{
-    const cvp9_job_t &job = s.jc;
-    int j;
-    TxRef t = locate_item(b, item, &j);
-    if (t.coeff + (uint64_t)(t.n * t.n) > (uint64_t)job.num_coeffs) return;
-    if ((t.px0 + t.n > (t.plane ? 32 : 64) || t.py0 + t.n > (t.plane ? 32 : 64))) return;
-    const int16_t *X = staged ? s.coef + (t.coeff - c_base) : job.coeffs + t.coeff;
-    if (A == CVP9_ARITH_FULL) {
-        /* FULL: rows first, item j = row j; intra luma by its mode's type */
-        const int qdc = t.plane ? job.q_dc_uv : job.q_dc, qac = t.plane ? job.q_ac_uv : job.q_ac;
-        const bool adst = full_tx_type(b, job, t) >= 2;
-        bool any;
-        switch (t.txl) {
-        case 0: any = full_row<4>(s, X, j, t.plane, t.px0, t.py0, qdc, qac, job.lossless, adst); break;
-        case 1: any = full_row<8>(s, X, j, t.plane, t.px0, t.py0, qdc, qac, job.lossless, adst); break;
-        case 2: any = full_row<16>(s, X, j, t.plane, t.px0, t.py0, qdc, qac, job.lossless, adst); break;
-        default: any = full_row<32>(s, X, j, t.plane, t.px0, t.py0, qdc, qac, job.lossless, false); break;
-        }
-        if (any) atomicOr(&s.txmask[t.mask_idx], 1u);
-    } else {
-        switch (t.txl) {
-        case 0: spec_col<4>(s, X, j, t, job.q_dc, job.q_ac); break;
-        case 1: spec_col<8>(s, X, j, t, job.q_dc, job.q_ac); break;
-        case 2: spec_col<16>(s, X, j, t, job.q_dc, job.q_ac); break;
-        default: spec_col<32>(s, X, j, t, job.q_dc, job.q_ac); break;
-        }
-    }
-}
-
-template <int A>
-__device__ __forceinline__ void item_pass2(ReconSmem &s, const BlkS &b, int item)
-{
-    const cvp9_job_t &job = s.jc;
-    int i;
-    TxRef t = locate_item(b, item, &i);
-    unsigned mask = s.txmask[t.mask_idx];
-    if (!mask) return;
-    int16_t *res = (b.flags & 1) ? s.coef : nullptr;
-    if (A == CVP9_ARITH_FULL) {
-        /* item i = column i */
-        const bool adst = full_tx_type(b, job, t) & 1;
-        switch (t.txl) {
-        case 0: full_col<4>(s, i, t.plane, t.px0, t.py0, job.lossless, adst, res); break;
-        case 1: full_col<8>(s, i, t.plane, t.px0, t.py0, job.lossless, adst, res); break;
-        case 2: full_col<16>(s, i, t.plane, t.px0, t.py0, job.lossless, adst, res); break;
-        default: full_col<32>(s, i, t.plane, t.px0, t.py0, job.lossless, false, res); break;
-        }
-    } else {
-        switch (t.txl) {
-        case 0: spec_row<4>(s, i, t, res); break;
-        case 1: spec_row<8>(s, i, t, res); break;
-        case 2: spec_row<16>(s, i, t, res); break;
-        default: spec_row<32>(s, i, t, res); break;
-        }
-    }
 }
 
 /* ── Synchronisation helpers ────────────────────────────────────────────── */
@@ -1886,59 +1678,6 @@ __device__ __forceinline__ bool wait_flag(const unsigned *flag, unsigned epoch)
         __nanosleep(it < 64 ? 32 : 256);
     }
     return false;
-}
-
-__device__ __forceinline__ void pf_l2(const void *p)
-{
-    asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
-}
-
-/* Prefetch into L2 the rows of a reference window (clamped like the
- * prediction reads) — first and last 128-byte line of each row. */
-__device__ __forceinline__ void pf_window(const uint8_t *plane, int stride, int pw, int ph,
-                                          int x0, int y0, int w, int h, int lane)
-{
-    int xm = pw > 0 ? pw - 1 : 0, ym = ph > 0 ? ph - 1 : 0;
-    int xa = clampi(x0, 0, xm), xb = clampi(x0 + w - 1, 0, xm);
-    for (int r = lane; r < h; r += 32) {
-        const uint8_t *row = plane + (size_t)clampi(y0 + r, 0, ym) * stride;
-        pf_l2(row + xa);
-        if ((xb >> 7) != (xa >> 7)) pf_l2(row + xb);
-    }
-}
-
-/* One warp per block, right after the descriptors are read: pull the
- * block's reference windows towards L2 so the prediction phase finds them
- * there. Addresses are clamped into the buffers exactly as the later reads
- * are. */
-template <int A>
-__device__ void prefetch_block(const BlkS &b, const cvp9_job_t &job, int sbx, int sby, int lane)
-{
-    if (b.flags & 1) return;
-    const cvp9_ref_t *R;
-    if (A == CVP9_ARITH_REFCPU) {
-        int slot = (int)b.ref0 - 1;
-        R = (slot >= 0 && slot < 8) ? &job.ref[slot] : nullptr;
-    } else {
-        R = &job.ref[job.ref_slot_of[clampi((int)b.ref0 - 1, 0, 2)] & 7];
-    }
-    if (!R || !R->plane) return;
-    const int rw = R->w, rh = R->h, rcs = (rw + 1) >> 1;
-    const uint8_t *ru = R->plane + (size_t)rw * rh;
-    const uint8_t *rv = ru + (size_t)rcs * ((rh + 1) >> 1);
-    const int gx = sbx + b.x, gy = sby + b.y, cbw = (b.cw + 1) >> 1, cbh = (b.ch + 1) >> 1;
-    if (A == CVP9_ARITH_REFCPU) {
-        int px8 = gx * 8 + b.mvx, py8 = gy * 8 + b.mvy;
-        pf_window(R->plane, rw, rw, rh, px8 >> 3, py8 >> 3, b.cw + 1, b.ch + 1, lane);
-        int cx8 = (gx >> 1) * 8 + b.mvx / 2, cy8 = (gy >> 1) * 8 + b.mvy / 2;
-        pf_window(ru, rcs, rw >> 1, rh >> 1, cx8 >> 3, cy8 >> 3, cbw + 1, cbh + 1, lane);
-        pf_window(rv, rcs, rw >> 1, rh >> 1, cx8 >> 3, cy8 >> 3, cbw + 1, cbh + 1, lane);
-    } else {
-        pf_window(R->plane, rw, rw, rh, gx + (b.mvx >> 3) - 3, gy + (b.mvy >> 3) - 3, b.cw + 7, b.ch + 7, lane);
-        int cx = (gx >> 1) + (b.mvx >> 4) - 3, cy = (gy >> 1) + (b.mvy >> 4) - 3;
-        pf_window(ru, rcs, rcs, (rh + 1) >> 1, cx, cy, cbw + 7, cbh + 7, lane);
-        pf_window(rv, rcs, rcs, (rh + 1) >> 1, cx, cy, cbw + 7, cbh + 7, lane);
-    }
 }
 
 /* Exclusive prefix sums of two per-thread counts over the CTA (thread order).
@@ -2068,7 +1807,7 @@ __device__ __forceinline__ void recon_inter(ReconSmem &s, const BlkS *one, int n
         const cvp9_job_t &job = s.jc;
         const uint32_t (*P)[2] = A == CVP9_ARITH_FULL ? c_subpel4_pk[job.interp_filter & 3] : c_subpel_pk;
         const int g = lane >> 3, k = lane & 7;
-        uint8_t *rows = reinterpret_cast<uint8_t *>(s.temp.i) + (warp * 4 + g) * 128;
+        uint8_t *rows = s.temp.mc + (warp * 4 + g) * 128;
         for (int base = warp * 4; base < n; base += 4 * kWarps) {
             const int chk = base + g;
             const bool on = chk < n;
@@ -2079,7 +1818,7 @@ __device__ __forceinline__ void recon_inter(ReconSmem &s, const BlkS *one, int n
             if (on) mc_chunk_at(one ? chk : chk - s.chunk_off[bi], b.cw, b.ch, ccw, cch, p, x, y, w, h);
             const int lx = (p ? b.x >> 1 : b.x) + x, ly = (p ? b.y >> 1 : b.y) + y;
             uint8_t *dst = p == 0 ? &TY(s, lx, ly + k) : &TC(s, p, lx, ly + k);
-            mc_chunk<uint8_t>(job, P, b, on, p, (p ? sbx >> 1 : sbx) + lx, (p ? sby >> 1 : sby) + ly, w, h, 128, rows,
+            mc_chunk<uint8_t, A == CVP9_ARITH_FULL>(job, P, b, on, p, (p ? sbx >> 1 : sbx) + lx, (p ? sby >> 1 : sby) + ly, w, h, 128, rows,
                               dst, k);
         }
     }
@@ -2173,13 +1912,12 @@ __device__ __forceinline__ S &smem_as()
     return *reinterpret_cast<S *>(smem_raw);
 }
 
-template <int A>
 __device__ __forceinline__ IntraView<uint8_t> recon_view(ReconSmem &s)
 {
     IntraView<uint8_t> V;
     V.tile0 = &TY(s, 0, 0);
     V.col0 = s.col;
-    V.res = A == CVP9_ARITH_REFCPU ? s.temp.a.res : s.coef;
+    V.res = s.res;
     return V;
 }
 
@@ -2209,29 +1947,277 @@ __device__ __noinline__ void phase_inter(int one, int n, int sbx, int sby)
     recon_inter<A>(s, one < 0 ? nullptr : &s.blk[one], n, sbx, sby, threadIdx.x >> 5, threadIdx.x & 31);
 }
 
-/* Both transform passes of n items of the whole SB (one < 0), or of block
- * `one`; zero: clear the residual grid (the coefficient staging, spent after
- * the first pass) in between. Barriers at both ends. */
+/* The residual TXs of a superblock, sorted by size, largest first. What
+ * bounds them is the length of a transform on one thread and how evenly
+ * threads are busy, so a warp takes 32 / N TXs of N x N at a time, a lane a row
+ * and then a column of one, with warp barriers only: no warp mixes sizes, no
+ * CTA barrier waits for the longest. The rows pass through 4 KB a warp, laid
+ * out in 16-byte chunks that are permuted within 128 bytes (tx_word), so that
+ * rows and columns both go through all banks. (A thread per row and column
+ * over all sizes, CTA barriers between the passes, rows 256 bytes apart: 24 k
+ * cycles a superblock of FULL inter blocks, 48 k at 10 bits; this 21 k and
+ * 33 k, 5 k of it the list.) */
+template <int N> struct std_int { static constexpr int value = N; };
+
+struct TxRef {       /* x: first coefficient; y: x / 4 | y / 4 << 4 | plane << 8 | TX type << 10 | flags */
+    static constexpr uint32_t kIntra = 1u << 12, kNone = 1u << 13;
+};
+
+/* Place of word e in a permuted buffer. */
+__device__ __forceinline__ int tx_word(int e)
+{
+    const int a = e >> 2;
+    return ((a ^ ((a >> 3) & 7)) << 2) | (e & 3);
+}
+
+/* List the TXs of blocks [lo, hi), whole CTA: W.tx sorted by size, W.ntx their
+ * numbers. layout(b, p, txl, nx, ny): plane p's TXs of block b (0 for a
+ * skipped one); type(b, p, txl): the TX type. Barriers inside and at the end. */
+template <class S, class L, class Y>
+__device__ __forceinline__ void list_txs(S &s, int lo, int hi, int nb, uint32_t num_coeffs, int tid, int nthreads, L layout,
+                                         Y type)
+{
+    const int lane = tid & 31, warp = tid >> 5, nwarps = nthreads >> 5, cnt = min(hi, nb) - lo;
+    if (tid < 4) s.ntx[tid] = 0;
+    __syncthreads();
+    /* a thread a block and plane: its TXs' place among those of their size */
+    for (int t = tid; t < 3 * cnt; t += nthreads) {
+        const int p = t >= 2 * cnt ? 2 : (t >= cnt ? 1 : 0), b = lo + t - p * cnt;
+        int txl, nx, ny;
+        layout(s.blk[b], p, txl, nx, ny);
+        s.tx_at[p][b] = nx * ny ? (uint16_t)atomicAdd(&s.ntx[txl], nx * ny) : (uint16_t)0;
+    }
+    __syncthreads();
+    const int n32 = s.ntx[3], n16 = s.ntx[2], n8 = s.ntx[1];
+    for (int t0 = 0; t0 < 3 * cnt; t0 += nthreads) {
+        auto of = [&](int i) { return t0 + i * nwarps + warp; };     /* dealt over the warps */
+        auto pair = [&](int t, int &p, int &b) {
+            p = t >= 2 * cnt ? 2 : (t >= cnt ? 1 : 0);
+            b = lo + t - p * cnt;
+        };
+        int count = 0;
+        if (of(lane) < 3 * cnt) {
+            int p, b, txl, nx, ny;
+            pair(of(lane), p, b);
+            layout(s.blk[b], p, txl, nx, ny);
+            count = nx * ny;
+        }
+        warp_spread(count, lane, [&](int i, int k) {
+            int p, b, txl, nx, ny;
+            pair(of(i), p, b);
+            const auto &m = s.blk[b];
+            uint64_t off = m.coeff;
+            for (int q = 0; q < p; q++) {
+                layout(m, q, txl, nx, ny);
+                off += (uint64_t)(nx * ny) << (4 + 2 * txl);
+            }
+            layout(m, p, txl, nx, ny);
+            const int n = 4 << txl, tile = p ? 32 : 64, ty = div_small(k, nx);
+            const int x = (p ? m.x >> 1 : m.x) + (k - ty * nx) * n, y = (p ? m.y >> 1 : m.y) + ty * n;
+            const int to = s.tx_at[p][b] + k + (txl < 3 ? n32 : 0) + (txl < 2 ? n16 : 0) + (txl < 1 ? n8 : 0);
+            const uint64_t co = off + ((uint64_t)k << (4 + 2 * txl));
+            const bool none = co + (uint64_t)(n * n) > (uint64_t)num_coeffs || x + n > tile || y + n > tile;
+            if (to < kMaxTasks)
+                s.tx[to] = make_uint2((uint32_t)co, (uint32_t)(x >> 2) | (uint32_t)(y >> 2) << 4 | (uint32_t)p << 8 |
+                                                        (uint32_t)type(m, p, txl) << 10 |
+                                                        (m.flags & 1 ? TxRef::kIntra : 0u) | (none ? TxRef::kNone : 0u));
+        });
+    }
+    __syncthreads();
+}
+
+/* Deal the listed TXs to the warps: unit(N, first, count, part) for 32 / N TXs
+ * of size N; N = 32 in `parts` parts each. */
+template <class F>
+__device__ __forceinline__ void deal_txs(const int *ntx, int parts, int warp, int nwarps, F unit)
+{
+    const int n32 = ntx[3], n16 = ntx[2], n8 = ntx[1], n4 = ntx[0];
+    const int u16 = parts * n32, u8 = u16 + ((n16 + 1) >> 1), u4 = u8 + ((n8 + 3) >> 2), end = u4 + ((n4 + 7) >> 3);
+    if (n32 + n16 + n8 + n4 > kMaxTasks) return;
+    for (int u = warp; u < end; u += nwarps) {
+        if (u < u16) {
+            unit(std_int<32>(), u / parts, 1, u % parts);
+        } else if (u < u8) {
+            const int f = (u - u16) * 2;
+            unit(std_int<16>(), n32 + f, min(2, n16 - f), 0);
+        } else if (u < u4) {
+            const int f = (u - u8) * 4;
+            unit(std_int<8>(), n32 + n16 + f, min(4, n8 - f), 0);
+        } else {
+            const int f = (u - u4) * 8;
+            unit(std_int<4>(), n32 + n16 + n8 + f, min(8, n4 - f), 0);
+        }
+    }
+}
+
+/* N coefficients of a row, as ints: 16-byte loads where they are aligned. */
+template <int N>
+__device__ __forceinline__ void row_coeffs(int (&c)[N], const int16_t *row)
+{
+    if (!((uintptr_t)row & (N == 4 ? 7 : 15))) {
+#pragma unroll
+        for (int k = 0; k < N; k += (N == 4 ? 4 : 8)) {
+            uint32_t w[4] = { 0, 0, 0, 0 };
+            if (N == 4) {
+                const uint2 v = *reinterpret_cast<const uint2 *>(row);
+                w[0] = v.x;
+                w[1] = v.y;
+            } else {
+                const uint4 v = *reinterpret_cast<const uint4 *>(row + k);
+                w[0] = v.x;
+                w[1] = v.y;
+                w[2] = v.z;
+                w[3] = v.w;
+            }
+#pragma unroll
+            for (int q = 0; q < (N == 4 ? 2 : 4); q++) {
+                c[k + 2 * q] = (int16_t)(w[q] & 0xffffu);
+                c[k + 2 * q + 1] = (int)w[q] >> 16;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) c[k] = row[k];
+    }
+}
+
+/* Four residuals, each within int16, of a row of an intra block into the
+ * grid, of an inter block onto its samples (x a multiple of 4). */
+__device__ __forceinline__ void put_residual4(ReconSmem &s, int p, int x, int y, const int (&r)[4], bool intra)
+{
+    if (intra) {
+        *reinterpret_cast<uint2 *>(&s.res[plane_at(p, x, y)]) =
+            make_uint2((uint32_t)(r[0] & 0xffff) | (uint32_t)r[1] << 16, (uint32_t)(r[2] & 0xffff) | (uint32_t)r[3] << 16);
+    } else {
+        uint32_t *d = reinterpret_cast<uint32_t *>(p == 0 ? &TY(s, x, y) : &TC(s, p, x, y));
+        const uint32_t o = *d;
+        *d = (uint32_t)clampi((int)(o & 255u) + r[0], 0, 255) | (uint32_t)clampi((int)((o >> 8) & 255u) + r[1], 0, 255) << 8 |
+             (uint32_t)clampi((int)((o >> 16) & 255u) + r[2], 0, 255) << 16 |
+             (uint32_t)clampi((int)(o >> 24) + r[3], 0, 255) << 24;
+    }
+}
+
+/* SPEC and FULL: 32 / N TXs by a warp. SPEC (vp9_idct.comp.glsl:666-789):
+ * dequantise (DC step at [0][0] only), columns, then rows; FULL: dequantise
+ * with the plane's steps (32x32 halved toward zero), rows, then columns, ADST
+ * by the TX type, WHT when lossless. Then the rounding shift 4/5/6/6 (none
+ * after the WHT); added to an inter block's samples, left in the grid, saturated
+ * to int16 (which no sum with a sample notices), for an intra one. */
+template <int A, int N>
+__device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, int count, bool staged, unsigned c_base, int lane)
+{
+    const cvp9_job_t &job = s.jc;
+    const int sub = lane / N, i = lane & (N - 1);
+    const bool on = sub < count;
+    const uint2 tx = s.tx[first + (on ? sub : 0)];
+    const int p = (int)(tx.y >> 8) & 3, type = (int)(tx.y >> 10) & 3;
+    const bool go = on && !(tx.y & TxRef::kNone);
+    const int16_t *X = staged ? s.coef + (tx.x - c_base) : job.coeffs + tx.x;
+    wi v[N];
+    bool any = false;
+    if (go) {
+        if (A == CVP9_ARITH_FULL) {
+            const int qdc = p ? job.q_dc_uv : job.q_dc, qac = p ? job.q_ac_uv : job.q_ac;
+            int c[N];
+            row_coeffs<N>(c, X + i * N);
+#pragma unroll
+            for (int k = 0; k < N; k++) {
+                any |= c[k] != 0;
+                const int d = c[k] * (i == 0 && k == 0 ? qdc : qac);
+                v[k] = wi(N == 32 ? d / 2 : d);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; k++) {
+                const int c = X[k * N + i];
+                any |= c != 0;
+                v[k] = wi(c) * (k == 0 && i == 0 ? job.q_dc : job.q_ac);
+            }
+        }
+    }
+    const uint32_t live = __ballot_sync(0xffffffffu, any);
+    if (!live) return;
+    const bool mine = N == 32 || ((live >> (sub * N)) & ((1u << (N & 31)) - 1u));
+    const bool wht = A == CVP9_ARITH_FULL && N == 4 && job.lossless;
+    if (mine) {
+        if (any) {
+            if (wht) iwht4(v, true);
+            else if (A == CVP9_ARITH_FULL) itx1<N>(v, type >= 2);
+            else idct_n(v, N);
+        }
+        if (A == CVP9_ARITH_FULL) {
+#pragma unroll
+            for (int k = 0; k < N; k += 4)
+                *reinterpret_cast<int4 *>(&buf[tx_word(lane * N + k)]) =
+                    any ? make_int4(v[k].v, v[k + 1].v, v[k + 2].v, v[k + 3].v) : make_int4(0, 0, 0, 0);
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; k++) buf[tx_word(sub * N * N + k * N + i)] = any ? v[k].v : 0;
+        }
+    }
+    __syncwarp();
+    if (mine) {
+        const int x = (int)(tx.y & 15u) * 4, y = (int)((tx.y >> 4) & 15u) * 4;
+        const bool intra = tx.y & TxRef::kIntra;
+        const int sh = N == 4 ? 4 : (N == 8 ? 5 : 6);
+        if (A == CVP9_ARITH_FULL) {
+#pragma unroll
+            for (int k = 0; k < N; k++) v[k] = wi(buf[tx_word(sub * N * N + k * N + i)]);
+            if (wht) iwht4(v, false);
+            else itx1<N>(v, type & 1);
+            uint8_t *d = p == 0 ? &TY(s, x + i, y) : &TC(s, p, x + i, y);
+            int16_t *r = s.res + plane_at(p, x + i, y);
+            const int dp = p ? kCPitch : kYPitch, rp = p ? 32 : 64;
+#pragma unroll
+            for (int k = 0; k < N; k++) {
+                const int q = wht ? v[k].v : ((int)((unsigned)v[k].v + (1u << (sh - 1)))) >> sh;
+                if (intra) r[k * rp] = (int16_t)clampi(q, -32768, 32767);
+                else d[k * dp] = (uint8_t)clampi((int)d[k * dp] + q, 0, 255);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; k += 4) {
+                const int4 w = *reinterpret_cast<const int4 *>(&buf[tx_word(lane * N + k)]);
+                v[k] = wi(w.x);
+                v[k + 1] = wi(w.y);
+                v[k + 2] = wi(w.z);
+                v[k + 3] = wi(w.w);
+            }
+            idct_n(v, N);
+#pragma unroll
+            for (int k = 0; k < N; k += 4) {
+                int q[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    q[j] = clampi(((int)((unsigned)v[k + j].v + (1u << (sh - 1)))) >> sh, -32768, 32767);
+                put_residual4(s, p, x + k, y + i, q, intra);
+            }
+        }
+    }
+    __syncwarp();
+}
+
+/* SPEC and FULL: every residual of blocks [lo, hi) of the SB. Barriers at both ends. */
 template <int A>
-__device__ __noinline__ void phase_residual(int one, int n, bool staged, unsigned c_base, bool zero)
+__device__ __noinline__ void phase_residual(int lo, int hi, bool staged, unsigned c_base, int sbx, int sby)
 {
     ReconSmem &s = smem_as<ReconSmem>();
-    const int tid = threadIdx.x;
-    __syncthreads();
-    for (int it = tid; it < n; it += kThreads) {
-        const int b = one < 0 ? s.item_blk[it] : one;
-        item_pass1<A>(s, s.blk[b], one < 0 ? it - s.item_off[b] : it, staged, c_base);
-    }
-    __syncthreads();
-    if (zero) {
-        uint4 *z = reinterpret_cast<uint4 *>(s.coef);
-        for (int i = tid; i < kCoefStage / 8; i += kThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
-        __syncthreads();
-    }
-    for (int it = tid; it < n; it += kThreads) {
-        const int b = one < 0 ? s.item_blk[it] : one;
-        item_pass2<A>(s, s.blk[b], one < 0 ? it - s.item_off[b] : it);
-    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int k = tid; k < kResidGrid / 8; k += kThreads) reinterpret_cast<uint4 *>(s.res)[k] = make_uint4(0u, 0u, 0u, 0u);
+    const cvp9_job_t &job = s.jc;
+    list_txs(s, lo, hi, hi, job.num_coeffs, tid, kThreads,
+             [&](const BlkS &b, int p, int &txl, int &nx, int &ny) {
+                 txl = b.ptxl[p];
+                 nx = b.pnx[p];
+                 ny = b.pny[p];
+             },
+             [&](const BlkS &b, int p, int txl) {
+                 return A == CVP9_ARITH_FULL && (b.flags & 1) && p == 0 && !job.lossless && txl < 3 && b.ymode < 10
+                            ? (int)c_tx_type[b.ymode] : 0;
+             });
+    deal_txs(s.ntx, 1, warp, kWarps, [&](auto n, int first, int count, int) {
+        tx_unit<A, decltype(n)::value>(s, s.temp.tx[warp], first, count, staged, c_base, lane);
+    });
     __syncthreads();
 }
 
@@ -2247,10 +2233,6 @@ __device__ __noinline__ void phase_residual(int one, int n, bool staged, unsigne
  * and its latency; a thread per column and then per row, with the basis read
  * from constant memory at addresses that differ from lane to lane, took 56 k
  * cycles a superblock of mixed sizes, this 27 k. */
-struct RefTx {                       /* x: first coefficient; y: */
-    static constexpr uint32_t kIntra = 1u << 8, kNone = 1u << 9;   /* x / 4 | y / 4 << 4 | flags */
-};
-
 template <int N>
 __device__ __forceinline__ void ref_tx_unit(ReconSmem &s, int first, int count, int half, bool staged, unsigned c_base, int lane)
 {
@@ -2261,7 +2243,7 @@ __device__ __forceinline__ void ref_tx_unit(ReconSmem &s, int first, int count, 
     const int16_t *X = staged ? s.coef + (tx.x - c_base) : s.jc.coeffs + tx.x;
     const double *M = g_dct + (N == 4 ? 0 : N == 8 ? 16 : N == 16 ? 80 : 336);
     uint32_t nz = 0;                 /* this row's nonzero columns */
-    if (on && !(tx.y & RefTx::kNone)) {
+    if (on && !(tx.y & TxRef::kNone)) {
         const int16_t *row = X + i * N;
         if (!((uintptr_t)row & (N == 4 ? 7 : 15))) {
             uint32_t w[N / 2];
@@ -2317,7 +2299,7 @@ __device__ __forceinline__ void ref_tx_unit(ReconSmem &s, int first, int count, 
     }
     if (!any) return;
     const int px = (int)(tx.y & 15u) * 4 + j0, py = (int)((tx.y >> 4) & 15u) * 4 + i;
-    const bool intra = tx.y & RefTx::kIntra;
+    const bool intra = tx.y & TxRef::kIntra;
 #pragma unroll
     for (int j = 0; j < kCols; j += 4) {
         int r[4];
@@ -2326,16 +2308,7 @@ __device__ __forceinline__ void ref_tx_unit(ReconSmem &s, int first, int count, 
             const double v = acc[j + q];
             r[q] = clampi(__double2int_rz(__dadd_rn(v, v >= 0.0 ? 0.5 : -0.5)), -32768, 32767);
         }
-        if (intra) {
-            *reinterpret_cast<uint2 *>(&s.temp.a.res[py * 64 + px + j]) =
-                make_uint2((uint32_t)(r[0] & 0xffff) | (uint32_t)r[1] << 16, (uint32_t)(r[2] & 0xffff) | (uint32_t)r[3] << 16);
-        } else {
-            uint32_t *d = reinterpret_cast<uint32_t *>(&TY(s, px + j, py));
-            const uint32_t o = *d;
-            *d = (uint32_t)clampi((int)(o & 255u) + r[0], 0, 255) | (uint32_t)clampi((int)((o >> 8) & 255u) + r[1], 0, 255) << 8 |
-                 (uint32_t)clampi((int)((o >> 16) & 255u) + r[2], 0, 255) << 16 |
-                 (uint32_t)clampi((int)(o >> 24) + r[3], 0, 255) << 24;
-        }
+        put_residual4(s, 0, px + j, py, r, intra);
     }
 }
 
@@ -2344,53 +2317,17 @@ __device__ __noinline__ void phase_residual_ref(int lo, int hi, bool staged, uns
 {
     ReconSmem &s = smem_as<ReconSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < 4) s.ntx[tid] = 0;
-    __syncthreads();
-    {
-        uint4 *z = reinterpret_cast<uint4 *>(s.temp.a.res);
-        for (int k = tid; k < kResidGrid / 8; k += kThreads) z[k] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    /* the TXs, largest first: count each size, then list them, a warp a block */
-    const bool in = tid >= lo && tid < hi && s.blk[tid].pnt[0];
-    int at = 0;
-    if (in) at = atomicAdd(&s.ntx[s.blk[tid].txl], (int)s.blk[tid].pnt[0]);
-    __syncthreads();
-    const int n32 = s.ntx[3], n16 = s.ntx[2], n8 = s.ntx[1], n4 = s.ntx[0];
-    if (n32 + n16 + n8 + n4 <= 256) {
-        if (in) {
-            const int c = s.blk[tid].txl;
-            s.chunk_off[tid] = (uint16_t)(at + (c < 3 ? n32 : 0) + (c < 2 ? n16 : 0) + (c < 1 ? n8 : 0));
-        }
-        __syncthreads();
-        for (int b = lo + warp; b < hi; b += kWarps) {
-            const BlkS &k = s.blk[b];
-            const int n = 4 << k.txl, nx = k.pnx[0];
-            for (int t = lane; t < k.pnt[0]; t += 32) {
-                const int ty = div_small(t, nx), tx = t - ty * nx;
-                const uint64_t co = (uint64_t)k.coeff + (uint64_t)t * (uint64_t)(n * n);
-                s.tx[s.chunk_off[b] + t] = make_uint2(
-                    (uint32_t)co, (uint32_t)((k.x + tx * n) >> 2) | (uint32_t)((k.y + ty * n) >> 2) << 4 |
-                                      (k.flags & 1 ? RefTx::kIntra : 0u) |
-                                      (co + (uint64_t)(n * n) > (uint64_t)s.jc.num_coeffs ? RefTx::kNone : 0u));
-            }
-        }
-        __syncthreads();
-        const int u16 = 2 * n32, u8 = u16 + ((n16 + 1) >> 1), u4 = u8 + ((n8 + 3) >> 2), end = u4 + ((n4 + 7) >> 3);
-        for (int u = warp; u < end; u += kWarps) {
-            if (u < u16) {
-                ref_tx_unit<32>(s, u >> 1, 1, u & 1, staged, c_base, lane);
-            } else if (u < u8) {
-                const int f = (u - u16) * 2;
-                ref_tx_unit<16>(s, n32 + f, min(2, n16 - f), 0, staged, c_base, lane);
-            } else if (u < u4) {
-                const int f = (u - u8) * 4;
-                ref_tx_unit<8>(s, n32 + n16 + f, min(4, n8 - f), 0, staged, c_base, lane);
-            } else {
-                const int f = (u - u4) * 8;
-                ref_tx_unit<4>(s, n32 + n16 + n8 + f, min(8, n4 - f), 0, staged, c_base, lane);
-            }
-        }
-    }
+    for (int k = tid; k < kResidGrid / 8; k += kThreads) reinterpret_cast<uint4 *>(s.res)[k] = make_uint4(0u, 0u, 0u, 0u);
+    list_txs(s, lo, hi, hi, s.jc.num_coeffs, tid, kThreads,
+             [&](const BlkS &b, int p, int &txl, int &nx, int &ny) {
+                 txl = b.ptxl[p];
+                 nx = b.pnx[p];
+                 ny = b.pny[p];
+             },
+             [](const BlkS &, int, int) { return 0; });
+    deal_txs(s.ntx, 2, warp, kWarps, [&](auto n, int first, int count, int part) {
+        ref_tx_unit<decltype(n)::value>(s, first, count, part, staged, c_base, lane);
+    });
     __syncthreads();
 }
 
@@ -2400,10 +2337,10 @@ __device__ __noinline__ void phase_plan(int nb, int sbx, int sby)
 {
     ReconSmem &s = smem_as<ReconSmem>();
     const cvp9_job_t &job = s.jc;
-    IntraWork &W = s.temp.a.w;
+    IntraWork &W = s.temp.w;
     const int tid = threadIdx.x;
     const bool mine = tid < nb && (s.blk[tid].flags & 1);
-    intra_fill_cols(recon_view<A>(s), tid, kThreads);
+    intra_fill_cols(recon_view(s), tid, kThreads);
     int ntask;
     if (A == CVP9_ARITH_FULL) {
         const int at = cta_scan1(s, mine ? intra_tx_count(s.blk[tid], job, sbx, sby) : 0, &ntask);
@@ -2444,7 +2381,7 @@ template <int A>
 __device__ __noinline__ void phase_levels()
 {
     ReconSmem &s = smem_as<ReconSmem>();
-    intra_run<A, 255, uint8_t>(s.temp.a.w, recon_view<A>(s), threadIdx.x, kThreads);
+    intra_run<A, 255, uint8_t>(s.temp.w, recon_view(s), threadIdx.x, kThreads);
 }
 
 /* Intra block b on its own, its residual in the grid. */
@@ -2453,9 +2390,9 @@ __device__ __noinline__ void phase_ordered(int b, int sbx, int sby)
 {
     ReconSmem &s = smem_as<ReconSmem>();
     const cvp9_job_t &job = s.jc;
-    IntraWork &W = s.temp.a.w;
+    IntraWork &W = s.temp.w;
     const int tid = threadIdx.x;
-    const IntraView<uint8_t> V = recon_view<A>(s);
+    const IntraView<uint8_t> V = recon_view(s);
     intra_fill_cols(V, tid, kThreads);
     if (A == CVP9_ARITH_FULL) {
         const int n = min(intra_tx_count(s.blk[b], job, sbx, sby), kMaxTasks);
@@ -2495,7 +2432,7 @@ __device__ __noinline__ void phase_neighbours(unsigned need, int sb)
 {
     ReconSmem &s = smem_as<ReconSmem>();
     constexpr int fill_a = A == CVP9_ARITH_SPEC ? 128 : 127, fill_l = A == CVP9_ARITH_FULL ? 129 : fill_a;
-    wait_halo<ReconSmem, uint8_t>(s, recon_view<A>(s), need, sb, A == CVP9_ARITH_FULL, fill_a, fill_l, threadIdx.x, kThreads);
+    wait_halo<ReconSmem, uint8_t>(s, recon_view(s), need, sb, A == CVP9_ARITH_FULL, fill_a, fill_l, threadIdx.x, kThreads);
 }
 
 template <int A>
@@ -2541,7 +2478,6 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             const uint4 fill = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
             for (int i = tid; i < (kTyBytes + 2 * kTcBytes) / 16; i += kThreads) t4[i] = fill;
         }
-        for (int i = tid; i < 256 + 128; i += kThreads) s.txmask[i] = 0;
         for (int i = tid; i < 256; i += kThreads) s.cell[i] = 0;
         if (tid < 16) s.rows[tid] = 0;
         if (tid == 0) { s.c_lo = 0xFFFFFFFFu; s.c_hi = 0u; s.needs = 0u; }
@@ -2552,7 +2488,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
          * grid), then mark the 4x4 cells each one covers */
         bool my_intra = false, my_seq = false, my_bad = false;
         BlkS mb;
-        int nch = 0, nit = 0;
+        int nch = 0;
         if (tid < nb) {
             vp9_macroblock_info_t g = job.blocks[start + tid];
             int lx = (int)g.x - sbx, ly = (int)g.y - sby;
@@ -2603,7 +2539,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             s.blk[tid] = mb;
             my_intra = g.is_intra != 0;
             nch = my_intra ? 0 : block_chunks<A>(mb);
-            nit = A == CVP9_ARITH_REFCPU ? 0 : block_items(mb);
+
         }
         if (__syncthreads_or(my_bad)) {
             /* leave the tile at 128 and flag the frame */
@@ -2611,14 +2547,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             nb = 0;
             my_intra = my_seq = false;
         }
-        for (int b = warp; b < nb; b += kWarps) prefetch_block<A>(s.blk[b], job, sbx, sby, lane);
         {
             /* span of coefficients the residual pass reads */
             unsigned lo = 0xFFFFFFFFu, hi = 0u;
             if (tid < nb) {
                 uint64_t n = 0;
 #pragma unroll
-                for (int q = 0; q < 3; q++) n += (uint64_t)mb.pnt[q] * (uint64_t)(16 << (2 * mb.ptxl[q]));
+                for (int q = 0; q < 3; q++) n += (uint64_t)(mb.pnx[q] * mb.pny[q]) * (uint64_t)(16 << (2 * mb.ptxl[q]));
                 uint64_t e = (uint64_t)mb.coeff + n;
                 if (n) { lo = mb.coeff; hi = e > 0xFFFFFFFFull ? 0xFFFFFFFFu : (unsigned)e; }
             }
@@ -2658,11 +2593,18 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
          * corner: where one of them comes later in the list, the superblock
          * runs in list order (as it does when blocks overlap) */
         if (any_intra) {
-            for (int b = warp; b < nb; b += kWarps) {
+            int n = 0;
+            if (lane * kWarps + warp < nb) {      /* the blocks dealt over the warps */
+                int x0, x1, y0, y1;
+                block_cells<A>(s.blk[lane * kWarps + warp], job, sbx, sby, x0, x1, y0, y1);
+                n = (x1 - x0 + 1) * (y1 - y0 + 1);
+            }
+            warp_spread(n, lane, [&](int i, int k) {
+                const int b = i * kWarps + warp;
                 int x0, x1, y0, y1;
                 block_cells<A>(s.blk[b], job, sbx, sby, x0, x1, y0, y1);
-                own_cells(s.cell, b, x0, x1, y0, y1, lane);
-            }
+                own_cell(s.cell, b, x0, x1, y0, k);
+            });
             __syncthreads();
             bool late = false;
             if (tid < nb && my_intra) {
@@ -2672,36 +2614,32 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             }
             seq |= __syncthreads_or(late) != 0;
         }
-        /* chunk and item offsets in list order */
+        /* inter chunks in list order: offsets, and chunk -> block */
         {
-            int ec, ei, tc, ti;
-            cta_scan2(tid < nb ? nch : 0, tid < nb ? nit : 0, &ec, &ei, &tc, &ti, s.scan_tmp);
-            if (tid < nb) {
-                s.chunk_off[tid] = (uint16_t)ec;
-                s.item_off[tid] = (uint16_t)ei;
-            }
-            if (tid == 0) { s.chunk_off[nb] = (uint16_t)tc; s.item_off[nb] = (uint16_t)ti; }
+            int n;
+            const int at = cta_scan1(s, tid < nb ? nch : 0, &n);
+            if (tid < nb) s.chunk_off[tid] = (uint16_t)at;
+            if (tid == 0) s.chunk_off[nb] = (uint16_t)n;
         }
         __syncthreads();
-        /* chunk -> block and TX item -> block maps, a warp per block */
-        for (int p = warp; p < nb; p += kWarps) {
-            int c0 = s.chunk_off[p], c1 = s.chunk_off[p + 1];
-            for (int c = c0 + lane; c < c1 && c < 256; c += 32) s.chunk_blk[c] = (uint8_t)p;
-            int i0 = s.item_off[p], i1 = s.item_off[p + 1];
-            for (int i = i0 + lane; i < i1 && i < kMaxItems; i += 32) s.item_blk[i] = (uint8_t)p;
+        {
+            const int mine = lane * kWarps + warp;
+            warp_spread(mine < nb ? s.chunk_off[mine + 1] - s.chunk_off[mine] : 0, lane, [&](int i, int k) {
+                const int b = i * kWarps + warp, c = s.chunk_off[b] + k;
+                if (c < 256) s.chunk_blk[c] = (uint8_t)b;
+            });
         }
         __syncthreads();
 
         if (!seq) {
-            /* 3. everything that reads no neighbour: inter predictions, the
-             * first transform pass of every TX, then the second, which adds
-             * to the inter blocks and leaves the intra blocks' residuals in
-             * the (spent) coefficient staging */
-            const int n_chunks = min((int)s.chunk_off[nb], 256), n_items = min((int)s.item_off[nb], kMaxItems);
+            /* 3. everything that reads no neighbour: inter predictions, then
+             * the residual of every TX, added to the inter blocks and left in
+             * the grid for the intra ones */
+            const int n_chunks = min((int)s.chunk_off[nb], 256);
             if (n_chunks) phase_inter<A>(-1, n_chunks, sbx, sby);
             cp_async_wait_all();
             if (A == CVP9_ARITH_REFCPU) phase_residual_ref(0, nb, staged, c_base);
-            else phase_residual<A>(-1, n_items, staged, c_base, any_intra);
+            else phase_residual<A>(0, nb, staged, c_base, sbx, sby);
             if (any_intra) {
                 /* 4. the intra tasks and their levels; 5. the neighbours'
                  * samples, then level by level */
@@ -2710,16 +2648,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
                 phase_levels<A>();
             }
         } else {
-            /* list order, block by block; the staging holds residuals only */
+            /* list order, block by block */
             cp_async_wait_all();
             __syncthreads();
             if (any_intra) phase_neighbours<A>(7u, sb);
             for (int b = 0; b < nb; b++) {
                 const bool intra = s.blk[b].flags & 1;
                 if (!intra) phase_inter<A>(b, block_chunks<A>(s.blk[b]), sbx, sby);
-                for (int i = tid; i < 256 + 128; i += kThreads) s.txmask[i] = 0;
-                if (A == CVP9_ARITH_REFCPU) phase_residual_ref(b, b + 1, false, 0u);
-                else phase_residual<A>(b, block_items(s.blk[b]), false, 0u, true);
+                if (A == CVP9_ARITH_REFCPU) phase_residual_ref(b, b + 1, staged, c_base);
+                else phase_residual<A>(b, b + 1, staged, c_base, sbx, sby);
                 if (intra) phase_ordered<A>(b, sbx, sby);
             }
         }
@@ -5089,8 +5026,8 @@ __global__ void __launch_bounds__(kLfThreads, 2) k_lf_full(const cvp9_job_t *__r
  *
  * One CTA per superblock ticket (SB-diagonal order over the step's jobs,
  * persistent, as k_recon). What reads no neighbour goes first and together:
- * the inter predictions a thread per column strip of up to 8 rows, then every
- * residual a thread per TX row, then per TX column. The intra blocks follow
+ * the inter predictions eight lanes a chunk, then every residual, a warp for
+ * TXs of one size. The intra blocks follow
  * as in k_recon, TX by TX in dependency levels over the whole CTA (8x1080p
  * key step 15.6 -> 3.9 ms against a warp per block, prediction and
  * transforms in turn). A superblock whose blocks overlap, or
@@ -5099,7 +5036,7 @@ __global__ void __launch_bounds__(kLfThreads, 2) k_lf_full(const cvp9_job_t *__r
 namespace {
 
 constexpr int kHbdThreads = 256, kHbdWarps = kHbdThreads / 32;
-constexpr int kHbdMaxBlocks = 256, kHbdMaxTx = 384;
+constexpr int kHbdMaxBlocks = 256;
 constexpr int kHYP = 72, kHCP = 40;      /* tile pitches in samples; column -1 at index 3 */
 constexpr int kHbdMax = 1023, kHbdMid = 512;
 
@@ -5116,29 +5053,23 @@ struct HbdBlk {
     uint32_t coeff;
 };
 
-struct HbdTx {
-    uint32_t coeff;
-    uint8_t  plane;              /* | TX type << 2, 16 intra, 32 no coefficients */
-    uint8_t  txl, x, y;          /* plane-local tile position */
-};
-
 struct HbdSmem {
     uint16_t ty[65 * kHYP];                /* luma tile, row 0 = the row above */
     uint16_t tc[2][33 * kHCP];
     union {
-        int32_t i[64 * 64 + 2 * 32 * 32];  /* row-pass output at tile positions */
+        int32_t i[kResidGrid + 32];        /* coefficients (tx_word), then the row pass's output */
         IntraWork w;                       /* then the intra tasks             */
     } tmp;
-    int16_t  res[kResidGrid];              /* residuals of the intra blocks    */
+    alignas(16) int16_t res[kResidGrid];   /* prediction rows; then residuals of intra blocks */
     uint16_t col[16 * 64 + 2 * 16 * 32];   /* left-column copies (IntraView)   */
     HbdBlk   blk[kHbdMaxBlocks];
-    HbdTx    tx[kHbdMaxTx];
-    uint16_t tx_base[kHbdMaxTx + 1];       /* prefix over TXs of their sizes   */
-    uint16_t it_base[kHbdMaxBlocks + 1];   /* prefix over blocks of their items */
+    uint2    tx[kMaxTasks];                /* residual TXs by size (TxRef)     */
+    uint16_t tx_at[3][kHbdMaxBlocks];      /* first TX of a block's plane in tx */
+    int      ntx[4];                       /* TXs of each size                 */
+    uint16_t it_base[kHbdMaxBlocks + 1];   /* prefix over blocks of their chunks, tasks */
     uint16_t cell[256];                    /* owner block + 1 per 4x4          */
     uint32_t rows[16];                     /* claimed cells, a bit each        */
-    uint8_t  txnz[kHbdMaxTx];              /* a TX has a nonzero coefficient   */
-    uint8_t  txwide[kHbdMaxTx];            /* and one that needs 64-bit values */
+    unsigned c_lo, c_hi;                   /* coefficient span of the SB       */
     int      scan[kHbdWarps];
     cvp9_job_t jc;
     unsigned needs;                        /* intra_needs of its blocks        */
@@ -5148,11 +5079,6 @@ struct HbdSmem {
 __device__ __forceinline__ uint16_t &HT(HbdSmem &s, int p, int x, int y)
 {
     return p == 0 ? s.ty[(y + 1) * kHYP + x + 4] : s.tc[p - 1][(y + 1) * kHCP + x + 4];
-}
-
-__device__ __forceinline__ int32_t *hbd_tmp(HbdSmem &s, int p, int x, int y)
-{
-    return &s.tmp.i[plane_at(p, x, y)];
 }
 
 /* Exclusive prefix of v over the CTA's threads (thread order); *total: the
@@ -5180,159 +5106,6 @@ __device__ __forceinline__ int hbd_scan(HbdSmem &s, int v, int *total)
     return off + x - v;
 }
 
-/* The residual TXs of a block in coefficient order (planes, then raster) as
- * s.tx[at ...], by one warp. A TX
- * whose coefficients do not end inside num_coeffs is marked empty: offsets
- * ascend, so every later one of the block is, too (as is one reaching past
- * the SB, which no block that its TXs tile has). */
-__device__ __forceinline__ void hbd_list_txs(HbdSmem &s, const HbdBlk &b, int sbx, int sby, int at, int lane)
-{
-    const cvp9_job_t &job = s.jc;
-    const int gx = sbx + b.x, gy = sby + b.y;
-    uint64_t off = b.coeff;
-    for (int p = 0; p < 3; p++) {
-        int txl, nx, ny, pbw;
-        plane_layout(b, job, gx, gy, p, txl, nx, ny, pbw);
-        const int sz = 16 << (2 * txl), ts = 4 << txl;
-        const int ox = p ? (b.x >> 1) : b.x, oy = p ? (b.y >> 1) : b.y;
-        const int type = ((b.flags & 1) && p == 0 && !job.lossless && txl < 3 && b.ymode < 10) ? c_tx_type[b.ymode] : 0;
-        for (int k = lane; k < nx * ny && at + k < kHbdMaxTx; k += 32) {
-            const int ty = div_small(k, nx), tx = k - ty * nx;
-            const uint64_t o = off + (uint64_t)k * (uint64_t)sz;
-            HbdTx &t = s.tx[at + k];
-            t.coeff = (uint32_t)o;
-            const bool none = o + (uint64_t)sz > (uint64_t)job.num_coeffs || ox + (tx + 1) * ts > (p ? 32 : 64) ||
-                              oy + (ty + 1) * ts > (p ? 32 : 64);
-            t.plane = (uint8_t)(p | (type << 2) | ((b.flags & 1) << 4) | (none ? 0x20 : 0));
-            t.txl = (uint8_t)txl;
-            t.x = (uint8_t)(ox + tx * ts);
-            t.y = (uint8_t)(oy + ty * ts);
-        }
-        at += nx * ny;
-        off += (uint64_t)(nx * ny) * (uint64_t)sz;
-    }
-}
-
-/* Row pass of TX row i: the frame's dequantised coefficients through the
- * 1-D inverse (DCT, ADST along the row when row_adst, WHT when lossless),
- * 64-bit products inside, 32-bit out into the temp rows. Returns 0 when the
- * row has no nonzero coefficient, 2 when one is outside +-2^18 (a 10-bit
- * stream's reach +-2^17): then the row, and its TX's columns, run on 64-bit
- * values (wl). The 32-bit values (wn) took six steps of six 2160p inter pictures
- * from 30.1 to 29.6 ms. */
-template <int N, class T>
-__device__ __forceinline__ void hbd_row_as(T (&v)[N], int32_t *d, bool lossless, bool row_adst)
-{
-    if (N == 4 && lossless) iwht4(v, true);
-    else itx1<N>(v, row_adst);
-#pragma unroll
-    for (int k = 0; k < N; k++) d[k] = (int32_t)v[k].v;
-}
-
-template <int N>
-__device__ __noinline__ void hbd_row_wide(const int32_t *X, int32_t *d, bool lossless, bool row_adst)
-{
-    wl v[N];
-    for (int k = 0; k < N; k++) v[k] = wl(X[k]);
-    hbd_row_as<N>(v, d, lossless, row_adst);
-}
-
-template <int N>
-__device__ __forceinline__ int hbd_row(HbdSmem &s, const int32_t *X, int i, int p, int px0, int py0,
-                                       bool lossless, bool row_adst)
-{
-    wn v[N];
-    int any = 0;
-    unsigned wide = 0;
-    X += i * N;
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        const int c = __ldg(X + k);
-        any |= c;
-        wide |= ((unsigned)c + (1u << 18)) >> 19;
-        v[k] = wn(c);
-    }
-    int32_t *d = hbd_tmp(s, p, px0, py0 + i);
-    if (!any) {
-#pragma unroll
-        for (int k = 0; k < N; k++) d[k] = 0;
-        return 0;
-    }
-    if (wide) {
-        hbd_row_wide<N>(X, d, lossless, row_adst);
-        return 2;
-    }
-    hbd_row_as<N>(v, d, lossless, row_adst);
-    return 1;
-}
-
-/* Column pass of TX column j: the 1-D inverse down the column, rounding
- * shift 4/5/6/6 (none after the WHT); an inter block's residual is added and
- * clipped to 10 bits, an intra block's (intra) goes to the residual grid,
- * saturated to int16, which no sum with a sample notices. wide: a row of the
- * TX left the 32-bit range. */
-template <int N, class T>
-__device__ __forceinline__ void hbd_col_as(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst,
-                                           bool intra)
-{
-    T v[N];
-    const int32_t *c = hbd_tmp(s, p, px0 + j, py0);
-    const int pitch = p ? 32 : 64;
-#pragma unroll
-    for (int k = 0; k < N; k++) v[k] = T(c[k * pitch]);
-    const bool wht = N == 4 && lossless;
-    if (wht) iwht4(v, false);
-    else itx1<N>(v, col_adst);
-    const int sh = wht ? 0 : N == 4 ? 4 : (N == 8 ? 5 : 6);
-    const int round = wht ? 0 : 1 << (sh - 1);
-    int16_t *r = s.res + plane_at(p, px0 + j, py0);
-    uint16_t *px = &HT(s, p, px0 + j, py0);
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        const auto x = (v[k].v + round) >> sh;
-        const int q = x < -32768 ? -32768 : (x > 32767 ? 32767 : (int)x);
-        if (intra) r[k * pitch] = (int16_t)q;
-        else px[k * (p ? kHCP : kHYP)] = (uint16_t)clampi((int)px[k * (p ? kHCP : kHYP)] + q, 0, kHbdMax);
-    }
-}
-
-template <int N>
-__device__ __noinline__ void hbd_col_wide(int j, int p, int px0, int py0, bool lossless, bool col_adst,
-                                          bool intra)
-{
-    hbd_col_as<N, wl>(smem_as<HbdSmem>(), j, p, px0, py0, lossless, col_adst, intra);
-}
-
-template <int N>
-__device__ __forceinline__ void hbd_col(HbdSmem &s, int j, int p, int px0, int py0, bool lossless, bool col_adst,
-                                        bool intra, bool wide)
-{
-    if (wide) hbd_col_wide<N>(j, p, px0, py0, lossless, col_adst, intra);
-    else hbd_col_as<N, wn>(s, j, p, px0, py0, lossless, col_adst, intra);
-}
-
-__device__ __forceinline__ int hbd_row_n(HbdSmem &s, int txl, const int32_t *X, int i, int p, int x, int y,
-                                         bool lossless, bool row_adst)
-{
-    switch (txl) {
-    case 0: return hbd_row<4>(s, X, i, p, x, y, lossless, row_adst);
-    case 1: return hbd_row<8>(s, X, i, p, x, y, lossless, row_adst);
-    case 2: return hbd_row<16>(s, X, i, p, x, y, lossless, row_adst);
-    default: return hbd_row<32>(s, X, i, p, x, y, lossless, false);
-    }
-}
-
-__device__ __forceinline__ void hbd_col_n(HbdSmem &s, int txl, int j, int p, int x, int y, bool lossless,
-                                          bool col_adst, bool intra, bool wide)
-{
-    switch (txl) {
-    case 0: hbd_col<4>(s, j, p, x, y, lossless, col_adst, intra, wide); break;
-    case 1: hbd_col<8>(s, j, p, x, y, lossless, col_adst, intra, wide); break;
-    case 2: hbd_col<16>(s, j, p, x, y, lossless, col_adst, intra, wide); break;
-    default: hbd_col<32>(s, j, p, x, y, lossless, false, intra, wide); break;
-    }
-}
-
 /* The inter predictions of blocks [lo, hi) of the SB, whole CTA, four chunks
  * a warp. */
 __device__ __noinline__ void hbd_predict(int lo, int hi, int nb, int sbx, int sby)
@@ -5346,7 +5119,7 @@ __device__ __noinline__ void hbd_predict(int lo, int hi, int nb, int sbx, int sb
     if (tid < kHbdMaxBlocks) s.it_base[tid] = (uint16_t)min(at, 0xFFFF);
     __syncthreads();
     const uint32_t (*P)[2] = c_subpel4_pk[job.interp_filter & 3];
-    uint16_t *rows = reinterpret_cast<uint16_t *>(s.tmp.i) + (warp * 4 + g) * 128;
+    uint16_t *rows = reinterpret_cast<uint16_t *>(s.res) + (warp * 4 + g) * 128;
     for (int base = warp * 4; base < n; base += 4 * kHbdWarps) {
         const int chk = base + g;
         const bool on = chk < n;
@@ -5355,68 +5128,132 @@ __device__ __noinline__ void hbd_predict(int lo, int hi, int nb, int sbx, int sb
         int p = 0, x = 0, y = 0, w = 0, h = 0;
         if (on) mc_chunk_at(chk - s.it_base[bi], b.cw, b.ch, b.ccw, b.cch, p, x, y, w, h);
         const int lx = (p ? b.x >> 1 : b.x) + x, ly = (p ? b.y >> 1 : b.y) + y;
-        mc_chunk<uint16_t>(job, P, b, on, p, (p ? sbx >> 1 : sbx) + lx, (p ? sby >> 1 : sby) + ly, w, h, kHbdMid, rows,
+        mc_chunk<uint16_t, true>(job, P, b, on, p, (p ? sbx >> 1 : sbx) + lx, (p ? sby >> 1 : sby) + ly, w, h, kHbdMid, rows,
                            &HT(s, p, lx, ly + k), k);
     }
     __syncthreads();
 }
 
-/* Blocks [lo, hi) of the SB, whole CTA: the TX rows and the TX columns of every block's residual (an intra block's
- * into the residual grid, which starts at zero). */
-__device__ __noinline__ void hbd_residual(int lo, int hi, int nb, int sbx, int sby)
+/* 32 / N TXs by a warp, T the type of the butterflies' values: the rows of the
+ * frame's dequantised coefficients (DCT, ADST along the row by the TX type, WHT
+ * when lossless) in place in the permuted coefficient buffer — 64-bit products
+ * inside, 32 bits between the passes —, then the columns, rounding shift
+ * 4/5/6/6 (none after the WHT); an inter block's residual is added and clipped
+ * to 10 bits, an intra block's goes to the grid, saturated to int16, which no
+ * sum with a sample notices. c: the lane's row, at: its TX's place. */
+template <int N, class T>
+__device__ __forceinline__ void hbd_tx_passes(HbdSmem &s, const int (&c)[N], int at, uint2 tx, bool any, bool mine, int i)
+{
+    const bool lossless = s.jc.lossless;
+    const int p = (int)(tx.y >> 8) & 3, type = (int)(tx.y >> 10) & 3;
+    const bool wht = N == 4 && lossless;
+    int32_t *buf = s.tmp.i;
+    T v[N];
+    if (mine && any) {               /* a row of zeros stays as it is */
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = T(c[k]);
+        if (wht) iwht4(v, true);
+        else itx1<N>(v, type >= 2);
+#pragma unroll
+        for (int k = 0; k < N; k += 4)
+            *reinterpret_cast<int4 *>(&buf[tx_word(at + i * N + k)]) =
+                make_int4((int)v[k].v, (int)v[k + 1].v, (int)v[k + 2].v, (int)v[k + 3].v);
+    }
+    __syncwarp();
+    if (mine) {
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = T(buf[tx_word(at + k * N + i)]);
+        if (wht) iwht4(v, false);
+        else itx1<N>(v, type & 1);
+        const int sh = wht ? 0 : N == 4 ? 4 : (N == 8 ? 5 : 6), round = wht ? 0 : 1 << (sh - 1);
+        const int x = (int)(tx.y & 15u) * 4 + i, y = (int)((tx.y >> 4) & 15u) * 4;
+        const bool intra = tx.y & TxRef::kIntra;
+        int16_t *r = s.res + plane_at(p, x, y);
+        uint16_t *d = &HT(s, p, x, y);
+        const int rp = p ? 32 : 64, dp = p ? kHCP : kHYP;
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const auto q = (v[k].v + round) >> sh;
+            const int e = q < -32768 ? -32768 : (q > 32767 ? 32767 : (int)q);
+            if (intra) r[k * rp] = (int16_t)e;
+            else d[k * dp] = (uint16_t)clampi((int)d[k * dp] + e, 0, kHbdMax);
+        }
+    }
+}
+
+template <int N>
+__device__ __noinline__ void hbd_tx_wide(int at, uint2 tx, bool any, bool mine, int i)
+{
+    HbdSmem &s = smem_as<HbdSmem>();
+    int c[N];
+    for (int k = 0; k < N; k++) c[k] = s.tmp.i[tx_word(at + i * N + k)];
+    __syncwarp();
+    hbd_tx_passes<N, wl>(s, c, at, tx, any, mine, i);
+}
+
+/* The butterflies run on 32-bit values (wn) unless one of the warp's
+ * coefficients is outside +-2^18 (a 10-bit stream's reach +-2^17): then on
+ * 64-bit ones (wl), with the same results. */
+template <int N>
+__device__ __forceinline__ void hbd_tx_unit(HbdSmem &s, int first, int count, bool staged, unsigned c_base, int slot, int lane)
+{
+    const int sub = lane / N, i = lane & (N - 1);
+    const bool on = sub < count;
+    const uint2 tx = s.tx[first + (on ? sub : 0)];
+    const bool go = on && !(tx.y & TxRef::kNone);
+    const int at = !go ? 0 : staged ? (int)(tx.x - c_base) : slot + sub * N * N;
+    if (!staged) {                   /* bring the TXs here */
+        if (go)
+            for (int k = 0; k < N; k++) s.tmp.i[tx_word(at + k * N + i)] = __ldg(s.jc.coeffs32 + tx.x + k * N + i);
+        __syncwarp();
+    }
+    int c[N], any = 0;
+    unsigned wide = 0;
+#pragma unroll
+    for (int k = 0; k < N; k += 4) {
+        const int4 w = go ? *reinterpret_cast<const int4 *>(&s.tmp.i[tx_word(at + i * N + k)]) : make_int4(0, 0, 0, 0);
+        c[k] = w.x;
+        c[k + 1] = w.y;
+        c[k + 2] = w.z;
+        c[k + 3] = w.w;
+        any |= w.x | w.y | w.z | w.w;
+        wide |= (((unsigned)w.x + (1u << 18)) | ((unsigned)w.y + (1u << 18)) | ((unsigned)w.z + (1u << 18)) |
+                 ((unsigned)w.w + (1u << 18))) >> 19;
+    }
+    const uint32_t live = __ballot_sync(0xffffffffu, any != 0);
+    if (live) {
+        const bool mine = go && (N == 32 || ((live >> (sub * N)) & ((1u << (N & 31)) - 1u)));
+        if (__any_sync(0xffffffffu, wide != 0)) hbd_tx_wide<N>(at, tx, any != 0, mine, i);
+        else hbd_tx_passes<N, wn>(s, c, at, tx, any != 0, mine, i);
+    }
+    __syncwarp();
+}
+
+/* Every residual of blocks [lo, hi) of the SB, whole CTA; staged: their
+ * coefficients are in the permuted buffer, from c_base on. */
+__device__ __noinline__ void hbd_residual(int lo, int hi, int nb, bool staged, unsigned c_base, int sbx, int sby)
 {
     HbdSmem &s = smem_as<HbdSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const cvp9_job_t &job = s.jc;
-    const bool in = tid >= lo && tid < hi && tid < nb;
-    int total;
     for (int i = tid; i < kResidGrid / 8; i += kHbdThreads) reinterpret_cast<uint4 *>(s.res)[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    /* the residual TXs, a warp per block listing them */
-    int cnt = in && !(s.blk[tid].flags & 2) && s.blk[tid].txl <= 3 ? intra_tx_count(s.blk[tid], job, sbx, sby) : 0;
-    int base = hbd_scan(s, cnt, &total);
-    if (total > kHbdMaxTx) {
-        if (tid == 0) atomicOr(job.status, (unsigned)CVP9_JOB_TOO_MANY);
-        total = kHbdMaxTx;
-    }
-    if (tid < kHbdMaxBlocks) s.it_base[tid] = (uint16_t)min(base, 0xFFFF);
-    __syncthreads();
-    for (int b = lo + warp; b < min(hi, nb); b += kHbdWarps)
-        if (!(s.blk[b].flags & 2) && s.blk[b].txl <= 3) hbd_list_txs(s, s.blk[b], sbx, sby, s.it_base[b], lane);
-    __syncthreads();
-    const int ntx = total;
-    /* prefix over TXs of their edge length (their rows, and columns), two
-     * consecutive TXs a thread */
-    {
-        const int t0 = 2 * tid, t1 = 2 * tid + 1;
-        const int a = t0 < ntx ? 4 << s.tx[t0].txl : 0, c = t1 < ntx ? 4 << s.tx[t1].txl : 0;
-        int nrow_all;
-        const int b0 = hbd_scan(s, a + c, &nrow_all);
-        if (t0 <= ntx) s.tx_base[t0] = (uint16_t)b0;
-        if (t1 <= ntx) s.tx_base[t1] = (uint16_t)(b0 + a);
-        if (t0 < ntx) s.txnz[t0] = s.txwide[t0] = 0;
-        if (t1 < ntx) s.txnz[t1] = s.txwide[t1] = 0;
-    }
-    if (ntx > 0) {
-        __syncthreads();
-        const int nrow = s.tx_base[ntx];
-        for (int it = tid; it < nrow; it += kHbdThreads) {
-            const int t = find_base(s.tx_base, ntx, it);
-            const HbdTx x = s.tx[t];
-            if (x.plane & 0x20) continue;
-            const int got = hbd_row_n(s, x.txl, job.coeffs32 + x.coeff, it - s.tx_base[t], x.plane & 3, x.x, x.y,
-                                      job.lossless, ((x.plane >> 2) & 3) >= 2);
-            if (got) s.txnz[t] = 1;
-            if (got == 2) s.txwide[t] = 1;
-        }
-        __syncthreads();
-        for (int it = tid; it < nrow; it += kHbdThreads) {
-            const int t = find_base(s.tx_base, ntx, it);
-            const HbdTx x = s.tx[t];
-            if (s.txnz[t]) hbd_col_n(s, x.txl, it - s.tx_base[t], x.plane & 3, x.x, x.y, job.lossless,
-                                     (x.plane >> 2) & 1, (x.plane >> 4) & 1, s.txwide[t] != 0);
-        }
-    }
+    list_txs(s, lo, hi, nb, job.num_coeffs, tid, kHbdThreads,
+             [&](const HbdBlk &b, int p, int &txl, int &nx, int &ny) {
+                 int pbw;
+                 plane_layout(b, job, sbx + b.x, sby + b.y, p, txl, nx, ny, pbw);
+                 if (b.flags & 2) nx = ny = 0;
+             },
+             [&](const HbdBlk &b, int p, int txl) {
+                 return (b.flags & 1) && p == 0 && !job.lossless && txl < 3 && b.ymode < 10 ? (int)c_tx_type[b.ymode] : 0;
+             });
+    if (tid == 0 && s.ntx[0] + s.ntx[1] + s.ntx[2] + s.ntx[3] > kMaxTasks) atomicOr(job.status, (unsigned)CVP9_JOB_TOO_MANY);
+    const int n32 = s.ntx[3], n16 = s.ntx[2], n8 = s.ntx[1];
+    deal_txs(s.ntx, 1, warp, kHbdWarps, [&](auto n, int first, int count, int) {
+        constexpr int N = decltype(n)::value;
+        const int before = N == 32 ? 0 : N == 16 ? n32 * 1024 : N == 8 ? n32 * 1024 + n16 * 256 : n32 * 1024 + n16 * 256 + n8 * 64;
+        const int skip = N == 32 ? 0 : N == 16 ? n32 : N == 8 ? n32 + n16 : n32 + n16 + n8;
+        hbd_tx_unit<N>(s, first, count, staged, c_base, before + (first - skip) * N * N, lane);
+    });
     __syncthreads();
 }
 
@@ -5522,7 +5359,7 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
         }
         for (int i = tid; i < 256; i += kHbdThreads) s.cell[i] = 0;
         if (tid < 16) s.rows[tid] = 0;
-        if (tid == 0) s.needs = 0u;
+        if (tid == 0) { s.needs = 0u; s.c_lo = 0xFFFFFFFFu; s.c_hi = 0u; }
         __syncthreads();
 
         /* 1. blocks (each inside this SB, 4-aligned, 4..64 px, tx_size <= 3,
@@ -5574,12 +5411,48 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
             const HbdBlk &b = s.blk[tid];
             my_seq |= claim_cells(s.rows, b.x >> 2, (b.x + b.cw - 1) >> 2, b.y >> 2, (b.y + b.ch - 1) >> 2);
         }
-        const bool any_intra = __syncthreads_or(my_intra) != 0;
-        if (any_intra) {
-            for (int i = warp; i < nb; i += kHbdWarps) {
-                const HbdBlk &b = s.blk[i];
-                own_cells(s.cell, i, b.x >> 2, (b.x + b.cw - 1) >> 2, b.y >> 2, (b.y + b.ch - 1) >> 2, lane);
+        /* stage the coefficients in the permuted buffer, where 16-byte copies
+         * can: every block's start a multiple of 4, the span no longer than the
+         * SB's samples */
+        bool odd = false;
+        {
+            unsigned lo = 0xFFFFFFFFu, hi = 0u;
+            if (tid < nb && !(s.blk[tid].flags & 2)) {
+                const HbdBlk &b = s.blk[tid];
+                uint64_t n = 0;
+                for (int p = 0; p < 3; p++) {
+                    int txl, nx, ny, pbw;
+                    plane_layout(b, job, sbx + b.x, sby + b.y, p, txl, nx, ny, pbw);
+                    n += (uint64_t)(nx * ny) << (4 + 2 * txl);
+                }
+                const uint64_t e = (uint64_t)b.coeff + n;
+                if (n) {
+                    lo = b.coeff;
+                    hi = e > 0xFFFFFFFFull ? 0xFFFFFFFFu : (unsigned)e;
+                    odd = b.coeff & 3u;
+                }
             }
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            if (lane == 0) { atomicMin(&s.c_lo, lo); atomicMax(&s.c_hi, hi); }
+        }
+        const bool any_intra = __syncthreads_or(my_intra) != 0;
+        odd = __syncthreads_or(odd) != 0;
+        const unsigned c_base = s.c_lo, c_hi = s.c_hi;
+        const bool staged = c_hi > c_base && !odd && c_hi <= job.num_coeffs && c_hi - c_base <= (unsigned)kResidGrid &&
+                            !((uintptr_t)job.coeffs32 & 15);
+        if (staged)
+            for (unsigned e = 4u * (unsigned)tid; e < c_hi - c_base; e += 4u * kHbdThreads)
+                cp_async16(&s.tmp.i[tx_word((int)e)], job.coeffs32 + c_base + e);
+        cp_async_commit();
+        if (any_intra) {
+            const int mb = lane * kHbdWarps + warp;     /* the blocks dealt over the warps */
+            const HbdBlk &m = s.blk[mb];
+            warp_spread(mb < nb ? (((m.x + m.cw + 3) >> 2) - (m.x >> 2)) * (((m.y + m.ch + 3) >> 2) - (m.y >> 2)) : 0, lane,
+                        [&](int i, int k) {
+                            const HbdBlk &b = s.blk[i * kHbdWarps + warp];
+                            own_cell(s.cell, i * kHbdWarps + warp, b.x >> 2, (b.x + b.cw - 1) >> 2, b.y >> 2, k);
+                        });
             __syncthreads();
         }
         /* an intra block reading samples of a block later in the list: the
@@ -5600,17 +5473,21 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
          * by level; or block by block in list order */
         if (!seq) {
             hbd_predict(0, nb, nb, sbx, sby);
-            hbd_residual(0, nb, nb, sbx, sby);
+            cp_async_wait_all();
+            __syncthreads();
+            hbd_residual(0, nb, nb, staged, c_base, sbx, sby);
             if (any_intra) {
                 hbd_plan(nb, sbx, sby);
                 hbd_neighbours(s.needs, sb);
                 hbd_levels();
             }
         } else {
+            cp_async_wait_all();
+            __syncthreads();
             if (any_intra) hbd_neighbours(7u, sb);
             for (int i = 0; i < nb; i++) {
                 hbd_predict(i, i + 1, nb, sbx, sby);
-                hbd_residual(i, i + 1, nb, sbx, sby);
+                hbd_residual(i, i + 1, nb, false, 0u, sbx, sby);
                 if (s.blk[i].flags & 1) hbd_ordered(i, sbx, sby);
             }
         }
