@@ -18,7 +18,7 @@
  *  - every process that loads the library holds the array (~200 KB) on every
  *    GPU it uses until exit;
  *  - all calls share the array: everything that must start at zero is
- *    cleared at the start of each call, and calls whose work overlaps on the
+ *    cleared by each call's first kernel, and calls whose work overlaps on the
  *    GPU (different streams, or different host threads) race with each
  *    other — serialise them on one stream;
  *  - the first call on a device does the one-time set-up for that device
@@ -55,26 +55,32 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 constexpr int kMaxDev = 64;
 static unsigned char *g_scratch_ptr[kMaxDev];
 
-__global__ void k_put_job(cvp9_job_t job, cvp9_job_t *dst)
+/* Everything that a call's kernels find in the array, in one launch: the job
+ * descriptor, the words that start at zero (superblock ranges and done flags,
+ * ticket counter, status), and the SB-diagonal ticket order: SB (r, c) goes
+ * after every SB of a smaller anti-diagonal, in row order within its own. A
+ * small picture's call is bound by its launches: as three memsets and two
+ * kernels it was 10 of a 352x288 picture's 45 us. */
+__global__ void __launch_bounds__(256) k_prepare(cvp9_job_t job, cvp9_job_t *dst, uint32_t *misc, uint32_t *tickets)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *dst = job;
-}
-
-/* SB-diagonal ticket order computed on the device: SB (r, c) goes after
- * every SB of a smaller anti-diagonal, in row order within its diagonal. */
-__global__ void k_diag_tickets(int sb_cols, int sb_rows, uint32_t *tickets)
-{
-    int sb = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sb >= sb_cols * sb_rows) return;
-    int r = sb / sb_cols, c = sb - r * sb_cols, d = r + c;
-    int before = 0;
-    for (int e = 0; e < d; e++) {
-        int lo = e - (sb_cols - 1) > 0 ? e - (sb_cols - 1) : 0;
-        int hi = e < sb_rows - 1 ? e : sb_rows - 1;
-        before += hi - lo + 1;
+    const int sb = blockIdx.x * blockDim.x + threadIdx.x, sb_cols = job.sb_cols, sb_rows = job.sb_rows;
+    if (sb == 0) {
+        *dst = job;
+        misc[0] = misc[1] = 0u;
+        *job.status = 0u;
     }
-    int lo = d - (sb_cols - 1) > 0 ? d - (sb_cols - 1) : 0;
-    tickets[before + (r - lo)] = (uint32_t)sb;
+    if (sb >= sb_cols * sb_rows) return;
+    reinterpret_cast<uint4 *>(job.sb_range)[sb] = make_uint4(0u, 0u, 0u, 0u);
+    job.sb_done[sb] = 0u;
+    const int r = sb / sb_cols, d = r + (sb - r * sb_cols);
+    /* SBs of the diagonals before d: a triangle, a band, and what the last
+     * corner lacks of one */
+    const int m = min(sb_cols, sb_rows), n = max(sb_cols, sb_rows);
+    const int t = d <= m ? d * (d + 1) / 2
+                         : d <= n ? m * (m + 1) / 2 + (d - m) * m
+                                  : sb_cols * sb_rows - (m + n - 1 - d) * (m + n - d) / 2;
+    const int lo = max(0, d - (sb_cols - 1));
+    tickets[t + (r - lo)] = (uint32_t)sb;
 }
 
 static int setup_device(int dev)
@@ -145,15 +151,11 @@ extern "C" cvp9_err_t cuda_reconstruct_noalloc(const vp9_parsed_frame_t *pf,
     job.epoch = 1;
     job.sb_range = (uint32_t *)(base + kOffRange);
     job.sb_done = (uint32_t *)(base + kOffDone);
-    job.status = (uint32_t *)(base + kOffMisc) + 1;
+    job.status = status_dev ? status_dev : (uint32_t *)(base + kOffMisc) + 1;
 
-    /* the array keeps the previous call's contents: clear what starts at 0 */
-    if (cudaMemsetAsync(base + kOffMisc, 0, 64, st) != cudaSuccess ||
-        cudaMemsetAsync(base + kOffRange, 0, (size_t)n_sb * 16, st) != cudaSuccess ||
-        cudaMemsetAsync(base + kOffDone, 0, (size_t)n_sb * 4, st) != cudaSuccess)
-        return CVP9_ERR_GPU;
-    k_put_job<<<1, 1, 0, st>>>(job, (cvp9_job_t *)(base + kOffJob));
-    k_diag_tickets<<<(n_sb + 255) / 256, 256, 0, st>>>(sb_cols, sb_rows, (uint32_t *)(base + kOffTickets));
+    /* the array keeps the previous call's contents */
+    k_prepare<<<(n_sb + 255) / 256, 256, 0, st>>>(job, (cvp9_job_t *)(base + kOffJob), (uint32_t *)(base + kOffMisc),
+                                                  (uint32_t *)(base + kOffTickets));
     if (cudaGetLastError() != cudaSuccess) return CVP9_ERR_GPU;
 
     int sms = 148;
@@ -176,9 +178,5 @@ extern "C" cvp9_err_t cuda_reconstruct_noalloc(const vp9_parsed_frame_t *pf,
         L.flat_lf_max_w = W;
         L.flat_lf_max_h = H;
     }
-    if (cvp9k_launch_frame(&L, st) != 0) return CVP9_ERR_GPU;
-    if (status_dev &&
-        cudaMemcpyAsync(status_dev, base + kOffMisc + 4, 4, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-        return CVP9_ERR_GPU;
-    return CVP9_OK;
+    return cvp9k_launch_frame(&L, st) == 0 ? CVP9_OK : CVP9_ERR_GPU;
 }
