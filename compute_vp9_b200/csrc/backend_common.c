@@ -195,6 +195,18 @@ double cvp9_now(void)
     return (double)ts.tv_sec + 1e-9 * (double)ts.tv_nsec;
 }
 
+void cvp9_poll_pause(double waited)
+{
+    if (waited < 200e-6) {
+#if defined(__x86_64__)
+        for (int k = 0; k < 16; k++) __builtin_ia32_pause();
+#endif
+        return;
+    }
+    struct timespec ts = { 0, 20000 };
+    nanosleep(&ts, NULL);
+}
+
 /* ── Autotuner ─────────────────────────────────────────────────────────── */
 
 static int ceil_log2_u64(uint64_t v)

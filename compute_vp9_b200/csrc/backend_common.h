@@ -76,6 +76,11 @@ void cvp9_job_geometry(cvp9_job_t *job, const vp9_parsed_frame_t *pf);
 /* Monotonic clock in seconds. */
 double cvp9_now(void);
 
+/* Between two looks at an event that was not ready after `waited` seconds:
+ * nothing much at first, as a sleep of 20 us takes 70 us to return and a
+ * small frame's kernels as long; sleep from 0.2 ms on. */
+void cvp9_poll_pause(double waited);
+
 #ifdef __cplusplus
 }
 #endif

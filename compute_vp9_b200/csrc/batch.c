@@ -562,8 +562,7 @@ static cvp9_err_t wait_slot(cvp9_batch_t *b, bslot_t *s)
             snprintf(b->err, sizeof(b->err), "step did not complete within %.0f s", WAIT_LIMIT_S);
             return CVP9_ERR_GPU;
         }
-        struct timespec ts = { 0, 20000 };
-        nanosleep(&ts, NULL);
+        cvp9_poll_pause(cvp9_now() - t0);
     }
     complete_slot(b, s);
     return CVP9_OK;
@@ -1416,8 +1415,7 @@ cvp9_err_t cvp9_batch_timer_stop(cvp9_batch_t *b, float *ms)
         if (e == cudaSuccess) break;
         if (e != cudaErrorNotReady) return bfail(b, e, "timer");
         if (cvp9_now() - t0 > WAIT_LIMIT_S) return CVP9_ERR_GPU;
-        struct timespec ts = { 0, 20000 };
-        nanosleep(&ts, NULL);
+        cvp9_poll_pause(cvp9_now() - t0);
     }
     BCK(cudaEventElapsedTime(ms, b->ev_t0, b->ev_t1), "timer");
     return CVP9_OK;

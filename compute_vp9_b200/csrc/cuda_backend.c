@@ -4,8 +4,13 @@
  * kernels are reached through the launch shim in recon.cu.
  *
  * Per context:
- *   - one CUDA stream; every frame is upload -> scan/recon/filter -> output
- *     copy on it, so stream order carries all cross-frame hazards;
+ *   - three CUDA streams, uploads, kernels and downloads: while the kernels
+ *     of one frame run, the inputs of the next one arrive and the samples of
+ *     the one before leave (one stream for all three: 0.31 ms a 720p frame,
+ *     of which 0.07 ms are kernels). Per frame the kernels wait for its
+ *     upload and its download for the kernels; the kernels share the
+ *     reference pool and the scratch in stream order, and a device frame is
+ *     written again only after its download (dframe_t.read);
  *   - a device-resident reference pool: up to 8 slots pointing at device
  *     I420 frames (pointer swaps, no copies — the Vulkan backend copies
  *     luma into images, vulkan_backend.c:1310-1354);
@@ -48,40 +53,42 @@ typedef struct {
     size_t   cap;
     int32_t  w, h;
     int      users;       /* reference slots pointing here */
+    cudaEvent_t read;     /* its last download */
 } dframe_t;
 
 typedef struct {
     int          pending;
     int64_t      pts;
     int32_t      w, h;
-    cudaEvent_t  ev_start, ev_k0, ev_k1, ev_end;
+    cudaEvent_t  ev_start, ev_up, ev_k0, ev_k1, ev_end;
     int          tune_idx;             /* tuner bucket this frame measures, -1 none */
     cvp9_tcfg_t  tune_cfg;
-    /* pinned staging */
+    /* pinned staging: the job and the blocks in one piece (JOB_BYTES apart) */
     void        *h_blocks;  size_t h_blocks_cap;
     void        *h_coeffs;  size_t h_coeffs_cap;
-    cvp9_job_t  *h_job;
     uint32_t    *h_status;
     int          out;                  /* output buffer of this frame */
     /* device inputs */
     void        *d_blocks;  size_t d_blocks_cap;
     void        *d_coeffs;  size_t d_coeffs_cap;
-    cvp9_job_t  *d_job;
+    uint32_t    *d_misc;    /* [0] status, [1] ticket counter, [2] filter tickets, from MISC_WORDS
+                             * on 4 * n_sb of sb_range: all zeroed per frame */
 } slot_t;
+
+#define JOB_BYTES  ((sizeof(cvp9_job_t) + 255) & ~(size_t)255)
+#define MISC_WORDS 16
 
 typedef struct {
     int          device;
     int          arith;
-    cudaStream_t stream;
+    cudaStream_t stream, up, down;
     int32_t      W, H;                 /* current geometry */
     int          sb_cols, sb_rows, n_sb;
     dframe_t     frames[MAX_DFRAMES];
     int          ref_slot[8];          /* index into frames, -1 = empty */
     uint32_t     epoch;
     /* per-geometry scratch */
-    uint32_t    *d_sb_range;           /* 4 * n_sb, zeroed per frame    */
     uint32_t    *d_sb_done;            /* n_sb                          */
-    uint32_t    *d_misc;               /* [0] status, [1] ticket counter, [2] filter tickets */
     uint32_t    *d_tickets;
     uint32_t    *d_fast;               /* inter fast path: general flags, tickets, count */
     uint32_t    *d_mi_map;             /* FULL loop filter: mode info per 8x8 MI          */
@@ -110,27 +117,40 @@ static cvp9_err_t fail(cuctx_t *c, cudaError_t e, const char *what)
 static void free_slot(slot_t *s)
 {
     if (s->ev_start) cudaEventDestroy(s->ev_start);
+    if (s->ev_up) cudaEventDestroy(s->ev_up);
     if (s->ev_k0) cudaEventDestroy(s->ev_k0);
     if (s->ev_k1) cudaEventDestroy(s->ev_k1);
     if (s->ev_end) cudaEventDestroy(s->ev_end);
     cudaFreeHost(s->h_blocks);
     cudaFreeHost(s->h_coeffs);
-    cudaFreeHost(s->h_job);
     cudaFreeHost(s->h_status);
     cudaFree(s->d_blocks);
     cudaFree(s->d_coeffs);
-    cudaFree(s->d_job);
+    cudaFree(s->d_misc);
     memset(s, 0, sizeof(*s));
+}
+
+/* every stream of the context, whether or not it was made */
+static cudaError_t drain(cuctx_t *c)
+{
+    cudaError_t e = cudaSuccess, r;
+    cudaStream_t all[3] = { c->up, c->stream, c->down };
+    for (int k = 0; k < 3; k++)
+        if (all[k] && (r = cudaStreamSynchronize(all[k])) != cudaSuccess) e = r;
+    return e;
 }
 
 static void free_geometry(cuctx_t *c)
 {
-    cudaFree(c->d_sb_range);
+    for (int i = 0; i < CVP9_CUDA_INFLIGHT; i++) {
+        cudaFree(c->slots[i].d_misc);
+        c->slots[i].d_misc = NULL;
+    }
     cudaFree(c->d_sb_done);
     cudaFree(c->d_tickets);
     cudaFree(c->d_fast);
     cudaFree(c->d_mi_map);
-    c->d_sb_range = c->d_sb_done = c->d_tickets = c->d_fast = c->d_mi_map = NULL;
+    c->d_sb_done = c->d_tickets = c->d_fast = c->d_mi_map = NULL;
     c->n_tickets = 0;
 }
 
@@ -153,21 +173,26 @@ cvp9_err_t cuda_backend_init_ex(void **out, const cuda_backend_options_t *opt)
     if (c->device >= dev_count || cvp9_device_setup(c->device) != 0) { free(c); return CVP9_ERR_NO_BACKEND; }
     for (int i = 0; i < 8; i++) c->ref_slot[i] = -1;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc((void **)&c->d_misc, 64) != cudaSuccess) {
+        cudaStreamCreateWithFlags(&c->up, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->down, cudaStreamNonBlocking) != cudaSuccess) {
         cuda_backend_destroy(c);
         return CVP9_ERR_GPU;
     }
     for (int i = 0; i < CVP9_CUDA_INFLIGHT; i++) {
         slot_t *s = &c->slots[i];
-        if (cudaEventCreate(&s->ev_start) != cudaSuccess || cudaEventCreate(&s->ev_k0) != cudaSuccess ||
+        if (cudaEventCreate(&s->ev_start) != cudaSuccess ||
+            cudaEventCreateWithFlags(&s->ev_up, cudaEventDisableTiming) != cudaSuccess || cudaEventCreate(&s->ev_k0) != cudaSuccess ||
             cudaEventCreate(&s->ev_k1) != cudaSuccess || cudaEventCreate(&s->ev_end) != cudaSuccess ||
-            cudaMallocHost((void **)&s->h_job, sizeof(cvp9_job_t)) != cudaSuccess ||
-            cudaMallocHost((void **)&s->h_status, 64) != cudaSuccess ||
-            cudaMalloc((void **)&s->d_job, sizeof(cvp9_job_t)) != cudaSuccess) {
+            cudaMallocHost((void **)&s->h_status, 64) != cudaSuccess) {
             cuda_backend_destroy(c);
             return CVP9_ERR_GPU;
         }
     }
+    for (int i = 0; i < MAX_DFRAMES; i++)
+        if (cudaEventCreateWithFlags(&c->frames[i].read, cudaEventDisableTiming) != cudaSuccess) {
+            cuda_backend_destroy(c);
+            return CVP9_ERR_GPU;
+        }
     c->epoch = 0;
     *out = c;
     return CVP9_OK;
@@ -183,13 +208,17 @@ void cuda_backend_destroy(void *ctx)
     cuctx_t *c = (cuctx_t *)ctx;
     if (!c) return;
     cudaSetDevice(c->device);
-    if (c->stream) cudaStreamSynchronize(c->stream);
+    drain(c);
     for (int i = 0; i < CVP9_CUDA_INFLIGHT; i++) free_slot(&c->slots[i]);
     for (int i = 0; i < OUTBUFS; i++) cudaFreeHost(c->outs[i].h);
-    for (int i = 0; i < MAX_DFRAMES; i++) cudaFree(c->frames[i].dev);
+    for (int i = 0; i < MAX_DFRAMES; i++) {
+        cudaFree(c->frames[i].dev);
+        if (c->frames[i].read) cudaEventDestroy(c->frames[i].read);
+    }
     free_geometry(c);
-    cudaFree(c->d_misc);
     if (c->stream) cudaStreamDestroy(c->stream);
+    if (c->up) cudaStreamDestroy(c->up);
+    if (c->down) cudaStreamDestroy(c->down);
     free(c);
 }
 
@@ -198,14 +227,15 @@ void cuda_backend_destroy(void *ctx)
  * into each reference's own extent as the CPU path does). */
 static cvp9_err_t set_geometry(cuctx_t *c, int32_t W, int32_t H)
 {
-    CK(cudaStreamSynchronize(c->stream), "sync before resize");
+    CK(drain(c), "sync before resize");
     free_geometry(c);
     c->W = W;
     c->H = H;
     c->sb_cols = (W + 63) / 64;
     c->sb_rows = (H + 63) / 64;
     c->n_sb = c->sb_cols * c->sb_rows;
-    CK(cudaMalloc((void **)&c->d_sb_range, (size_t)c->n_sb * 16), "alloc sb_range");
+    for (int i = 0; i < CVP9_CUDA_INFLIGHT; i++)
+        CK(cudaMalloc((void **)&c->slots[i].d_misc, (MISC_WORDS + (size_t)c->n_sb * 4) * 4), "alloc sb_range");
     CK(cudaMalloc((void **)&c->d_sb_done, (size_t)c->n_sb * 4), "alloc sb_done");
     CK(cudaMemset(c->d_sb_done, 0, (size_t)c->n_sb * 4), "clear sb_done");
     CK(cudaMalloc((void **)&c->d_tickets, (size_t)c->n_sb * 4), "alloc tickets");
@@ -248,8 +278,8 @@ static cvp9_err_t grow_pinned(cuctx_t *c, void **p, size_t *cap, size_t need)
 static cvp9_err_t grow_device(cuctx_t *c, void **p, size_t *cap, size_t need)
 {
     if (*cap >= need) return CVP9_OK;
-    /* the previous user of this slot's buffer finished (slot not pending
-     * and stream-ordered), so free is safe */
+    /* the previous user of this slot's buffer finished (the slot is not
+     * pending, and a frame that failed to start drained the streams) */
     cudaFree(*p);
     *p = NULL;
     *cap = 0;
@@ -259,7 +289,8 @@ static cvp9_err_t grow_device(cuctx_t *c, void **p, size_t *cap, size_t need)
     return CVP9_OK;
 }
 
-/* A device frame no reference slot uses (stream order makes reuse safe). */
+/* A device frame no reference slot uses. Kernels that read it as a reference
+ * precede the new frame's in their stream; its download is waited for there. */
 static int acquire_dframe(cuctx_t *c, int32_t W, int32_t H)
 {
     size_t need = (size_t)W * H + 2 * (size_t)((W + 1) / 2) * ((H + 1) / 2);
@@ -272,7 +303,7 @@ static int acquire_dframe(cuctx_t *c, int32_t W, int32_t H)
     if (pick < 0) return -1;
     dframe_t *f = &c->frames[pick];
     if (!f->dev || f->cap < need) {
-        if (f->dev) { cudaStreamSynchronize(c->stream); cudaFree(f->dev); }
+        if (f->dev) { drain(c); cudaFree(f->dev); }
         f->dev = NULL;
         f->cap = 0;
         if (cudaMalloc((void **)&f->dev, need) != cudaSuccess) return -1;
@@ -288,6 +319,94 @@ static void set_ref(cuctx_t *c, int slot, int frame)
     if (c->ref_slot[slot] >= 0) c->frames[c->ref_slot[slot]].users--;
     c->ref_slot[slot] = frame;
     if (frame >= 0) c->frames[frame].users++;
+}
+
+/* The frame's upload, kernels and download; its blocks and coefficients are staged. */
+static cvp9_err_t enqueue(cuctx_t *c, const vp9_parsed_frame_t *pf, slot_t *s, outbuf_t *o, int of, cvp9_tcfg_t tc)
+{
+    const int32_t W = c->W, H = c->H;
+    const size_t nbb = (size_t)pf->num_blocks * sizeof(vp9_macroblock_info_t);
+    const size_t ncb = (size_t)pf->num_coeffs * sizeof(int16_t);
+    cvp9_job_t *job = (cvp9_job_t *)s->h_blocks;
+    memset(job, 0, sizeof(*job));
+    cvp9_job_geometry(job, pf);
+    const int full = c->arith == CVP9_ARITH_FULL;
+    if (full) {
+        cvp9_job_full(job, pf);
+        job->mi_map = c->d_mi_map;
+    }
+    job->blocks = (const vp9_macroblock_info_t *)((uint8_t *)s->d_blocks + JOB_BYTES);
+    job->coeffs = (const int16_t *)s->d_coeffs;
+    job->out = c->frames[of].dev;
+    job->nv12 = (uint8_t *)c->pending_target;
+    if (job->lf_tiled && !tc.lf32 && !(W & 3) && !job->nv12) job->lf_tiled = 2;   /* register strips */
+    for (int i = 0; i < 8; i++) {
+        int f = c->ref_slot[i];
+        if (f >= 0) {
+            job->ref[i].plane = c->frames[f].dev;
+            job->ref[i].w = c->frames[f].w;
+            job->ref[i].h = c->frames[f].h;
+        }
+    }
+    job->epoch = ++c->epoch;
+    job->sb_range = s->d_misc + MISC_WORDS;
+    job->sb_done = c->d_sb_done;
+    job->status = s->d_misc;
+
+    cudaStream_t st = c->stream;
+    CK(cudaEventRecord(s->ev_start, c->up), "event");
+    CK(cudaMemcpyAsync(s->d_blocks, s->h_blocks, JOB_BYTES + nbb, cudaMemcpyHostToDevice, c->up), "upload blocks");
+    if (ncb) CK(cudaMemcpyAsync(s->d_coeffs, s->h_coeffs, ncb, cudaMemcpyHostToDevice, c->up), "upload coeffs");
+    CK(cudaMemsetAsync(s->d_misc, 0, (MISC_WORDS + (size_t)c->n_sb * 4) * 4, c->up), "clear status");
+    CK(cudaEventRecord(s->ev_up, c->up), "event");
+    CK(cudaStreamWaitEvent(st, s->ev_up, 0), "wait for the upload");
+    CK(cudaStreamWaitEvent(st, c->frames[of].read, 0), "wait for the frame");
+    CK(cudaEventRecord(s->ev_k0, st), "event");
+
+    cvp9k_launch_t L;
+    memset(&L, 0, sizeof(L));
+    L.jobs = (const cvp9_job_t *)s->d_blocks;
+    L.njobs = 1;
+    L.arith = full ? CVP9_ARITH_SPEC : c->arith;
+    L.max_blocks = (int)pf->num_blocks;
+    L.tickets = c->d_tickets;
+    L.n_tickets = c->n_tickets;
+    L.ticket_counter = s->d_misc + 1;
+    L.recon_ctas = tc.half ? (c->recon_ctas + 1) / 2 : c->recon_ctas;
+    L.lf_tile_h = tc.lf32 ? 32 : 64;
+    if (tc.inter) {
+        L.general = c->d_fast;
+        L.general_tickets = c->d_fast + c->n_sb;
+        L.n_general = c->d_fast + 2 * c->n_sb;
+        L.inter_variant = tc.inter;
+    }
+    if (full) {
+        L.full = 1;
+        L.lf_counter = s->d_misc + 2;
+        L.lf_tickets = (uint32_t)c->sb_rows;
+        L.lf_ctas = c->sb_rows;
+        L.full_nv12_max_px = job->nv12 ? W * H : 0;
+    } else if (job->lf_tiled == 2) {
+        L.lf_strips_x = ((W + 4 + 7) / 8 + 127) / 128;
+        L.lf_strips_y = (H + 4 + 15) / 16;
+    } else if (job->lf_tiled) {
+        L.lf_tiles_x = (W + 4 + 63) / 64;
+        L.lf_tiles_y = (H + 4 + 63) / 64;
+    } else {
+        L.flat_lf_max_w = W;
+        L.flat_lf_max_h = H;
+        L.flat_nv12 = job->nv12 != NULL;
+    }
+    int lrc = cvp9k_launch_frame(&L, st);
+    if (lrc != 0) return fail(c, (cudaError_t)lrc, "launch");
+    CK(cudaEventRecord(s->ev_k1, st), "event");
+    CK(cudaStreamWaitEvent(c->down, s->ev_k1, 0), "wait for the kernels");
+    CK(cudaMemcpyAsync(s->h_status, s->d_misc, 4, cudaMemcpyDeviceToHost, c->down), "download status");
+    CK(cudaMemcpyAsync(o->h, c->frames[of].dev, (size_t)W * H + 2 * (size_t)((W + 1) / 2) * ((H + 1) / 2),
+                       cudaMemcpyDeviceToHost, c->down), "download frame");
+    CK(cudaEventRecord(c->frames[of].read, c->down), "event");
+    CK(cudaEventRecord(s->ev_end, c->down), "event");
+    return CVP9_OK;
 }
 
 cvp9_err_t cuda_decode_frame(void *ctx, const vp9_parsed_frame_t *pf, int64_t pts)
@@ -332,99 +451,28 @@ cvp9_err_t cuda_decode_frame(void *ctx, const vp9_parsed_frame_t *pf, int64_t pt
         if (!c->outs[i].busy && c->outs[i].free_after <= c->decodes) ob = i;
     if (ob < 0) return fail(c, cudaErrorMemoryAllocation, "output buffers");
     outbuf_t *o = &c->outs[ob];
-    if ((err = grow_pinned(c, &s->h_blocks, &s->h_blocks_cap, nbb ? nbb : 64)) ||
+    if ((err = grow_pinned(c, &s->h_blocks, &s->h_blocks_cap, JOB_BYTES + nbb)) ||
         (err = grow_pinned(c, &s->h_coeffs, &s->h_coeffs_cap, ncb ? ncb : 64)) ||
         (err = grow_pinned(c, (void **)&o->h, &o->cap, outb)) ||
-        (err = grow_device(c, &s->d_blocks, &s->d_blocks_cap, nbb ? nbb : 64)) ||
+        (err = grow_device(c, &s->d_blocks, &s->d_blocks_cap, JOB_BYTES + nbb)) ||
         (err = grow_device(c, &s->d_coeffs, &s->d_coeffs_cap, ncb ? ncb : 64)))
         return err;
     /* the parser's arrays are borrowed for this call only: stage them now */
-    if (nbb) cvp9_parallel_memcpy(s->h_blocks, pf->blocks, nbb);
+    if (nbb) cvp9_parallel_memcpy((uint8_t *)s->h_blocks + JOB_BYTES, pf->blocks, nbb);
     if (ncb) cvp9_parallel_memcpy(s->h_coeffs, pf->coeffs, ncb);
 
     int of = acquire_dframe(c, W, H);
     if (of < 0) return fail(c, cudaErrorMemoryAllocation, "frame pool");
 
-    cvp9_job_t *job = s->h_job;
-    memset(job, 0, sizeof(*job));
-    cvp9_job_geometry(job, pf);
-    const int full = c->arith == CVP9_ARITH_FULL;
-    if (full) {
-        cvp9_job_full(job, pf);
-        job->mi_map = c->d_mi_map;
-    }
     cvp9_tcfg_t tc;
     s->tune_idx = cvp9_tuner_pick(&c->tuner, cvp9_tune_key(c->arith, 1, (uint64_t)c->n_sb), 1, &tc);
     s->tune_cfg = tc;
-    job->blocks = (const vp9_macroblock_info_t *)s->d_blocks;
-    job->coeffs = (const int16_t *)s->d_coeffs;
-    job->out = c->frames[of].dev;
-    job->nv12 = (uint8_t *)c->pending_target;
-    if (job->lf_tiled && !tc.lf32 && !(W & 3) && !job->nv12) job->lf_tiled = 2;   /* register strips */
-    for (int i = 0; i < 8; i++) {
-        int f = c->ref_slot[i];
-        if (f >= 0) {
-            job->ref[i].plane = c->frames[f].dev;
-            job->ref[i].w = c->frames[f].w;
-            job->ref[i].h = c->frames[f].h;
-        }
+    if ((err = enqueue(c, pf, s, o, of, tc)) != CVP9_OK) {
+        drain(c);           /* the slot's buffers are free again */
+        return err;
     }
-    job->epoch = ++c->epoch;
-    job->sb_range = c->d_sb_range;
-    job->sb_done = c->d_sb_done;
-    job->status = c->d_misc;
 
-    cudaStream_t st = c->stream;
-    CK(cudaEventRecord(s->ev_start, st), "event");
-    if (nbb) CK(cudaMemcpyAsync(s->d_blocks, s->h_blocks, nbb, cudaMemcpyHostToDevice, st), "upload blocks");
-    if (ncb) CK(cudaMemcpyAsync(s->d_coeffs, s->h_coeffs, ncb, cudaMemcpyHostToDevice, st), "upload coeffs");
-    CK(cudaMemcpyAsync(s->d_job, job, sizeof(*job), cudaMemcpyHostToDevice, st), "upload job");
-    CK(cudaMemsetAsync(c->d_sb_range, 0, (size_t)c->n_sb * 16, st), "clear sb_range");
-    CK(cudaMemsetAsync(c->d_misc, 0, 12, st), "clear status");
-    CK(cudaEventRecord(s->ev_k0, st), "event");
-
-    cvp9k_launch_t L;
-    memset(&L, 0, sizeof(L));
-    L.jobs = s->d_job;
-    L.njobs = 1;
-    L.arith = full ? CVP9_ARITH_SPEC : c->arith;
-    L.max_blocks = (int)pf->num_blocks;
-    L.tickets = c->d_tickets;
-    L.n_tickets = c->n_tickets;
-    L.ticket_counter = c->d_misc + 1;
-    L.recon_ctas = tc.half ? (c->recon_ctas + 1) / 2 : c->recon_ctas;
-    L.lf_tile_h = tc.lf32 ? 32 : 64;
-    if (tc.inter) {
-        L.general = c->d_fast;
-        L.general_tickets = c->d_fast + c->n_sb;
-        L.n_general = c->d_fast + 2 * c->n_sb;
-        L.inter_variant = tc.inter;
-    }
-    if (full) {
-        L.full = 1;
-        L.lf_counter = c->d_misc + 2;
-        L.lf_tickets = (uint32_t)c->sb_rows;
-        L.lf_ctas = c->sb_rows;
-        L.full_nv12_max_px = job->nv12 ? W * H : 0;
-    } else if (job->lf_tiled == 2) {
-        L.lf_strips_x = ((W + 4 + 7) / 8 + 127) / 128;
-        L.lf_strips_y = (H + 4 + 15) / 16;
-    } else if (job->lf_tiled) {
-        L.lf_tiles_x = (W + 4 + 63) / 64;
-        L.lf_tiles_y = (H + 4 + 63) / 64;
-    } else {
-        L.flat_lf_max_w = W;
-        L.flat_lf_max_h = H;
-        L.flat_nv12 = job->nv12 != NULL;
-    }
-    int lrc = cvp9k_launch_frame(&L, st);
-    if (lrc != 0) return fail(c, (cudaError_t)lrc, "launch");
-    CK(cudaEventRecord(s->ev_k1, st), "event");
-    CK(cudaMemcpyAsync(o->h, c->frames[of].dev, outb, cudaMemcpyDeviceToHost, st), "download frame");
-    CK(cudaMemcpyAsync(s->h_status, c->d_misc, 4, cudaMemcpyDeviceToHost, st), "download status");
-    CK(cudaEventRecord(s->ev_end, st), "event");
-
-    /* reference pool update (host bookkeeping; stream order protects reuse) */
+    /* reference pool update (host bookkeeping) */
     if (c->arith != CVP9_ARITH_REFCPU) {
         unsigned refresh = pf->hdr.refresh_frame_flags ? pf->hdr.refresh_frame_flags : 0x01u;
         for (int i = 0; i < 8; i++) if (refresh & (1u << i)) set_ref(c, i, of);
@@ -458,8 +506,7 @@ static cvp9_err_t wait_event(cuctx_t *c, cudaEvent_t ev)
             snprintf(c->last_error, sizeof(c->last_error), "frame did not complete within %.0f s", WAIT_LIMIT_S);
             return CVP9_ERR_GPU;
         }
-        struct timespec ts = { 0, 20000 };
-        nanosleep(&ts, NULL);
+        cvp9_poll_pause(cvp9_now() - t0);
     }
 }
 
