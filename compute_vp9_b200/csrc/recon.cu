@@ -432,11 +432,16 @@ __device__ __forceinline__ void st_task(uint4 *t, int x, int y, int w, int h, in
 constexpr int kMaxTasks = 384;       /* 4x4 TXs of an SB's three planes; 3 x kMaxBlocks */
 constexpr uint32_t kNoQuad = 0xFFFFFFFFu;
 constexpr int kResidGrid = 64 * 64 + 2 * 32 * 32;
-constexpr int kMaxQuads = 2048;      /* 16 a luma row, at most 11 a chroma row */
+constexpr int kMaxQuads = 2048;      /* 16 a luma row, at most 16 a chroma row */
+/* A level's kind of quads fills its last warp in part, and there are no more
+ * of those than tasks; full warps hold 8 (kind 2) or 32 quads. */
+constexpr int kMaxJobs = kMaxTasks + kMaxQuads / 8;
 
 struct IntraWork {
-    uint32_t qtab[kMaxQuads];        /* by level: task | row << 9 | quad << 15 */
-    uint32_t lvlq[kMaxTasks + 1];    /* quads per level, then each level's first */
+    uint2    qtab[kMaxQuads];        /* quads by level and kind (quad_word)  */
+    uint32_t job[kMaxJobs];          /* a warp's quads: first | count - 1 << 11 | kind << 16 */
+    uint32_t lvlq[kMaxTasks][2];     /* quads of each level and kind, then the first of each: 16 bits a kind */
+    uint16_t lvlj[kMaxTasks + 1];    /* first job of each level              */
     uint4    task[kMaxTasks];        /* ITask                                */
     uint16_t lvl[kMaxTasks];
     uint16_t qat[kMaxTasks];         /* a task's first quad in its level     */
@@ -1453,45 +1458,102 @@ __device__ __forceinline__ void intra_tx_levels(IntraWork &W, int ntask, int tid
     for (int i = 0; i < 2; i++) if (have[i]) W.lvl[tid + i * nthreads] = (uint16_t)max(0, lt[i].level);
 }
 
-/* Sort the quads of all tasks by level, whole CTA: W.lvlq[L] .. W.lvlq[L + 1]
- * of W.qtab are level L's. A thread per four-sample group of the SB finds its
+/* How intra_run predicts a task's quads: 0 DC, 1 from the row above and the
+ * left column (V, H, TM), 2 FULL's directional modes, 3 what does not consist
+ * of aligned words (a clipped area, chroma two samples wide, a repeated edge,
+ * no edge at all): as IntraQuad has it. */
+template <int A>
+__device__ __forceinline__ int intra_kind(const ITask &k)
+{
+    const int mode = k.mode();
+    if (A == CVP9_ARITH_FULL && mode >= 3 && mode <= 8) return 2;
+    const bool words = !((k.x() | k.w()) & 3) &&
+                       (A != CVP9_ARITH_SPEC || (k.w() == k.pw() && k.h() == k.ph()));
+    if (!words) return 3;
+    if (mode) return k.acl() >= k.w() - 1 ? 1 : 3;
+    return !((k.y() | k.h() | k.pw() | k.ph()) & 3) && k.acl() >= k.pw() - 1 && k.lcl() >= k.ph() - 1 && k.avail() ? 0 : 3;
+}
+
+/* A quad: x: its place in the tile (13 bits, from luma's (0, 0)), row (6),
+ * column / 4 (4), task (9); y: its row in the left column (11 bits, from
+ * column 0), residual / 4 (11), chroma (1), mode (4). */
+template <class T>
+__device__ __forceinline__ uint2 quad_word(const ITask &k, int t, int r, int q)
+{
+    using V = IntraView<T>;
+    const int p = k.plane(), pitch = p ? kCPitch : kYPitch, y = k.y() + r, x = k.x() + 4 * q;
+    const int at = (p ? V::kU + (p - 1) * V::kUV : 0) + y * pitch + x;
+    const int lf = p ? 1024 + (p - 1) * 512 + (k.x() >> 1) * 32 + y : (k.x() >> 2) * 64 + y;
+    return make_uint2((uint32_t)at | (uint32_t)r << 13 | (uint32_t)q << 19 | (uint32_t)t << 23,
+                      (uint32_t)lf | (uint32_t)(plane_at(p, x, y) >> 2) << 11 | (p ? 1u << 22 : 0u) |
+                      (uint32_t)(k.mode() & 15) << 23);
+}
+
+/* Sort the quads of all tasks by level and kind, whole CTA, and deal each
+ * level's to warps: W.job[W.lvlj[L]] .. W.job[W.lvlj[L + 1]] are level L's,
+ * each of one kind, so that a warp runs one path: a level waits for the
+ * instructions of its longest warp, about 8 cycles each, and not for data.
+ * With all kinds in one warp and places and residuals worked out by the
+ * thread that predicts: three 1080p SPEC pictures, one of them key, 0.84 ms,
+ * eight 10-bit 1080p key pictures 3.05 ms; by kind and prepared a level
+ * ahead: 0.70 and 2.66 ms. A thread per four-sample group of the SB finds its
  * task from the owner map of the cells: W.own of each plane's (FULL), or the
  * block map `cell` of the luma ones, whose chroma groups start at even
  * samples. */
-template <int A, class C>
+template <int A, class T, class C>
 __device__ __forceinline__ void intra_sort(IntraWork &W, const C *cell, int ntask, int tid, int nthreads)
 {
     const int lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i <= kMaxTasks; i += nthreads) W.lvlq[i] = 0;
-    for (int i = tid; i < kMaxQuads; i += nthreads) W.qtab[i] = kNoQuad;
+    for (int i = tid; i < kMaxTasks * 2; i += nthreads) (&W.lvlq[0][0])[i] = 0;
+    for (int i = tid; i < kMaxQuads; i += nthreads) W.qtab[i] = make_uint2(kNoQuad, 0u);
     if (tid == 0) W.nlev = 0;
     __syncthreads();
     int top = 0;
     for (int t = tid; t < ntask; t += nthreads) {
         const ITask k = ld_task(&W.task[t]);
-        W.qat[t] = (uint16_t)atomicAdd(&W.lvlq[W.lvl[t]], (unsigned)(((k.w() + 3) >> 2) * k.h()));
+        const int kind = intra_kind<A>(k), sh = 16 * (kind & 1);
+        W.qat[t] = (uint16_t)(atomicAdd(&W.lvlq[W.lvl[t]][kind >> 1], (unsigned)(((k.w() + 3) >> 2) * k.h()) << sh) >> sh);
         top = max(top, (int)W.lvl[t] + 1);
     }
     top = __reduce_max_sync(0xffffffffu, top);
     if (lane == 0 && top) atomicMax(&W.nlev, top);
     __syncthreads();
     if (warp == 0) {
-        const int nlev = W.nlev, per = (nlev + 31) >> 5, b0 = lane * per;
-        unsigned sum = 0;
-        for (int l = b0; l < b0 + per && l < nlev; l++) sum += W.lvlq[l];
-        unsigned x = sum;
+        const int nlev = W.nlev, per = (nlev + 31) >> 5, b0 = lane * per, b1 = min(b0 + per, nlev);
+        auto jobs = [](unsigned a, unsigned b) {
+            return ((a & 0xffffu) + 31) / 32 + ((a >> 16) + 31) / 32 + ((b & 0xffffu) + 7) / 8 + ((b >> 16) + 31) / 32;
+        };
+        unsigned sum = 0, js = 0;
+        for (int l = b0; l < b1; l++) {
+            const unsigned a = W.lvlq[l][0], b = W.lvlq[l][1];
+            sum += (a & 0xffffu) + (a >> 16) + (b & 0xffffu) + (b >> 16);
+            js += jobs(a, b);
+        }
+        unsigned x = sum | js << 16;         /* at most kMaxQuads, kMaxJobs  */
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned z = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += z;
         }
-        unsigned at = x - sum;
-        for (int l = b0; l < b0 + per && l < nlev; l++) {
-            const unsigned n = W.lvlq[l];
-            W.lvlq[l] = at;
-            at += n;
+        if (lane == 31) W.lvlj[nlev] = (uint16_t)min(x >> 16, (unsigned)kMaxJobs);
+        x -= sum | js << 16;
+        unsigned at = x & 0xffffu, j = x >> 16;
+        for (int l = b0; l < b1; l++) {
+            const unsigned a = W.lvlq[l][0], b = W.lvlq[l][1];
+            unsigned first[4];
+            W.lvlj[l] = (uint16_t)min(j, (unsigned)kMaxJobs);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned n = ((k < 2 ? a : b) >> (16 * (k & 1))) & 0xffffu, step = k == 2 ? 8u : 32u;
+                first[k] = at;
+                for (unsigned i = 0; i < n; i += step, j++)
+                    if (j < (unsigned)kMaxJobs && at + i < (unsigned)kMaxQuads)
+                        W.job[j] = (at + i) | (min(step, n - i) - 1u) << 11 | (unsigned)k << 16;
+                at += n;
+            }
+            W.lvlq[l][0] = first[0] | first[1] << 16;
+            W.lvlq[l][1] = first[2] | first[3] << 16;
         }
-        if (lane == 31) W.lvlq[nlev] = x;
     }
     __syncthreads();
     constexpr int kGroups = A == CVP9_ARITH_FULL ? 1024 + 2 * 256 : 1024 + 2 * 512;
@@ -1519,39 +1581,203 @@ __device__ __forceinline__ void intra_sort(IntraWork &W, const C *cell, int ntas
         const ITask k = ld_task(&W.task[t]);
         const int r = y - k.y(), c = x - k.x();
         if (r >= k.h() || c >= k.w() || (c & 3)) continue;
-        const unsigned at = W.lvlq[W.lvl[t]] + W.qat[t] + (unsigned)(r * ((k.w() + 3) >> 2) + (c >> 2));
-        if (at < (unsigned)kMaxQuads) W.qtab[at] = (uint32_t)t | (uint32_t)r << 9 | (uint32_t)(c >> 2) << 15;
+        const int kind = intra_kind<A>(k);
+        const unsigned at = ((W.lvlq[W.lvl[t]][kind >> 1] >> (16 * (kind & 1))) & 0xffffu) + W.qat[t] +
+                            (unsigned)(r * ((k.w() + 3) >> 2) + (c >> 2));
+        if (at < (unsigned)kMaxQuads) W.qtab[at] = quad_word<T>(k, t, r, c >> 2);
     }
     __syncthreads();
 }
 
-/* The levels, whole CTA: one barrier each. The next level's first quad and
- * its task are loaded before the barrier. */
+__device__ __forceinline__ uint32_t min2_s16(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("min.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+__device__ __forceinline__ uint32_t max2_s16(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("max.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+/* What a lane of intra_run does for a level, before (prepare) and after (run)
+ * the samples it reads are there: four samples of a quad, or one of a
+ * directional mode's, four lanes a quad. A level waits for the instructions
+ * of run, so all that can be is done in prepare; places are bytes from luma's
+ * (0, 0), which shared memory loads take without pointer arithmetic. */
+template <int A, int MAXV, class T>
+struct IntraLane {
+    static constexpr int kPer = 4 / (int)sizeof(T);      /* samples a word   */
+    static constexpr uint32_t kHi = (uint32_t)MAXV << 16 | MAXV;
+    int a0, a1, a2;                  /* edge samples: DC up, left less the words above; V, H, TM: up, left,
+                                      * corner; else E(i) .. E(i + 2)        */
+    int dst, cl;                     /* its sample(s); their column copy (cl[-32]: of the second, chroma) */
+    uint32_t r0, r1;                 /* residuals                            */
+    uint32_t m;                      /* DC: reciprocal; V, H, TM: 0 leaves out the row and the corner; 2: weights */
+    int nu, n;                       /* DC: words of the edge above, of both */
+    int kind;
+    unsigned put;                    /* 1: dst, 2: cl, 4: cl[-32]            */
+    uint32_t word;                   /* quad_word's x                        */
+
+    template <class E>
+    static __device__ __forceinline__ const E &at(const IntraView<T> &V, int off)
+    {
+        return *reinterpret_cast<const E *>(reinterpret_cast<const char *>(V.tile0) + off);
+    }
+    template <class E>
+    static __device__ __forceinline__ void put_at(const IntraView<T> &V, int off, E v)
+    {
+        *reinterpret_cast<E *>(reinterpret_cast<char *>(V.tile0) + off) = v;
+    }
+
+    __device__ __forceinline__ void prepare(const IntraWork &W, const IntraView<T> &V, uint32_t job, int lane)
+    {
+        constexpr int S = (int)sizeof(T);
+        kind = (int)(job >> 16);
+        const int cnt = (int)((job >> 11) & 31u), i0 = kind == 2 ? lane >> 2 : lane;
+        const uint2 d = W.qtab[(job & 2047u) + min(i0, cnt)];
+        const bool have = i0 <= cnt && d.x != kNoQuad;
+        word = d.x;
+        const bool chroma = (d.y >> 22) & 1u;
+        const int pitch = chroma ? kCPitch : kYPitch, r = (int)(d.x >> 13) & 63, q = (int)(d.x >> 19) & 15;
+        const int lf = (int)(d.y & 2047u), left = (int)(reinterpret_cast<const char *>(V.col0) -
+                                                        reinterpret_cast<const char *>(V.tile0)) + lf * S;
+        dst = (int)(d.x & 8191u) * S;
+        const int up = dst - (r + 1) * pitch * S;
+        const int16_t *const rs = V.res + ((d.y >> 11) & 2047u) * 4;
+        put = have;
+        if (kind <= 1) {
+            const uint2 w = *reinterpret_cast<const uint2 *>(rs);
+            /* the samples are clamped: so may the residuals be, and sums stay in 16 bits */
+            constexpr uint32_t lo = (uint32_t)(-MAXV & 0xffff) * 0x10001u;
+            r0 = min2_s16(max2_s16(w.x, lo), kHi);
+            r1 = min2_s16(max2_s16(w.y, lo), kHi);
+            cl = left + (q + 1) * 64 * S;
+            const int c = chroma ? ((lf >> 5) & 15) + 2 * q + 1 : (lf >> 6) + q;
+            if (have && c < 15) put = 3u;
+            if (have && chroma && c < 16) put |= 4u;
+        }
+        if (kind == 0) {
+            const ITask t = ld_task(&W.task[min(d.x >> 23, kMaxTasks - 1u)]);
+            nu = t.avail() & 1u ? t.pw() / kPer : 0;
+            n = nu + (t.avail() & 2u ? t.ph() / kPer : 0);
+            a0 = up - 4 * q * S;
+            a1 = left - r * S - nu * 4;
+            m = t.inv;
+        } else if (kind == 1) {
+            const int mode = (int)(d.y >> 23) & 15;
+            a0 = up;
+            a2 = up - (4 * q + 1) * S;
+            a1 = mode == 1 ? a2 : left;
+            m = mode == 2 ? 0u : 0xFFFFFFFFu;
+        } else if (A == CVP9_ARITH_FULL && kind == 2) {
+            const ITask t = ld_task(&W.task[min(d.x >> 23, kMaxTasks - 1u)]);
+            const int mode = t.mode(), c = 4 * q + (lane & 3), size = t.pw(), acl = t.acl(), lcl = t.lcl();
+            /* the place and the weights, in quarters, of the sample's taps */
+            int i;
+            bool two = false, one = false;
+            if (mode == 3) {
+                i = r + c;
+                one = i + 2 >= 2 * size;
+                if (one) i = 2 * size - 1;
+            } else if (mode == 8) {
+                i = (r >> 1) + c;
+                two = !(r & 1);
+            } else if (mode == 4) {
+                i = c - r - 2;
+            } else if (mode == 5) {
+                const int d5 = r - 2 * c;
+                two = d5 < 2 && !(r & 1);
+                i = d5 >= 2 ? -d5 - 1 : c - (r >> 1) - 2 + !(r & 1);
+            } else if (mode == 6) {
+                const int d6 = c - 2 * r;
+                two = d6 < 2 && !(c & 1);
+                i = d6 >= 2 ? d6 - 3 : (c >> 1) - r - 2;
+            } else {
+                i = -r - (c >> 1) - 4 + !(c & 1);
+                two = !(c & 1);
+            }
+            m = one ? 4u : two ? 2u | 2u << 8 : 1u | 2u << 8 | 1u << 16;
+            const int u = up - 4 * q * S, l = left - r * S;
+            auto E = [&](int k) { return k >= -1 ? u + min(k, acl) * S : l + min(-k - 2, lcl) * S; };
+            a0 = E(i);
+            a1 = E(i + 1);
+            a2 = E(i + 2);
+            r0 = (uint32_t)(int)rs[lane & 3];
+            dst += (lane & 3) * S;
+            const int e = c + 1;
+            cl = left + (chroma ? (e >> 1) * 32 : (e >> 2) * 64) * S;
+            const bool copy = chroma ? !(e & 1) && ((lf >> 5) & 15) + (e >> 1) < 16 : !(e & 3) && (lf >> 6) + (e >> 2) < 16;
+            put = have && c < t.w() ? (copy ? 3u : 1u) : 0u;
+        }
+    }
+
+    __device__ __forceinline__ void run(const IntraWork &W, const IntraView<T> &V, int lane) const
+    {
+        if (kind <= 1) {
+            uint32_t v0, v1;
+            if (kind == 0) {
+                /* the four lanes are of one task: its quads come in fours */
+                unsigned s = 0;
+                for (int j = lane & 3; j < n; j += 4) {
+                    const uint32_t w = at<uint32_t>(V, (j < nu ? a0 : a1) + 4 * j);
+                    s = sizeof(T) == 1 ? __dp4a(w, 0x01010101u, s) : s + (w & 0xffffu) + (w >> 16);
+                }
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                v0 = v1 = __umulhi(s + (unsigned)(n * kPer >> 1), m) * 0x10001u;
+            } else {
+                const uint32_t w0 = at<uint32_t>(V, a0) & m, w1 = sizeof(T) == 1 ? 0u : at<uint32_t>(V, a0 + 4) & m;
+                const uint32_t d = (uint32_t)at<T>(V, a1) - ((uint32_t)at<T>(V, a2) & m), dd = __byte_perm(d, 0u, 0x1010);
+                v0 = sizeof(T) == 1 ? __byte_perm(w0, 0u, 0x4140) : w0;
+                v1 = sizeof(T) == 1 ? __byte_perm(w0, 0u, 0x4342) : w1;
+                v0 = min2_s16(__viaddmax_s16x2(v0, dd, 0u), kHi);
+                v1 = min2_s16(__viaddmax_s16x2(v1, dd, 0u), kHi);
+            }
+            v0 = min2_s16(__viaddmax_s16x2(v0, r0, 0u), kHi);
+            v1 = min2_s16(__viaddmax_s16x2(v1, r1, 0u), kHi);
+            if (put & 1u) {
+                if (sizeof(T) == 1) put_at<uint32_t>(V, dst, __byte_perm(v0, v1, 0x6420));
+                else put_at<uint2>(V, dst, make_uint2(v0, v1));
+            }
+            if (put & 2u) put_at<T>(V, cl, (T)(v1 >> 16));
+            if (put & 4u) put_at<T>(V, cl - 32 * (int)sizeof(T), (T)(v0 >> 16));
+        } else if (A == CVP9_ARITH_FULL && kind == 2) {
+            const int e = at<T>(V, a0) * (int)(m & 255u) + at<T>(V, a1) * (int)((m >> 8) & 255u) + at<T>(V, a2) * (int)(m >> 16);
+            const T v = (T)clampi(((e + 2) >> 2) + (int)r0, 0, MAXV);
+            if (put & 1u) put_at<T>(V, dst, v);
+            if (put & 2u) put_at<T>(V, cl, v);
+        } else if (put) {
+            IntraQuad<T> k;
+            k.load(V, ld_task(&W.task[min(word >> 23, kMaxTasks - 1u)]), (int)(word >> 13) & 63, (int)(word >> 19) & 15);
+            k.template run<A, MAXV>();
+        }
+    }
+};
+
+/* The levels, whole CTA: one barrier each. A warp has a job of a level at
+ * most, in general; odd levels begin at the middle warp, so that the warps
+ * which a level leaves idle prepare the next one. */
 template <int A, int MAXV, class T>
 __device__ __forceinline__ void intra_run(const IntraWork &W, const IntraView<T> &V, int tid, int nthreads)
 {
-    const int nlev = W.nlev;
-    int q = tid, q1 = min((int)W.lvlq[1], kMaxQuads);
-    uint32_t e = q < q1 ? W.qtab[q] : kNoQuad;
-    ITask t = ld_task(&W.task[e != kNoQuad ? e & 511u : 0u]);
+    const int nlev = W.nlev, nw = nthreads >> 5, warp = tid >> 5, lane = tid & 31;
+    IntraLane<A, MAXV, T> k;
+    int j = warp, end = nlev ? W.lvlj[1] : 0;
+    if (j < end) k.prepare(W, V, W.job[j], lane);
     for (int L = 0; L < nlev; L++) {
-        while (q < q1) {
-            if (e != kNoQuad) {
-                IntraQuad<T> k;
-                k.load(V, t, (int)(e >> 9) & 63, (int)(e >> 15));
-                k.template run<A, MAXV>();
-            }
-            q += nthreads;
-            if (q < q1) {
-                e = W.qtab[q];
-                t = ld_task(&W.task[e != kNoQuad ? e & 511u : 0u]);
-            }
+        while (j < end) {
+            k.run(W, V, lane);
+            j += nw;
+            if (j < end) k.prepare(W, V, W.job[j], lane);
         }
         if (L + 1 < nlev) {
-            q = q1 + tid;
-            q1 = min((int)W.lvlq[L + 2], kMaxQuads);
-            e = q < q1 ? W.qtab[q] : kNoQuad;
-            t = ld_task(&W.task[e != kNoQuad ? e & 511u : 0u]);
+            j = end + ((warp + (L & 1 ? 0 : nw >> 1)) & (nw - 1));
+            end = W.lvlj[L + 2];
+            if (j < end) k.prepare(W, V, W.job[j], lane);
         }
         __syncthreads();
     }
@@ -2380,7 +2606,7 @@ __device__ __noinline__ void phase_plan(int nb, int sbx, int sby)
         if (mine) intra_block_tasks<A>(W, s.blk[tid], job, sbx, sby, at, max(0, lt[0].level));
     }
     __syncthreads();
-    intra_sort<A>(W, s.cell, ntask, tid, kThreads);
+    intra_sort<A, uint8_t>(W, s.cell, ntask, tid, kThreads);
 }
 
 template <int A>
@@ -5087,6 +5313,8 @@ struct HbdSmem {
     int      ticket;
 };
 
+static_assert(sizeof(HbdSmem) <= 75 * 1024, "three CTAs per SM");
+
 __device__ __forceinline__ uint16_t &HT(HbdSmem &s, int p, int x, int y)
 {
     return p == 0 ? s.ty[(y + 1) * kHYP + x + 4] : s.tc[p - 1][(y + 1) * kHCP + x + 4];
@@ -5299,7 +5527,7 @@ __device__ __noinline__ void hbd_plan(int nb, int sbx, int sby)
     __syncthreads();
     intra_tx_levels(W, ntask, tid, kHbdThreads);
     __syncthreads();
-    intra_sort<CVP9_ARITH_FULL>(W, s.cell, ntask, tid, kHbdThreads);
+    intra_sort<CVP9_ARITH_FULL, uint16_t>(W, s.cell, ntask, tid, kHbdThreads);
 }
 
 __device__ __noinline__ void hbd_levels()
