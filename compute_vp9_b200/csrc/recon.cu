@@ -72,7 +72,38 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-__device__ __forceinline__ uint32_t tap_round(int acc) { return (uint32_t)clampi((acc + 64) >> 7, 0, 255); }
+/* Saturated and packed, the first in the low bits: one instruction for two
+ * values, where clamping and shifting them in takes five. */
+__device__ __forceinline__ uint32_t pack4_u8(int a, int b, int c, int d)
+{
+    uint32_t hi, r;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(d), "r"(c), "r"(0));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(b), "r"(a), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ uint32_t pack2_s16(int a, int b)
+{
+    uint32_t r;
+    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(r) : "r"(b), "r"(a));
+    return r;
+}
+__device__ __forceinline__ uint32_t min2_s16(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("min.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t max2_s16(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("max.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+/* two 10-bit samples */
+__device__ __forceinline__ uint32_t pack2_u10(int a, int b)
+{
+    return max2_s16(min2_s16(pack2_s16(a, b), 0x03ff03ffu), 0u);
+}
 
 __device__ __forceinline__ int dp4a_su(uint32_t taps, uint32_t px, int c)
 {
@@ -83,9 +114,10 @@ __device__ __forceinline__ int dp4a_su(uint32_t taps, uint32_t px, int c)
 
 /* One 8-tap output from samples s0 (samples 0-3 of the window) and s1
  * (4-7): phase 0 is the centre sample itself. */
-__device__ __forceinline__ uint32_t tap8(uint32_t ta, uint32_t tb, int phase, uint32_t s0, uint32_t s1)
+/* not clamped to a sample yet */
+__device__ __forceinline__ int tap8(uint32_t ta, uint32_t tb, int phase, uint32_t s0, uint32_t s1)
 {
-    return phase ? tap_round(dp4a_su(tb, s1, dp4a_su(ta, s0, 0))) : (s0 >> 24);
+    return phase ? dp4a_su(tb, s1, dp4a_su(ta, s0, 64)) >> 7 : (int)(s0 >> 24);
 }
 
 /* t / d for 0 <= t < 4096 and 1 <= d <= 16 without an integer divide:
@@ -599,12 +631,15 @@ __device__ __forceinline__ void tr4(uint32_t a, uint32_t b, uint32_t c, uint32_t
  * permutes. Both passes round and clip, as vp9_mc.comp.glsl:61-110 does;
  * every fetch is clamped into the reference plane. What bounded this was
  * instructions and L1 requests, not bytes: a warp per chunk with a load per
- * sample took 50 k cycles a superblock (8 bits), a load per tap and sample 75 k
- * (10 bits), this 25 k and 42 k. */
+ * sample took 50 k cycles a superblock (8 bits, SPEC), a load per tap and
+ * sample 75 k (10 bits), this 21 k and 42 k. Samples are clamped and packed by
+ * cvt.pack and stay packed, also where two predictions are averaged: of 29 k
+ * cycles a superblock that took 4 k (FULL). */
 template <class T> struct McRow;
 
 template <> struct McRow<uint8_t> {
     static constexpr int kWords = 4, kLoads = 3;      /* 16 samples; 15 + 7 bytes */
+    static constexpr uint32_t kOne = 0x01010101u;     /* 1 in every sample of a word */
     /* 8 outputs of the horizontal pass, packed as two words */
     static __device__ __forceinline__ void filter(const uint32_t (&w)[4], int f, uint32_t ta, uint32_t tb, uint8_t *d)
     {
@@ -619,23 +654,20 @@ template <> struct McRow<uint8_t> {
         for (int c = 0; c < 12; c++) s[c] = (c & 3) ? __funnelshift_r(w[c >> 2], w[(c >> 2) + 1], 8 * (c & 3)) : w[c >> 2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            uint32_t r[4];
+            int r[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) r[c] = tap_round(dp4a_su(tb, s[4 * h + c + 4], dp4a_su(ta, s[4 * h + c], 0)));
-            o[h] = r[0] | r[1] << 8 | r[2] << 16 | r[3] << 24;
+            for (int c = 0; c < 4; c++) r[c] = dp4a_su(tb, s[4 * h + c + 4], dp4a_su(ta, s[4 * h + c], 64)) >> 7;
+            o[h] = pack4_u8(r[0], r[1], r[2], r[3]);
         }
     }
-    /* output row from the 8 rows at h (8 samples each) */
-    static __device__ __forceinline__ void down(const uint8_t *h, int f, uint32_t ta, uint32_t tb, int (&v)[8])
+    /* output row, packed, from the 8 rows at h (8 samples each) */
+    static __device__ __forceinline__ void down(const uint8_t *h, int f, uint32_t ta, uint32_t tb, uint32_t (&v)[2])
     {
         const uint2 *r = reinterpret_cast<const uint2 *>(h);
         if (f == 0) {
             const uint2 m = r[3];
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                v[c] = (int)((m.x >> (8 * c)) & 255u);
-                v[4 + c] = (int)((m.y >> (8 * c)) & 255u);
-            }
+            v[0] = m.x;
+            v[1] = m.y;
             return;
         }
         uint2 a[8];
@@ -646,8 +678,10 @@ template <> struct McRow<uint8_t> {
             uint32_t lo[4], hi[4];
             tr4(s ? a[0].y : a[0].x, s ? a[1].y : a[1].x, s ? a[2].y : a[2].x, s ? a[3].y : a[3].x, lo);
             tr4(s ? a[4].y : a[4].x, s ? a[5].y : a[5].x, s ? a[6].y : a[6].x, s ? a[7].y : a[7].x, hi);
+            int u[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) v[4 * s + c] = (int)tap_round(dp4a_su(tb, hi[c], dp4a_su(ta, lo[c], 0)));
+            for (int c = 0; c < 4; c++) u[c] = dp4a_su(tb, hi[c], dp4a_su(ta, lo[c], 64)) >> 7;
+            v[s] = pack4_u8(u[0], u[1], u[2], u[3]);
         }
     }
 };
@@ -667,10 +701,10 @@ __device__ __forceinline__ int dp2a_hi_su(uint32_t px, uint32_t taps, int c)
 
 template <> struct McRow<uint16_t> {
     static constexpr int kWords = 8, kLoads = 5;      /* 16 samples; 30 + 6 bytes */
+    static constexpr uint32_t kOne = 0x00010001u;
     static __device__ __forceinline__ int tap(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t ta, uint32_t tb)
     {
-        const int s = dp2a_hi_su(d, tb, dp2a_lo_su(c, tb, dp2a_hi_su(b, ta, dp2a_lo_su(a, ta, 64))));
-        return clampi(s >> 7, 0, 1023);
+        return dp2a_hi_su(d, tb, dp2a_lo_su(c, tb, dp2a_hi_su(b, ta, dp2a_lo_su(a, ta, 64)))) >> 7;
     }
     static __device__ __forceinline__ void filter(const uint32_t (&w)[8], int f, uint32_t ta, uint32_t tb, uint16_t *d)
     {
@@ -685,18 +719,15 @@ template <> struct McRow<uint16_t> {
         uint32_t r[4];
 #pragma unroll
         for (int i = 0; i < 4; i++)
-            r[i] = (uint32_t)tap(w[i], w[i + 1], w[i + 2], w[i + 3], ta, tb) |
-                   (uint32_t)tap(s[i], s[i + 1], s[i + 2], s[i + 3], ta, tb) << 16;
+            r[i] = pack2_u10(tap(w[i], w[i + 1], w[i + 2], w[i + 3], ta, tb), tap(s[i], s[i + 1], s[i + 2], s[i + 3], ta, tb));
         *o = make_uint4(r[0], r[1], r[2], r[3]);
     }
-    static __device__ __forceinline__ void down(const uint16_t *h, int f, uint32_t ta, uint32_t tb, int (&v)[8])
+    static __device__ __forceinline__ void down(const uint16_t *h, int f, uint32_t ta, uint32_t tb, uint32_t (&v)[4])
     {
         const uint4 *r = reinterpret_cast<const uint4 *>(h);
         if (f == 0) {
             const uint4 m = r[3];
-            const uint32_t x[4] = { m.x, m.y, m.z, m.w };
-#pragma unroll
-            for (int i = 0; i < 4; i++) { v[2 * i] = (int)(x[i] & 0xffffu); v[2 * i + 1] = (int)(x[i] >> 16); }
+            v[0] = m.x; v[1] = m.y; v[2] = m.z; v[3] = m.w;
             return;
         }
         int acc[8];
@@ -715,7 +746,7 @@ template <> struct McRow<uint16_t> {
             }
         }
 #pragma unroll
-        for (int c = 0; c < 8; c++) v[c] = clampi(acc[c] >> 7, 0, 1023);
+        for (int i = 0; i < 4; i++) v[i] = pack2_u10(acc[2 * i] >> 7, acc[2 * i + 1] >> 7);
     }
 };
 
@@ -790,9 +821,10 @@ template <class T, bool COMPOUND, class B>
 __device__ __forceinline__ void mc_chunk(const cvp9_job_t &job, const uint32_t (*P)[2], const B &b, bool on, int p, int gx,
                                          int gy, int w, int h, int mid, T *rows, T *dst, int k)
 {
-    int v[8];
+    constexpr int kV = 2 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);
+    uint32_t v[kV];                    /* the row's samples, packed            */
 #pragma unroll
-    for (int c = 0; c < 8; c++) v[c] = mid;
+    for (int c = 0; c < kV; c++) v[c] = (uint32_t)mid * McRow<T>::kOne;
 #pragma unroll 1
     for (int q = 0; q < (COMPOUND ? 2 : 1); q++) {
         const int rf = on ? (q ? b.ref1 : b.ref0) : 0;
@@ -813,26 +845,24 @@ __device__ __forceinline__ void mc_chunk(const cvp9_job_t &job, const uint32_t (
         }
         __syncwarp();
         if (go && k < h) {
-            int u[8];
+            uint32_t u[kV];
             McRow<T>::down(rows + k * 8, m.fy, P[m.fy][0], P[m.fy][1], u);
+            /* (a + b + 1) >> 1 of each sample: a | b less half of a ^ b, no bit crossing into the next */
+            constexpr uint32_t half = ~(McRow<T>::kOne << (8 * sizeof(T) - 1));
 #pragma unroll
-            for (int c = 0; c < 8; c++) v[c] = q ? (v[c] + u[c] + 1) >> 1 : u[c];
+            for (int c = 0; c < kV; c++) v[c] = q ? (v[c] | u[c]) - (((v[c] ^ u[c]) >> 1) & half) : u[c];
         }
         __syncwarp();
     }
     if (k < h) {
         if (w == 8 && !((uintptr_t)dst & 3)) {
             uint32_t *d = reinterpret_cast<uint32_t *>(dst);
-            if (sizeof(T) == 1) {
-                d[0] = (uint32_t)v[0] | (uint32_t)v[1] << 8 | (uint32_t)v[2] << 16 | (uint32_t)v[3] << 24;
-                d[1] = (uint32_t)v[4] | (uint32_t)v[5] << 8 | (uint32_t)v[6] << 16 | (uint32_t)v[7] << 24;
-            } else {
 #pragma unroll
-                for (int i = 0; i < 4; i++) d[i] = (uint32_t)v[2 * i] | (uint32_t)v[2 * i + 1] << 16;
-            }
+            for (int c = 0; c < kV; c++) d[c] = v[c];
         } else {
 #pragma unroll
-            for (int c = 0; c < 8; c++) if (c < w) dst[c] = (T)v[c];
+            for (int c = 0; c < 8; c++)
+                if (c < w) dst[c] = (T)(v[c / kPer] >> (8 * (int)sizeof(T) * (c & (kPer - 1))));
         }
     }
 }
@@ -1589,20 +1619,6 @@ __device__ __forceinline__ void intra_sort(IntraWork &W, const C *cell, int ntas
     __syncthreads();
 }
 
-__device__ __forceinline__ uint32_t min2_s16(uint32_t a, uint32_t b)
-{
-    uint32_t r;
-    asm("min.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-
-__device__ __forceinline__ uint32_t max2_s16(uint32_t a, uint32_t b)
-{
-    uint32_t r;
-    asm("max.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-
 /* What a lane of intra_run does for a level, before (prepare) and after (run)
  * the samples it reads are there: four samples of a quad, or one of a
  * directional mode's, four lanes a quad. A level waits for the instructions
@@ -2319,13 +2335,11 @@ __device__ __forceinline__ void put_residual4(ReconSmem &s, int p, int x, int y,
 {
     if (intra) {
         *reinterpret_cast<uint2 *>(&s.res[plane_at(p, x, y)]) =
-            make_uint2((uint32_t)(r[0] & 0xffff) | (uint32_t)r[1] << 16, (uint32_t)(r[2] & 0xffff) | (uint32_t)r[3] << 16);
+            make_uint2(pack2_s16(r[0], r[1]), pack2_s16(r[2], r[3]));
     } else {
         uint32_t *d = reinterpret_cast<uint32_t *>(p == 0 ? &TY(s, x, y) : &TC(s, p, x, y));
         const uint32_t o = *d;
-        *d = (uint32_t)clampi((int)(o & 255u) + r[0], 0, 255) | (uint32_t)clampi((int)((o >> 8) & 255u) + r[1], 0, 255) << 8 |
-             (uint32_t)clampi((int)((o >> 16) & 255u) + r[2], 0, 255) << 16 |
-             (uint32_t)clampi((int)(o >> 24) + r[3], 0, 255) << 24;
+        *d = pack4_u8((int)(o & 255u) + r[0], (int)((o >> 8) & 255u) + r[1], (int)((o >> 16) & 255u) + r[2], (int)(o >> 24) + r[3]);
     }
 }
 
@@ -2421,7 +2435,7 @@ __device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, i
                 int q[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++)
-                    q[j] = clampi(((int)((unsigned)v[k + j].v + (1u << (sh - 1)))) >> sh, -32768, 32767);
+                    q[j] = ((int)((unsigned)v[k + j].v + (1u << (sh - 1)))) >> sh;
                 put_residual4(s, p, x + k, y + i, q, intra);
             }
         }
@@ -3395,7 +3409,8 @@ __device__ void fast_residual(S &w, uint8_t *dst, int pitch, const cvp9_job_t &j
                 if (have) {
 #pragma unroll
                     for (int j4 = 0; j4 < NJ / 4; j4++) {
-                        uint32_t word = GLOBAL ? pix[j4] : reinterpret_cast<const uint32_t *>(rowp)[j4], outw = 0;
+                        const uint32_t word = GLOBAL ? pix[j4] : reinterpret_cast<const uint32_t *>(rowp)[j4];
+                        int o[4];
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
                             /* round half away from zero; the int16 saturation of
@@ -3403,8 +3418,9 @@ __device__ void fast_residual(S &w, uint8_t *dst, int pitch, const cvp9_job_t &j
                              * the 0..255 clamp that follows, so it is folded in */
                             const int r = __double2int_rz(__dadd_rn(acc[j4 * 4 + e], copysign(0.5, acc[j4 * 4 + e])));
                             const int px = (int)((word >> (8 * e)) & 0xffu);
-                            outw |= (uint32_t)clampi(px + r, 0, 255) << (8 * e);
+                            o[e] = px + r;
                         }
+                        const uint32_t outw = pack4_u8(o[0], o[1], o[2], o[3]);
                         if (words) {
                             reinterpret_cast<uint32_t *>(rowp)[j4] = outw;
                         } else {
@@ -3511,7 +3527,7 @@ __device__ void fast_residual_d(S &w, uint8_t *dst, int pitch, const cvp9_job_t 
 #pragma unroll
             for (int j4 = 0; j4 < N / 4; j4++) {
                 const uint32_t word = GLOBAL ? pix[j4] : reinterpret_cast<const uint32_t *>(rowp)[j4];
-                uint32_t outw = 0;
+                int o[4];
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     /* round half away from zero; the int16 saturation of
@@ -3519,8 +3535,9 @@ __device__ void fast_residual_d(S &w, uint8_t *dst, int pitch, const cvp9_job_t 
                      * the 0..255 clamp that follows, so it is folded in */
                     const int r = __double2int_rz(__dadd_rn(acc[j4 * 4 + e], copysign(0.5, acc[j4 * 4 + e])));
                     const int px = (int)((word >> (8 * e)) & 0xffu);
-                    outw |= (uint32_t)clampi(px + r, 0, 255) << (8 * e);
+                    o[e] = px + r;
                 }
+                const uint32_t outw = pack4_u8(o[0], o[1], o[2], o[3]);
                 if (words) {
                     reinterpret_cast<uint32_t *>(rowp)[j4] = outw;
                 } else {
@@ -3605,15 +3622,12 @@ __device__ void spec_luma_pass(S &w, const PredDst &D, const cvp9_job_t &job, in
                 uint32_t o[4];
                 if (x0 >= 0 && x0 + lw + 6 < rw && y >= 0 && y < rh) ld16w(rp + (size_t)y * rw + x0, o);
                 else ld16c(rp, rw, rw, rh, x0, y, o);
-                uint32_t out0 = 0, out1 = 0;
+                int v[8];
 #pragma unroll
-                for (int cc = 0; cc < 8; cc++) {
-                    const uint32_t v = tap8(ta, tb, fx, win4(o, cc), win4(o, cc + 4));
-                    if (cc < 4) out0 |= v << (8 * cc); else out1 |= v << (8 * (cc - 4));
-                }
+                for (int cc = 0; cc < 8; cc++) v[cc] = tap8(ta, tb, fx, win4(o, cc), win4(o, cc + 4));
                 uint32_t *hrow = reinterpret_cast<uint32_t *>(hb + (q * 15 + hr) * 8);
-                hrow[0] = out0;
-                hrow[1] = out1;
+                hrow[0] = pack4_u8(v[0], v[1], v[2], v[3]);
+                hrow[1] = pack4_u8(v[4], v[5], v[6], v[7]);
             }
         }
     }
@@ -3639,9 +3653,10 @@ __device__ void spec_luma_pass(S &w, const PredDst &D, const cvp9_job_t &job, in
                 uint32_t ca[4], cb[4];
                 tr4(rw8[0], rw8[1], rw8[2], rw8[3], ca);
                 tr4(rw8[4], rw8[5], rw8[6], rw8[7], cb);
-                uint32_t word = 0;
+                int v[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) word |= tap8(va, vb, fy, ca[j], cb[j]) << (8 * j);
+                for (int j = 0; j < 4; j++) v[j] = tap8(va, vb, fy, ca[j], cb[j]);
+                const uint32_t word = pack4_u8(v[0], v[1], v[2], v[3]);
                 if (half) o1 = word; else o0 = word;
             }
         }
@@ -3694,10 +3709,10 @@ __device__ void spec_chroma_pass(S &w, const PredDst &D, const cvp9_job_t &job, 
                 /* a further chroma row exists below: word reads stay inside */
                 if (x0 >= 0 && x0 + clw + 6 < cw2 && y >= 0 && y + 1 < ch2) ld16w(pl + (size_t)y * rcs + x0, o);
                 else ld16c(pl, rcs, cw2, ch2, x0, y, o);
-                uint32_t out = 0;
+                int v[4];
 #pragma unroll
-                for (int cc = 0; cc < 4; cc++) out |= tap8(ta, tb, fx, win4(o, cc), win4(o, cc + 4)) << (8 * cc);
-                *reinterpret_cast<uint32_t *>(hb + ((q * 2 + p) * 11 + hr) * 4) = out;
+                for (int cc = 0; cc < 4; cc++) v[cc] = tap8(ta, tb, fx, win4(o, cc), win4(o, cc + 4));
+                *reinterpret_cast<uint32_t *>(hb + ((q * 2 + p) * 11 + hr) * 4) = pack4_u8(v[0], v[1], v[2], v[3]);
             }
         }
     }
@@ -3705,14 +3720,15 @@ __device__ void spec_chroma_pass(S &w, const PredDst &D, const cvp9_job_t &job, 
     if (c < nchunks && clw > 0 && r < clh) {
         uint32_t o = 0x80808080u;                             /* missing reference: 128 */
         if (pl) {
-            o = 0;
             const uint32_t *hrows = reinterpret_cast<const uint32_t *>(hb + ((q * 2 + p) * 11 + r) * 4);
             uint32_t ca[4], cb[4];
             tr4(hrows[0], hrows[1], hrows[2], hrows[3], ca);
             tr4(hrows[4], hrows[5], hrows[6], hrows[7], cb);
             const uint32_t va = c_subpel_pk[fy][0], vb = c_subpel_pk[fy][1];
+            int v[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) o |= tap8(va, vb, fy, ca[j], cb[j]) << (8 * j);
+            for (int j = 0; j < 4; j++) v[j] = tap8(va, vb, fy, ca[j], cb[j]);
+            o = pack4_u8(v[0], v[1], v[2], v[3]);
         }
         uint8_t *d = (p ? D.v : D.u) + (cy0 + r) * D.pc + cx0;
         if (clw == 4 && !((uintptr_t)d & 3)) {
@@ -3826,12 +3842,11 @@ __device__ void spec_fast_residual(S &w, const PredDst &D, const cvp9_job_t &job
                         for (int e = 0; e < 4; e++)
                             if (4 * j4 + e < xin) word |= (uint32_t)rowp[4 * j4 + e] << (8 * e);
                     }
-                    uint32_t outw = 0;
+                    int o[4];
 #pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const int r = ((int)((unsigned)v[j4 * 4 + e].v + (1u << (sh - 1)))) >> sh;
-                        outw |= (uint32_t)clampi((int)((word >> (8 * e)) & 0xffu) + r, 0, 255) << (8 * e);
-                    }
+                    for (int e = 0; e < 4; e++)
+                        o[e] = (int)((word >> (8 * e)) & 0xffu) + (((int)((unsigned)v[j4 * 4 + e].v + (1u << (sh - 1)))) >> sh);
+                    const uint32_t outw = pack4_u8(o[0], o[1], o[2], o[3]);
                     if (words) {
                         reinterpret_cast<uint32_t *>(rowp)[j4] = outw;
                     } else {
