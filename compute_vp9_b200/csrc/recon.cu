@@ -420,9 +420,9 @@ struct BlkS {
  * prediction has no cases for them.
  * Measured (one B200), against a warp per block with transform and
  * prediction in turn and the inter blocks after the wait: 16x1080p REFCPU
- * key step with its download 3.77 -> 2.82 ms, three FULL 1080p pictures (one
- * key) 21.5 -> 6.0 ms, a step of 24 1366x768 REFCPU inter pictures with 5%
- * intra blocks 2.2 -> 1.4 ms. */
+ * key step with its download 3.77 -> 2.43 ms, three FULL 1080p pictures (one
+ * key) 21.5 -> 2.95 ms, a step of 24 1366x768 REFCPU inter pictures with 5%
+ * intra blocks 2.2 -> 0.92 ms (with the steps noted further down). */
 
 struct ITask {           /* four words, read as one 16-byte load            */
     uint32_t xywh;       /* plane position in the SB tile; samples written   */
@@ -5300,7 +5300,7 @@ __global__ void __launch_bounds__(kLfThreads, 2) k_lf_full(const cvp9_job_t *__r
  * the inter predictions eight lanes a chunk, then every residual, a warp for
  * TXs of one size. The intra blocks follow
  * as in k_recon, TX by TX in dependency levels over the whole CTA (8x1080p
- * key step 15.6 -> 3.9 ms against a warp per block, prediction and
+ * key step 15.6 -> 2.65 ms against a warp per block, prediction and
  * transforms in turn). A superblock whose blocks overlap, or
  * whose intra blocks read samples of blocks later in the list, runs block by
  * block in list order, so every sample is what the list order makes it. */
