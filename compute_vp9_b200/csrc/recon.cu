@@ -5693,8 +5693,11 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
         }
         /* stage the coefficients in the permuted buffer, where 16-byte copies
          * can: every block's start a multiple of 4, the span no longer than the
-         * SB's samples */
+         * SB's samples. The row passes go over the coefficients in place, so
+         * only where no two blocks share any: each block's begin where those
+         * listed before it have ended, or later */
         bool odd = false;
+        unsigned begin, ended;           /* this block's first; the largest end before it */
         {
             unsigned lo = 0xFFFFFFFFu, hi = 0u;
             if (tid < nb && !(s.blk[tid].flags & 2)) {
@@ -5712,12 +5715,26 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
                     odd = b.coeff & 3u;
                 }
             }
+            begin = lo;
+            unsigned most = hi;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, most, o);
+                if (lane >= o) most = max(most, y);
+            }
+            ended = __shfl_up_sync(0xffffffffu, most, 1);
+            if (lane == 0) ended = 0u;
+            if (lane == 31) {
+                s.scan[warp] = (int)most;
+                atomicMax(&s.c_hi, most);
+            }
             lo = __reduce_min_sync(0xffffffffu, lo);
-            hi = __reduce_max_sync(0xffffffffu, hi);
-            if (lane == 0) { atomicMin(&s.c_lo, lo); atomicMax(&s.c_hi, hi); }
+            if (lane == 0) atomicMin(&s.c_lo, lo);
         }
         const bool any_intra = __syncthreads_or(my_intra) != 0;
-        odd = __syncthreads_or(odd) != 0;
+#pragma unroll
+        for (int w = 0; w < kHbdWarps; w++) if (w < warp) ended = max(ended, (unsigned)s.scan[w]);
+        odd = __syncthreads_or(odd || begin < ended) != 0;
         const unsigned c_base = s.c_lo, c_hi = s.c_hi;
         const bool staged = c_hi > c_base && !odd && c_hi <= job.num_coeffs && c_hi - c_base <= (unsigned)kResidGrid &&
                             !((uintptr_t)job.coeffs32 & 15);
