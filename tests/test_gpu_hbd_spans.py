@@ -1,7 +1,7 @@
 """10-bit blocks whose coefficient spans overlap, or lie out of list order.
 The block record asks for neither, so every sample must be the list-order
 oracle's: blocks of a superblock at one offset, spans that share a part,
-offsets exchanged between blocks of one size; DCT beside ADST, inter beside
+offsets exchanged between blocks of one size, gaps; DCT beside ADST, inter beside
 intra, transforms of one warp and of several. Tolerance: none."""
 import numpy as np
 import pytest
@@ -35,12 +35,15 @@ def _respan(pf, how):
                 offsets = [b.coeff_offset for b in same]
                 for b, o in zip(same, offsets[::-1]):
                     b.coeff_offset = o
+        elif how == "gaps":
+            for b in blocks[1::3]:
+                b.skip = 1
         else:
             for b in blocks:
                 b.coeff_offset = first if how == "one" else first + (b.coeff_offset - first) // 8 * 4
 
 
-@pytest.mark.parametrize("how", ["one", "part", "exchanged"])
+@pytest.mark.parametrize("how", ["one", "part", "exchanged", "gaps"])
 @pytest.mark.parametrize("content", list(CONTENT))
 @pytest.mark.parametrize("size", [(64, 64), (136, 72), (328, 200)])
 def test_spans(size, content, how):
