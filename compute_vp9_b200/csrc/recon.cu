@@ -1276,11 +1276,17 @@ struct IntraQuad {
     }
     /* A: the profile; directional modes are FULL's. Every directional sample
      * is a copy, a two-tap or a three-tap average at one place of the edge E:
-     * E(i) = above[i] for i >= -1 (-1 the corner), left[-i - 2] below. */
-    template <int A, int MAXV>
+     * E(i) = above[i] for i >= -1 (-1 the corner), left[-i - 2] below. LIST:
+     * the superblock runs in list order; only there FULL misses an edge that
+     * is not the tile's (a block off the 8x8 grid whose first MI is the
+     * picture's or tile column's first), so that the halo does not hold it. */
+    template <int A, int MAXV, bool LIST>
     __device__ __forceinline__ void run() const
     {
         const int mode = t.mode();
+        const bool no_up = LIST && A == CVP9_ARITH_FULL && !(t.avail() & 1u), no_lf = LIST && A == CVP9_ARITH_FULL && !(t.avail() & 2u);
+        auto above = [&](int i) -> int { return no_up ? MAXV / 2 : no_lf && i < 0 ? MAXV / 2 + 2 : up[min(i, t.acl())]; };
+        auto left = [&](int i) -> int { return no_lf ? MAXV / 2 + 2 : lf[min(i, t.lcl())]; };
         int v[4];
         if (mode == 0) {
             const unsigned av = t.avail(), n = (av & 1u ? t.pw() : 0) + (av & 2u ? t.ph() : 0);
@@ -1290,15 +1296,18 @@ struct IntraQuad {
 #pragma unroll
             for (int i = 0; i < 4; i++) v[i] = (int)dc;
         } else if (A != CVP9_ARITH_FULL || mode == 9 || mode <= 2) {
-            const int l = lf[min(r, t.lcl())], tl = up[-1], acl = t.acl();
+            const int l = left(r), tl = above(-1);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int a = up[min(c0 + i, acl)];
+                const int a = above(c0 + i);
                 v[i] = mode == 1 ? a : mode == 2 ? l : clampi(a + l - tl, 0, MAXV);
             }
         } else {
-            const int n = t.pw(), acl = t.acl(), lcl = t.lcl();
-            auto E = [&](int i) -> int { return *(i >= -1 ? up + min(i, acl) : lf + min(-i - 2, lcl)); };
+            const int n = t.pw();
+            auto E = [&](int i) -> int {
+                if (LIST) return i >= -1 ? above(i) : left(-i - 2);
+                return *(i >= -1 ? up + min(i, t.acl()) : lf + min(-i - 2, t.lcl()));
+            };
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int c = c0 + k;
@@ -1391,7 +1400,8 @@ __device__ __forceinline__ void intra_tx_task(IntraWork &W, const B &b, const cv
     const int ty = div_small(k, nx), tx = k - ty * nx;
     const int lx = (p ? (b.x >> 1) : b.x) + tx * n, ly = (p ? (b.y >> 1) : b.y) + ty * n;
     const int X0 = (p ? (gx >> 1) : gx) + tx * n, Y0 = (p ? (gy >> 1) : gy) + ty * n;
-    const bool top = Y0 > 0, right = n == 4 && (tx + 1) * n < pbw;
+    /* above-right: not past the block's last whole 4x4 (6 samples of chroma have one) */
+    const bool top = ty > 0 || gy >= 8, right = n == 4 && (tx + 1) * n < (pbw & ~3);
     const int avail = (top ? 1 : 0) | (tx > 0 || left_ok ? 2 : 0);
     st_task(&W.task[id], lx, ly, max(0, min(n, min(pw - X0, tile - lx))), max(0, min(n, min(ph - Y0, tile - ly))), p, mode,
             top ? max(1, min(n + (right ? 4 : 0), pw - X0)) - 1 : n - 1, max(0, min(n - 1, ph - 1 - Y0)), avail, n, n,
@@ -1769,7 +1779,7 @@ struct IntraLane {
         } else if (put) {
             IntraQuad<T> k;
             k.load(V, ld_task(&W.task[min(word >> 23, kMaxTasks - 1u)]), (int)(word >> 13) & 63, (int)(word >> 19) & 15);
-            k.template run<A, MAXV>();
+            k.template run<A, MAXV, false>();
         }
     }
 };
@@ -1812,7 +1822,7 @@ __device__ __forceinline__ void intra_run_ordered(const IntraWork &W, const Intr
             const int r = div_small(i, qw);
             IntraQuad<T> quad;
             quad.load(V, k, r, i - r * qw);
-            quad.template run<A, MAXV>();
+            quad.template run<A, MAXV, true>();
         }
         __syncthreads();
     }
