@@ -2218,8 +2218,17 @@ __device__ __noinline__ void phase_inter(int one, int n, int sbx, int sby)
  * 33 k, 5 k of it the list.) */
 template <int N> struct std_int { static constexpr int value = N; };
 
-struct TxRef {       /* x: first coefficient; y: x / 4 | y / 4 << 4 | plane << 8 | TX type << 10 | flags */
-    static constexpr uint32_t kIntra = 1u << 12, kNone = 1u << 13;
+/* x: first coefficient; y: x / 4 | y / 4 << 4 | plane << 8 | TX type << 10 |
+ * flags. LIST: a superblock in list order, the only one with blocks off the
+ * 8x8 grid, whose chroma TXs lie between 4x4 cells: kX2, kY2 two samples on. */
+struct TxRef {
+    static constexpr uint32_t kIntra = 1u << 12, kNone = 1u << 13, kX2 = 1u << 14, kY2 = 1u << 15;
+    template <bool LIST>
+    static __device__ __forceinline__ int x(uint32_t y) { return (int)(y & 15u) * 4 + (LIST && (y & kX2) ? 2 : 0); }
+    template <bool LIST>
+    static __device__ __forceinline__ int y(uint32_t y) { return (int)((y >> 4) & 15u) * 4 + (LIST && (y & kY2) ? 2 : 0); }
+    static __device__ __forceinline__ int plane(uint32_t y) { return (int)(y >> 8) & 3; }
+    static __device__ __forceinline__ int type(uint32_t y) { return (int)(y >> 10) & 3; }
 };
 
 /* Place of word e in a permuted buffer. */
@@ -2231,8 +2240,9 @@ __device__ __forceinline__ int tx_word(int e)
 
 /* List the TXs of blocks [lo, hi), whole CTA: W.tx sorted by size, W.ntx their
  * numbers. layout(b, p, txl, nx, ny): plane p's TXs of block b (0 for a
- * skipped one); type(b, p, txl): the TX type. Barriers inside and at the end. */
-template <class S, class L, class Y>
+ * skipped one); type(b, p, txl): the TX type. LIST: the SB runs in list order.
+ * Barriers inside and at the end. */
+template <bool LIST, class S, class L, class Y>
 __device__ __forceinline__ void list_txs(S &s, int lo, int hi, int nb, uint32_t num_coeffs, int tid, int nthreads, L layout,
                                          Y type)
 {
@@ -2279,7 +2289,8 @@ __device__ __forceinline__ void list_txs(S &s, int lo, int hi, int nb, uint32_t 
             if (to < kMaxTasks)
                 s.tx[to] = make_uint2((uint32_t)co, (uint32_t)(x >> 2) | (uint32_t)(y >> 2) << 4 | (uint32_t)p << 8 |
                                                         (uint32_t)type(m, p, txl) << 10 |
-                                                        (m.flags & 1 ? TxRef::kIntra : 0u) | (none ? TxRef::kNone : 0u));
+                                                        (m.flags & 1 ? TxRef::kIntra : 0u) | (none ? TxRef::kNone : 0u) |
+                                                        (LIST ? (uint32_t)(x & 2) << 13 | (uint32_t)(y & 2) << 14 : 0u));
         });
     }
     __syncthreads();
@@ -2341,9 +2352,20 @@ __device__ __forceinline__ void row_coeffs(int (&c)[N], const int16_t *row)
 }
 
 /* Four residuals, each within int16, of a row of an intra block into the
- * grid, of an inter block onto its samples (x a multiple of 4). */
+ * grid, of an inter block onto its samples. x: even, and a multiple of 4
+ * unless LIST. */
+template <bool LIST>
 __device__ __forceinline__ void put_residual4(ReconSmem &s, int p, int x, int y, const int (&r)[4], bool intra)
 {
+    if (LIST) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            uint8_t &d = p == 0 ? TY(s, x + k, y) : TC(s, p, x + k, y);
+            if (intra) s.res[plane_at(p, x + k, y)] = (int16_t)clampi(r[k], -32768, 32767);
+            else d = (uint8_t)clampi((int)d + r[k], 0, 255);
+        }
+        return;
+    }
     if (intra) {
         *reinterpret_cast<uint2 *>(&s.res[plane_at(p, x, y)]) =
             make_uint2(pack2_s16(r[0], r[1]), pack2_s16(r[2], r[3]));
@@ -2360,14 +2382,14 @@ __device__ __forceinline__ void put_residual4(ReconSmem &s, int p, int x, int y,
  * by the TX type, WHT when lossless. Then the rounding shift 4/5/6/6 (none
  * after the WHT); added to an inter block's samples, left in the grid, saturated
  * to int16 (which no sum with a sample notices), for an intra one. */
-template <int A, int N>
+template <int A, int N, bool LIST>
 __device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, int count, bool staged, unsigned c_base, int lane)
 {
     const cvp9_job_t &job = s.jc;
     const int sub = lane / N, i = lane & (N - 1);
     const bool on = sub < count;
     const uint2 tx = s.tx[first + (on ? sub : 0)];
-    const int p = (int)(tx.y >> 8) & 3, type = (int)(tx.y >> 10) & 3;
+    const int p = TxRef::plane(tx.y), type = TxRef::type(tx.y);
     const bool go = on && !(tx.y & TxRef::kNone);
     const int16_t *X = staged ? s.coef + (tx.x - c_base) : job.coeffs + tx.x;
     wi v[N];
@@ -2414,7 +2436,7 @@ __device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, i
     }
     __syncwarp();
     if (mine) {
-        const int x = (int)(tx.y & 15u) * 4, y = (int)((tx.y >> 4) & 15u) * 4;
+        const int x = TxRef::x<LIST>(tx.y), y = TxRef::y<LIST>(tx.y);
         const bool intra = tx.y & TxRef::kIntra;
         const int sh = N == 4 ? 4 : (N == 8 ? 5 : 6);
         if (A == CVP9_ARITH_FULL) {
@@ -2447,22 +2469,23 @@ __device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, i
 #pragma unroll
                 for (int j = 0; j < 4; j++)
                     q[j] = ((int)((unsigned)v[k + j].v + (1u << (sh - 1)))) >> sh;
-                put_residual4(s, p, x + k, y + i, q, intra);
+                put_residual4<LIST>(s, p, x + k, y + i, q, intra);
             }
         }
     }
     __syncwarp();
 }
 
-/* SPEC and FULL: every residual of blocks [lo, hi) of the SB. Barriers at both ends. */
-template <int A>
+/* SPEC and FULL: every residual of blocks [lo, hi) of the SB. LIST: it runs in
+ * list order, the only one for blocks off the 8x8 grid. Barriers at both ends. */
+template <int A, bool LIST>
 __device__ __noinline__ void phase_residual(int lo, int hi, bool staged, unsigned c_base, int sbx, int sby)
 {
     ReconSmem &s = smem_as<ReconSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int k = tid; k < kResidGrid / 8; k += kThreads) reinterpret_cast<uint4 *>(s.res)[k] = make_uint4(0u, 0u, 0u, 0u);
     const cvp9_job_t &job = s.jc;
-    list_txs(s, lo, hi, hi, job.num_coeffs, tid, kThreads,
+    list_txs<LIST>(s, lo, hi, hi, job.num_coeffs, tid, kThreads,
              [&](const BlkS &b, int p, int &txl, int &nx, int &ny) {
                  txl = b.ptxl[p];
                  nx = b.pnx[p];
@@ -2473,7 +2496,7 @@ __device__ __noinline__ void phase_residual(int lo, int hi, bool staged, unsigne
                             ? (int)c_tx_type[b.ymode] : 0;
              });
     deal_txs(s.ntx, 1, warp, kWarps, [&](auto n, int first, int count, int) {
-        tx_unit<A, decltype(n)::value>(s, s.temp.tx[warp], first, count, staged, c_base, lane);
+        tx_unit<A, decltype(n)::value, LIST>(s, s.temp.tx[warp], first, count, staged, c_base, lane);
     });
     __syncthreads();
 }
@@ -2555,7 +2578,7 @@ __device__ __forceinline__ void ref_tx_unit(ReconSmem &s, int first, int count, 
         }
     }
     if (!any) return;
-    const int px = (int)(tx.y & 15u) * 4 + j0, py = (int)((tx.y >> 4) & 15u) * 4 + i;
+    const int px = TxRef::x<false>(tx.y) + j0, py = TxRef::y<false>(tx.y) + i;
     const bool intra = tx.y & TxRef::kIntra;
 #pragma unroll
     for (int j = 0; j < kCols; j += 4) {
@@ -2565,7 +2588,7 @@ __device__ __forceinline__ void ref_tx_unit(ReconSmem &s, int first, int count, 
             const double v = acc[j + q];
             r[q] = clampi(__double2int_rz(__dadd_rn(v, v >= 0.0 ? 0.5 : -0.5)), -32768, 32767);
         }
-        put_residual4(s, 0, px + j, py, r, intra);
+        put_residual4<false>(s, 0, px + j, py, r, intra);
     }
 }
 
@@ -2575,7 +2598,7 @@ __device__ __noinline__ void phase_residual_ref(int lo, int hi, bool staged, uns
     ReconSmem &s = smem_as<ReconSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int k = tid; k < kResidGrid / 8; k += kThreads) reinterpret_cast<uint4 *>(s.res)[k] = make_uint4(0u, 0u, 0u, 0u);
-    list_txs(s, lo, hi, hi, s.jc.num_coeffs, tid, kThreads,
+    list_txs<false>(s, lo, hi, hi, s.jc.num_coeffs, tid, kThreads,
              [&](const BlkS &b, int p, int &txl, int &nx, int &ny) {
                  txl = b.ptxl[p];
                  nx = b.pnx[p];
@@ -2929,7 +2952,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
             if (n_chunks) phase_inter<A>(-1, n_chunks, sbx, sby);
             cp_async_wait_all();
             if (A == CVP9_ARITH_REFCPU) phase_residual_ref(0, nb, staged, c_base);
-            else phase_residual<A>(0, nb, staged, c_base, sbx, sby);
+            else phase_residual<A, false>(0, nb, staged, c_base, sbx, sby);
             if (any_intra) {
                 /* 4. the intra tasks and their levels; 5. the neighbours'
                  * samples, then level by level */
@@ -2945,7 +2968,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
                 const bool intra = s.blk[b].flags & 1;
                 if (!intra) phase_inter<A>(b, block_chunks<A>(s.blk[b]), sbx, sby);
                 if (A == CVP9_ARITH_REFCPU) phase_residual_ref(b, b + 1, staged, c_base);
-                else phase_residual<A>(b, b + 1, staged, c_base, sbx, sby);
+                else phase_residual<A, true>(b, b + 1, staged, c_base, sbx, sby);
                 if (intra) phase_ordered<A>(b, sbx, sby);
             }
         }
@@ -5424,11 +5447,11 @@ __device__ __noinline__ void hbd_predict(int lo, int hi, int nb, int sbx, int sb
  * 4/5/6/6 (none after the WHT); an inter block's residual is added and clipped
  * to 10 bits, an intra block's goes to the grid, saturated to int16, which no
  * sum with a sample notices. c: the lane's row, at: its TX's place. */
-template <int N, class T>
+template <int N, class T, bool LIST>
 __device__ __forceinline__ void hbd_tx_passes(HbdSmem &s, const int (&c)[N], int at, uint2 tx, bool any, bool mine, int i)
 {
     const bool lossless = s.jc.lossless;
-    const int p = (int)(tx.y >> 8) & 3, type = (int)(tx.y >> 10) & 3;
+    const int p = TxRef::plane(tx.y), type = TxRef::type(tx.y);
     const bool wht = N == 4 && lossless;
     int32_t *buf = s.tmp.i;
     T v[N];
@@ -5449,7 +5472,7 @@ __device__ __forceinline__ void hbd_tx_passes(HbdSmem &s, const int (&c)[N], int
         if (wht) iwht4(v, false);
         else itx1<N>(v, type & 1);
         const int sh = wht ? 0 : N == 4 ? 4 : (N == 8 ? 5 : 6), round = wht ? 0 : 1 << (sh - 1);
-        const int x = (int)(tx.y & 15u) * 4 + i, y = (int)((tx.y >> 4) & 15u) * 4;
+        const int x = TxRef::x<LIST>(tx.y) + i, y = TxRef::y<LIST>(tx.y);
         const bool intra = tx.y & TxRef::kIntra;
         int16_t *r = s.res + plane_at(p, x, y);
         uint16_t *d = &HT(s, p, x, y);
@@ -5464,20 +5487,20 @@ __device__ __forceinline__ void hbd_tx_passes(HbdSmem &s, const int (&c)[N], int
     }
 }
 
-template <int N>
+template <int N, bool LIST>
 __device__ __noinline__ void hbd_tx_wide(int at, uint2 tx, bool any, bool mine, int i)
 {
     HbdSmem &s = smem_as<HbdSmem>();
     int c[N];
     for (int k = 0; k < N; k++) c[k] = s.tmp.i[tx_word(at + i * N + k)];
     __syncwarp();
-    hbd_tx_passes<N, wl>(s, c, at, tx, any, mine, i);
+    hbd_tx_passes<N, wl, LIST>(s, c, at, tx, any, mine, i);
 }
 
 /* The butterflies run on 32-bit values (wn) unless one of the warp's
  * coefficients is outside +-2^18 (a 10-bit stream's reach +-2^17): then on
  * 64-bit ones (wl), with the same results. */
-template <int N>
+template <int N, bool LIST>
 __device__ __forceinline__ void hbd_tx_unit(HbdSmem &s, int first, int count, bool staged, unsigned c_base, int slot, int lane)
 {
     const int sub = lane / N, i = lane & (N - 1);
@@ -5506,21 +5529,22 @@ __device__ __forceinline__ void hbd_tx_unit(HbdSmem &s, int first, int count, bo
     const uint32_t live = __ballot_sync(0xffffffffu, any != 0);
     if (live) {
         const bool mine = go && (N == 32 || ((live >> (sub * N)) & ((1u << (N & 31)) - 1u)));
-        if (__any_sync(0xffffffffu, wide != 0)) hbd_tx_wide<N>(at, tx, any != 0, mine, i);
-        else hbd_tx_passes<N, wn>(s, c, at, tx, any != 0, mine, i);
+        if (__any_sync(0xffffffffu, wide != 0)) hbd_tx_wide<N, LIST>(at, tx, any != 0, mine, i);
+        else hbd_tx_passes<N, wn, LIST>(s, c, at, tx, any != 0, mine, i);
     }
     __syncwarp();
 }
 
 /* Every residual of blocks [lo, hi) of the SB, whole CTA; staged: their
  * coefficients are in the permuted buffer, from c_base on. */
+template <bool LIST>
 __device__ __noinline__ void hbd_residual(int lo, int hi, int nb, bool staged, unsigned c_base, int sbx, int sby)
 {
     HbdSmem &s = smem_as<HbdSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const cvp9_job_t &job = s.jc;
     for (int i = tid; i < kResidGrid / 8; i += kHbdThreads) reinterpret_cast<uint4 *>(s.res)[i] = make_uint4(0u, 0u, 0u, 0u);
-    list_txs(s, lo, hi, nb, job.num_coeffs, tid, kHbdThreads,
+    list_txs<LIST>(s, lo, hi, nb, job.num_coeffs, tid, kHbdThreads,
              [&](const HbdBlk &b, int p, int &txl, int &nx, int &ny) {
                  int pbw;
                  plane_layout(b, job, sbx + b.x, sby + b.y, p, txl, nx, ny, pbw);
@@ -5535,7 +5559,7 @@ __device__ __noinline__ void hbd_residual(int lo, int hi, int nb, bool staged, u
         constexpr int N = decltype(n)::value;
         const int before = N == 32 ? 0 : N == 16 ? n32 * 1024 : N == 8 ? n32 * 1024 + n16 * 256 : n32 * 1024 + n16 * 256 + n8 * 64;
         const int skip = N == 32 ? 0 : N == 16 ? n32 : N == 8 ? n32 + n16 : n32 + n16 + n8;
-        hbd_tx_unit<N>(s, first, count, staged, c_base, before + (first - skip) * N * N, lane);
+        hbd_tx_unit<N, LIST>(s, first, count, staged, c_base, before + (first - skip) * N * N, lane);
     });
     __syncthreads();
 }
@@ -5787,7 +5811,7 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
             hbd_predict(0, nb, nb, sbx, sby);
             cp_async_wait_all();
             __syncthreads();
-            hbd_residual(0, nb, nb, staged, c_base, sbx, sby);
+            hbd_residual<false>(0, nb, nb, staged, c_base, sbx, sby);
             if (any_intra) {
                 hbd_plan(nb, sbx, sby);
                 hbd_intra(s.needs, sb, sbx, sby);
@@ -5798,7 +5822,7 @@ __global__ void __launch_bounds__(kHbdThreads, 3) k_hbd_recon(const cvp9_job_t *
             if (any_intra) hbd_neighbours(7u, sb);
             for (int i = 0; i < nb; i++) {
                 hbd_predict(i, i + 1, nb, sbx, sby);
-                hbd_residual(i, i + 1, nb, false, 0u, sbx, sby);
+                hbd_residual<true>(i, i + 1, nb, false, 0u, sbx, sby);
                 if (s.blk[i].flags & 1) hbd_ordered(i, sbx, sby);
             }
         }

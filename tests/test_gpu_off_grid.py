@@ -18,7 +18,7 @@ from oracle.oracle_py import FULL, REFCPU, SPEC, HbdOracleStream, OracleStream
 pytestmark = pytest.mark.gpu
 
 HBD = 3
-CONTENT = ["skipped"]
+CONTENT = ["skipped", "4x4"]
 
 
 def _split(rng, x, y, w, h, out):
