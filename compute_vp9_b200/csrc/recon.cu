@@ -2240,9 +2240,11 @@ __device__ __forceinline__ int tx_word(int e)
 
 /* List the TXs of blocks [lo, hi), whole CTA: W.tx sorted by size, W.ntx their
  * numbers. layout(b, p, txl, nx, ny): plane p's TXs of block b (0 for a
- * skipped one); type(b, p, txl): the TX type. LIST: the SB runs in list order.
- * Barriers inside and at the end. */
-template <bool LIST, class S, class L, class Y>
+ * skipped one); type(b, p, txl): the TX type. LIST: the SB runs in list order;
+ * only there TXs reach past their block, some past the SB, where the passes
+ * clip them. GRID: residuals of intra blocks go to the grid. Barriers inside
+ * and at the end. */
+template <bool LIST, bool GRID, class S, class L, class Y>
 __device__ __forceinline__ void list_txs(S &s, int lo, int hi, int nb, uint32_t num_coeffs, int tid, int nthreads, L layout,
                                          Y type)
 {
@@ -2285,11 +2287,11 @@ __device__ __forceinline__ void list_txs(S &s, int lo, int hi, int nb, uint32_t 
             const int x = (p ? m.x >> 1 : m.x) + (k - ty * nx) * n, y = (p ? m.y >> 1 : m.y) + ty * n;
             const int to = s.tx_at[p][b] + k + (txl < 3 ? n32 : 0) + (txl < 2 ? n16 : 0) + (txl < 1 ? n8 : 0);
             const uint64_t co = off + ((uint64_t)k << (4 + 2 * txl));
-            const bool none = co + (uint64_t)(n * n) > (uint64_t)num_coeffs || x + n > tile || y + n > tile;
+            const bool none = co + (uint64_t)(n * n) > (uint64_t)num_coeffs || (!LIST && (x + n > tile || y + n > tile));
             if (to < kMaxTasks)
                 s.tx[to] = make_uint2((uint32_t)co, (uint32_t)(x >> 2) | (uint32_t)(y >> 2) << 4 | (uint32_t)p << 8 |
                                                         (uint32_t)type(m, p, txl) << 10 |
-                                                        (m.flags & 1 ? TxRef::kIntra : 0u) | (none ? TxRef::kNone : 0u) |
+                                                        (GRID && (m.flags & 1) ? TxRef::kIntra : 0u) | (none ? TxRef::kNone : 0u) |
                                                         (LIST ? (uint32_t)(x & 2) << 13 | (uint32_t)(y & 2) << 14 : 0u));
         });
     }
@@ -2352,17 +2354,18 @@ __device__ __forceinline__ void row_coeffs(int (&c)[N], const int16_t *row)
 }
 
 /* Four residuals, each within int16, of a row of an intra block into the
- * grid, of an inter block onto its samples. x: even, and a multiple of 4
- * unless LIST. */
+ * grid, of an inter block onto its samples (x a multiple of 4). LIST: onto the
+ * samples in either case, clipped to the SB (x even). */
 template <bool LIST>
 __device__ __forceinline__ void put_residual4(ReconSmem &s, int p, int x, int y, const int (&r)[4], bool intra)
 {
     if (LIST) {
+        const int tile = p ? 32 : 64;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
+            if (x + k >= tile || y >= tile) continue;
             uint8_t &d = p == 0 ? TY(s, x + k, y) : TC(s, p, x + k, y);
-            if (intra) s.res[plane_at(p, x + k, y)] = (int16_t)clampi(r[k], -32768, 32767);
-            else d = (uint8_t)clampi((int)d + r[k], 0, 255);
+            d = (uint8_t)clampi((int)d + r[k], 0, 255);
         }
         return;
     }
@@ -2439,6 +2442,7 @@ __device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, i
         const int x = TxRef::x<LIST>(tx.y), y = TxRef::y<LIST>(tx.y);
         const bool intra = tx.y & TxRef::kIntra;
         const int sh = N == 4 ? 4 : (N == 8 ? 5 : 6);
+        const int tile = p ? 32 : 64;
         if (A == CVP9_ARITH_FULL) {
 #pragma unroll
             for (int k = 0; k < N; k++) v[k] = wi(buf[tx_word(sub * N * N + k * N + i)]);
@@ -2450,6 +2454,7 @@ __device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, i
 #pragma unroll
             for (int k = 0; k < N; k++) {
                 const int q = wht ? v[k].v : ((int)((unsigned)v[k].v + (1u << (sh - 1)))) >> sh;
+                if (LIST && (x + i >= tile || y + k >= tile)) continue;
                 if (intra) r[k * rp] = (int16_t)clampi(q, -32768, 32767);
                 else d[k * dp] = (uint8_t)clampi((int)d[k * dp] + q, 0, 255);
             }
@@ -2477,7 +2482,9 @@ __device__ __forceinline__ void tx_unit(ReconSmem &s, int32_t *buf, int first, i
 }
 
 /* SPEC and FULL: every residual of blocks [lo, hi) of the SB. LIST: it runs in
- * list order, the only one for blocks off the 8x8 grid. Barriers at both ends. */
+ * list order, the only one for blocks off the 8x8 grid or smaller than their
+ * transforms. There SPEC adds an intra block's residual after its prediction,
+ * since it may reach past what is predicted. Barriers at both ends. */
 template <int A, bool LIST>
 __device__ __noinline__ void phase_residual(int lo, int hi, bool staged, unsigned c_base, int sbx, int sby)
 {
@@ -2485,7 +2492,7 @@ __device__ __noinline__ void phase_residual(int lo, int hi, bool staged, unsigne
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int k = tid; k < kResidGrid / 8; k += kThreads) reinterpret_cast<uint4 *>(s.res)[k] = make_uint4(0u, 0u, 0u, 0u);
     const cvp9_job_t &job = s.jc;
-    list_txs<LIST>(s, lo, hi, hi, job.num_coeffs, tid, kThreads,
+    list_txs<LIST, !(LIST && A == CVP9_ARITH_SPEC)>(s, lo, hi, hi, job.num_coeffs, tid, kThreads,
              [&](const BlkS &b, int p, int &txl, int &nx, int &ny) {
                  txl = b.ptxl[p];
                  nx = b.pnx[p];
@@ -2598,7 +2605,7 @@ __device__ __noinline__ void phase_residual_ref(int lo, int hi, bool staged, uns
     ReconSmem &s = smem_as<ReconSmem>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int k = tid; k < kResidGrid / 8; k += kThreads) reinterpret_cast<uint4 *>(s.res)[k] = make_uint4(0u, 0u, 0u, 0u);
-    list_txs<false>(s, lo, hi, hi, s.jc.num_coeffs, tid, kThreads,
+    list_txs<false, true>(s, lo, hi, hi, s.jc.num_coeffs, tid, kThreads,
              [&](const BlkS &b, int p, int &txl, int &nx, int &ny) {
                  txl = b.ptxl[p];
                  nx = b.pnx[p];
@@ -2962,14 +2969,17 @@ __global__ void __launch_bounds__(kThreads, 3) k_recon(const cvp9_job_t *__restr
         } else {
             /* list order, block by block */
             cp_async_wait_all();
+            if (A == CVP9_ARITH_SPEC)        /* what phase_ordered adds there */
+                for (int k = tid; k < kResidGrid / 8; k += kThreads) reinterpret_cast<uint4 *>(s.res)[k] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
             if (any_intra) phase_neighbours<A>(7u, sb);
             for (int b = 0; b < nb; b++) {
                 const bool intra = s.blk[b].flags & 1;
                 if (!intra) phase_inter<A>(b, block_chunks<A>(s.blk[b]), sbx, sby);
+                if (A == CVP9_ARITH_SPEC && intra) phase_ordered<A>(b, sbx, sby);
                 if (A == CVP9_ARITH_REFCPU) phase_residual_ref(b, b + 1, staged, c_base);
                 else phase_residual<A, true>(b, b + 1, staged, c_base, sbx, sby);
-                if (intra) phase_ordered<A>(b, sbx, sby);
+                if (A != CVP9_ARITH_SPEC && intra) phase_ordered<A>(b, sbx, sby);
             }
         }
 
@@ -5481,6 +5491,7 @@ __device__ __forceinline__ void hbd_tx_passes(HbdSmem &s, const int (&c)[N], int
         for (int k = 0; k < N; k++) {
             const auto q = (v[k].v + round) >> sh;
             const int e = q < -32768 ? -32768 : (q > 32767 ? 32767 : (int)q);
+            if (LIST && (x >= (p ? 32 : 64) || y + k >= (p ? 32 : 64))) continue;
             if (intra) r[k * rp] = (int16_t)e;
             else d[k * dp] = (uint16_t)clampi((int)d[k * dp] + e, 0, kHbdMax);
         }
@@ -5544,7 +5555,7 @@ __device__ __noinline__ void hbd_residual(int lo, int hi, int nb, bool staged, u
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const cvp9_job_t &job = s.jc;
     for (int i = tid; i < kResidGrid / 8; i += kHbdThreads) reinterpret_cast<uint4 *>(s.res)[i] = make_uint4(0u, 0u, 0u, 0u);
-    list_txs<LIST>(s, lo, hi, nb, job.num_coeffs, tid, kHbdThreads,
+    list_txs<LIST, true>(s, lo, hi, nb, job.num_coeffs, tid, kHbdThreads,
              [&](const HbdBlk &b, int p, int &txl, int &nx, int &ny) {
                  int pbw;
                  plane_layout(b, job, sbx + b.x, sby + b.y, p, txl, nx, ny, pbw);

@@ -1,9 +1,15 @@
-"""Blocks off the 8x8 grid. No parser makes them, but the layout checks take
-them: such a superblock runs in list order, and its samples are the list-order
-oracle's. Tolerance: none.
+"""Blocks off the 8x8 grid, and blocks whose transforms reach past them. No
+parser makes them, but the layout checks take them: such a superblock runs in
+list order, and its samples are the list-order oracle's. Tolerance: none.
 
 CONTENT: "skipped" has predictions alone (edges by MI, chroma of 6 samples),
-"4x4" the smallest transforms too (chroma between 4x4 cells)."""
+"4x4" the smallest transforms too (chroma between 4x4 cells), "any" those
+that are no divisor of the block, or larger (10 bits: not larger), some across
+the superblock's edge. FULL and 10 bits predict by transform and so read edges
+past the superblock there: a picture of one superblock only. Blocks are
+shuffled, so that transforms reach over finished ones; not in larger pictures
+of "any", where the oracle's reach into superblocks that shuffled blocks would
+read before their prediction."""
 import ctypes as C
 import random
 
@@ -18,7 +24,7 @@ from oracle.oracle_py import FULL, REFCPU, SPEC, HbdOracleStream, OracleStream
 pytestmark = pytest.mark.gpu
 
 HBD = 3
-CONTENT = ["skipped", "4x4"]
+CONTENT = ["skipped", "4x4", "any"]
 
 
 def _split(rng, x, y, w, h, out):
@@ -43,12 +49,16 @@ def _frame(rng, header, arith, w, h, key, content):
         for sx in range(0, w, 64):
             rects = []
             _split(rng, 0, 0, 64, 64, rects)
-            rng.shuffle(rects)
+            if content != "any" or w <= 64:
+                rng.shuffle(rects)
             for x, y, bw, bh in rects:
                 if sx + x >= w or sy + y >= h:
                     continue
+                tx = rng.randrange(4) if content == "any" else 0
+                if arith == HBD:
+                    tx = min(tx, 1 if min(bw, bh) < 16 else 2 if min(bw, bh) < 32 else 3)
                 intra = key or rng.random() < 0.4
-                b = BlockInfo(x=sx + x, y=sy + y, width=bw, height=bh, tx_size=0, is_intra=int(intra),
+                b = BlockInfo(x=sx + x, y=sy + y, width=bw, height=bh, tx_size=tx, is_intra=int(intra),
                               y_mode=rng.randrange(10), uv_mode=rng.randrange(10),
                               skip=int(content == "skipped" or rng.random() < 0.2), coeff_offset=coeffs)
                 b.ref_frame[0] = 0 if intra else rng.randrange(1, 4)
@@ -79,6 +89,8 @@ def _frame(rng, header, arith, w, h, key, content):
                                          (ARITH_FULL, (136, 72)), (HBD, (64, 64)), (HBD, (136, 72))])
 def test_off_grid(arith, size, content, seed):
     w, h = size
+    if content == "any" and arith in (ARITH_FULL, HBD) and w > 64:
+        pytest.skip("edges past the superblock")
     rng = random.Random(seed * 1000 + w)
     syn = Synth(synth_config(2, w, h, seed=seed, gop=2, **({} if arith == ARITH_REFCPU else {"interp_filter": 0})))
     if arith == HBD:
