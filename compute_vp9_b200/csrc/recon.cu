@@ -2107,13 +2107,15 @@ __device__ __forceinline__ void intra_block_tasks(IntraWork &W, const BlkS &b, c
     }
 }
 
-/* The tile of the superblock into the picture, clipped to it. */
+/* The tile of the superblock into the picture, clipped to it: as words where the
+ * picture's address (a caller's own, any) and its rows are multiples of 4. */
 __device__ __forceinline__ void recon_write(ReconSmem &s, int sbx, int sby, int tid)
 {
     const cvp9_job_t &job = s.jc;
     const int vw = min(64, job.W - sbx), vh = min(64, job.H - sby);
     uint8_t *Y = job.out;
-    if ((job.W & 3) == 0) {
+    const bool aligned = !((uintptr_t)Y & 3);
+    if (aligned && (job.W & 3) == 0) {
         for (int i = tid; i < vh * 16; i += kThreads) {
             int r = i >> 4, c4 = (i & 15) * 4;
             if (c4 >= vw) continue;
@@ -2129,7 +2131,7 @@ __device__ __forceinline__ void recon_write(ReconSmem &s, int sbx, int sby, int 
     const int cvw = min(32, job.CW - (sbx >> 1)), cvh = min(32, job.CH - (sby >> 1));
     uint8_t *U = job.out + (size_t)job.W * job.H;
     uint8_t *V = U + (size_t)job.CW * job.CH;
-    if ((job.CW & 3) == 0 && ((size_t)job.W * job.H & 3) == 0) {
+    if (aligned && (job.CW & 3) == 0 && ((size_t)job.W * job.H & 3) == 0) {
         for (int i = tid; i < 2 * cvh * 8; i += kThreads) {
             int p = i >= cvh * 8;
             int k = p ? i - cvh * 8 : i;
