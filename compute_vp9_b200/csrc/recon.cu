@@ -756,8 +756,10 @@ template <class T>
 __device__ __forceinline__ void mc_load(const T *row, int X, int pw, uint32_t (&w)[McRow<T>::kWords])
 {
     constexpr int kW = McRow<T>::kWords, kL = McRow<T>::kLoads, kPer = 4 / (int)sizeof(T);
-    if (X >= 0 && X + 16 + 8 / (int)sizeof(T) <= pw) {   /* every byte read is the row's */
-        const uintptr_t at = (uintptr_t)(row + X);
+    const uintptr_t at = (uintptr_t)(row + X);
+    /* every byte read is the row's, which may begin anywhere: the loads begin
+     * up to 7 bytes before sample X and end up to 8 after the 16 */
+    if (X * (int)sizeof(T) >= (int)(at & 7) && X + 16 + 8 / (int)sizeof(T) <= pw) {
         const uint2 *q = reinterpret_cast<const uint2 *>(at & ~(uintptr_t)7);
         uint32_t u[2 * kL];
 #pragma unroll
