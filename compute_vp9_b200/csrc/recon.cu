@@ -1847,11 +1847,14 @@ __device__ __forceinline__ void intra_fill_cols(const IntraView<T> &V, int tid, 
 /* The halo of a superblock, whole CTA: the row above (x = -1 .. 63) and the
  * left column of each plane, from the picture where `top` / `left` say that
  * they are available, else the profile's fill values (above, left). The
- * corner is a sample only where both are. */
+ * corner is a sample only where both are. need: the neighbours whose samples
+ * are read (intra_needs) and that have been waited for; the others' may still
+ * be in the middle of being written, and are left alone. */
 template <class T>
 __device__ __forceinline__ void intra_halo(const IntraView<T> &V, const cvp9_job_t &job, int sbx, int sby, bool top,
-                                           bool left, int fill_a, int fill_l, int tid, int nthreads)
+                                           bool left, unsigned need, int fill_a, int fill_l, int tid, int nthreads)
 {
+    const bool load_t = top && (need & 2u), load_l = left && (need & 1u), load_c = top && left && (need & 4u);
     const T *base = reinterpret_cast<const T *>(job.out);
     /* 128 samples above, 128 to the left: one each for 256 threads, and the
      * corner for three of them at the same time */
@@ -1864,12 +1867,12 @@ __device__ __forceinline__ void intra_halo(const IntraView<T> &V, const cvp9_job
         const int pitch = p ? kCPitch : kYPitch;
         if (!half) {
             T c = (T)(top ? fill_l : fill_a);
-            if (k == 0 && top && left) c = __ldcg(g + (size_t)(Y - 1) * w + X - 1);
-            const T v = top ? (X + k < w ? __ldcg(g + (size_t)(Y - 1) * w + X + k) : (T)0) : (T)fill_a;
+            if (k == 0 && load_c) c = __ldcg(g + (size_t)(Y - 1) * w + X - 1);
+            const T v = load_t ? (X + k < w ? __ldcg(g + (size_t)(Y - 1) * w + X + k) : (T)0) : (T)fill_a;
             tile[-pitch + k] = v;
             if (k == 0) tile[-pitch - 1] = c;
         } else {
-            const T v = left ? (Y + k < h ? __ldcg(g + (size_t)(Y + k) * w + X - 1) : (T)0) : (T)fill_l;
+            const T v = load_l ? (Y + k < h ? __ldcg(g + (size_t)(Y + k) * w + X - 1) : (T)0) : (T)fill_l;
             col[k] = v;
             tile[k * pitch - 1] = v;
         }
@@ -2707,7 +2710,7 @@ __device__ __forceinline__ void wait_halo(S &s, const IntraView<T> &V, unsigned 
             atomicOr(job.status, (unsigned)CVP9_JOB_TIMEOUT);
     }
     __syncthreads();
-    intra_halo<T>(V, job, sbc * 64, sbr * 64, sbr > 0, have_l, fill_a, fill_l, tid, nthreads);
+    intra_halo<T>(V, job, sbc * 64, sbr * 64, sbr > 0, have_l, need, fill_a, fill_l, tid, nthreads);
     __syncthreads();
 }
 
