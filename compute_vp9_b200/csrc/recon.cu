@@ -51,7 +51,14 @@ constexpr int kYPitch = 72;          /* luma tile row pitch; x = 0 at byte 4 */
 constexpr int kCPitch = 40;          /* chroma tile row pitch; x = 0 at byte 4 */
 constexpr int kTyBytes = (65 * kYPitch + 15) / 16 * 16;
 constexpr int kTcBytes = (33 * kCPitch + 15) / 16 * 16;
-constexpr long long kSpinLimit = 1ll << 20;   /* ~0.25 s of polling */
+/* Looks at a flag before a wait gives up, and what one takes (measured, ns):
+ * superblocks' flags (wait_flag) 0.9 s in all, the loop filter's rows
+ * (wait_at_least) 1.1 s, its counts in shared memory (lf_wait) 2.1 s: who waits
+ * for these waits for a thread that may itself be waiting for a row. */
+constexpr int kFlagLooks = 1 << 22, kRowLooks = 1 << 21, kShmLooks = 1 << 24;
+constexpr double kFlagLookNs = 213, kRowLookNs = 512, kShmLookNs = 128;
+static_assert(kShmLooks * kShmLookNs > 1.5 * kRowLooks * kRowLookNs && kFlagLooks * kFlagLookNs > 0.5e9,
+              "an inner wait outlasts the one it depends on; none gives up within half a second");
 
 __constant__ double c_dct[16 + 64 + 256 + 1024];      /* N = 4, 8, 16, 32 */
 /* The basis again in global memory: lane-varying reads are served by L1
@@ -1936,7 +1943,7 @@ __device__ __forceinline__ void st_release(unsigned *p, unsigned v)
 /* Bounded wait until flag == epoch; returns false on timeout. */
 __device__ __forceinline__ bool wait_flag(const unsigned *flag, unsigned epoch)
 {
-    for (long long it = 0; it < kSpinLimit; it++) {
+    for (int it = 0; it < kFlagLooks; it++) {
         if (ld_acquire(flag) == epoch) return true;
         __nanosleep(32);
     }
@@ -5026,7 +5033,7 @@ __device__ __forceinline__ int lf_unit_edge(const LfGeom &job, int plane, int ux
 
 __device__ bool wait_at_least(const unsigned *flag, unsigned v)
 {
-    for (long long it = 0; it < kSpinLimit; it++) {
+    for (int it = 0; it < kRowLooks; it++) {
         if (ld_acquire(flag) >= v) return true;
         __nanosleep(it < 64 ? 32 : 256);
     }
@@ -5061,8 +5068,8 @@ __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.ar
 /* Bounded wait on a shared-memory count. */
 __device__ __forceinline__ bool lf_wait(const volatile int *count, int v)
 {
-    for (long long it = 0; *count < v; it++) {
-        if (it >= kSpinLimit) return false;
+    for (int it = 0; *count < v; it++) {
+        if (it >= kShmLooks) return false;
         if (it > 64) __nanosleep(64);
     }
     __threadfence_block();
@@ -5221,12 +5228,12 @@ __global__ void __launch_bounds__(kLfThreads, 2) k_lf_full(const cvp9_job_t *__r
                 }
                 if (++k == 10) { k = 0; c++; }
                 /* the next step's first horizontal edges need the rows above */
-                if (ph10 == 1 && row > 0 && cc < ncols) ok &= lf_wait(&s.halo, cc + 1);
+                if (ph10 == 1 && row > 0 && cc < ncols) ok = ok && lf_wait(&s.halo, cc + 1);
                 bar_sync(kBarStep, kLfWork);
                 if (ph10 == 7) {
                     /* superblock cc - 1 is final; cc + 1 must be there, and the
                      * copying warps past the last of these barriers */
-                    ok &= lf_wait(&s.body, cc + 2);
+                    ok = ok && lf_wait(&s.body, cc + 2);
                     bar_arrive(kBarCycle, kLfWork + kLfCopy);
                 }
                 if (++ph10 == 10) { ph10 = 0; cc++; }
@@ -5236,10 +5243,11 @@ __global__ void __launch_bounds__(kLfThreads, 2) k_lf_full(const cvp9_job_t *__r
             /* the 8 rows above, as the row above publishes them */
             const int ht = tid - kLfWork, r = ht >> 3, v = ht & 7;
             const unsigned *const prev = job.sb_range + 4 * (size_t)(row - 1) * ncols + 3;
+            bool ok = true;                  /* a wait that gave up is not repeated */
             for (int c = 0; row > 0 && c < ncols; c++) {
                 const int slot = c & 3;
-                bool ok = c < 4 || lf_wait(&s.done, c - 3);      /* its slot is free */
-                if (ht == 0) ok &= wait_at_least(prev, (unsigned)c + 1u);
+                ok = ok && (c < 4 || lf_wait(&s.done, c - 3));   /* its slot is free */
+                if (ht == 0) ok = ok && wait_at_least(prev, (unsigned)c + 1u);
                 if (!ok) atomicOr(status, (unsigned)CVP9_JOB_TIMEOUT);
                 bar_sync(kBarHalo, kLfHalo);
                 const int x = c * 64 + 8 * v, xc = c * 32 + 4 * v;
