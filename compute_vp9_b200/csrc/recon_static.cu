@@ -151,7 +151,10 @@ extern "C" cvp9_err_t cuda_reconstruct_noalloc(const vp9_parsed_frame_t *pf,
     job.epoch = 1;
     job.sb_range = (uint32_t *)(base + kOffRange);
     job.sb_done = (uint32_t *)(base + kOffDone);
-    job.status = status_dev ? status_dev : (uint32_t *)(base + kOffMisc) + 1;
+    /* the kernels write the caller's word in place; one that is not on a word
+     * boundary gets a copy at the end */
+    const bool in_place = status_dev && !((uintptr_t)status_dev & 3);
+    job.status = in_place ? status_dev : (uint32_t *)(base + kOffMisc) + 1;
 
     /* the array keeps the previous call's contents */
     k_prepare<<<(n_sb + 255) / 256, 256, 0, st>>>(job, (cvp9_job_t *)(base + kOffJob), (uint32_t *)(base + kOffMisc),
@@ -178,5 +181,9 @@ extern "C" cvp9_err_t cuda_reconstruct_noalloc(const vp9_parsed_frame_t *pf,
         L.flat_lf_max_w = W;
         L.flat_lf_max_h = H;
     }
-    return cvp9k_launch_frame(&L, st) == 0 ? CVP9_OK : CVP9_ERR_GPU;
+    if (cvp9k_launch_frame(&L, st) != 0) return CVP9_ERR_GPU;
+    if (status_dev && !in_place &&
+        cudaMemcpyAsync(status_dev, base + kOffMisc + 4, 4, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+        return CVP9_ERR_GPU;
+    return CVP9_OK;
 }

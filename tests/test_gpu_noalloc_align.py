@@ -1,7 +1,7 @@
 """cuda_reconstruct_noalloc on a caller's memory at any byte: frames carved out of
-a pool at odd offsets, which the next picture takes as references, must be
-those at aligned addresses. Sizes: rows of whole words and odd ones, chroma
-rows of whole words and not. Tolerance: none."""
+a pool at odd offsets, which the next picture takes as references, and status
+words, must be those at aligned addresses. Sizes: rows of whole words and odd
+ones, chroma rows of whole words and not. Tolerance: none."""
 import ctypes as C
 
 import numpy as np
@@ -28,7 +28,7 @@ def _decode(arith, w, h, offset):
     fn, n = _call(), i420_size(w, h)
     syn = Synth(synth_config(2, w, h, seed=5, gop=60, intra_in_inter=0.1, interp_filter=0, mv_range_px=48))
     pools = [torch.full((n + 2 * GUARD,), 0xA5, dtype=torch.uint8, device="cuda") for _ in range(3)]
-    status = torch.full((3,), -1, dtype=torch.int32, device="cuda")
+    status = torch.full((8 * 3 + 8,), 0xA5, dtype=torch.uint8, device="cuda")
     sizes = (C.c_uint32 * 8)(*([w] * 8)), (C.c_uint32 * 8)(*([h] * 8))
     keep, refs = [], (C.c_void_p * 8)()
     for f in range(3):
@@ -43,10 +43,12 @@ def _decode(arith, w, h, offset):
         pf.coeffs = C.cast(C.c_void_p(coeffs.data_ptr()), C.POINTER(C.c_int16))
         torch.cuda.synchronize()
         out = pools[f].data_ptr() + GUARD + offset
-        assert fn(C.byref(pf), refs, *sizes, out, arith, status.data_ptr() + 4 * f, None) == CVP9_OK
+        assert fn(C.byref(pf), refs, *sizes, out, arith, status.data_ptr() + 8 * f + offset, None) == CVP9_OK
         refs = (C.c_void_p * 8)(*([out] * 8))
     torch.cuda.synchronize()
-    assert status.cpu().tolist() == [0, 0, 0]
+    status = status.cpu().numpy()
+    assert all((status[8 * f + offset:8 * f + offset + 4] == 0).all() for f in range(3))
+    assert (status == 0xA5).sum() == 8 * 3 + 8 - 12
     for p in pools:
         p = p.cpu().numpy()
         assert (p[:GUARD + offset] == 0xA5).all() and (p[GUARD + offset + n:] == 0xA5).all()
