@@ -13,6 +13,9 @@
 #include <stdlib.h>
 #include <string.h>
 #include <time.h>
+#if defined(__linux__)
+#include <sys/prctl.h>
+#endif
 
 static const int16_t k_dc_q[256] = CVP9_QTABLE_DC_INIT;
 static const int16_t k_ac_q[256] = CVP9_QTABLE_AC_INIT;
@@ -197,13 +200,16 @@ double cvp9_now(void)
 
 void cvp9_poll_pause(double waited)
 {
-    if (waited < 200e-6) {
-#if defined(__x86_64__)
-        for (int k = 0; k < 16; k++) __builtin_ia32_pause();
-#endif
+    struct timespec ts = { 0, waited < 200e-6 ? 10000 : 20000 };
+#if defined(__linux__)
+    const int slack = waited < 200e-6 ? prctl(PR_GET_TIMERSLACK, 0, 0, 0, 0) : 0;
+    if (slack > 1) {
+        prctl(PR_SET_TIMERSLACK, 1, 0, 0, 0);
+        nanosleep(&ts, NULL);
+        prctl(PR_SET_TIMERSLACK, slack, 0, 0, 0);
         return;
     }
-    struct timespec ts = { 0, 20000 };
+#endif
     nanosleep(&ts, NULL);
 }
 
