@@ -2106,8 +2106,8 @@ __device__ __forceinline__ void intra_block_tasks(IntraWork &W, const BlkS &b, c
         const int mode = A == CVP9_ARITH_REFCPU ? (m <= 2 ? m : 9) : (m == 0 || m == 2 || m == 9 ? m : 1);
         const int pw = p ? (b.cw + 1) >> 1 : b.cw, ph = p ? (b.ch + 1) >> 1 : b.ch;
         int w = pw, h = ph;
-        if (A == CVP9_ARITH_SPEC && (b.w < 8 || b.h < 8)) {   /* the residual's area: the whole MI */
-            const int ow = min(8, job.W - (sbx + b.x)), oh = min(8, job.H - (sby + b.y));
+        if (A == CVP9_ARITH_SPEC && (b.w < 8 || b.h < 8)) {   /* the residual's area too: the whole MI */
+            const int ow = max((int)b.cw, min(8, job.W - (sbx + b.x))), oh = max((int)b.ch, min(8, job.H - (sby + b.y)));
             w = p ? (ow + 1) >> 1 : ow;
             h = p ? (oh + 1) >> 1 : oh;
         }
@@ -2196,15 +2196,15 @@ __device__ __forceinline__ IntraView<uint8_t> recon_view(ReconSmem &s)
 
 /* The 4x4 cells of a block: its prediction area; under SPEC and FULL a
  * sub-8x8 block's residual spans the whole 8x8 MI (vp9_kf_tile.c:327-330),
- * so it owns that area too. */
+ * so it owns that area too (a block 4 samples wide may be taller than it). */
 template <int A>
 __device__ __forceinline__ void block_cells(const BlkS &b, const cvp9_job_t &job, int sbx, int sby, int &c0x, int &c1x,
                                             int &c0y, int &c1y)
 {
     int ow = b.cw, oh = b.ch;
     if (A != CVP9_ARITH_REFCPU && (b.w < 8 || b.h < 8)) {
-        ow = min(8, job.W - (sbx + b.x));
-        oh = min(8, job.H - (sby + b.y));
+        ow = max(ow, min(8, job.W - (sbx + b.x)));
+        oh = max(oh, min(8, job.H - (sby + b.y)));
     }
     c0x = b.x >> 2;
     c0y = b.y >> 2;

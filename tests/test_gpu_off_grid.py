@@ -1,6 +1,7 @@
-"""Blocks off the 8x8 grid, and blocks whose transforms reach past them. No
-parser makes them, but the layout checks take them: such a superblock runs in
-list order, and its samples are the list-order oracle's. Tolerance: none.
+"""Blocks off the 8x8 grid, blocks whose transforms reach past them, blocks 4
+samples wide and more than 8 tall. No parser makes them, but the layout checks
+take them: the first two kinds run in list order, and all samples are the
+list-order oracle's. Tolerance: none.
 
 CONTENT: "skipped" has predictions alone (edges by MI, chroma of 6 samples),
 "4x4" the smallest transforms too (chroma between 4x4 cells), "any" those
@@ -9,7 +10,8 @@ the superblock's edge. FULL and 10 bits predict by transform and so read edges
 past the superblock there: a picture of one superblock only. Blocks are
 shuffled, so that transforms reach over finished ones; not in larger pictures
 of "any", where the oracle's reach into superblocks that shuffled blocks would
-read before their prediction."""
+read before their prediction. "narrow" has blocks on the 8x8 grid, many of them
+cut to 4 samples in one direction."""
 import ctypes as C
 import random
 
@@ -24,22 +26,22 @@ from oracle.oracle_py import FULL, REFCPU, SPEC, HbdOracleStream, OracleStream
 pytestmark = pytest.mark.gpu
 
 HBD = 3
-CONTENT = ["skipped", "4x4", "any"]
+CONTENT = ["skipped", "4x4", "any", "narrow"]
 
 
-def _split(rng, x, y, w, h, out):
-    """Rectangles of at least 8x8 at multiples of 4."""
+def _split(rng, x, y, w, h, out, step):
+    """Rectangles of at least 8x8 at multiples of `step`."""
     cuts = [c for c, n in (("w", w), ("h", h)) if n >= 16]
     if not cuts or (w <= 40 and h <= 40 and rng.random() < 0.3):
         out.append((x, y, w, h))
     elif rng.choice(cuts) == "w":
-        k = rng.randrange(8, w - 7, 4)
-        _split(rng, x, y, k, h, out)
-        _split(rng, x + k, y, w - k, h, out)
+        k = rng.randrange(8, w - 7, step)
+        _split(rng, x, y, k, h, out, step)
+        _split(rng, x + k, y, w - k, h, out, step)
     else:
-        k = rng.randrange(8, h - 7, 4)
-        _split(rng, x, y, w, k, out)
-        _split(rng, x, y + k, w, h - k, out)
+        k = rng.randrange(8, h - 7, step)
+        _split(rng, x, y, w, k, out, step)
+        _split(rng, x, y + k, w, h - k, out, step)
 
 
 def _frame(rng, header, arith, w, h, key, content):
@@ -48,13 +50,16 @@ def _frame(rng, header, arith, w, h, key, content):
     for sy in range(0, h, 64):
         for sx in range(0, w, 64):
             rects = []
-            _split(rng, 0, 0, 64, 64, rects)
+            _split(rng, 0, 0, 64, 64, rects, 8 if content == "narrow" else 4)
             if content != "any" or w <= 64:
                 rng.shuffle(rects)
             for x, y, bw, bh in rects:
                 if sx + x >= w or sy + y >= h:
                     continue
                 tx = rng.randrange(4) if content == "any" else 0
+                if content == "narrow" and rng.random() < 0.5:
+                    bw, bh = (4, bh) if rng.random() < 0.5 else (bw, 4)
+                    tx = rng.randrange(2)
                 if arith == HBD:
                     tx = min(tx, 1 if min(bw, bh) < 16 else 2 if min(bw, bh) < 32 else 3)
                 intra = key or rng.random() < 0.4
