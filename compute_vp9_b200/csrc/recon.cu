@@ -119,9 +119,8 @@ __device__ __forceinline__ int dp4a_su(uint32_t taps, uint32_t px, int c)
     return d;
 }
 
-/* One 8-tap output from samples s0 (samples 0-3 of the window) and s1
- * (4-7): phase 0 is the centre sample itself. */
-/* not clamped to a sample yet */
+/* One 8-tap output from samples s0 (samples 0-3 of the window) and s1 (4-7),
+ * not clamped to a sample yet; phase 0 is the centre sample itself. */
 __device__ __forceinline__ int tap8(uint32_t ta, uint32_t tb, int phase, uint32_t s0, uint32_t s1)
 {
     return phase ? dp4a_su(tb, s1, dp4a_su(ta, s0, 64)) >> 7 : (int)(s0 >> 24);
@@ -547,10 +546,6 @@ __device__ __forceinline__ int max_tx_for(int w, int h)
     return m >= 32 ? 3 : (m >= 16 ? 2 : (m >= 8 ? 1 : 0));
 }
 
-/* Residual TX layout of one block (plane TX size, TXs per row, TX count).
- * REFCPU: luma only, counts from the frame-clamped size
- * (vp9_reconstruct.c:336-347). SPEC: every plane in the tile parser's layout
- * (vp9_kf_tile.c:320-396): coded area clipped at the MI-aligned frame edge. */
 /* The tile parser's TX layout of one plane of a block (vp9_kf_tile.c:
  * 320-396): TX size, TXs per row and per column over the coded area clipped
  * at the MI-aligned frame edge, and the plane block width (sub-8x8 blocks
@@ -579,6 +574,9 @@ __device__ __forceinline__ void plane_layout(const B &b, const cvp9_job_t &job, 
     pbw = pw;
 }
 
+/* Residual TX layout of one block (plane TX size, TXs per row and column).
+ * REFCPU: luma only, counts from the frame-clamped size
+ * (vp9_reconstruct.c:336-347). SPEC, FULL: every plane as plane_layout has it. */
 template <int A>
 __device__ __forceinline__ void residual_layout(BlkS &b, const cvp9_job_t &job, int gx, int gy)
 {
@@ -612,9 +610,6 @@ __device__ __forceinline__ int block_chunks(const BlkS &b)
     return A == CVP9_ARITH_REFCPU ? ((b.cw + 7) >> 3) * ((b.ch + 7) >> 3)
                                   : mc_chunks(b.cw, b.ch, (b.cw + 1) >> 1, (b.ch + 1) >> 1);
 }
-
-/* c + the dot product of four signed taps with four unsigned samples */
-
 
 /* 4x4 byte transpose: rows a..d (one word of four columns each) to four
  * words, one column each (its bytes in row order) */
@@ -693,13 +688,14 @@ template <> struct McRow<uint8_t> {
     }
 };
 
-__device__ __forceinline__ int dp2a_lo_su(uint32_t px, uint32_t taps, int c)
+/* Two 10-bit samples (signed halves hold them) with taps 0-1 or 2-3 of a word. */
+__device__ __forceinline__ int dp2a_lo_ss(uint32_t px, uint32_t taps, int c)
 {
     int d;
     asm("dp2a.lo.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(px), "r"(taps), "r"(c));
     return d;
 }
-__device__ __forceinline__ int dp2a_hi_su(uint32_t px, uint32_t taps, int c)
+__device__ __forceinline__ int dp2a_hi_ss(uint32_t px, uint32_t taps, int c)
 {
     int d;
     asm("dp2a.hi.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(px), "r"(taps), "r"(c));
@@ -711,7 +707,7 @@ template <> struct McRow<uint16_t> {
     static constexpr uint32_t kOne = 0x00010001u;
     static __device__ __forceinline__ int tap(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t ta, uint32_t tb)
     {
-        return dp2a_hi_su(d, tb, dp2a_lo_su(c, tb, dp2a_hi_su(b, ta, dp2a_lo_su(a, ta, 64)))) >> 7;
+        return dp2a_hi_ss(d, tb, dp2a_lo_ss(c, tb, dp2a_hi_ss(b, ta, dp2a_lo_ss(a, ta, 64)))) >> 7;
     }
     static __device__ __forceinline__ void filter(const uint32_t (&w)[8], int f, uint32_t ta, uint32_t tb, uint16_t *d)
     {
@@ -748,8 +744,8 @@ template <> struct McRow<uint16_t> {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const uint32_t e = __byte_perm(x[i], y[i], 0x5410), o = __byte_perm(x[i], y[i], 0x7632);
-                acc[2 * i] = t & 1 ? dp2a_hi_su(e, tp, acc[2 * i]) : dp2a_lo_su(e, tp, acc[2 * i]);
-                acc[2 * i + 1] = t & 1 ? dp2a_hi_su(o, tp, acc[2 * i + 1]) : dp2a_lo_su(o, tp, acc[2 * i + 1]);
+                acc[2 * i] = t & 1 ? dp2a_hi_ss(e, tp, acc[2 * i]) : dp2a_lo_ss(e, tp, acc[2 * i]);
+                acc[2 * i + 1] = t & 1 ? dp2a_hi_ss(o, tp, acc[2 * i + 1]) : dp2a_lo_ss(o, tp, acc[2 * i + 1]);
             }
         }
 #pragma unroll
@@ -1285,7 +1281,8 @@ struct IntraQuad {
     }
     /* A: the profile; directional modes are FULL's. Every directional sample
      * is a copy, a two-tap or a three-tap average at one place of the edge E:
-     * E(i) = above[i] for i >= -1 (-1 the corner), left[-i - 2] below. LIST:
+     * E(i) = above[i] for i >= -1 (-1 the corner), left[-i - 2] below (the same
+     * places as in IntraLane::prepare, which has a sample a lane). LIST:
      * the superblock runs in list order; only there FULL misses an edge that
      * is not the tile's (a block off the 8x8 grid whose first MI is the
      * picture's or tile column's first), so that the halo does not hold it. */
@@ -1711,7 +1708,8 @@ struct IntraLane {
         } else if (A == CVP9_ARITH_FULL && kind == 2) {
             const ITask t = ld_task(&W.task[min(d.x >> 23, kMaxTasks - 1u)]);
             const int mode = t.mode(), c = 4 * q + (lane & 3), size = t.pw(), acl = t.acl(), lcl = t.lcl();
-            /* the place and the weights, in quarters, of the sample's taps */
+            /* the place (as in IntraQuad::run) and the weights, in quarters, of
+             * the sample's taps */
             int i;
             bool two = false, one = false;
             if (mode == 3) {
@@ -5346,9 +5344,10 @@ __global__ void __launch_bounds__(kLfThreads, 2) k_lf_full(const cvp9_job_t *__r
  *
  * The FULL profile's reconstruction on 16-bit samples in [0, 1023]. The
  * frame brings its coefficients dequantised, as int32 (coeffs32, the dense
- * layout of coeffs; the 32x32 halving already applied): the butterflies run
- * in 64-bit integers (wl) with 32-bit values between the row and the column
- * pass, both 8-tap passes of a prediction round and clip to 10 bits, intra
+ * layout of coeffs; the 32x32 halving already applied): the butterflies give
+ * what 64-bit integers would (wn: 32-bit values, 64-bit products; wl where a
+ * coefficient is outside +-2^18), with 32-bit values between the row and the
+ * column pass, both 8-tap passes of a prediction round and clip to 10 bits, intra
  * edges that are missing read 511 above and 513 on the left (512 for a DC
  * with neither), and every residual add clips to [0, 1023]. The loop filter
  * is k_lf_full<uint16_t, 2>.
@@ -5359,9 +5358,10 @@ __global__ void __launch_bounds__(kLfThreads, 2) k_lf_full(const cvp9_job_t *__r
  * TXs of one size. The intra blocks follow
  * as in k_recon, TX by TX in dependency levels over the whole CTA (8x1080p
  * key step 15.6 -> 2.65 ms against a warp per block, prediction and
- * transforms in turn). A superblock whose blocks overlap, or
- * whose intra blocks read samples of blocks later in the list, runs block by
- * block in list order, so every sample is what the list order makes it. */
+ * transforms in turn). A superblock whose blocks overlap, lie
+ * off the 8x8 grid or are no multiple of their transforms, or whose intra
+ * blocks read samples of blocks later in the list, runs block by block in list
+ * order, so every sample is what the list order makes it. */
 namespace {
 
 constexpr int kHbdThreads = 256, kHbdWarps = kHbdThreads / 32;
