@@ -9,6 +9,7 @@
 
 #include <math.h>
 #include <pthread.h>
+#include <sched.h>
 #include <unistd.h>
 #include <stdlib.h>
 #include <string.h>
@@ -198,11 +199,11 @@ double cvp9_now(void)
     return (double)ts.tv_sec + 1e-9 * (double)ts.tv_nsec;
 }
 
-void cvp9_poll_pause(double waited)
+static void nap(long ns)
 {
-    struct timespec ts = { 0, waited < 200e-6 ? 10000 : 20000 };
+    struct timespec ts = { 0, ns };
 #if defined(__linux__)
-    const int slack = waited < 200e-6 ? prctl(PR_GET_TIMERSLACK, 0, 0, 0, 0) : 0;
+    const int slack = prctl(PR_GET_TIMERSLACK, 0, 0, 0, 0);
     if (slack > 1) {
         prctl(PR_SET_TIMERSLACK, 1, 0, 0, 0);
         nanosleep(&ts, NULL);
@@ -211,6 +212,21 @@ void cvp9_poll_pause(double waited)
     }
 #endif
     nanosleep(&ts, NULL);
+}
+
+void cvp9_poll_pause(unsigned *naps, double waited)
+{
+    if (waited >= 200e-6) {
+        struct timespec ts = { 0, 20000 };
+        nanosleep(&ts, NULL);
+    } else if (*naps) {
+        (*naps)--;
+        nap(10000);
+    } else {
+        const double t0 = cvp9_now();
+        sched_yield();
+        if (cvp9_now() - t0 > 20e-6) *naps = 4096;
+    }
 }
 
 /* ── Autotuner ─────────────────────────────────────────────────────────── */

@@ -76,15 +76,18 @@ void cvp9_job_geometry(cvp9_job_t *job, const vp9_parsed_frame_t *pf);
 /* Monotonic clock in seconds. */
 double cvp9_now(void);
 
-/* Between two looks at an event that was not ready after `waited` seconds: a
- * sleep of 10 us, 20 us from 0.2 ms on. With the 50 us of slack that a thread's
- * timers have, such a sleep takes 70 us to return and a small frame's kernels
- * as long, so the first ones go without (the thread's slack is put back):
- * measured, a wait ends 2.6 us late instead of 45. Looking without a sleep
- * (0.2 us) takes the core from the threads that stage and pack: four engines
- * and four busy threads on four cores waited 500 us too long so, 40 us with
- * these sleeps, 66 with the slack. */
-void cvp9_poll_pause(double waited);
+/* Between two looks at an event that was not ready after `waited` seconds: 20
+ * us of sleep from 0.2 ms on. With the 50 us of slack that a thread's timers
+ * have, such a sleep takes 70 us to return and a small frame's kernels as long,
+ * so at first the core is offered to another thread instead. Where one takes
+ * it (20 us, *naps: the engine's, 0 at its start), there are more threads
+ * than cores, and the next looks are 10 us of sleep apart, the timer slack set
+ * aside meanwhile: looking on would take the core from the threads that stage
+ * and pack. Measured, a wait of 0.1 ms on a free core ends 0.2 us late (sleeps
+ * of 20 us: 45, of 10 without slack: 2.6); waits of 0.3 ms by 16 threads
+ * beside 16 busy ones on 16 cores 73 us late (66, 40; looking all the time:
+ * 270, and 30% of the others' work lost). */
+void cvp9_poll_pause(unsigned *naps, double waited);
 
 #ifdef __cplusplus
 }

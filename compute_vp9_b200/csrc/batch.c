@@ -134,6 +134,7 @@ struct cvp9_batch {
     int          pack_q;     /* large steps: frames packed, in 16ths of the step (0..16) */
     int          pack_fixed; /* $CVP9_PACK_SHARE=0..16 pins pack_q (-1: the feedback sets it) */
     cvp9_tuner_t tuner;      /* kernel configuration per shape bucket */
+    unsigned     naps;       /* cvp9_poll_pause */
     uint64_t     budget, reserved;
     cudaStream_t cs, hs, ds;
     bstream_t   *st;
@@ -562,7 +563,7 @@ static cvp9_err_t wait_slot(cvp9_batch_t *b, bslot_t *s)
             snprintf(b->err, sizeof(b->err), "step did not complete within %.0f s", WAIT_LIMIT_S);
             return CVP9_ERR_GPU;
         }
-        cvp9_poll_pause(cvp9_now() - t0);
+        cvp9_poll_pause(&b->naps, cvp9_now() - t0);
     }
     complete_slot(b, s);
     return CVP9_OK;
@@ -1415,7 +1416,7 @@ cvp9_err_t cvp9_batch_timer_stop(cvp9_batch_t *b, float *ms)
         if (e == cudaSuccess) break;
         if (e != cudaErrorNotReady) return bfail(b, e, "timer");
         if (cvp9_now() - t0 > WAIT_LIMIT_S) return CVP9_ERR_GPU;
-        cvp9_poll_pause(cvp9_now() - t0);
+        cvp9_poll_pause(&b->naps, cvp9_now() - t0);
     }
     BCK(cudaEventElapsedTime(ms, b->ev_t0, b->ev_t1), "timer");
     return CVP9_OK;

@@ -93,6 +93,7 @@ typedef struct {
     uint32_t    *d_fast;               /* inter fast path: general flags, tickets, count */
     uint32_t    *d_mi_map;             /* FULL loop filter: mode info per 8x8 MI          */
     cvp9_tuner_t tuner;                /* kernel configuration per frame size */
+    unsigned     naps;                 /* cvp9_poll_pause */
     int          resident_ctas;
     uint32_t     n_tickets;
     int          recon_ctas;
@@ -506,7 +507,7 @@ static cvp9_err_t wait_event(cuctx_t *c, cudaEvent_t ev)
             snprintf(c->last_error, sizeof(c->last_error), "frame did not complete within %.0f s", WAIT_LIMIT_S);
             return CVP9_ERR_GPU;
         }
-        cvp9_poll_pause(cvp9_now() - t0);
+        cvp9_poll_pause(&c->naps, cvp9_now() - t0);
     }
 }
 
