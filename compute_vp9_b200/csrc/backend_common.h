@@ -83,10 +83,10 @@ double cvp9_now(void);
  * it (20 us, *naps: the engine's, 0 at its start), there are more threads
  * than cores, and the next looks are 10 us of sleep apart, the timer slack set
  * aside meanwhile: looking on would take the core from the threads that stage
- * and pack. Measured, a wait of 0.1 ms on a free core ends 0.2 us late (sleeps
- * of 20 us: 45, of 10 without slack: 2.6); waits of 0.3 ms by 16 threads
- * beside 16 busy ones on 16 cores 73 us late (66, 40; looking all the time:
- * 270, and 30% of the others' work lost). */
+ * and pack. Measured, a wait of 0.1 ms on a free core ends 2 us late (sleeps of
+ * 20 us: 45, of 10 without slack: 2.6, looking all the time: 0.2); waits of 0.3
+ * ms by 16 threads beside 16 busy ones on 16 cores 63-77 us late (66, 40, 250-
+ * 300) with 8% of the others' work lost (0, 21%, 35%). */
 void cvp9_poll_pause(unsigned *naps, double waited);
 
 #ifdef __cplusplus

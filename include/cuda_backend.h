@@ -19,6 +19,9 @@
  *    backend-owned pinned memory and stay valid for the next two
  *    cuda_decode_frame calls (include/compute_vp9/decoder.h:100-104),
  *    however many frames the ring holds when the frame is delivered.
+ *    A call that waits looks at the GPU without sleeping for its first 0.2 ms
+ *    (offering its core to other threads in between), then sleeps 20 us
+ *    between looks.
  *  - Errors found on the device (invalid block layout, an expired bounded
  *    wait) are reported by the cuda_get_frame call that delivers the frame:
  *    CVP9_ERR_INVALID_DATA or CVP9_ERR_GPU.
@@ -114,8 +117,10 @@ cvp9_err_t cuda_backend_selftest_wait_limit(int device, uint32_t *status, float 
  * owns every buffer: pf->blocks and pf->coeffs are DEVICE pointers,
  * ref_planes[i] are device I420 frames (NULL = empty slot) of size
  * ref_width[i] x ref_height[i], out_i420 receives the frame
- * (W*H + 2*ceil(W/2)*ceil(H/2) bytes), status_dev (optional, device) receives
- * the CVP9_JOB_* status word. Work is enqueued on `stream` (a cudaStream_t,
+ * (W*H + 2*ceil(W/2)*ceil(H/2) bytes), status_dev (optional, device memory)
+ * receives the CVP9_JOB_* status word, which the kernels write while they run
+ * (0 first): read it when the work is done. Frames and status word may lie at
+ * any byte address; blocks and coefficients at their types' alignment. Work is enqueued on `stream` (a cudaStream_t,
  * NULL = legacy default stream); nothing is allocated or freed.
  * The kernels' scratch is a fixed ~200 KB __device__ array in the library:
  *  - frames above CVP9_NOALLOC_MAX_SB superblocks (7680x4320) are rejected
